@@ -106,6 +106,17 @@ struct AdamArgs {
   int decoupled;  // 1 = AdamW, 0 = Adam (L2 added to the gradient)
 };
 
+__device__ __forceinline__ void adam_update(float& p, float& m, float& v, float g, const AdamArgs& a) {
+  float gj = g * a.grad_scale;
+  if (!a.decoupled) gj += a.wd * p;
+  m = a.beta1 * m + (1.f - a.beta1) * gj;
+  v = a.beta2 * v + (1.f - a.beta2) * gj * gj;
+  const float mh = m / a.bc1, vh = v / a.bc2;
+  float pj = p;
+  if (a.decoupled) pj *= (1.f - a.lr * a.wd);
+  p = pj - a.lr * mh / (sqrtf(vh) + a.eps);
+}
+
 // grad is bf16 or fp32; p/m/v fp32; optional bf16 copy of the updated weights. `skip` (device int)
 // non-zero turns the launch into a no-op (loss-scaler found inf/nan).
 template <typename G>
@@ -137,16 +148,7 @@ __global__ void adam_flat_kernel(float* __restrict__ p, float* __restrict__ m, f
     float* mp = reinterpret_cast<float*>(&mv);
     float* vp = reinterpret_cast<float*>(&vv);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float gj = gr[j] * a.grad_scale;
-      if (!a.decoupled) gj += a.wd * pp[j];
-      mp[j] = a.beta1 * mp[j] + (1.f - a.beta1) * gj;
-      vp[j] = a.beta2 * vp[j] + (1.f - a.beta2) * gj * gj;
-      const float mh = mp[j] / a.bc1, vh = vp[j] / a.bc2;
-      float pj = pp[j];
-      if (a.decoupled) pj *= (1.f - a.lr * a.wd);
-      pp[j] = pj - a.lr * mh / (sqrtf(vh) + a.eps);
-    }
+    for (int j = 0; j < 4; ++j) adam_update(pp[j], mp[j], vp[j], gr[j], a);
     reinterpret_cast<float4*>(p)[i] = pv;
     reinterpret_cast<float4*>(m)[i] = mv;
     reinterpret_cast<float4*>(v)[i] = vv;
@@ -160,17 +162,93 @@ __global__ void adam_flat_kernel(float* __restrict__ p, float* __restrict__ m, f
   // tail (n % 4) handled by the first threads of block 0
   if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
     const long long i = (nvec << 2) + threadIdx.x;
-    float gj = (sizeof(G) == 4 ? reinterpret_cast<const float*>(g)[i]
-                               : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(g)[i])) *
-               a.grad_scale;
-    if (!a.decoupled) gj += a.wd * p[i];
-    m[i] = a.beta1 * m[i] + (1.f - a.beta1) * gj;
-    v[i] = a.beta2 * v[i] + (1.f - a.beta2) * gj * gj;
-    float pj = p[i];
-    if (a.decoupled) pj *= (1.f - a.lr * a.wd);
-    pj -= a.lr * (m[i] / a.bc1) / (sqrtf(v[i] / a.bc2) + a.eps);
-    p[i] = pj;
-    if (p_lp) p_lp[i] = __float2bfloat16(pj);
+    const float gi = sizeof(G) == 4 ? reinterpret_cast<const float*>(g)[i]
+                                    : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(g)[i]);
+    adam_update(p[i], m[i], v[i], gi, a);
+    if (p_lp) p_lp[i] = __float2bfloat16(p[i]);
+  }
+}
+
+// Adam / AdamW over many parameter tensors in one launch: master weights and moments are one flat buffer, every
+// gradient and every bf16 weight is read and written where it lies. Bound by memory: 24 bytes per weight for master
+// and moments plus the gradient and the bf16 copy, each moved once. Gathering the gradients into a flat fp32 buffer
+// first and copying the weights out afterwards moved 40 bytes per bf16 weight instead of 28, in two launches per tensor:
+// 50.4 M weights in 48 tensors took 879 us, this kernel takes 235 us (6.0 TB/s).
+// The tensor table travels in the kernel's parameters (gradients move from step to step, and nothing has to be copied
+// to the device or outlive the launch); a CTA finds its tensor by bisection over the first-CTA column.
+constexpr int ADAM_MULTI_TENSORS = 100;                      // 100 table rows + arguments < 4 KB of parameters
+constexpr int ADAM_MULTI_THREADS = 256, ADAM_MULTI_VECS = 2; // vectors of four in flight per thread and round
+constexpr int ADAM_MULTI_CHUNK = ADAM_MULTI_THREADS * 4 * ADAM_MULTI_VECS * 2;
+
+struct AdamTable {
+  const void* grad[ADAM_MULTI_TENSORS];
+  __nv_bfloat16* lp[ADAM_MULTI_TENSORS];       // bf16 weights to write, or null
+  long long off[ADAM_MULTI_TENSORS];           // first element in the flat buffers, a multiple of four
+  long long n[ADAM_MULTI_TENSORS];
+  int first_cta[ADAM_MULTI_TENSORS];
+  unsigned char grad_bf16[ADAM_MULTI_TENSORS];
+  int count;
+};
+
+__global__ void __launch_bounds__(ADAM_MULTI_THREADS)
+adam_multi_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, const __grid_constant__ AdamTable tab,
+                  const AdamArgs a) {
+  int lo = 0, hi = tab.count;                  // last row whose first CTA is not behind this one
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (tab.first_cta[mid] <= (int)blockIdx.x) lo = mid; else hi = mid;
+  }
+  const long long n = tab.n[lo], off = tab.off[lo];
+  const long long e0 = (long long)((int)blockIdx.x - tab.first_cta[lo]) * ADAM_MULTI_CHUNK;
+  const bool gb = tab.grad_bf16[lo] != 0;
+  const void* grad = tab.grad[lo];
+  __nv_bfloat16* lp = tab.lp[lo];
+  // whole vectors only where gradient and bf16 weights start on a vector boundary (views may not)
+  const bool wide = ((reinterpret_cast<uintptr_t>(grad) & (gb ? 7 : 15)) | (reinterpret_cast<uintptr_t>(lp) & 7)) == 0;
+  p += off; m += off; v += off;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    float4 pv[ADAM_MULTI_VECS], mv[ADAM_MULTI_VECS], vv[ADAM_MULTI_VECS], gv[ADAM_MULTI_VECS];
+    const long long e = e0 + ((long long)r * ADAM_MULTI_VECS * ADAM_MULTI_THREADS + threadIdx.x) * 4;
+    bool full[ADAM_MULTI_VECS];
+#pragma unroll
+    for (int k = 0; k < ADAM_MULTI_VECS; ++k) {
+      const long long i = e + (long long)k * ADAM_MULTI_THREADS * 4;
+      full[k] = wide && i + 4 <= n;
+      if (full[k]) {
+        pv[k] = *reinterpret_cast<const float4*>(p + i);
+        mv[k] = *reinterpret_cast<const float4*>(m + i);
+        vv[k] = *reinterpret_cast<const float4*>(v + i);
+        if (gb) {
+          const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(grad) + i);
+          const float2 x = unpack_bf16x2(u.x), y = unpack_bf16x2(u.y);
+          gv[k] = make_float4(x.x, x.y, y.x, y.y);
+        } else {
+          gv[k] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(grad) + i);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < ADAM_MULTI_VECS; ++k) {
+      const long long i = e + (long long)k * ADAM_MULTI_THREADS * 4;
+      if (full[k]) {
+        adam_update(pv[k].x, mv[k].x, vv[k].x, gv[k].x, a);
+        adam_update(pv[k].y, mv[k].y, vv[k].y, gv[k].y, a);
+        adam_update(pv[k].z, mv[k].z, vv[k].z, gv[k].z, a);
+        adam_update(pv[k].w, mv[k].w, vv[k].w, gv[k].w, a);
+        *reinterpret_cast<float4*>(p + i) = pv[k];
+        *reinterpret_cast<float4*>(m + i) = mv[k];
+        *reinterpret_cast<float4*>(v + i) = vv[k];
+        if (lp) *reinterpret_cast<uint2*>(lp + i) = make_uint2(pack_bf16x2(pv[k].x, pv[k].y), pack_bf16x2(pv[k].z, pv[k].w));
+      } else {
+        for (long long j = i; j < i + 4 && j < n; ++j) {
+          const float gj = gb ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(grad)[j])
+                              : reinterpret_cast<const float*>(grad)[j];
+          adam_update(p[j], m[j], v[j], gj, a);
+          if (lp) lp[j] = __float2bfloat16(p[j]);
+        }
+      }
+    }
   }
 }
 
@@ -279,6 +357,50 @@ GF_API int gf_adam_flat_dev(float* p, float* m, float* v, const void* g, void* p
   else
     adam_flat_kernel<float><<<flat_grid(n), 256, 0, (cudaStream_t)stream>>>(
         p, m, v, (const float*)g, (__nv_bfloat16*)p_lp, n, a, skip, step_dev);
+  return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
+}
+
+// Adam / AdamW over `count` tensors. p / m / v: fp32 flat buffers; table (host memory, read before the call returns):
+// five values per tensor {gradient pointer, bf16 weight pointer or 0, first element in the flat buffers (a multiple of
+// four), number of elements, 1 when the gradient is bf16 and 0 when it is fp32}.
+GF_API int gf_adam_multi(float* p, float* m, float* v, const long long* table, int count, float lr, float beta1,
+                         float beta2, float eps, float wd, int step, float grad_scale, int decoupled, void* stream) {
+  gf::enter();
+  if (count < 0 || (count && !table)) return GFH_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v)) & 15)
+    return GFH_BAD_ARG;
+  AdamArgs a;
+  a.lr = lr; a.beta1 = beta1; a.beta2 = beta2; a.eps = eps; a.wd = wd; a.grad_scale = grad_scale;
+  a.bc1 = 1.f - powf(beta1, (float)step);
+  a.bc2 = 1.f - powf(beta2, (float)step);
+  a.decoupled = decoupled;
+  for (int i = 0; i < count; ++i)
+    if (!table[5 * i] || table[5 * i + 2] < 0 || (table[5 * i + 2] & 3) || table[5 * i + 3] < 0) return GFH_BAD_ARG;
+  AdamTable t;
+  t.count = 0;
+  long long ctas = 0;
+  int launches = 0;
+  for (int i = 0; i <= count; ++i) {
+    const long long n = i < count ? table[5 * i + 3] : 0;
+    const long long need = (n + ADAM_MULTI_CHUNK - 1) / ADAM_MULTI_CHUNK;
+    if (need > 0x7fffffffLL) return GFH_TOO_LARGE;
+    if (t.count && (i == count || t.count == ADAM_MULTI_TENSORS || ctas + need > 0x7fffffffLL)) {
+      adam_multi_kernel<<<(unsigned)ctas, ADAM_MULTI_THREADS, 0, (cudaStream_t)stream>>>(p, m, v, t, a);
+      ++launches;
+      t.count = 0;
+      ctas = 0;
+    }
+    if (i == count || n == 0) continue;
+    const int k = t.count++;
+    t.grad[k] = reinterpret_cast<const void*>(table[5 * i]);
+    t.lp[k] = reinterpret_cast<__nv_bfloat16*>(table[5 * i + 1]);
+    t.off[k] = table[5 * i + 2];
+    t.n[k] = n;
+    t.first_cta[k] = (int)ctas;
+    t.grad_bf16[k] = table[5 * i + 4] != 0;
+    ctas += need;
+  }
+  if (launches > 1) gf::note_extra_launches(launches - 1);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
 }
 

@@ -46,6 +46,7 @@ _SIGS = {
     "gf_xent_fused": [P, P, P, P, I, I, L, F, L, P],
     "gf_adam_flat": [P, P, P, P, P, L, F, F, F, F, F, I, F, I, I, P, P],
     "gf_adam_flat_dev": [P, P, P, P, P, L, F, F, F, F, F, I, F, I, I, P, P, P],
+    "gf_adam_multi": [P, P, P, P, I, F, F, F, F, F, I, F, I, P],
     "gf_counter_add": [P, I, P],
     "gf_colsum_bf16": [P, L, P, P, I, I, I, P],
     "gf_sgd_flat": [P, P, P, P, L, F, F, F, F, I, I, F, I, P],

@@ -6,6 +6,8 @@ Formulas: ghostflow-optim/src/adam.rs:52-95,162-197 and ghostflow-optim/src/sgd.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -32,6 +34,22 @@ def adam_flat(p, m, v, g, p_lp=None, *, lr, beta1=0.9, beta2=0.999, eps=1e-8, we
         1 if decoupled else 0, _gd(g), skip_flag.data_ptr() if skip_flag is not None else None,
         step_dev.data_ptr() if step_dev is not None else None, _lib.stream_ptr())
     _lib.check_rc(rc, "gf_adam_flat")
+
+
+def adam_multi(p, m, v, tensors, *, lr, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0, step=1, grad_scale=1.0,
+               decoupled=True):
+    """Adam / AdamW over many tensors whose fp32 master weights and moments lie in the flat buffers ``p, m, v``.
+    ``tensors``: ``(gradient, bf16 weight or None, first element in the flat buffers)`` per tensor; gradients are
+    contiguous, bf16 or fp32, and read in place; the bf16 weight gets the rounded result."""
+    assert p.is_cuda and p.dtype == torch.float32 and p.is_contiguous()
+    rows = []
+    for g, w, off in tensors:
+        rows += (g.data_ptr(), w.data_ptr() if w is not None else 0, off, g.numel(), _gd(g))
+    rc = _lib.cuda_lib().gf_adam_multi(
+        p.data_ptr(), m.data_ptr(), v.data_ptr(), (ctypes.c_longlong * len(rows))(*rows), len(tensors), float(lr),
+        float(beta1), float(beta2), float(eps), float(weight_decay), int(step), float(grad_scale),
+        1 if decoupled else 0, _lib.stream_ptr())
+    _lib.check_rc(rc, "gf_adam_multi")
 
 
 def sgd_flat(p, buf, g, p_lp=None, *, lr, momentum=0.0, dampening=0.0, weight_decay=0.0, nesterov=False,

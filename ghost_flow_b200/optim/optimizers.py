@@ -92,7 +92,8 @@ class Optimizer:
                 p.data = master[o:o + p.numel()].view(p.shape)
         f = {"params": ps, "offs": offs, "n": n, "master": master,
              "state": [torch.zeros(n, dtype=torch.float32, device=dev) for _ in range(n_state)],
-             "grad": torch.zeros(n, dtype=torch.float32, device=dev),
+             "grad": None,
+             "repeats": len({id(p) for p in ps}) < len(ps),
              "is_view": [p.dtype == torch.float32 and p.data_ptr() == master[o:o + 1].data_ptr()
                          for p, o in zip(ps, offs)],
              "versions": [p._version for p in ps]}
@@ -117,6 +118,8 @@ class Optimizer:
         """Copies the gradients into the flat buffer and returns it with the element ranges ``[(lo, hi), ...]``
         that have one. A parameter without a gradient in this step is left out of the update altogether (no
         weight decay, no decay of its moments), like the per-tensor path and the reference's loop do."""
+        if f["grad"] is None:
+            f["grad"] = torch.zeros_like(f["master"])
         g = f["grad"]
         runs, lo, hi = [], None, None
         for p, o in zip(f["params"], f["offs"]):
@@ -133,6 +136,25 @@ class Optimizer:
         if lo is not None:
             runs.append((lo, hi))
         return g, runs
+
+    @staticmethod
+    def _tensors_in_place(f):
+        """``(gradient, bf16 weight or None, offset)`` of every parameter with a gradient, for a kernel that reads and
+        writes them where they lie; ``None`` when one of them has a layout, type or device that needs the flat copy."""
+        if f["repeats"]:
+            return None
+        out, dev = [], f["master"].device
+        for p, o, view in zip(f["params"], f["offs"], f["is_view"]):
+            g = p.grad
+            if g is None:
+                continue
+            if g.dtype not in (torch.bfloat16, torch.float32) or g.device != dev or g.layout != torch.strided \
+                    or not g.is_contiguous() or type(g) not in (torch.Tensor, torch.nn.Parameter):
+                return None
+            if not view and (p.dtype != torch.bfloat16 or p.device != dev or not p.is_contiguous()):
+                return None
+            out.append((g, None if view else p, o))
+        return out
 
     @staticmethod
     def _scatter_params(f):
@@ -243,16 +265,24 @@ class Adam(Optimizer):
             b1, b2 = g["betas"]
             f = self._flat_group(gi, 2)
             if f is not None:
-                from ..ops.optim_kernels import adam_flat
+                from ..ops.optim_kernels import adam_flat, adam_multi
 
                 self._sync_master(f)
-                grads, runs = self._gather_grads(f)
-                with torch.cuda.device(f["master"].device):
-                    for lo, hi in runs:
-                        adam_flat(f["master"][lo:hi], f["state"][0][lo:hi], f["state"][1][lo:hi], grads[lo:hi], None,
-                                  lr=g["lr"], beta1=b1, beta2=b2, eps=g["eps"], weight_decay=g["weight_decay"], step=t,
-                                  decoupled=self.decoupled)
-                self._scatter_params(f)
+                tensors = self._tensors_in_place(f)
+                hyper = dict(lr=g["lr"], beta1=b1, beta2=b2, eps=g["eps"], weight_decay=g["weight_decay"], step=t,
+                             decoupled=self.decoupled)
+                if tensors is not None:
+                    # a parameter that has no gradient keeps its bf16 value: its master copy did not move either
+                    with torch.cuda.device(f["master"].device):
+                        if tensors:
+                            adam_multi(f["master"], *f["state"], tensors, **hyper)
+                else:
+                    grads, runs = self._gather_grads(f)
+                    with torch.cuda.device(f["master"].device):
+                        for lo, hi in runs:
+                            adam_flat(f["master"][lo:hi], f["state"][0][lo:hi], f["state"][1][lo:hi], grads[lo:hi],
+                                      None, **hyper)
+                    self._scatter_params(f)
             for p in g["params"]:
                 if p.is_cuda or p.grad is None:
                     continue
