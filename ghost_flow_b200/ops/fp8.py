@@ -18,6 +18,7 @@ import ctypes
 import torch
 
 from . import _lib
+from .gemm import _colsum
 
 E4M3_MAX = 448.0
 _BOUND = False
@@ -30,8 +31,9 @@ def _bind():
         P, I, L = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
         lib.gf_quant_fp8_rows.argtypes = [P, L, P, L, P, I, I, I, P]
         lib.gf_quant_fp8_block128.argtypes = [P, L, P, L, P, I, I, P]
+        lib.gf_quant_fp8_transpose.argtypes = [P, L, P, P, P, P, I, I, P, P]
         lib.gf_gemm_fp8.argtypes = [P, P, P, I, I, I, L, L, L, P, P, P, I, P, P]
-        for n in ("gf_quant_fp8_rows", "gf_quant_fp8_block128", "gf_gemm_fp8"):
+        for n in ("gf_quant_fp8_rows", "gf_quant_fp8_block128", "gf_quant_fp8_transpose", "gf_gemm_fp8"):
             getattr(lib, n).restype = I
         _BOUND = True
     return lib
@@ -56,6 +58,28 @@ def quantize_rows(x: torch.Tensor, mode: int = 0):
     s = xb.abs().amax(2).clamp_min(1e-12) / E4M3_MAX
     q = (xb / s[:, :, None]).clamp(-E4M3_MAX, E4M3_MAX).to(torch.float8_e4m3fn).view(torch.uint8).view(T, K)
     return q, s.t().contiguous()
+
+
+def quantize_transposed(x: torch.Tensor, rows: bool = False):
+    """``quantize_rows(x^T)`` for x [R, K] bf16: ``(qt uint8 [K, R], scale fp32 [K])``; with ``rows`` also
+    ``quantize_rows(x)``, as ``(q, scale, qt, scale_t)``, from the same reads of x."""
+    R, K = x.shape
+    if x.is_cuda and x.dtype == torch.bfloat16 and R % 16 == 0 and K % 16 == 0 and R and K \
+            and (R + 63) // 64 < 65536:
+        x = x.contiguous()
+        if x.data_ptr() % 16:
+            x = x.clone()
+        qt = torch.empty(K, R, dtype=torch.uint8, device=x.device)
+        q = torch.empty(R, K, dtype=torch.uint8, device=x.device) if rows else None
+        st = torch.empty(K, dtype=torch.float32, device=x.device)
+        s = torch.empty(R, dtype=torch.float32, device=x.device) if rows else None
+        scratch = torch.empty(R + K, dtype=torch.float32, device=x.device)
+        _lib.check_rc(_bind().gf_quant_fp8_transpose(
+            x.data_ptr(), x.stride(0), q.data_ptr() if rows else None, s.data_ptr() if rows else None, qt.data_ptr(),
+            st.data_ptr(), R, K, scratch.data_ptr(), _lib.stream_ptr()), "gf_quant_fp8_transpose")
+        return (q, s, qt, st) if rows else (qt, st)
+    t = quantize_rows(x.t().contiguous(), 0)
+    return (*quantize_rows(x.contiguous(), 0), *t) if rows else t
 
 
 def quantize_block128(w: torch.Tensor):
@@ -165,16 +189,21 @@ class _Fp8LinearFn(torch.autograd.Function):
         x2, w = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1]).to(torch.bfloat16)
         dx = dw = db = None
-        if ctx.needs_input_grad[0]:
+        if ctx.needs_input_grad[0] and ctx.needs_input_grad[1]:
+            gq, gs, gtq, gts = quantize_transposed(dy2, rows=True)
+        elif ctx.needs_input_grad[0]:
             gq, gs = quantize_rows(dy2.contiguous(), 0)
-            wtq, wts = quantize_rows(w.to(torch.bfloat16).t().contiguous(), 0)
+        elif ctx.needs_input_grad[1]:
+            gtq, gts = quantize_transposed(dy2)
+        if ctx.needs_input_grad[0]:
+            wtq, wts = quantize_transposed(w.to(torch.bfloat16))
             dx = gemm_fp8(gq, gs, wtq, wts, 0).view(ctx.x_shape).to(ctx.x_dtype)
         if ctx.needs_input_grad[1]:
-            gtq, gts = quantize_rows(dy2.t().contiguous(), 0)
-            xtq, xts = quantize_rows(x2.t().contiguous(), 0)
+            xtq, xts = quantize_transposed(x2)
             dw = gemm_fp8(gtq, gts, xtq, xts, 0).to(w.dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.float().sum(0).to(dy.dtype)
+            # fp32 sums either way; the kernel's result is bf16, the type of a bf16 dy
+            db = _colsum(dy2) if dy.dtype == torch.bfloat16 else dy2.float().sum(0).to(dy.dtype)
         return dx, dw, db
 
 

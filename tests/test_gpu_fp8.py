@@ -96,3 +96,45 @@ def test_fp8_training_linear_matches_the_emulation_and_fp32(kernel_status):
     for got, emu, ref in zip(outs["cuda"], outs["cpu"], (yr.detach(), xr.grad, wr.grad, br.grad)):
         assert rel(got, emu) < 2e-2, rel(got, emu)          # same quantisation, different summation order
         assert rel(got, ref) < 7e-2, rel(got, ref)          # e4m3 against fp32
+
+
+# columns around the steps of the row kernel (registers per thread, threads per row, the loop beyond 16384), rows that
+# leave the last block part empty
+@pytest.mark.parametrize("T,K", [(1, 8), (9, 256), (3, 264), (7, 1024), (5, 1032), (3, 2056), (2, 4096), (3, 4104), (2, 8200),
+                                 (2, 12296), (3, 16384), (2, 16392)])
+def test_quantise_rows_gives_the_oracle_bytes(T, K):
+    from ghost_flow_b200.ops import fp8
+
+    x = torch.randn(T, K, device="cuda", dtype=torch.bfloat16) * 3
+    x[0] = 0                                           # an all-zero row keeps the smallest scale
+    if T > 2:
+        x[2, K // 2] = float("nan")                    # ignored by the maximum, kept as NaN
+    q, s = fp8.quantize_rows(x, 0)
+    f = x.float()
+    amax = torch.nan_to_num(f.abs(), nan=0.0).amax(1)
+    scale = amax.clamp_min(1e-12) / torch.full_like(amax, 448.0)     # a true division (by a number, torch multiplies)
+    assert torch.equal(s, scale)
+    want = (f * (torch.ones_like(scale) / scale)[:, None]).clamp(-448, 448).to(torch.float8_e4m3fn)
+    # the same fp32 operations and one conversion: equal up to the sign of NaN
+    assert torch.equal(torch.nan_to_num(q.view(torch.float8_e4m3fn).float(), nan=999.0), torch.nan_to_num(want.float(), nan=999.0))
+
+
+@pytest.mark.parametrize("R,K", [(16, 16), (128, 64), (144, 80), (112, 528), (1040, 1008), (4096, 2048), (16, 5008)])
+def test_transposed_quantisation_equals_quantising_the_transpose(R, K):
+    from ghost_flow_b200.ops import fp8
+
+    buf = torch.randn(R * K + 8, device="cuda", dtype=torch.bfloat16)
+    x = buf[8:].view(R, K)
+    x[0, 0], x[-1, -1], x[:, 3] = 300.0, -1e30, 0.0
+    x[5, 7] = float("nan")
+    q, s, qt, st = fp8.quantize_transposed(x, rows=True)
+    q1, s1 = fp8.quantize_rows(x, 0)
+    qt1, st1 = fp8.quantize_rows(x.t().contiguous(), 0)
+    assert torch.equal(q, q1) and torch.equal(s, s1) and torch.equal(qt, qt1) and torch.equal(st, st1)
+    qt2, st2 = fp8.quantize_transposed(x)
+    assert torch.equal(qt2, qt1) and torch.equal(st2, st1)
+    # a start off the 16-byte boundary is copied first; sizes the kernel does not take go through the plain transpose
+    odd = buf[1:1 + R * K].view(R, K)
+    assert torch.equal(fp8.quantize_transposed(odd)[0], fp8.quantize_rows(odd.clone().t().contiguous(), 0)[0])
+    part = x[:, :8].contiguous()
+    assert torch.equal(fp8.quantize_transposed(part)[0], fp8.quantize_rows(part.t().contiguous(), 0)[0])
