@@ -31,24 +31,25 @@ class LLaMAAttention(Module):
         B, S, _ = x.shape
         H, Hk, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim
         qkv = self.wqkv(x).view(B, S, H + 2 * Hk, D)
-        q, k, v = ops.split_qkv(qkv, H, Hk)
-        q = ops.rope(q, cos, sin, c.rope_interleaved, start_pos)
-        k = ops.rope(k, cos, sin, c.rope_interleaved, start_pos)
         if cache is not None:
             # decoding: append to the cache and attend over everything seen so far
             kc, vc = cache
-            kc[:, start_pos:start_pos + S] = k
-            vc[:, start_pos:start_pos + S] = v
             kernels = x.is_cuda and x.dtype == torch.bfloat16 and D in (64, 128) and not torch.is_grad_enabled()
-            if kernels and S == 1:
+            if kernels and start_pos == 0 and S > 1:
+                # prompt: nothing older than itself to attend to
+                q, k, v = ops.rope_qkv(qkv, H, Hk, cos, sin, c.rope_interleaved, start_pos)
+                kc[:, :S] = k
+                vc[:, :S] = v
+                o = ops.flash_attention(q, k, v, causal=True)
+            elif kernels and S == 1:
+                q = ops.rope_qkv_to_cache(qkv, H, Hk, cos, sin, kc, vc, c.rope_interleaved, start_pos)
                 # one new token per sequence: the decode kernel streams the cache once (GQA groups share the reads)
                 from ..ops import raw
 
                 o = raw.attn_decode(q.reshape(B, H * D), kc.view(B, kc.shape[1], Hk * D), vc.view(B, vc.shape[1], Hk * D),
                                     start_pos + 1, B, H, Hk, D).view(B, 1, H, D)
-            elif kernels and start_pos == 0:
-                o = ops.flash_attention(q, k, v, causal=True)        # prompt: nothing older than itself to attend to
             else:
+                q = ops.rope_qkv_to_cache(qkv, H, Hk, cos, sin, kc, vc, c.rope_interleaved, start_pos)
                 kk, vv = kc[:, :start_pos + S], vc[:, :start_pos + S]
                 G = H // Hk
                 qf = q.transpose(1, 2).float()
@@ -60,6 +61,7 @@ class LLaMAAttention(Module):
                 s = s.masked_fill(~mask, float("-inf"))
                 o = (torch.softmax(s, -1) @ vf).transpose(1, 2).to(x.dtype)
         else:
+            q, k, v = ops.rope_qkv(qkv, H, Hk, cos, sin, c.rope_interleaved, start_pos)
             o = ops.flash_attention(q, k, v, causal=True)
         return self.wo(o.reshape(B, S, H * D), residual)
 

@@ -62,11 +62,12 @@ class MultiHeadAttention(Module):
         """x: ``[B, S, E]``. ``rope`` = (cos, sin, interleaved) applies rotary embedding to q and k."""
         causal = self.causal if causal is None else causal
         B, S, _ = x.shape
-        q, k, v = self._split(x)
         if rope is not None:
             cos, sin, inter = rope
-            q = ops.rope(q, cos, sin, inter)
-            k = ops.rope(k, cos, sin, inter)
+            H, Hk, D = self.num_heads, self.num_kv_heads, self.head_dim
+            q, k, v = ops.rope_qkv(self.qkv(x).view(B, S, H + 2 * Hk, D), H, Hk, cos, sin, inter)
+        else:
+            q, k, v = self._split(x)
         if mask is None and not (self.dropout > 0 and self.training):
             o = ops.flash_attention(q, k, v, causal=causal)
         else:

@@ -7,6 +7,7 @@ numerical reference the GPU tests compare against.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -233,6 +234,94 @@ def rope(x, cos, sin, interleaved: bool = False, pos_offset: int = 0, inplace: b
     if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] % 16 == 0:
         return _call(_RopeFn, x, cos, sin, interleaved, pos_offset, inplace)
     return rope_ref(x, cos, sin, interleaved, pos_offset)
+
+
+def _packed_rows(t):
+    """``t [B, S, H, D]`` as it is when its rows can be addressed as ``base + (b * S + s) * pitch`` on 16-byte boundaries
+    with the heads packed, else a contiguous copy; with the row pitch."""
+    ld = _rows_view(t)
+    if ld is None or ld % 8 or t.data_ptr() % 16:
+        t = t.clone(memory_format=torch.contiguous_format)
+        ld = t.shape[2] * t.shape[3]
+    return t, ld
+
+
+def _rope_qkv_launch(q, k, v, qd, kd, vd, cos, sin, interleaved, pos_offset, backward):
+    """Rotates ``q, k [B, S, *, D]`` into ``qd, kd`` and copies ``v`` into ``vd`` (``None``: left alone). Destinations are
+    ``[B, S, *, D]`` views with packed heads and free row and sequence pitch."""
+    B, S, H, D = q.shape
+    q, ldq = _packed_rows(q)
+    k, ldk = _packed_rows(k)
+    ldv = 0
+    if vd is not None:
+        v, ldv = _packed_rows(v)
+    table = (ctypes.c_longlong * 9)(ldq, ldk, ldv, qd.stride(1), qd.stride(0), kd.stride(1), kd.stride(0),
+                                    vd.stride(1) if vd is not None else 0, vd.stride(0) if vd is not None else 0)
+    _rc(_lib.cuda_lib().gf_rope_qkv(q.data_ptr(), k.data_ptr(), v.data_ptr() if vd is not None else None, qd.data_ptr(),
+                                    kd.data_ptr(), vd.data_ptr() if vd is not None else None, table, cos.data_ptr(),
+                                    sin.data_ptr(), B * S, S, H, k.shape[2], D, pos_offset, 1 if interleaved else 0,
+                                    1 if backward else 0, _lib.stream_ptr()), "gf_rope_qkv")
+
+
+class _RopeQKVFn(torch.autograd.Function):
+    """Split and rotation of a packed projection in one launch per direction: the backward pass rotates the gradients of
+    q and k back and packs the three gradients in the same pass."""
+
+    @staticmethod
+    def forward(ctx, qkv, H, Hk, cos, sin, interleaved, pos_offset):
+        B, S, G, D = qkv.shape
+        q = torch.empty((B, S, H, D), dtype=qkv.dtype, device=qkv.device)
+        k = torch.empty((B, S, Hk, D), dtype=qkv.dtype, device=qkv.device)
+        v = qkv[:, :, H + Hk:]
+        _rope_qkv_launch(qkv[:, :, :H], qkv[:, :, H:H + Hk], None, q, k, None, cos, sin, interleaved, pos_offset, False)
+        ctx.save_for_backward(cos, sin)
+        ctx.args = (H, Hk, interleaved, pos_offset)
+        return q, k, v
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        cos, sin = ctx.saved_tensors
+        H, Hk, interleaved, pos_offset = ctx.args
+        B, S, _, D = dq.shape
+        g = torch.empty((B, S, H + 2 * Hk, D), dtype=dq.dtype, device=dq.device)
+        _rope_qkv_launch(dq, dk, dv, g[:, :, :H], g[:, :, H:H + Hk], g[:, :, H + Hk:], cos, sin, interleaved, pos_offset,
+                         True)
+        return g, None, None, None, None, None, None
+
+
+def _rope_qkv_ok(qkv, cos, sin) -> bool:
+    return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.shape[-1] % 16 == 0 and qkv.numel() > 0
+            and cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0)
+
+
+def rope_qkv(qkv, num_heads: int, num_kv_heads: int, cos, sin, interleaved: bool = False, pos_offset: int = 0):
+    """``q, k, v`` of a packed projection output ``[B, S, H + 2 Hk, D]`` with q and k rotated (see :func:`rope`)."""
+    H, Hk = num_heads, num_kv_heads
+    if _rope_qkv_ok(qkv, cos, sin):
+        return _call(_RopeQKVFn, qkv, H, Hk, cos, sin, interleaved, pos_offset)
+    q, k, v = split_qkv(qkv, H, Hk)
+    return rope(q, cos, sin, interleaved, pos_offset), rope(k, cos, sin, interleaved, pos_offset), v
+
+
+def rope_qkv_to_cache(qkv, num_heads: int, num_kv_heads: int, cos, sin, kcache, vcache, interleaved: bool = False,
+                      pos_offset: int = 0):
+    """Rotated q of a packed projection output; rotated k and v go to rows ``pos_offset ..`` of the caches
+    ``[B, max_len, Hk, D]``. Inference only: nothing is recorded for autograd."""
+    B, S, _, D = qkv.shape
+    H, Hk = num_heads, num_kv_heads
+    if not torch.is_grad_enabled() and _rope_qkv_ok(qkv, cos, sin) and pos_offset + S <= kcache.shape[1] \
+            and all(c.is_cuda and c.device == qkv.device and c.dtype == qkv.dtype and c.shape == (B, kcache.shape[1], Hk, D)
+                    and c.stride(3) == 1 and c.stride(2) == D and c.stride(1) % 8 == 0 and c.stride(0) % 8 == 0
+                    and c.data_ptr() % 16 == 0 for c in (kcache, vcache)):
+        q = torch.empty((B, S, H, D), dtype=qkv.dtype, device=qkv.device)
+        _rope_qkv_launch(qkv[:, :, :H], qkv[:, :, H:H + Hk], qkv[:, :, H + Hk:], q, kcache[:, pos_offset:pos_offset + S],
+                         vcache[:, pos_offset:pos_offset + S], cos, sin, interleaved, pos_offset, False)
+        return q
+    q, k, v = rope_qkv(qkv, H, Hk, cos, sin, interleaved, pos_offset)
+    kcache[:, pos_offset:pos_offset + S] = k
+    vcache[:, pos_offset:pos_offset + S] = v
+    return q
 
 
 # ------------------------------------------------------------------------------------------ SwiGLU / unary

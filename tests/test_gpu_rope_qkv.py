@@ -1,0 +1,62 @@
+"""Rotary embedding of a packed projection in one launch (``rope_qkv``) against split + ``rope`` one by one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(a, b):
+    # the same fp32 formula, contracted differently at most: equal up to one bf16 rounding (2^-8 relative, and 2^-8 of a
+    # product that cancelled)
+    return torch.allclose(a.float(), b.float(), rtol=2 ** -7, atol=2 ** -7)
+
+
+@pytest.mark.parametrize("B,S,H,Hk,D", [(1, 1, 1, 1, 16), (2, 37, 3, 3, 48), (2, 5, 8, 2, 64), (1, 130, 40, 8, 128), (3, 1, 4, 4, 256)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rope_qkv_forward_and_backward(B, S, H, Hk, D, interleaved):
+    from ghost_flow_b200 import ops
+
+    pos = 3
+    cos, sin = ops.rope_tables(S + pos, D, 1e4, "cuda")
+    x = torch.randn(B, S, H + 2 * Hk, D, device="cuda", dtype=torch.bfloat16)
+    a, b = x.clone().requires_grad_(), x.clone().requires_grad_()
+    got = ops.rope_qkv(a, H, Hk, cos, sin, interleaved, pos)
+    q, k, v = ops.split_qkv(b, H, Hk)
+    want = ops.rope(q, cos, sin, interleaved, pos), ops.rope(k, cos, sin, interleaved, pos), v
+    # gradients as three tensors, one of them strided so that it has to be copied first
+    gs = [torch.randn_like(t) for t in want]
+    gs[1] = torch.randn(B, Hk, S, D, device="cuda", dtype=torch.bfloat16).transpose(1, 2)
+    for g, w in zip(got, want):
+        assert _close(g, w)
+    torch.autograd.backward(got, gs)
+    torch.autograd.backward(want, gs)
+    assert _close(a.grad, b.grad)
+    with torch.no_grad():
+        for g, w in zip(ops.rope_qkv(x, H, Hk, cos, sin, interleaved, pos), want):
+            assert _close(g, w)
+
+
+@pytest.mark.parametrize("B,S,H,Hk,D", [(3, 1, 4, 2, 64), (2, 7, 8, 8, 128), (1, 1, 5, 5, 24)])
+@pytest.mark.parametrize("layout", ["plain", "heads_first"])
+def test_rope_qkv_to_cache(B, S, H, Hk, D, layout):
+    from ghost_flow_b200 import ops
+
+    pos, n = 11, 32
+    cos, sin = ops.rope_tables(n, D, 1e4, "cuda")
+    qkv = torch.randn(B, S, H + 2 * Hk, D, device="cuda", dtype=torch.bfloat16)
+    if layout == "plain":
+        caches = [torch.randn(B, n, Hk, D, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    else:                                  # a layout the kernel does not write: takes the assignments
+        caches = [torch.randn(B, Hk, n, D, device="cuda", dtype=torch.bfloat16).transpose(1, 2) for _ in range(2)]
+    want = [c.clone() for c in caches]
+    with torch.no_grad():
+        q = ops.rope_qkv_to_cache(qkv, H, Hk, cos, sin, *caches, False, pos)
+        qs, ks, vs = ops.split_qkv(qkv, H, Hk)
+        want[0][:, pos:pos + S] = ops.rope(ks, cos, sin, False, pos)
+        want[1][:, pos:pos + S] = vs
+    assert _close(q, ops.rope(qs, cos, sin, False, pos))
+    for c, w in zip(caches, want):
+        assert _close(c, w)
+        rest = torch.ones(n, dtype=torch.bool)
+        rest[pos:pos + S] = False
+        assert torch.equal(c[:, rest], w[:, rest])
