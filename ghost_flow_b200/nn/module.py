@@ -16,6 +16,9 @@ ModuleDict = torch.nn.ModuleDict
 Identity = torch.nn.Identity
 
 
+_MAY_WRAP = (Tensor, list, tuple)
+
+
 def _unwrap_args(args, kwargs):
     wrapped = False
 
@@ -47,8 +50,11 @@ class Module(torch.nn.Module):
     _profile_hook = None  # set by ghost_flow_b200.utils.profiler when profiling of modules is enabled
 
     def __call__(self, *args, **kwargs):
-        a, k, wrapped = _unwrap_args(args, kwargs)
         hook = Module._profile_hook
+        if hook is None and not any(isinstance(x, _MAY_WRAP) for x in args) \
+                and not (kwargs and any(isinstance(x, _MAY_WRAP) for x in kwargs.values())):
+            return super().__call__(*args, **kwargs)     # nothing to unwrap: the usual call of a layer by a layer
+        a, k, wrapped = _unwrap_args(args, kwargs)
         if hook is not None:
             with hook(type(self).__name__):
                 out = super().__call__(*a, **k)

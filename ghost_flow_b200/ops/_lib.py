@@ -132,6 +132,8 @@ def host_lib():
 
 
 _BOUND_DEVICE = -1
+# the handle without the Python stream object around it (3 us of every launch); absent in some torch builds
+_RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def stream_ptr() -> int:
@@ -142,7 +144,7 @@ def stream_ptr() -> int:
     if dev != _BOUND_DEVICE:
         cuda_lib().gf_set_device(dev)
         _BOUND_DEVICE = dev
-    return torch.cuda.current_stream().cuda_stream
+    return _RAW_STREAM(dev) if _RAW_STREAM is not None else torch.cuda.current_stream().cuda_stream
 
 
 _STATUS = {}

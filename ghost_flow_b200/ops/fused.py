@@ -61,48 +61,47 @@ def _rc(rc, what):
 
 
 # ------------------------------------------------------------------------------------------ RMSNorm
+def _dense(t):
+    return t if t.is_contiguous() else t.contiguous()
+
+
 class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps, residual):
         D = x.shape[-1]
-        x2 = x.reshape(-1, D).contiguous()
-        T = x2.shape[0]
-        y = torch.empty_like(x2)
-        rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-        h = None
-        res2 = None
+        x = _dense(x)
+        T = x.numel() // D
+        y = torch.empty_like(x)
+        # the row statistics are kept for the backward pass only
+        rstd = torch.empty(T, dtype=torch.float32, device=x.device) if type(ctx) is not _NoGraph else None
+        h = res = None
         if residual is not None:
-            res2 = residual.reshape(-1, D).contiguous()
-            h = torch.empty_like(x2)
-        lib = _lib.cuda_lib()
-        _rc(lib.gf_rmsnorm_fwd(x2.data_ptr(), res2.data_ptr() if res2 is not None else None, w.data_ptr(),
-                               y.data_ptr(), h.data_ptr() if h is not None else None, rstd.data_ptr(), T, D,
-                               float(eps), _lib.stream_ptr()), "gf_rmsnorm_fwd")
-        ctx.save_for_backward(h if h is not None else x2, w, rstd)
-        ctx.shape = x.shape
+            res = _dense(residual)
+            h = torch.empty_like(x)
+        _rc(_lib.cuda_lib().gf_rmsnorm_fwd(
+            x.data_ptr(), None if res is None else res.data_ptr(), w.data_ptr(), y.data_ptr(),
+            None if h is None else h.data_ptr(), None if rstd is None else rstd.data_ptr(), T, D, float(eps),
+            _lib.stream_ptr()), "gf_rmsnorm_fwd")
+        ctx.save_for_backward(h if h is not None else x, w, rstd)
         ctx.has_res = residual is not None
-        if residual is not None:
-            return y.view(x.shape), h.view(x.shape)
-        return y.view(x.shape)
+        return (y, h) if residual is not None else y
 
     @staticmethod
     def backward(ctx, dy, dh=None):
-        x2, w, rstd = ctx.saved_tensors
-        T, D = x2.shape
-        dy2 = dy.reshape(-1, D).contiguous()
-        dres = dh.reshape(-1, D).contiguous() if (ctx.has_res and dh is not None) else None
-        dx = torch.empty_like(x2)
+        x, w, rstd = ctx.saved_tensors
+        D = x.shape[-1]
+        T = x.numel() // D
+        dy = _dense(dy)
+        dres = _dense(dh) if (ctx.has_res and dh is not None) else None
+        dx = torch.empty_like(x)
         dw = torch.empty_like(w)
         lib = _lib.cuda_lib()
         g = lib.gf_norm_bwd_grid(T)
-        scratch = _scratch(x2.device, g * D)
-        _rc(lib.gf_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), rstd.data_ptr(),
-                               dres.data_ptr() if dres is not None else None, dx.data_ptr(), dw.data_ptr(),
+        scratch = _scratch(x.device, g * D)
+        _rc(lib.gf_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(),
+                               None if dres is None else dres.data_ptr(), dx.data_ptr(), dw.data_ptr(),
                                scratch.data_ptr(), T, D, 0, _lib.stream_ptr()), "gf_rmsnorm_bwd")
-        dxv = dx.view(ctx.shape)
-        if ctx.has_res:
-            return dxv, dw, None, dxv
-        return dxv, dw, None, None
+        return dx, dw, None, dx if ctx.has_res else None
 
 
 def rms_norm_ref(x, w, eps=1e-6):
@@ -126,35 +125,35 @@ class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, eps):
         D = x.shape[-1]
-        x2 = x.reshape(-1, D).contiguous()
-        T = x2.shape[0]
-        y = torch.empty_like(x2)
-        mean = torch.empty(T, dtype=torch.float32, device=x.device)
-        rstd = torch.empty(T, dtype=torch.float32, device=x.device)
+        x = _dense(x)
+        T = x.numel() // D
+        y = torch.empty_like(x)
+        stats = torch.empty((2, T), dtype=torch.float32, device=x.device) if type(ctx) is not _NoGraph else None
         lib = _lib.cuda_lib()
-        _rc(lib.gf_layernorm_fwd(x2.data_ptr(), w.data_ptr(), b.data_ptr() if b is not None else None, y.data_ptr(),
-                                 mean.data_ptr(), rstd.data_ptr(), T, D, float(eps), _lib.stream_ptr()),
-            "gf_layernorm_fwd")
-        ctx.save_for_backward(x2, w, mean, rstd)
-        ctx.shape = x.shape
+        _rc(lib.gf_layernorm_fwd(x.data_ptr(), w.data_ptr(), b.data_ptr() if b is not None else None, y.data_ptr(),
+                                 None if stats is None else stats.data_ptr(),
+                                 None if stats is None else stats.data_ptr() + 4 * T, T, D, float(eps),
+                                 _lib.stream_ptr()), "gf_layernorm_fwd")
+        ctx.save_for_backward(x, w, stats)
         ctx.has_bias = b is not None
-        return y.view(x.shape)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w, mean, rstd = ctx.saved_tensors
-        T, D = x2.shape
-        dy2 = dy.reshape(-1, D).contiguous()
-        dx = torch.empty_like(x2)
+        x, w, stats = ctx.saved_tensors
+        D = x.shape[-1]
+        T = x.numel() // D
+        dy = _dense(dy)
+        dx = torch.empty_like(x)
         dw = torch.empty_like(w)
         db = torch.empty_like(w) if ctx.has_bias else None
         lib = _lib.cuda_lib()
         g = lib.gf_norm_bwd_grid(T)
-        scratch = _scratch(x2.device, 2 * g * D)
-        _rc(lib.gf_layernorm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+        scratch = _scratch(x.device, 2 * g * D)
+        _rc(lib.gf_layernorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), stats.data_ptr(), stats.data_ptr() + 4 * T,
                                  dx.data_ptr(), dw.data_ptr(), db.data_ptr() if db is not None else None,
                                  scratch.data_ptr(), T, D, 0, _lib.stream_ptr()), "gf_layernorm_bwd")
-        return dx.view(ctx.shape), dw, db, None
+        return dx, dw, db, None
 
 
 def layer_norm(x, w, b=None, eps: float = 1e-5):

@@ -15,6 +15,7 @@ from . import _lib
 
 
 _SMS: dict = {}
+_BF16 = torch.bfloat16
 
 
 def _sm_count(device) -> int:
@@ -36,33 +37,38 @@ def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bf
     ``[N, K]`` or ``[K, N]`` when ``b_mn_major``. Row pitches may exceed the row length. ``relu`` applies
     max(., 0) in the epilogue after bias and residual.
     """
-    assert a.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    assert _is_dense_2d(a) and _is_dense_2d(b), "operands must be 2-D with unit inner stride"
+    sa, sb = a.stride(), b.stride()
+    assert a.is_cuda and a.dtype is _BF16 and b.dtype is _BF16
+    assert len(sa) == 2 and len(sb) == 2 and sa[1] == 1 and sb[1] == 1 and sa[0] >= a.size(1) and sb[0] >= b.size(1), \
+        "operands must be 2-D with unit inner stride"
     if out is None:
         if N % 8:
             # rows of an [M, N] tensor with such an N do not start on 16-byte boundaries; give the result a padded
             # pitch (the caller gets an [M, N] view) so that it can feed the next kernel as it is
             out = torch.empty((M, (N + 63) // 64 * 64), dtype=out_dtype, device=a.device)[:, :N]
         else:
-            out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    assert _is_dense_2d(out)
+            out = a.new_empty((M, N), dtype=out_dtype)
+    else:
+        assert _is_dense_2d(out)
     lib = _lib.cuda_lib()
+    device = a.device
+    f32_out = out.dtype is torch.float32
     # few output tiles and a long K: the kernel splits K and needs an fp32 [M, N] workspace. It comes from torch's
     # allocator, so it belongs to the current stream (and to the graph's pool while a CUDA graph is recorded).
     ws = None
-    if (K >= 2048 and out.dtype == torch.bfloat16 and not accumulate and not relu and bn_hint == 0 and max_ctas == 0
+    if (K >= 2048 and out.dtype is _BF16 and not accumulate and not relu and bn_hint == 0 and max_ctas == 0
             and M * N < (1 << 31)
-            and 2 * ((M + 127) // 128) * ((N + (127 if N <= 128 else 255)) // (128 if N <= 128 else 256)) <= _sm_count(a.device)):
-        ws = torch.empty(M * N, dtype=torch.float32, device=a.device)
+            and 2 * ((M + 127) // 128) * ((N + (127 if N <= 128 else 255)) // (128 if N <= 128 else 256)) <= _sm_count(device)):
+        ws = torch.empty(M * N, dtype=torch.float32, device=device)
     rc = lib.gf_gemm_bf16(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K,
-        1 if a_mn_major else 0, a.stride(0), 1 if b_mn_major else 0, b.stride(0), out.stride(0),
-        1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0,
-        bias.data_ptr() if bias is not None else None,
-        residual.data_ptr() if residual is not None else None,
-        residual.stride(0) if residual is not None else 0,
-        float(alpha), _lib.status_word(a.device).data_ptr(), bn_hint, max_ctas,
-        ws.data_ptr() if ws is not None else None, 1 if relu else 0, ws.numel() if ws is not None else 0,
+        1 if a_mn_major else 0, sa[0], 1 if b_mn_major else 0, sb[0], out.stride(0),
+        1 if f32_out else 0, 1 if accumulate else 0,
+        None if bias is None else bias.data_ptr(),
+        None if residual is None else residual.data_ptr(),
+        0 if residual is None else residual.stride(0),
+        float(alpha), _lib.status_word(device).data_ptr(), bn_hint, max_ctas,
+        None if ws is None else ws.data_ptr(), 1 if relu else 0, 0 if ws is None else M * N,
         _lib.stream_ptr(),
     )
     _lib.check_rc(rc, "gf_gemm_bf16")
@@ -74,9 +80,10 @@ def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bf
 def _kernel_ok(*ts) -> bool:
     """bf16 CUDA operands whose 2-D view satisfies the TMA rules (16-byte base and row pitch)."""
     for t in ts:
-        if not (t.is_cuda and t.dtype == torch.bfloat16):
+        if not (t.is_cuda and t.dtype is _BF16):
             return False
-        if t.dim() >= 2 and (t.stride(-1) != 1 or (t.stride(-2) % 8) or (t.data_ptr() % 16)):
+        s = t.stride()
+        if len(s) >= 2 and (s[-1] != 1 or s[-2] % 8 or t.data_ptr() % 16):
             return False
     return True
 
@@ -123,7 +130,7 @@ def matmul_tt(a: torch.Tensor, b: torch.Tensor, **kw) -> torch.Tensor:
 
 
 def _as_2d(x: torch.Tensor) -> torch.Tensor:
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     return x2
@@ -181,7 +188,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
             r2 = _as_2d(residual) if residual is not None else None
             x2 = _as_2d(x)
             y = gemm_raw(x2, False, w, False, x2.shape[0], w.shape[0], x2.shape[1], bias=bias, residual=r2)
-            return y.view(*x.shape[:-1], w.shape[0])
+            return y if x.dim() == 2 else y.view(*x.shape[:-1], w.shape[0])
         return _LinearFn.apply(x, w, bias, residual)
     y = torch.nn.functional.linear(x, w, bias)
     if residual is not None:
