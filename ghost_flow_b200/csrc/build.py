@@ -33,6 +33,7 @@ CUDA_SOURCES = [
     "gf_host.cu",
     "gemm_bf16.cu",
     "gemm2sm_bf16.cu",
+    "gemm_skinny.cu",
     "norm.cu",
     "pointwise.cu",
     "xent_adamw.cu",

@@ -917,6 +917,12 @@ static float* splitk_workspace(size_t floats) {
 }  // namespace gf
 
 namespace gf {
+// kernel for at most 16 rows (gemm_skinny.cu)
+bool gemm_skinny_wanted(const void* A, const void* W, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
+                        long long ldb, int accumulate);
+int gemm_skinny_run(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
+                    int out_fp32, const void* bias, const void* residual, long long ldr, float alpha, int relu,
+                    cudaStream_t st);
 // CTA-pair kernel for plain GEMMs (gemm2sm_bf16.cu)
 int gemm2sm_wanted(int M, int N, int K);
 int gemm2sm_run(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda,
@@ -952,6 +958,9 @@ GF_API int gf_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int
   no_gather(p);
   p.act = activation == 1 ? 1 : 0;   // epilogue activation after bias and residual: 0 none, 1 ReLU
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
+  if (bn_hint == 0 && max_ctas == 0 &&
+      gf::gemm_skinny_wanted(A, B, M, N, K, a_mn_major, lda, b_mn_major, ldb, accumulate))
+    return gf::gemm_skinny_run(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, bias, residual, ldr, alpha, p.act, st);
   // Few output tiles and a long K (decode-sized M; weight gradients of narrow layers, [768, 2304] over 8192 tokens):
   // too few tiles to fill the machine. Split K until there is about one work item per SM; the slices add into an
   // fp32 workspace that a second kernel converts. The workspace is the caller's (splitk_ws, splitk_ws_floats >= M * N:

@@ -56,7 +56,7 @@ def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bf
     # few output tiles and a long K: the kernel splits K and needs an fp32 [M, N] workspace. It comes from torch's
     # allocator, so it belongs to the current stream (and to the graph's pool while a CUDA graph is recorded).
     ws = None
-    if (K >= 2048 and out.dtype is _BF16 and not accumulate and not relu and bn_hint == 0 and max_ctas == 0
+    if (K >= 2048 and (M > 16 or a_mn_major or b_mn_major or K % 8) and out.dtype is _BF16 and not accumulate and not relu and bn_hint == 0 and max_ctas == 0
             and M * N < (1 << 31)
             and 2 * ((M + 127) // 128) * ((N + (127 if N <= 128 else 255)) // (128 if N <= 128 else 256)) <= _sm_count(device)):
         ws = torch.empty(M * N, dtype=torch.float32, device=device)
