@@ -157,6 +157,21 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(const __grid_constant__ R
   }
 }
 
+// ---- rows of a table by index, zeros for an index outside it; one warp per 512 bytes of a row. The tensor-library form
+// (two comparisons, an or, a clamp, a lookup, a masked fill) takes six launches; for the three tokens of a small decode step
+// launches are all it costs (one token of a two-layer model for three sequences: 28 launches -> 24).
+template <typename I>
+__global__ void __launch_bounds__(256)
+embedding_rows_kernel(const I* __restrict__ ids, const uint4* __restrict__ table, uint4* __restrict__ out, long long n,
+                      long long rows, int vpr, int pieces) {
+  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long i = w / pieces;
+  const int v = (int)(w - i * pieces) * 32 + (threadIdx.x & 31);
+  if (i >= n || v >= vpr) return;
+  const long long id = (long long)ids[i];
+  out[i * vpr + v] = id >= 0 && id < rows ? table[id * vpr + v] : make_uint4(0, 0, 0, 0);
+}
+
 // ------------------------------------------------------------------ SwiGLU
 // gu is [T, 2F] (gate columns [0,F), up columns [F,2F)); y = silu(g) * u is [T, F].
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, long long T,
@@ -544,6 +559,24 @@ GF_API int gf_rope(void* x, const float* cos_t, const float* sin_t, int T, int H
   rope_kernel<<<ew_grid(total, 256), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)x, cos_t, sin_t, T, H, D,
                                                                     row_stride, head_stride, S, pos_offset, mode,
                                                                     backward ? -1.f : 1.f);
+  GF_RET();
+}
+// out[i] = table[ids[i]], rows of `row_bytes` (a multiple of 16) on 16-byte boundaries; ids int64 (wide) or int32.
+GF_API int gf_embedding_rows(const void* ids, int wide, const void* table, void* out, long long n, long long rows,
+                             int row_bytes, void* stream) {
+  gf::enter();
+  if (n <= 0 || rows <= 0 || row_bytes <= 0 || row_bytes % 16 || !ids || !table || !out ||
+      ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return GFH_BAD_ARG;
+  const int vpr = row_bytes / 16, pieces = (vpr + 31) / 32;
+  const long long ctas = (n * pieces + 7) / 8;
+  if (ctas > 0x7fffffffLL) return GFH_TOO_LARGE;
+  if (wide)
+    embedding_rows_kernel<long long><<<(unsigned)ctas, 256, 0, (cudaStream_t)stream>>>(
+        (const long long*)ids, (const uint4*)table, (uint4*)out, n, rows, vpr, pieces);
+  else
+    embedding_rows_kernel<int><<<(unsigned)ctas, 256, 0, (cudaStream_t)stream>>>(
+        (const int*)ids, (const uint4*)table, (uint4*)out, n, rows, vpr, pieces);
   GF_RET();
 }
 // q / k / v sources (head pitch D, row pitch ld*) to destinations with row and sequence pitches; see RopeQkv. `vd` may

@@ -34,6 +34,7 @@ _SIGS = {
     "gf_layernorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "gf_layernorm_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, P],
     "gf_rope": [P, P, P, I, I, I, L, L, I, I, I, I, P],
+    "gf_embedding_rows": [P, I, P, P, L, L, I, P],
     "gf_rope_qkv": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
     "gf_swiglu_fwd": [P, P, L, I, P],
     "gf_scale_by_dev_scalar": [P, L, P, P],

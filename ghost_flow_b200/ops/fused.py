@@ -356,6 +356,24 @@ def swiglu(gu):
     return F.silu(g) * u
 
 
+def embedding_rows(ids, table):
+    """``table[ids]`` with zero rows for ids outside the table, in one launch; ``None`` where the kernel does not apply
+    (CPU tensors, a gradient to record, rows that are no whole 16-byte vectors)."""
+    if not (table.is_cuda and ids.is_cuda and ids.device == table.device and table.dim() == 2 and ids.numel() > 0
+            and ids.dtype in (torch.int64, torch.int32) and table.dtype in (torch.bfloat16, torch.float32, torch.float16)
+            and not (torch.is_grad_enabled() and table.requires_grad) and table.is_contiguous() and table.shape[0] > 0):
+        return None
+    row_bytes = table.shape[1] * table.element_size()
+    if row_bytes == 0 or row_bytes % 16 or table.data_ptr() % 16:
+        return None
+    ids = _dense(ids)
+    out = table.new_empty((*ids.shape, table.shape[1]))
+    _rc(_lib.cuda_lib().gf_embedding_rows(ids.data_ptr(), 1 if ids.dtype is torch.int64 else 0, table.data_ptr(),
+                                          out.data_ptr(), ids.numel(), table.shape[0], row_bytes, _lib.stream_ptr()),
+        "gf_embedding_rows")
+    return out
+
+
 OPS = {"relu": 0, "gelu": 1, "sigmoid": 2, "tanh": 3, "silu": 4}
 
 

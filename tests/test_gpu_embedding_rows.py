@@ -1,0 +1,25 @@
+"""Embedding lookup in one launch against the tensor-library form, ids outside the table included."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# rows of one vector, of part of a warp's 512 bytes, of exactly that and of one vector more; 4 and 2 byte types
+@pytest.mark.parametrize("D,dtype", [(8, torch.bfloat16), (40, torch.float32), (256, torch.bfloat16), (264, torch.bfloat16),
+                                     (4096, torch.float16), (12, torch.bfloat16)])
+@pytest.mark.parametrize("shape", [(1,), (3, 1), (7, 33)])
+@pytest.mark.parametrize("kind", [torch.int64, torch.int32, torch.float32])
+def test_lookup_equals_the_masked_form(D, dtype, shape, kind):
+    from ghost_flow_b200.nn import Embedding
+
+    e = Embedding(11, D, device="cuda", dtype=dtype)
+    ids = torch.randint(-3, 14, shape, device="cuda").to(kind)
+    with torch.no_grad():
+        got = e(ids)
+    want = e(ids)                                    # with a gradient to record: the tensor-library form
+    assert want.requires_grad and not got.requires_grad
+    assert got.shape == (*shape, D) and torch.equal(got, want.detach())
+    if len(shape) == 2:
+        with torch.no_grad():
+            assert torch.equal(e(ids.t()), want.detach().transpose(0, 1))
