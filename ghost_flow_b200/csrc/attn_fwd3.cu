@@ -3,8 +3,8 @@
 // pipe busy while the softmax warps work:
 //
 //  * The probabilities never touch shared memory. A softmax thread reads its row of S = Q K^T from tensor
-//    memory, and writes P = exp2(...) as packed bf16 back into the first 64 columns of the same S region
-//    (tcgen05.st); O += P V then takes its A operand from tensor memory. The 64 KB of shared memory that held
+//    memory (once for the maximum, once for the exponentials), and writes P = exp2(...) as packed bf16 back into the
+//    first 64 columns of the same S region (tcgen05.st); O += P V then takes its A operand from tensor memory. The 64 KB of shared memory that held
 //    P now double-buffer K.
 //  * The MMA warp issues  P V (tile t, step j)  followed at once by  Q K^T (tile t, step j + 1)  and only then
 //    turns to the other tile. While the softmax warps of one tile are busy, the tensor pipe runs the two
@@ -16,6 +16,16 @@
 // The output accumulates in TMEM across KV tiles and is rescaled in place only when a row maximum has grown by
 // more than 2^8 since the last rescale; P is exp2 against that (possibly stale) reference maximum.
 //
+// What bounds it: the chain of one tile, S ready -> row maximum -> exponentials -> P V, Q K^T -> next S, of which two tiles
+// are in flight; tensor pipe and special-function unit are each busy half of the time. So the chain is kept short:
+//  * the MMA warp issues from uniform control flow, and P V in two parts, the first under the second half of
+//    the exponentials (four parts cost more in waits than they hide);
+//  * the exponential pass reads the scores from tensor memory again, 32 at a time with the next 32 on their way, rather
+//    than keep 128 of them in registers, and scale and row sum are packed two-wide instructions. A polynomial on the
+//    FMA pipe for a quarter of the exponentials was slower (148 against 145 us): issue slots are dearer than the unit.
+// Measured, before -> now: [1, 4096, 32 heads of 128] causal 155 -> 139 us, [2, 2987, 64 / 8 heads of 128] causal
+// 376 -> 325 us, [8, 1024, 12 heads of 64] causal 56 -> 42 us, [2, 4096, 16 heads of 128] full 287 -> 272 us.
+//
 // Replaces ghostflow-cuda/src/optimized_kernels.cu:185-248 and the CPU algorithm of
 // ghostflow-nn/src/flash_attention.rs:122-250.
 #include "gf_host.h"
@@ -25,11 +35,35 @@ namespace gf {
 
 constexpr int F3_TILE = 128;      // query rows per tile, kv rows per step
 constexpr int F3_THREADS = 384;   // warpgroup 0: TMA warp, MMA warp, two idle warps; warpgroups 1 and 2: softmax of tile 0 / 1
-// Registers move from warpgroup 0 to the softmax warpgroups (a softmax thread keeps its whole row of 128
-// scores in registers): 128 x 64 + 256 x 216 = 63488 of the 65536 registers of an SM.
+// Registers move from warpgroup 0 to the softmax warpgroups, whose loops over the scores are unrolled:
+// 128 x 64 + 256 x 216 = 63488 of the 65536 registers of an SM.
 constexpr int F3_REGS_CTRL = 64;
 constexpr int F3_REGS_SOFTMAX = 216;
+constexpr int F3_PARTS = 2;       // P V of a tile is issued in this many parts of the kv rows, each as soon as its P is there
 constexpr float F3_RESCALE_THRESHOLD = 8.0f;  // log2 units
+
+// ---- two fp32 at a time (one issue slot for two results)
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
 struct Fa3Params {
   int B, S, Hq, Hkv;
@@ -39,7 +73,7 @@ struct Fa3Params {
   long long ldo;
   float* lse;
   int* status;
-  int head_group;   // heads whose CTAs are dispatched together (see the kernel's block decoding)
+  int head_group;   // heads (of all sequences) whose CTAs are dispatched together (see the kernel's block decoding)
 };
 
 template <int HD>
@@ -74,17 +108,17 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint64_t* v_full = bars + 5;    // [2]
   uint64_t* v_empty = bars + 7;   // [2]
   uint64_t* s_full = bars + 9;    // [2] per tile
-  uint64_t* p_full = bars + 11;   // [2] per tile
-  uint64_t* o_done = bars + 13;   // [2] per tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* o_done = bars + 11;   // [2] per tile
+  uint64_t* p_full = bars + 13;   // [2][F3_PARTS] per tile and part of its columns
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13 + 2 * F3_PARTS);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qb = (p.S + 2 * F3_TILE - 1) / (2 * F3_TILE);
-  // CTAs are dispatched in linear block order. Heads are taken in groups of head_group: inside a group the heaviest
-  // query block (most KV tiles under a causal mask) of every head comes first, then the next block, so long CTAs
-  // start first and short ones fill the tail, while the CTAs in flight at any time belong to few heads, whose K / V
-  // (re-read by every query block) stay in L2.
-  int qb, h;
+  // CTAs are dispatched in linear block order. The heads of all sequences are taken in groups of head_group: inside a
+  // group the heaviest query block (most KV tiles under a causal mask) of every head comes first, then the next block,
+  // so long CTAs start first and short ones fill the tail, while the CTAs in flight at any time belong to one group,
+  // whose K / V (re-read by every query block) stay in L2.
+  int qb, h, b;
   {
     const int H = gridDim.x, NT = gridDim.y;
     const int lin = blockIdx.x + H * blockIdx.y;
@@ -94,8 +128,9 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const int gs_g = min(gs, H - g * gs);
     qb = n_qb - 1 - rem / gs_g;
     h = g * gs + rem % gs_g;
+    b = h / p.Hq;
+    h -= b * p.Hq;
   }
-  const int b = blockIdx.z;
   const int hk = h / (p.Hq / p.Hkv);
   const int n_kv_all = (p.S + F3_TILE - 1) / F3_TILE;
   const int row_base = b * p.S;
@@ -116,7 +151,7 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 4);
+      for (int c = 0; c < F3_PARTS; ++c) mbar_init(&p_full[i * F3_PARTS + c], 4);
       mbar_init(&o_done[i], 1);
     }
     mbar_fence_init();
@@ -170,68 +205,76 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(F3_TILE, F3_TILE, 0, 0);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16(F3_TILE, HD, 0, 1);
-      bool ok = mbar_wait(q_full, 0);
-      if (!ok && p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
-      // S_t = Q_t K(j)^T, announced on s_full[t]
-      auto issue_qk = [&](int t, int j) {
-        const uint32_t qa = smem_u32(sQ + t * Cfg::TILE_BYTES);
-        const uint32_t ka = smem_u32(sK + (j & 1) * Cfg::TILE_BYTES);
+    // The whole warp runs this in uniform control flow and one elected lane issues (see gf_ptx.cuh); the descriptors are
+    // bases plus constants. Issued from a single lane's branch an instruction took about 110 cycles to leave, twice
+    // what the tensor pipe needs for it, and the issue was what bounded the kernel.
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(F3_TILE, F3_TILE, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc_bf16(F3_TILE, HD, 0, 1);
+    const uint64_t dq0 = umma_desc_sw128(smem_u32(sQ), 16, 1024);
+    const uint64_t dk0 = umma_desc_sw128(smem_u32(sK), 16, 1024);
+    const uint64_t dv0 = umma_desc_sw128(smem_u32(sV), F3_TILE * 128, 1024);
+    constexpr uint64_t TILE_D = Cfg::TILE_BYTES >> 4;      // descriptor addresses count 16-byte units
+    bool ok = mbar_wait_warp(q_full, 0);
+    if (!ok && p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
+    // S_t = Q_t K(j)^T, announced on s_full[t]
+    auto issue_qk = [&](int t, int j) {
+      const uint64_t qa = dq0 + (t ? TILE_D : 0), ka = dk0 + ((j & 1) ? TILE_D : 0);
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * (F3_TILE * 128) + (kk & 3) * 32;
-          umma_bf16_ss(tmem_base + Cfg::TM_S + t * 128, umma_desc_sw128(qa + off, 16, 1024),
-                       umma_desc_sw128(ka + off, 16, 1024), idesc_qk, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[t]);
-      };
-      if (ok && n_j > 0) {
-        if (!mbar_wait(&k_full[0], 0)) {
-          if (p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
-          ok = false;
-        } else {
-          tc_fence_after();
-#pragma unroll
-          for (int t = 0; t < 2; ++t)
-            if (n_kv[t] > 0) issue_qk(t, 0);
-          umma_commit(&k_empty[0]);
-        }
+      for (int kk = 0; kk < HD / 16; ++kk) {
+        const uint64_t off = ((kk >> 2) * (F3_TILE * 128) + (kk & 3) * 32) >> 4;
+        umma_bf16_ss_u(leader, tmem_base + Cfg::TM_S + t * 128, qa + off, ka + off, idesc_qk, kk > 0 ? 1u : 0u);
       }
-      for (int j = 0; j < n_j && ok; ++j) {
-        const int st = j & 1;
-        const bool has_next = j + 1 < n_j;
-        if (!mbar_wait(&v_full[st], (j >> 1) & 1) ||
-            (has_next && !mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1))) {
-          if (p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
-          ok = false;
-          break;
-        }
-        const uint32_t va = smem_u32(sV + st * Cfg::TILE_BYTES);
+      umma_commit_u(leader, &s_full[t]);
+    };
+    if (ok && n_j > 0) {
+      if (!mbar_wait_warp(&k_full[0], 0)) {
+        if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
+        ok = false;
+      } else {
+        tc_fence_after();
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (j < n_kv[t]) {
-            if (!mbar_wait(&p_full[t], j & 1)) {
-              if (p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_SOFTMAX);
+        for (int t = 0; t < 2; ++t)
+          if (n_kv[t] > 0) issue_qk(t, 0);
+        umma_commit_u(leader, &k_empty[0]);
+      }
+    }
+    for (int j = 0; j < n_j && ok; ++j) {
+      const int st = j & 1;
+      const bool has_next = j + 1 < n_j;
+      if (!mbar_wait_warp(&v_full[st], (j >> 1) & 1) ||
+          (has_next && !mbar_wait_warp(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1))) {
+        if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
+        ok = false;
+        break;
+      }
+      const uint64_t va = dv0 + (st ? TILE_D : 0);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (j < n_kv[t]) {
+          // O_t += P_t V(j): A = P_t from tensor memory (8 columns per 16 kv rows), B = V(j) MN-major
+#pragma unroll
+          for (int c = 0; c < F3_PARTS; ++c) {
+            if (ok && !mbar_wait_warp(&p_full[t * F3_PARTS + c], j & 1)) {
+              if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_SOFTMAX);
               ok = false;
-              break;
             }
-            tc_fence_after();
-            // O_t += P_t V(j): A = P_t from tensor memory (8 columns per 16 kv rows), B = V(j) MN-major
+            if (ok) {
+              tc_fence_after();
 #pragma unroll
-            for (int kk = 0; kk < F3_TILE / 16; ++kk)
-              umma_bf16_ts(tmem_base + Cfg::TM_O + t * 128, tmem_base + Cfg::TM_S + t * 128 + kk * 8,
-                           umma_desc_sw128(va + kk * 2048, F3_TILE * 128, 1024), idesc_pv,
-                           (j > 0 || kk > 0) ? 1u : 0u);
-            if (j == n_kv[t] - 1) umma_commit(&o_done[t]);
+              for (int kk = c * (F3_TILE / 16 / F3_PARTS); kk < (c + 1) * (F3_TILE / 16 / F3_PARTS); ++kk)
+                umma_bf16_ts_u(leader, tmem_base + Cfg::TM_O + t * 128, tmem_base + Cfg::TM_S + t * 128 + kk * 8,
+                               va + ((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+            }
           }
-          if (j + 1 < n_kv[t]) issue_qk(t, j + 1);
+          if (!ok) break;
+          if (j == n_kv[t] - 1) umma_commit_u(leader, &o_done[t]);
         }
-        if (!ok) break;
-        umma_commit(&v_empty[st]);
-        if (has_next) umma_commit(&k_empty[(j + 1) & 1]);
+        if (j + 1 < n_kv[t]) issue_qk(t, j + 1);
       }
+      if (!ok) break;
+      umma_commit_u(leader, &v_empty[st]);
+      if (has_next) umma_commit_u(leader, &k_empty[(j + 1) & 1]);
     }
   }
   } else {
@@ -258,25 +301,30 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const int kv0 = j * F3_TILE;
       const bool need_mask = (p.causal && (kv0 + F3_TILE - 1 > qb * 2 * F3_TILE + t * F3_TILE)) ||
                              (kv0 + F3_TILE > p.S);
-      // ---- the whole row of raw scores into registers
-      uint32_t sv[F3_TILE];
-#pragma unroll
-      for (int c = 0; c < F3_TILE / 32; ++c) tmem_ld32(ts + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&sv[c * 32]));
-      tmem_ld_wait();
-      if (need_mask) {
-#pragma unroll
-        for (int i = 0; i < F3_TILE; ++i) {
-          const int kv = kv0 + i;
-          if (kv >= p.S || (p.causal && kv > q_idx)) sv[i] = 0xff800000u;  // -inf
-        }
-      }
-      // four independent chains: a single running maximum would serialise 64 dependent instructions
+      // ---- row maximum, 64 scores at a time (the exponential pass reads them from tensor memory again)
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < F3_TILE; i += 8) {
+      for (int c2 = 0; c2 < 2; ++c2) {
+        uint32_t sa[32], sb[32];
+        tmem_ld32(ts + c2 * 64, sa);
+        tmem_ld32(ts + c2 * 64 + 32, sb);
+        tmem_ld_wait();
+        if (need_mask) {
+          const int lim = min(p.causal ? q_idx : p.S - 1, p.S - 1) - kv0 - c2 * 64;   // last visible column here
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          mx4[e] = fmaxf(mx4[e], fmaxf(__uint_as_float(sv[i + 2 * e]), __uint_as_float(sv[i + 2 * e + 1])));
+          for (int i = 0; i < 32; ++i) {
+            if (i > lim) sa[i] = 0xff800000u;  // -inf
+            if (32 + i > lim) sb[i] = 0xff800000u;
+          }
+          tmem_st32(ts + c2 * 64, sa);
+          tmem_st32(ts + c2 * 64 + 32, sb);
+          tmem_st_wait();
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) mx4[e] = max3(mx4[e], __uint_as_float(sa[i + e]), __uint_as_float(sb[i + e]));
+        }
       }
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       // ---- reference maximum: move it (and rescale O, l) only when the row maximum grew a lot. The commit
@@ -302,26 +350,39 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
       const float mref_use = (m_ref == -INFINITY) ? 0.f : m_ref;  // row with no visible key yet
       const float mneg = -mref_use * sl2;
-      // ---- P = 2^(s*scale*log2e - m_ref*scale*log2e) as bf16 pairs into columns [0, 64) of the S region
-      float rs0 = 0.f, rs1 = 0.f;
-#pragma unroll
-      for (int c = 0; c < F3_TILE / 32; ++c) {
+      const uint64_t sl2x = pack2(sl2, sl2), mnegx = pack2(mneg, mneg);
+      uint64_t rsa = 0, rsb = 0;
+      uint32_t sa[32], sb[32];
+      auto chunk = [&](const uint32_t (&sv)[32], uint32_t dst) {
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          const float p0 = ex2_approx(fmaf(__uint_as_float(sv[c * 32 + i]), sl2, mneg));
-          const float p1 = ex2_approx(fmaf(__uint_as_float(sv[c * 32 + i + 1]), sl2, mneg));
-          rs0 += p0;
-          rs1 += p1;
+          float p0, p1;
+          unpack2(fma2(pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2x, mnegx), p0, p1);
+          p0 = ex2_approx(p0);
+          p1 = ex2_approx(p1);
+          if (i & 2) rsa = add2(rsa, pack2(p0, p1)); else rsb = add2(rsb, pack2(p0, p1));
           pk[i >> 1] = pack_bf16x2(p0, p1);
         }
-        tmem_st16(ts + c * 16, pk);
+        tmem_st16(dst, pk);
+      };
+      tmem_ld32(ts, sa);
+#pragma unroll
+      for (int c2 = 0; c2 < 2; ++c2) {
+        tmem_ld_wait();
+        tmem_ld32(ts + c2 * 64 + 32, sb);
+        chunk(sa, ts + c2 * 32);
+        tmem_ld_wait();
+        if (c2 == 0) tmem_ld32(ts + 64, sa);
+        chunk(sb, ts + c2 * 32 + 16);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[t * F3_PARTS + c2]);
       }
-      l += rs0 + rs1;
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[t]);
+      float r0, r1;
+      unpack2(add2(rsa, rsb), r0, r1);
+      l += r0 + r1;
     }
     // ---- epilogue: O / l
     if (ok && my_n > 0) {
@@ -385,7 +446,7 @@ static int launch_fa3(const void* q, const void* k, const void* v, long long ldq
   if (rc) return rc;
   rc = make_tmap_2d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, (uint64_t)p.Hkv * HD, ldv * 2, F3_TILE, 64);
   if (rc) return rc;
-  dim3 grid(p.Hq, (p.S + 2 * F3_TILE - 1) / (2 * F3_TILE), p.B);
+  dim3 grid(p.Hq * p.B, (p.S + 2 * F3_TILE - 1) / (2 * F3_TILE));
   kern<<<grid, F3_THREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
 }
@@ -403,7 +464,7 @@ GF_API int gf_flash_attn_fwd3(const void* q, const void* k, const void* v, void*
   Fa3Params p;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal; p.scale = scale;
   p.O = (__nv_bfloat16*)o; p.ldo = ldo; p.lse = lse; p.status = status;
-  p.head_group = attention_head_group(Hq);
+  p.head_group = attention_head_group_l2(B * Hq, 4ll * S * head_dim * Hkv / Hq);
   if (head_dim == 128) return launch_fa3<128>(q, k, v, ldq, ldk, ldv, p, (cudaStream_t)stream);
   if (head_dim == 64) return launch_fa3<64>(q, k, v, ldq, ldk, ldv, p, (cudaStream_t)stream);
   return GFH_BAD_ARG;

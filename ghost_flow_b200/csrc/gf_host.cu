@@ -114,6 +114,14 @@ int attention_head_group(int heads) {
   return g;
 }
 
+int attention_head_group_l2(int heads, long long bytes_per_head) {
+  if (const char* e = getenv("GF_ATT_GROUP"))
+    if (atoi(e) > 0) return attention_head_group(heads);
+  const long long fit = bytes_per_head > 0 ? (16ll << 20) / bytes_per_head : heads;
+  const long long g = fit < 8 ? 8 : fit;
+  return g < heads ? (int)g : heads;
+}
+
 static int* g_check_buffers[32] = {};
 int* check_buffer() {
   int dev = 0;

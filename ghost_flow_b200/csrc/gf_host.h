@@ -68,6 +68,11 @@ void set_check_buffer(int device, int* p);
 
 // Heads per dispatch group of the attention kernels: GF_ATT_GROUP when set (tuning), else 8, clamped to [1, heads].
 int attention_head_group(int heads);
+// The same for kernels that order all sequences' heads together: as many heads as have their re-read tensors in 16 MB,
+// but at least 8. The larger the group the better long CTAs come before short ones (8 sequences of 1024, 12 heads of 64,
+// forward: 48 us with groups inside a sequence, 42 us with all heads in one); with 64 or 256 MB, [2, 4096, 32, 128]
+// takes 2 to 5 % longer, because K and V then compete with the streamed Q and O for the L2.
+int attention_head_group_l2(int heads, long long bytes_per_head);
 
 // Binds the calling thread to the device selected with gf_set_device (see gf_host.cu).
 void enter();
