@@ -23,8 +23,8 @@
 //  * the exponential pass reads the scores from tensor memory again, 32 at a time with the next 32 on their way, rather
 //    than keep 128 of them in registers, and scale and row sum are packed two-wide instructions. A polynomial on the
 //    FMA pipe for a quarter of the exponentials was slower (148 against 145 us): issue slots are dearer than the unit.
-// Measured, before -> now: [1, 4096, 32 heads of 128] causal 155 -> 139 us, [2, 2987, 64 / 8 heads of 128] causal
-// 376 -> 325 us, [8, 1024, 12 heads of 64] causal 56 -> 42 us, [2, 4096, 16 heads of 128] full 287 -> 272 us.
+// Measured, before -> now: [1, 4096, 32 heads of 128] causal 155 -> 136 us, [2, 2987, 64 / 8 heads of 128] causal
+// 376 -> 318 us, [8, 1024, 12 heads of 64] causal 56 -> 42 us, [2, 4096, 16 heads of 128] full 287 -> 270 us.
 //
 // Replaces ghostflow-cuda/src/optimized_kernels.cu:185-248 and the CPU algorithm of
 // ghostflow-nn/src/flash_attention.rs:122-250.
@@ -36,9 +36,10 @@ namespace gf {
 constexpr int F3_TILE = 128;      // query rows per tile, kv rows per step
 constexpr int F3_THREADS = 384;   // warpgroup 0: TMA warp, MMA warp, two idle warps; warpgroups 1 and 2: softmax of tile 0 / 1
 // Registers move from warpgroup 0 to the softmax warpgroups, whose loops over the scores are unrolled:
-// 128 x 64 + 256 x 216 = 63488 of the 65536 registers of an SM.
-constexpr int F3_REGS_CTRL = 64;
-constexpr int F3_REGS_SOFTMAX = 216;
+// 128 x 104 + 256 x 200 = 64512, the block's own at launch
+// (384 x 168). With 64 for the first warpgroup the MMA warp spilled.
+constexpr int F3_REGS_CTRL = 104;
+constexpr int F3_REGS_SOFTMAX = 200;
 constexpr int F3_PARTS = 2;       // P V of a tile is issued in this many parts of the kv rows, each as soon as its P is there
 constexpr float F3_RESCALE_THRESHOLD = 8.0f;  // log2 units
 
@@ -215,7 +216,7 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const uint64_t dk0 = umma_desc_sw128(smem_u32(sK), 16, 1024);
     const uint64_t dv0 = umma_desc_sw128(smem_u32(sV), F3_TILE * 128, 1024);
     constexpr uint64_t TILE_D = Cfg::TILE_BYTES >> 4;      // descriptor addresses count 16-byte units
-    bool ok = mbar_wait_warp(q_full, 0);
+    bool ok = mbar_wait_warp_tight(q_full, 0);
     if (!ok && p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
     // S_t = Q_t K(j)^T, announced on s_full[t]
     auto issue_qk = [&](int t, int j) {
@@ -228,7 +229,7 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       umma_commit_u(leader, &s_full[t]);
     };
     if (ok && n_j > 0) {
-      if (!mbar_wait_warp(&k_full[0], 0)) {
+      if (!mbar_wait_warp_tight(&k_full[0], 0)) {
         if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
         ok = false;
       } else {
@@ -242,8 +243,8 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     for (int j = 0; j < n_j && ok; ++j) {
       const int st = j & 1;
       const bool has_next = j + 1 < n_j;
-      if (!mbar_wait_warp(&v_full[st], (j >> 1) & 1) ||
-          (has_next && !mbar_wait_warp(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1))) {
+      if (!mbar_wait_warp_tight(&v_full[st], (j >> 1) & 1) ||
+          (has_next && !mbar_wait_warp_tight(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1))) {
         if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
         ok = false;
         break;
@@ -255,7 +256,7 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           // O_t += P_t V(j): A = P_t from tensor memory (8 columns per 16 kv rows), B = V(j) MN-major
 #pragma unroll
           for (int c = 0; c < F3_PARTS; ++c) {
-            if (ok && !mbar_wait_warp(&p_full[t * F3_PARTS + c], j & 1)) {
+            if (ok && !mbar_wait_warp_tight(&p_full[t * F3_PARTS + c], j & 1)) {
               if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_SOFTMAX);
               ok = false;
             }
@@ -292,7 +293,7 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     bool ok = true;
     const int my_n = t ? n_kv[1] : n_kv[0];
     for (int j = 0; j < my_n && ok; ++j) {
-      if (!mbar_wait_warp(&s_full[t], j & 1)) {
+      if (!mbar_wait_warp_tight(&s_full[t], j & 1)) {
         if (p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_TMEM_FULL);
         ok = false;
         break;
@@ -386,7 +387,7 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
     // ---- epilogue: O / l
     if (ok && my_n > 0) {
-      if (!mbar_wait_warp(&o_done[t], 0)) {
+      if (!mbar_wait_warp_tight(&o_done[t], 0)) {
         if (p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_TMEM_FULL);
       } else {
         tc_fence_after();

@@ -127,6 +127,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
   return __all_sync(0xffffffffu, ok);
 }
 
+// The same with the least code: a warp whose every step is a chain of such waits runs cold code between other warps'
+// unrolled loops, and its own length is what it waits for. try_wait suspends the warp between polls.
+__device__ __forceinline__ bool mbar_wait_warp_tight(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+  for (uint32_t it = 0; it < GF_WAIT_LIMIT; ++it)
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return false;
+}
+
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

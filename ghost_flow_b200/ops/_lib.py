@@ -59,9 +59,9 @@ _SIGS = {
     "gf_attn_decode": [P, L, P, P, I, P, I, P, L, I, I, I, I, F, I, P, P],
     "gf_flash_attn_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, F, I, P, P],
     "gf_attn_bwd_prep": [P, P, P, P, I, I, I, I, L, L, P],
-    "gf_flash_attn_bwd2": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, F, I, P, P],
-    "gf_attn_bwd_prep2": [P, P, P, P, P, P, I, I, I, I, L, L, P],
-    "gf_dq_tiles_to_bf16": [P, P, I, I, I, I, L, F, P],
+    "gf_flash_attn_bwd3": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, F, I, P, P],
+    "gf_attn_bwd_prep3": [P, P, P, P, P, P, I, I, I, I, L, L, P],
+    "gf_dq_rows_to_bf16": [P, P, I, I, I, I, L, F, P],
     "gf_cast_f32_to_bf16_2d": [P, P, L, I, L, L, F, P],
 }
 
@@ -244,7 +244,7 @@ def flash_attn_backward(q, k, v, o, do, lse, dq, dk, dv, B, S, Hq, Hkv, D, ld, s
     delta = torch.empty((B, Hq, S), dtype=torch.float32, device=dev)
     dq_acc = torch.empty((B * S, Hq * D), dtype=torch.float32, device=dev)
     c = 1 if causal else 0
-    if os.environ.get("GF_FA_BWD", "2") == "1":
+    if os.environ.get("GF_FA_BWD", "3") == "1":
         check_rc(lib.gf_attn_bwd_prep(o.data_ptr(), do.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), B, S, Hq, D,
                                       ld["o"], ld["do"], st), "gf_attn_bwd_prep")
         check_rc(lib.gf_flash_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), do.data_ptr(), lse.data_ptr(),
@@ -255,13 +255,13 @@ def flash_attn_backward(q, k, v, o, do, lse, dq, dk, dv, B, S, Hq, Hkv, D, ld, s
                                             st), "gf_cast_f32_to_bf16_2d")
     else:
         nlse2 = torch.empty((B, Hq, S), dtype=torch.float32, device=dev)
-        check_rc(lib.gf_attn_bwd_prep2(o.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
+        check_rc(lib.gf_attn_bwd_prep3(o.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
                                        nlse2.data_ptr(), dq_acc.data_ptr(), B, S, Hq, D, ld["o"], ld["do"], st),
-                 "gf_attn_bwd_prep2")
-        check_rc(lib.gf_flash_attn_bwd2(q.data_ptr(), k.data_ptr(), v.data_ptr(), do.data_ptr(), nlse2.data_ptr(),
+                 "gf_attn_bwd_prep3")
+        check_rc(lib.gf_flash_attn_bwd3(q.data_ptr(), k.data_ptr(), v.data_ptr(), do.data_ptr(), nlse2.data_ptr(),
                                         delta.data_ptr(), dq_acc.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, S, Hq,
                                         Hkv, D, ld["q"], ld["k"], ld["v"], ld["do"], ld["dk"], ld["dv"],
-                                        float(scale), c, status, st), "gf_flash_attn_bwd2")
-        # the main kernel leaves dQ / scale in the accumulator, tile by tile ([B, Hq, S / 64, 64, D])
-        check_rc(lib.gf_dq_tiles_to_bf16(dq_acc.data_ptr(), dq.data_ptr(), B, S, Hq, D, ld["dq"], float(scale), st),
-                 "gf_dq_tiles_to_bf16")
+                                        float(scale), c, status, st), "gf_flash_attn_bwd3")
+        # the main kernel leaves dQ / scale in the accumulator [B, Hq, S, D]
+        check_rc(lib.gf_dq_rows_to_bf16(dq_acc.data_ptr(), dq.data_ptr(), B, S, Hq, D, ld["dq"], float(scale), st),
+                 "gf_dq_rows_to_bf16")
