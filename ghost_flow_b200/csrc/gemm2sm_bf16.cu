@@ -16,7 +16,8 @@
 //     that has gone).
 // Every wait is bounded; a wait that runs out records a code in the status word and the role leaves its loop.
 //
-// Plain GEMMs only (all four operand layouts, the epilogue options of the single-CTA kernel); the fused roles
+// Plain GEMMs only (all four operand layouts, the epilogue options of the single-CTA kernel, e4m3 operands with row and
+// column scales); the fused roles
 // (all-gather, reduce-scatter, grouped, split-K, implicit convolution) stay in gemm_bf16.cu.
 // Replaces, like that file, ghostflow-cuda/src/optimized_kernels.cu:22-119 and ghostflow-cuda/src/blas.rs:278-313.
 #include "gf_host.h"
@@ -39,6 +40,9 @@ struct Gemm2Params {
   int tiles_m, tiles_n;     // 256 x BN tiles
   int band;                 // rows of tiles walked together (keeps one wave's A and B panels in L2)
   int act;                  // 0 none, 1 ReLU
+  // e4m3 operands: C = sa[m] * sb[n] * A B^T + bias
+  const float* sa;
+  const float* sb;
 };
 
 constexpr int G2_BM = 128;        // rows of A per CTA
@@ -105,6 +109,16 @@ __device__ __forceinline__ void umma_bf16_ss_2sm(bool leader, uint32_t tmem_d, u
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
       : "memory");
 }
+__device__ __forceinline__ void umma_f8_ss_2sm(bool leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
+      : "memory");
+}
 // Arrive on the barrier at a shared::cluster address once all MMAs issued so far by this thread have completed.
 __device__ __forceinline__ void umma_commit_2sm(bool leader, uint32_t bar_cluster_addr) {
   asm volatile(
@@ -129,7 +143,9 @@ __device__ __forceinline__ void g2_tile_coords(const Gemm2Params& p, int tile, i
   tn = r / rows;
 }
 
-template <int BNH, bool A_MN, bool B_MN>
+// F8: e4m3 operands (both K-major). A k block is 128 bytes of every row either way, 64 bf16 or 128 e4m3 values, and so are
+// its four instructions (16 or 32 values deep): only counts, instruction and epilogue differ.
+template <int BNH, bool A_MN, bool B_MN, bool F8>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
 gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const Gemm2Params p) {
@@ -138,6 +154,8 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   constexpr int G2_BN = Cfg::BN;
   constexpr int G2_STAGES = Cfg::STAGES;
   constexpr int G2_STAGE_BYTES = Cfg::STAGE_BYTES;
+  constexpr int BKE = F8 ? 2 * G2_BK : G2_BK;     // values of a k block
+  static_assert(!F8 || (!A_MN && !B_MN), "e4m3 operands are K-major");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + G2_STAGES * G2_STAGE_BYTES);
@@ -149,7 +167,7 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
-  const int num_kb = (p.K + G2_BK - 1) / G2_BK;
+  const int num_kb = (p.K + BKE - 1) / BKE;
   const int num_tiles = p.tiles_m * p.tiles_n;
   const int pair = (int)blockIdx.x >> 1;
   const int npairs = (int)gridDim.x >> 1;
@@ -198,7 +216,7 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           uint8_t* sb = sa + G2_A_BYTES;
           if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * G2_STAGE_BYTES);   // both CTAs' bytes
           const uint32_t fb = mapa_u32(smem_u32(&full_bar[stage]), 0);
-          const int k0 = kb * G2_BK;
+          const int k0 = kb * BKE;
           if (!A_MN) {
             tma_load_2d_2sm(sa, &tmA, fb, k0, m0);
           } else {
@@ -222,7 +240,8 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ------------------------------------------------------------ MMA issuer (even CTA only; uniform warp, one lane issues)
     if (rank == 0) {
       const bool leader = elect_one();
-      constexpr uint32_t idesc = umma_idesc_bf16(2 * G2_BM, G2_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t idesc = F8 ? umma_idesc_e4m3(2 * G2_BM, G2_BN)
+                                    : umma_idesc_bf16(2 * G2_BM, G2_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -252,7 +271,8 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                         : umma_desc_sw128(sa + kk * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? umma_desc_sw128(sb + kk * 2048, G2_BK * 128, 1024)
                                         : umma_desc_sw128(sb + kk * 32, 16, 1024);
-            umma_bf16_ss_2sm(leader, tmem_d, adesc, bdesc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            if constexpr (F8) umma_f8_ss_2sm(leader, tmem_d, adesc, bdesc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            else umma_bf16_ss_2sm(leader, tmem_d, adesc, bdesc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
           }
           // the stage is free in both CTAs once these MMAs have read it
           const uint32_t eb = smem_u32(&empty_bar[stage]);
@@ -282,6 +302,7 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       g2_tile_coords(p, tile, tm, tn);
       const int row = tm * 2 * G2_BM + (int)rank * G2_BM + lane_grp * 32 + lane;
       const int n0 = tn * G2_BN;
+      const float row_scale = F8 ? (row < p.M ? p.sa[row] : 0.f) : p.alpha;
       const int buf = it & 1;
       const uint32_t bphase = (it >> 1) & 1;
       ++it;
@@ -308,7 +329,20 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (row < p.M && col0 < p.N) {
           float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * row_scale;
+          if constexpr (F8) {
+            if (full) {                 // sb is on a 16-byte boundary and so is every 32nd entry
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float4 t = *reinterpret_cast<const float4*>(p.sb + col0 + q * 4);
+                v[q * 4] *= t.x; v[q * 4 + 1] *= t.y; v[q * 4 + 2] *= t.z; v[q * 4 + 3] *= t.w;
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (col0 + j < p.N) v[j] *= p.sb[col0 + j];
+            }
+          }
           if (p.bias) {
             if (full && bias_wide) {
 #pragma unroll
@@ -411,14 +445,14 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
 }
 
-template <int BNH, bool A_MN, bool B_MN>
+template <int BNH, bool A_MN, bool B_MN, bool F8 = false>
 static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, cudaStream_t stream) {
   using Cfg = G2Cfg<BNH>;
   constexpr int G2_SMEM_BYTES = Cfg::SMEM_BYTES;
   constexpr int G2_BN = Cfg::BN;
   static gf::DeviceOnce configured;
   static int max_pairs = 0;
-  auto kern = gemm2sm_bf16_kernel<BNH, A_MN, B_MN>;
+  auto kern = gemm2sm_bf16_kernel<BNH, A_MN, B_MN, F8>;
   if (configured.todo()) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_BYTES) != cudaSuccess)
       return GFH_CUDA;
@@ -496,6 +530,7 @@ int gemm2sm_run(const void* A, const void* B, void* C, int M, int N, int K, int 
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   p.ldr = ldr; p.alpha = alpha; p.status = status; p.act = activation == 1 ? 1 : 0;
+  p.sa = p.sb = nullptr;
 #define GF_G2_DISPATCH(BNH_)                                                                        \
   if (!a_mn_major && !b_mn_major) return launch_gemm2<BNH_, false, false>(tmA, tmB, p, stream);     \
   if (!a_mn_major && b_mn_major) return launch_gemm2<BNH_, false, true>(tmA, tmB, p, stream);       \
@@ -504,6 +539,21 @@ int gemm2sm_run(const void* A, const void* B, void* C, int M, int N, int K, int 
   if (bn == 256) { GF_G2_DISPATCH(128) }
   GF_G2_DISPATCH(64)
 #undef GF_G2_DISPATCH
+}
+
+// C[M, N] (bf16) = sa[m] * sb[n] * A[M, K] B[N, K]^T + bias, A and B e4m3 bytes; sb on a 16-byte boundary.
+int gemm2sm_run_fp8(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
+                    const float* sa, const float* sb, const void* bias, int* status, cudaStream_t stream) {
+  CUtensorMap tmA, tmB;
+  int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, lda, G2_BM, 2 * G2_BK);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, ldb, 128, 2 * G2_BK);
+  if (rc) return rc;
+  Gemm2Params p;
+  p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_fp32 = 0; p.accumulate = 0;
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  p.residual = nullptr; p.ldr = 0; p.alpha = 1.f; p.status = status; p.act = 0; p.sa = sa; p.sb = sb;
+  return launch_gemm2<128, false, false, true>(tmA, tmB, p, stream);
 }
 
 }  // namespace gf

@@ -22,6 +22,11 @@
 
 namespace gf {
 
+// CTA-pair kernel (gemm2sm_bf16.cu)
+int gemm2sm_wanted(int M, int N, int K);
+int gemm2sm_run_fp8(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
+                    const float* sa, const float* sb, const void* bias, int* status, cudaStream_t stream);
+
 constexpr int F8_BM = 128;
 constexpr int F8_BK = 128;          // e4m3 elements = 128 bytes = one swizzle-128B row
 constexpr int F8_THREADS = 192;
@@ -723,6 +728,12 @@ GF_API int gf_gemm_fp8(const void* A, const void* B, void* C, int M, int N, int 
   gf::enter();
   if (M <= 0 || N <= 0 || K <= 0 || (K & 15) || (lda & 15) || (ldb & 15) || !sa || !sb) return GFH_BAD_ARG;
   if (mode == 1 && (K & 127)) return GFH_BAD_ARG;
+  // large products with row and column scales run on CTA pairs (gemm2sm_bf16.cu): half the operand bytes per SM and
+  // instruction, where the single-CTA tiles ask shared memory for more than it delivers. The rule is that of the bf16 products
+  // (every pair has a tile of 256 x 256), but for at most 256 rows, which would leave half of a tile empty or one row of tiles.
+  // [4096, 4096] x [11008, 4096]^T 162 -> 145 us, 8192^3 466 -> 392 us, [2048, 4096] x [4096, 4096]^T 40 -> 35 us.
+  if (mode == 0 && M > 256 && gf::gemm2sm_wanted(M, N, K) && !(reinterpret_cast<uintptr_t>(sb) & 15))
+    return gf::gemm2sm_run_fp8(A, B, C, M, N, K, lda, ldb, ldc, sa, sb, bias, status, (cudaStream_t)stream_v);
   const int bn = mode == 0 ? 256 : 128;
   CUtensorMap tmA, tmB;
   int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, lda, F8_BM, F8_BK);

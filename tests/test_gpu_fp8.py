@@ -138,3 +138,21 @@ def test_transposed_quantisation_equals_quantising_the_transpose(R, K):
     assert torch.equal(fp8.quantize_transposed(odd)[0], fp8.quantize_rows(odd.clone().t().contiguous(), 0)[0])
     part = x[:, :8].contiguous()
     assert torch.equal(fp8.quantize_transposed(part)[0], fp8.quantize_rows(part.t().contiguous(), 0)[0])
+
+
+# 256 x 256 tiles for 74 pairs and one fewer, ragged in every dimension, K of one block and of a part of one
+@pytest.mark.parametrize("M,N,K", [(2048, 2368, 128), (2000, 2600, 528), (2560, 1800, 272), (2304, 2100, 1040), (256, 18944, 256),
+                                   (257, 9500, 256)])
+@pytest.mark.parametrize("with_bias", [True, False])
+def test_large_products_with_row_and_column_scales(M, N, K, with_bias, kernel_status):
+    from ghost_flow_b200.ops import fp8
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    N = N // 8 * 8
+    aq, sa = fp8.quantize_rows(torch.randn(M, K, generator=g, device="cuda").bfloat16())
+    bq, sb = fp8.quantize_rows(torch.randn(N, K, generator=g, device="cuda").bfloat16() * torch.linspace(0.01, 3, N, device="cuda").bfloat16()[:, None])
+    bias = torch.randn(N, generator=g, device="cuda").bfloat16() if with_bias else None
+    y = fp8.gemm_fp8(aq, sa, bq, sb, 0, bias)
+    want = fp8.dequantize(aq, sa, 0).double() @ fp8.dequantize(bq, sb, 0).double().t() + (bias.double() if with_bias else 0)
+    # e4m3 products are exact in fp32; fp32 sums of K of them, of size one times the scale of the column, and one bf16 rounding
+    assert torch.allclose(y.double(), want, rtol=2 ** -8, atol=3 * K * 2 ** -20)
