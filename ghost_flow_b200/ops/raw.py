@@ -245,9 +245,14 @@ def attn_decode(q, kcache, vcache, length, B, Hq, Hkv, D, scale=None, splits=Non
         per_seq = torch.is_tensor(length)
         n = s_max if per_seq else int(length)
         if splits is None:
-            # enough CTAs for about eight per SM (the kernel hides DRAM latency with warps in flight), but no
-            # slice shorter than 128 cache rows
-            splits = max(1, min(32, -(-(148 * 8) // max(1, B * Hkv)), (n + 127) // 128))
+            # Sequences of one length: as many slices as still fit the machine at once (two CTAs to an SM, four with
+            # D = 64); a second wave or a merge costs more than idle SMs (8 sequences of 1501 keys, 32 heads of 128: 40 us
+            # with one slice, 49 with five). Mixed lengths: about four waves, so that short sequences even out the
+            # long ones (32 sequences of 1 .. 4096 keys, 8 heads: 72 us with one slice, 56 with four or five).
+            # No slice is shorter than 128 cache rows.
+            ctas = max(1, B * Hkv)
+            waves = -(-(148 * 8) // ctas) if per_seq else 148 * (2 if D > 64 else 4) // ctas
+            splits = max(1, min(32, waves, (n + 127) // 128))
         if out is None:
             out = torch.empty(B, Hq * D, dtype=q.dtype, device=q.device)
         scratch = torch.empty(B * Hq * splits * (D + 2), dtype=torch.float32, device=q.device)
