@@ -11,108 +11,20 @@
 
 namespace gf {
 
-constexpr int XENT_THREADS = 512;
-
-// One CTA per row. The row is staged in shared memory as bf16 while the max is found, so the
-// logits are read from global memory exactly once; dlogits overwrite the logits in place
-// (or go to a separate buffer). loss_rows[t] = logsumexp - x[target]; ignored rows give 0.
-__global__ void __launch_bounds__(XENT_THREADS)
-xent_fused_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
-                  float* __restrict__ loss_rows, __nv_bfloat16* __restrict__ dlogits, int T, int V, long long ld,
-                  float grad_scale, long long ignore_index) {
-  extern __shared__ __align__(16) uint8_t xs_raw[];
-  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(xs_raw);
-  __shared__ float red[32];
-  // Rows move as 16-byte vectors. The host guarantees ld % 8 == 0 and ld >= round_up(V, 8), so the last vector of a
-  // row whose V is not a multiple of 8 lies inside the row's pitch: its columns >= V are read as -inf (they add
-  // nothing to the sum) and get gradient 0.
-  const int nv = (V + 7) >> 3;
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    const __nv_bfloat16* xr = logits + (long long)row * ld;
-    const long long tgt = targets[row];
-    float m = -INFINITY;
-    for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
-      uint4 u = *reinterpret_cast<const uint4*>(xr + v * 8);
-      if (v * 8 + 8 > V) {
-        unsigned short* h = reinterpret_cast<unsigned short*>(&u);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (v * 8 + j >= V) h[j] = 0xFF80;   // bf16 -inf
-      }
-      *reinterpret_cast<uint4*>(xs + v * 8) = u;
-      const uint32_t* p = reinterpret_cast<const uint32_t*>(&u);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float2 a = unpack_bf16x2(p[q]);
-        m = fmaxf(m, fmaxf(a.x, a.y));
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
-    m = red[0];
-#pragma unroll
-    for (int w = 1; w < XENT_THREADS / 32; ++w) m = fmaxf(m, red[w]);
-    float s = 0.f;
-    for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
-      uint4 u = *reinterpret_cast<const uint4*>(xs + v * 8);
-      const uint32_t* p = reinterpret_cast<const uint32_t*>(&u);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float2 a = unpack_bf16x2(p[q]);
-        s += __expf(a.x - m) + __expf(a.y - m);
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    s = 0.f;
-#pragma unroll
-    for (int w = 0; w < XENT_THREADS / 32; ++w) s += red[w];
-    const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V;
-    if (threadIdx.x == 0)
-      loss_rows[row] = ignored ? 0.f : (logf(s) + m - __bfloat162float(xs[tgt]));
-    if (dlogits) {
-      const float inv = ignored ? 0.f : grad_scale / s;
-      __nv_bfloat16* dr = dlogits + (long long)row * ld;
-      for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
-        uint4 u = *reinterpret_cast<const uint4*>(xs + v * 8);
-        uint32_t* p = reinterpret_cast<uint32_t*>(&u);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float2 a = unpack_bf16x2(p[q]);
-          float g0 = __expf(a.x - m) * inv, g1 = __expf(a.y - m) * inv;
-          const int c = v * 8 + q * 2;
-          if (!ignored) {
-            if (c == tgt) g0 -= grad_scale;
-            if (c + 1 == tgt) g1 -= grad_scale;
-          }
-          p[q] = pack_bf16x2(g0, g1);
-        }
-        *reinterpret_cast<uint4*>(dr + v * 8) = u;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// Rows of 40 to 110 KB (the vocabularies of language models): one CTA of 1024 threads per SM walks its rows, which arrive
-// through a ring of bulk copies, so the next rows load while this one is worked on. A row goes from the ring into
-// registers (NV packed vectors a thread) and its slot is free again; maximum and sum take one reduction, because every
-// thread sums against its own maximum and the pairs are merged. The kernel above has its loads, sums and stores one after
-// the other, in two CTAs per SM.
-// What bounds it: the phases of a row (6.5 us for 50257 logits: two passes of exponentials at 1.7 us on the
-// special-function unit, 4.5 us of memory traffic that only partly overlap). A polynomial on the FMA pipe for a quarter of
-// the exponentials made it slower (396 against 362 us), 512 threads help the longest rows by 2 % and cost the others 8 %.
-// [8192, 50257] 438 -> 362 us, [8192, 30522] 258 -> 214 us, [4096, 32000] 138 -> 115 us; [8192, 8192] would take 106
-// instead of 85 us, so shorter rows stay with the kernel above.
-constexpr int XR_THREADS = 1024;
-constexpr int XR_MAX_SLOTS = 4;
-constexpr size_t XR_RING_BYTES = 220 * 1024;
+// One CTA of 256 threads per row, as many on an SM as have room for their row in shared memory, each walking its rows: a bulk
+// copy brings the row, the threads take maximum and sum in one reduction (every thread sums against its own maximum and
+// the pairs are merged) and write the gradient, and the next copy starts. Loads, exponentials (two per logit, a third of
+// the time by themselves) and stores of one CTA follow one another; it is the CTAs of an SM, each in another phase, that
+// keep memory and special-function unit busy together. So small CTAs win, with no more registers than six of them
+// have, and the arithmetic goes two logits to an instruction.
+// dlogits overwrite the logits in place or go to a separate buffer. loss_rows[t] = logsumexp - x[target]; ignored rows give 0.
+// Measured, before (512 threads per row, plain loads, three reductions) -> now: [8192, 50257] 438 -> 306 us (5.4 TB/s),
+// [8192, 30522] 258 -> 179, [4096, 32000] 138 -> 98, [8192, 16384] 145 -> 95, [8192, 8192] 85 -> 59, [8192, 1000] 34 -> 25.
+// Others tried at [8192, 50257] / [8192, 30522]: 512 threads 304 / 184, 1024 threads 330 / 235, one CTA of 1024 with a ring of
+// rows and the row in registers 362 / 214, a quarter of the exponentials by polynomial 396 / 220.
+constexpr int XENT_THREADS = 256;
+constexpr int XENT_CTAS = 6;
+constexpr size_t XENT_SMEM = 220 * 1024;    // of an SM, for rows
 
 __device__ __forceinline__ void bulk_load_row(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -156,67 +68,63 @@ __device__ __forceinline__ void warp_max_sum(float& m, float& s) {
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
 }
 
-template <int NV>
-__global__ void __launch_bounds__(XR_THREADS, 1)
-xent_ring_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targets, float* __restrict__ loss_rows,
-                 __nv_bfloat16* dlogits, int T, int V, long long ld, float grad_scale, long long ignore_index, int slots,
-                 int* status) {
-  extern __shared__ __align__(128) uint8_t ring[];
-  __shared__ uint64_t full[XR_MAX_SLOTS];
-  __shared__ float red[2][2][32];
+__global__ void __launch_bounds__(XENT_THREADS, XENT_CTAS)
+xent_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targets, float* __restrict__ loss_rows,
+                 __nv_bfloat16* dlogits, int T, int V, long long ld, float grad_scale, long long ignore_index, int* status) {
+  extern __shared__ __align__(128) uint8_t rowbuf[];
+  __shared__ uint64_t full;
+  __shared__ float red[2][2][32];     // of alternate rows: maximum and sum of every warp
   const int nv = (V + 7) >> 3;
   const uint32_t row_bytes = (uint32_t)nv * 16;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 32) {               // warps that there are not add nothing
+    red[0][0][threadIdx.x] = red[1][0][threadIdx.x] = -INFINITY;
+    red[0][1][threadIdx.x] = red[1][1][threadIdx.x] = 0.f;
+  }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < slots; ++i) mbar_init(&full[i], 1);
+    mbar_init(&full, 1);
     mbar_fence_init();
   }
   __syncthreads();
-  auto load = [&](int slot, int row) {
-    mbar_expect_tx(&full[slot], row_bytes);
-    bulk_load_row(ring + (size_t)slot * row_bytes, logits + (long long)row * ld, row_bytes, &full[slot]);
+  auto load = [&](long long row) {
+    mbar_expect_tx(&full, row_bytes);
+    bulk_load_row(rowbuf, logits + row * ld, row_bytes, &full);
   };
-  if (threadIdx.x == 0)
-    for (int i = 0; i < slots; ++i)
-      if (blockIdx.x + (long long)i * gridDim.x < T) load(i, blockIdx.x + i * gridDim.x);
-  int slot = 0;
-  uint32_t phase = 0;
-  bool go = true;
+  if (threadIdx.x == 0 && blockIdx.x < T) load(blockIdx.x);
+  uint4* xs = reinterpret_cast<uint4*>(rowbuf);
   int k = 0;
   for (long long row = blockIdx.x; row < T; row += gridDim.x, ++k) {
     const long long tgt = targets[row];
     const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V;
-    const bool ok = mbar_wait(&full[slot], phase);
-    const __nv_bfloat16* xs = reinterpret_cast<const __nv_bfloat16*>(ring + (size_t)slot * row_bytes);
-    uint4 u[NV];
-    float xt = 0.f;
-    if (threadIdx.x == 0 && !ignored && ok) xt = __bfloat162float(xs[tgt]);
+    const bool ok = mbar_wait(&full, k & 1);
     constexpr uint32_t NONE = 0xFF80FF80u;     // bf16 -inf twice: adds nothing to the sum and gets gradient 0
     uint32_t mp = NONE;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = threadIdx.x + i * XR_THREADS;
-      u[i] = v < nv ? *reinterpret_cast<const uint4*>(xs + v * 8) : make_uint4(NONE, NONE, NONE, NONE);
-      if (v == nv - 1) {                        // columns of the last vector behind the row
-        const int c = V - v * 8;                // 1 .. 8 belong to it
-        uint32_t w[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+    for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
+      uint4 u = xs[v];
+      // The host guarantees ld % 8 == 0 and ld >= round_up(V, 8): the last vector lies inside the row's pitch, and those
+      // of its columns that are behind the row do not count.
+      if (v == nv - 1) {
+        const int c = V - v * 8;
+        uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) w[q] = 2 * q >= c ? NONE : 2 * q + 1 >= c ? (w[q] & 0xffffu) | (NONE & 0xffff0000u) : w[q];
-        u[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        u = make_uint4(w[0], w[1], w[2], w[3]);
+        xs[v] = u;
       }
-      mp = max_bf16x2(max_bf16x2(mp, max_bf16x2(u[i].x, u[i].y)), max_bf16x2(u[i].z, u[i].w));
+      mp = max_bf16x2(max_bf16x2(mp, max_bf16x2(u.x, u.y)), max_bf16x2(u.z, u.w));
     }
     const float2 m2 = unpack_bf16x2(mp);
     float m = fmaxf(m2.x, m2.y);
     const float m0 = m == -INFINITY ? 0.f : -m;
     const uint64_t nm0 = two(m0, m0);
     uint64_t sa = 0, sb = 0;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      sa = add_two(sa, exp_two(u[i].x, nm0));
-      sb = add_two(sb, exp_two(u[i].y, nm0));
-      sa = add_two(sa, exp_two(u[i].z, nm0));
-      sb = add_two(sb, exp_two(u[i].w, nm0));
+#pragma unroll 2
+    for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
+      const uint4 u = xs[v];
+      sa = add_two(sa, exp_two(u.x, nm0));
+      sb = add_two(sb, exp_two(u.y, nm0));
+      sa = add_two(sa, exp_two(u.z, nm0));
+      sb = add_two(sb, exp_two(u.w, nm0));
     }
     sa = add_two(sa, sb);
     float s = first(sa) + second(sa);
@@ -225,44 +133,43 @@ xent_ring_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targ
       red[k & 1][0][warp] = m;
       red[k & 1][1][warp] = s;
     }
-    go = __syncthreads_and(ok);                // every thread has its part of the row: the slot may be refilled
-    if (!go) break;
-    if (threadIdx.x == 0 && row + (long long)slots * gridDim.x < T) load(slot, (int)(row + (long long)slots * gridDim.x));
-    if (++slot == slots) { slot = 0; phase ^= 1; }
+    if (!__syncthreads_and(ok)) {              // the copy never arrived: all threads give up together
+      if (status && threadIdx.x == 0) atomicCAS(status, 0, GF_ERR_WAIT_FULL);
+      error_drain_pause();
+      break;
+    }
     m = red[k & 1][0][lane];
     s = red[k & 1][1][lane];
     warp_max_sum(m, s);
     if (m == -INFINITY) s = __int_as_float(0x7fffffff);    // no finite logit in the row: no probabilities either
-    if (threadIdx.x == 0) loss_rows[row] = ignored ? 0.f : (logf(s) + m - xt);
+    if (threadIdx.x == 0)
+      loss_rows[row] = ignored ? 0.f : logf(s) + m - __bfloat162float(reinterpret_cast<__nv_bfloat16*>(rowbuf)[tgt]);
     if (dlogits) {
       const float inv = ignored ? 0.f : grad_scale / s;
-      __nv_bfloat16* dr = dlogits + row * ld;
+      uint4* dr = reinterpret_cast<uint4*>(dlogits + row * ld);
       const int tv = ignored ? -1 : (int)(tgt >> 3), tj = (int)(tgt & 7);
       const uint64_t nm = two(-m, -m), inv2 = two(inv, inv);
+#pragma unroll 2
+      for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
+        const uint4 u = xs[v];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        uint32_t o[4];
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int v = threadIdx.x + i * XR_THREADS;
-        if (v < nv) {
-          const uint32_t w[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
-          uint32_t o[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint64_t g = mul_two(exp_two(w[q], nm), inv2);
-            float g0 = first(g), g1 = second(g);
-            if (v == tv) {
-              g0 -= 2 * q == tj ? grad_scale : 0.f;
-              g1 -= 2 * q + 1 == tj ? grad_scale : 0.f;
-            }
-            o[q] = pack_bf16x2(g0, g1);
+        for (int q = 0; q < 4; ++q) {
+          const uint64_t g = mul_two(exp_two(w[q], nm), inv2);
+          float g0 = first(g), g1 = second(g);
+          if (v == tv) {
+            g0 -= 2 * q == tj ? grad_scale : 0.f;
+            g1 -= 2 * q + 1 == tj ? grad_scale : 0.f;
           }
-          *reinterpret_cast<uint4*>(dr + v * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+          o[q] = pack_bf16x2(g0, g1);
         }
+        dr[v] = make_uint4(o[0], o[1], o[2], o[3]);
       }
     }
-  }
-  if (!go) {
-    if (status && threadIdx.x == 0) atomicCAS(status, 0, GF_ERR_WAIT_FULL);
-    error_drain_pause();                       // copies in flight land before the CTA's shared memory goes
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (threadIdx.x == 0 && row + gridDim.x < T) load(row + gridDim.x);
   }
 }
 
@@ -485,37 +392,19 @@ GF_API int gf_xent_fused(const void* logits, const long long* targets, float* lo
   if (V <= 0 || ld % 8 || ld < v8 || T <= 0) return GFH_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(dlogits) & 15)) return GFH_BAD_ARG;
   const size_t smem = (size_t)v8 * 2;
-  // the ring needs two rows; short ones are too little work for 1024 threads (measured on both sides: see the kernel)
-  if (smem >= 40 * 1024 && 2 * smem <= XR_RING_BYTES && v8 / 8 <= 7 * XR_THREADS) {
-    const int nv = (int)((v8 / 8 + XR_THREADS - 1) / XR_THREADS);
-    int slots = (int)(XR_RING_BYTES / smem);
-    if (slots > XR_MAX_SLOTS) slots = XR_MAX_SLOTS;
-    const int grid = T < sm_count() ? T : sm_count();
-    auto kern = nv <= 3 ? xent_ring_kernel<3>
-                : nv == 4 ? xent_ring_kernel<4> : nv == 5 ? xent_ring_kernel<5> : nv == 6 ? xent_ring_kernel<6>
-                : xent_ring_kernel<7>;
-    static gf::DeviceOnce ring_configured[8];
-    if (ring_configured[nv].todo()) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XR_RING_BYTES) != cudaSuccess)
-        return GFH_CUDA;
-      ring_configured[nv].mark();
-    }
-    kern<<<grid, XR_THREADS, slots * smem, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, targets, loss_rows,
-                                                                  (__nv_bfloat16*)dlogits, T, V, ld, grad_scale,
-                                                                  ignore_index, slots, gf::check_buffer());
-    return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
-  }
   if (smem > 200 * 1024) return GFH_TOO_LARGE;
   static gf::DeviceMax configured;
   if (smem > configured.get()) {
-    if (cudaFuncSetAttribute(xent_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(xent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return GFH_CUDA;
     configured.set(smem);
   }
-  xent_fused_kernel<<<T, XENT_THREADS, smem, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, targets,
-                                                                    loss_rows, (__nv_bfloat16*)dlogits, T, V, ld,
-                                                                    grad_scale, ignore_index);
+  long long per_sm = (long long)(XENT_SMEM / (smem + 2048));   // 1 KB of static and reserved shared memory each, rounded up
+  per_sm = per_sm < 1 ? 1 : per_sm > XENT_CTAS ? XENT_CTAS : per_sm;
+  const long long most = per_sm * sm_count();
+  xent_kernel<<<(unsigned)(T < most ? T : most), XENT_THREADS, smem, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)logits, targets, loss_rows, (__nv_bfloat16*)dlogits, T, V, ld, grad_scale, ignore_index,
+      gf::check_buffer());
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
 }
 

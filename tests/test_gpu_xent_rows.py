@@ -1,4 +1,4 @@
-"""Cross-entropy over the row lengths at which the kernels change (shared-memory row, ring of rows, threads per row), against
+"""Cross-entropy over the row lengths at which the launch changes, against
 fp64: loss and gradient, ignored rows, in place, -inf and all-masked logits."""
 import pytest
 import torch
@@ -6,10 +6,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# 20472 / 20480: the rows on both sides of the ring's first length; 50257 and 24577: ragged last vectors; 56320 / 56328: the
-# longest two rows that fit and the next one
-@pytest.mark.parametrize("V", [5, 1000, 20472, 20480, 24577, 30522, 32000, 50257, 56320, 56328])
-@pytest.mark.parametrize("T", [1, 150, 460])
+# row lengths around a vector, a round of 256 threads, and those at which one CTA less fits an SM (six rows of 34.5 KB, two of
+# 108 KB, one above); ragged last vectors; the longest row of all
+@pytest.mark.parametrize("V", [5, 8, 1000, 2047, 2056, 17664, 17672, 30522, 50257, 55295, 55304, 102400])
+@pytest.mark.parametrize("T", [1, 150, 901])
 def test_loss_and_gradient_match_fp64(V, T):
     from ghost_flow_b200 import ops
 
@@ -22,14 +22,14 @@ def test_loss_and_gradient_match_fp64(V, T):
         buf[1, : V // 2] = float("-inf")           # a mask over half the classes
         tg[1] = V - 1
         tg[2] = -100
-    logits = buf[:, :V].clone(memory_format=torch.preserve_format) if V % 8 == 0 else buf[:, :V]
+    logits = buf[:, :V]
     logits.requires_grad_(True)
     lg = logits.detach().double().requires_grad_(True)
     want = torch.nn.functional.cross_entropy(lg, tg, ignore_index=-100)
     want.backward()
     loss = ops.cross_entropy(logits, tg, ignore_index=-100)
     (dl,) = torch.autograd.grad(loss, logits)
-    # fp32 sums of up to 56328 positive terms over T rows; the gradient is one bf16 rounding away (2^-9)
+    # fp32 sums of up to 102400 positive terms over T rows; the gradient is one bf16 rounding away (2^-9)
     assert abs(loss.item() - want.item()) < 1e-5 * abs(want.item())
     assert dl.shape == logits.shape and ((dl.double() - lg.grad).norm() / lg.grad.norm()).item() < 4e-3
     assert torch.allclose(dl.double(), lg.grad, rtol=2 ** -7, atol=1e-9)
