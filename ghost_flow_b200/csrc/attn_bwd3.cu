@@ -522,8 +522,15 @@ fa_bwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
 // Row statistics and the cleared dQ accumulator in one pass: ndelta[b, h, s] = -sum_d O dO, nlse2 = -lse * log2(e).
 // Bound by memory; HD / 8 lanes share a row with one 16-byte load of O and dO each, a thread takes four rows at once.
+// WIDE = false: rows on 8-byte boundaries only (a caller's own pitch), two loads for one.
 constexpr int P3_ROWS = 4;
-template <int HD>
+template <bool WIDE>
+__device__ __forceinline__ uint4 load_8_bf16(const __nv_bfloat16* p) {
+  if constexpr (WIDE) return *reinterpret_cast<const uint4*>(p);
+  const uint2 a = reinterpret_cast<const uint2*>(p)[0], b = reinterpret_cast<const uint2*>(p)[1];
+  return make_uint4(a.x, a.y, b.x, b.y);
+}
+template <int HD, bool WIDE>
 __global__ void __launch_bounds__(256)
 attn_bwd_prep3_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                       const float* __restrict__ lse, float* __restrict__ ndelta, float* __restrict__ nlse2,
@@ -539,8 +546,8 @@ attn_bwd_prep3_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* 
     const int s = s0 + k * RPB;
     if (s < S) {
       const long long t = (long long)b * S + s;
-      a[k] = *reinterpret_cast<const uint4*>(o + t * ldo + h * HD + l * 8);
-      g[k] = *reinterpret_cast<const uint4*>(dout + t * lddo + h * HD + l * 8);
+      a[k] = load_8_bf16<WIDE>(o + t * ldo + h * HD + l * 8);
+      g[k] = load_8_bf16<WIDE>(dout + t * lddo + h * HD + l * 8);
     }
   }
 #pragma unroll
@@ -571,7 +578,7 @@ attn_bwd_prep3_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* 
 }
 
 // dq[b * S + s, h * HD + d] = bf16(scale * acc[b, h, s, d]); eight elements to a thread and row, four rows at once.
-template <int HD>
+template <int HD, bool WIDE>
 __global__ void __launch_bounds__(256)
 dq_rows_to_bf16_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int S, int Hq, long long lddq,
                        float scale) {
@@ -599,7 +606,13 @@ dq_rows_to_bf16_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict_
       u.y = pack_bf16x2(f[k][0].z * scale, f[k][0].w * scale);
       u.z = pack_bf16x2(f[k][1].x * scale, f[k][1].y * scale);
       u.w = pack_bf16x2(f[k][1].z * scale, f[k][1].w * scale);
-      *reinterpret_cast<uint4*>(dq + ((long long)b * S + s) * lddq + (long long)h * HD + l * 8) = u;
+      __nv_bfloat16* out = dq + ((long long)b * S + s) * lddq + (long long)h * HD + l * 8;
+      if constexpr (WIDE) {
+        *reinterpret_cast<uint4*>(out) = u;
+      } else {
+        reinterpret_cast<uint2*>(out)[0] = make_uint2(u.x, u.y);
+        reinterpret_cast<uint2*>(out)[1] = make_uint2(u.z, u.w);
+      }
     }
   }
 }
@@ -634,16 +647,19 @@ static int launch_fa_bwd3(const void* q, const void* k, const void* v, const voi
 
 using namespace gf;
 
-// ndelta, nlse2: fp32 [B, Hq, S]; dq_acc: fp32 [B, Hq, S, HD], cleared. Rows of o and dout on 16-byte boundaries.
+// ndelta, nlse2: fp32 [B, Hq, S]; dq_acc: fp32 [B, Hq, S, HD], cleared. Rows of o and dout on 8-byte boundaries.
 GF_API int gf_attn_bwd_prep3(const void* o, const void* dout, const float* lse, float* ndelta, float* nlse2,
                              float* dq_acc, int B, int S, int Hq, int HD, long long ldo, long long lddo, void* stream) {
   gf::enter();
-  if (B <= 0 || S <= 0 || Hq <= 0 || B > 65535 || Hq > 65535 || (ldo % 8) || (lddo % 8) || (HD != 64 && HD != 128) ||
-      ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dq_acc)) & 15))
+  if (B <= 0 || S <= 0 || Hq <= 0 || B > 65535 || Hq > 65535 || (ldo % 4) || (lddo % 4) || (HD != 64 && HD != 128) ||
+      ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 7) || (reinterpret_cast<uintptr_t>(dq_acc) & 15))
     return GFH_BAD_ARG;
+  const bool wide = ldo % 8 == 0 && lddo % 8 == 0 &&
+                    ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0;
   const int rows = 256 / (HD / 8) * P3_ROWS;
   const dim3 grid((S + rows - 1) / rows, Hq, B);
-  auto kern = HD == 128 ? attn_bwd_prep3_kernel<128> : attn_bwd_prep3_kernel<64>;
+  auto kern = HD == 128 ? (wide ? attn_bwd_prep3_kernel<128, true> : attn_bwd_prep3_kernel<128, false>)
+                        : (wide ? attn_bwd_prep3_kernel<64, true> : attn_bwd_prep3_kernel<64, false>);
   kern<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, ndelta, nlse2,
                                                dq_acc, S, Hq, ldo, lddo);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
@@ -671,16 +687,18 @@ GF_API int gf_flash_attn_bwd3(const void* q, const void* k, const void* v, const
   return GFH_BAD_ARG;
 }
 
-// Converts the fp32 dQ accumulator [B, Hq, S, HD] into bf16 rows with pitch lddq.
+// Converts the fp32 dQ accumulator [B, Hq, S, HD] into bf16 rows with pitch lddq, on 8-byte boundaries.
 GF_API int gf_dq_rows_to_bf16(const float* acc, void* dq, int B, int S, int Hq, int HD, long long lddq, float scale,
                               void* stream) {
   gf::enter();
-  if (B <= 0 || S <= 0 || Hq <= 0 || B > 65535 || Hq > 65535 || (lddq % 8) || (HD != 64 && HD != 128) ||
-      ((reinterpret_cast<uintptr_t>(acc) | reinterpret_cast<uintptr_t>(dq)) & 15))
+  if (B <= 0 || S <= 0 || Hq <= 0 || B > 65535 || Hq > 65535 || (lddq % 4) || (HD != 64 && HD != 128) ||
+      (reinterpret_cast<uintptr_t>(acc) & 15) || (reinterpret_cast<uintptr_t>(dq) & 7))
     return GFH_BAD_ARG;
+  const bool wide = lddq % 8 == 0 && (reinterpret_cast<uintptr_t>(dq) & 15) == 0;
   const int rows = 256 / (HD / 8) * P3_ROWS;
   const dim3 grid((S + rows - 1) / rows, Hq, B);
-  auto kern = HD == 128 ? dq_rows_to_bf16_kernel<128> : dq_rows_to_bf16_kernel<64>;
+  auto kern = HD == 128 ? (wide ? dq_rows_to_bf16_kernel<128, true> : dq_rows_to_bf16_kernel<128, false>)
+                        : (wide ? dq_rows_to_bf16_kernel<64, true> : dq_rows_to_bf16_kernel<64, false>);
   kern<<<grid, 256, 0, (cudaStream_t)stream>>>(acc, (__nv_bfloat16*)dq, S, Hq, lddq, scale);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
 }

@@ -37,3 +37,30 @@ def test_gradients_match_fp64(B, S, H, Hk, D, causal, kernel_status):
         # while the typical row of a long causal sequence is only about 0.3 long
         err = (got.double() - want).norm(dim=-1) / want.norm(dim=-1).clamp_min(want.norm() / math.sqrt(want[..., 0].numel()))
         assert err.max().item() < 0.1 and ((got.double() - want).norm() / want.norm()).item() < 5e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("pad,shift", [(4, 0), (0, 4), (4, 4)])
+def test_rows_on_8_byte_boundaries(D, pad, shift, kernel_status):
+    """The caller's own pitch and offset for o and dq; same numbers as from packed rows."""
+    from ghost_flow_b200.ops import raw
+
+    B, S, H = 2, 256, 2
+    g = torch.Generator(device="cuda").manual_seed(D + pad)
+    q, k, v, do = (torch.randn(B * S, H * D, generator=g, device="cuda").bfloat16() for _ in range(4))
+    o, lse = raw.attn_fwd(q, k, v, B, S, H, H, D)
+
+    def strided(fill):
+        t = torch.zeros(B * S * (H * D + pad) + shift, device="cuda", dtype=torch.bfloat16)[shift:].view(B * S, H * D + pad)
+        return t, t[:, :H * D].copy_(fill)
+
+    got = []
+    for narrow in (False, True):
+        whole, dq = strided(torch.zeros_like(q)) if narrow else (None, torch.empty_like(q))
+        oo = strided(o)[1] if narrow else o
+        raw.attn_bwd(q, k, v, oo, do, lse, dq, torch.empty_like(k), torch.empty_like(v), B, S, H, H, D)
+        got.append(dq)
+        if narrow and pad:
+            assert whole[:, H * D:].count_nonzero().item() == 0
+    # sums of two key tiles in either order, rounded once to bf16
+    assert torch.allclose(got[0].float(), got[1].float(), rtol=2 ** -8, atol=1e-6)
