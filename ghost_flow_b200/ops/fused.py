@@ -12,6 +12,7 @@ import math
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import _lib
 
@@ -356,9 +357,19 @@ def swiglu(gu):
     return F.silu(g) * u
 
 
+def _observed() -> bool:
+    """Whether something follows the tensor operations of this call that a kernel launch would escape: tracing, compilation,
+    ``torch.func`` transforms, dispatch or function modes, forward-mode gradients."""
+    return (torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active()
+            or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
+            or forward_ad._current_level >= 0 or torch.compiler.is_compiling())
+
+
 def embedding_rows(ids, table):
     """``table[ids]`` with zero rows for ids outside the table, in one launch; ``None`` where the kernel does not apply
-    (CPU tensors, a gradient to record, rows that are no whole 16-byte vectors)."""
+    (CPU tensors, a gradient to record, rows that are no whole 16-byte vectors, tensors that are traced or transformed)."""
+    if type(ids) is not torch.Tensor or type(table) not in (torch.Tensor, torch.nn.Parameter) or _observed():
+        return None
     if not (table.is_cuda and ids.is_cuda and ids.device == table.device and table.dim() == 2 and ids.numel() > 0
             and ids.dtype in (torch.int64, torch.int32) and table.dtype in (torch.bfloat16, torch.float32, torch.float16)
             and not (torch.is_grad_enabled() and table.requires_grad) and table.is_contiguous() and table.shape[0] > 0):

@@ -23,3 +23,22 @@ def test_lookup_equals_the_masked_form(D, dtype, shape, kind):
     if len(shape) == 2:
         with torch.no_grad():
             assert torch.equal(e(ids.t()), want.detach().transpose(0, 1))
+
+
+def test_traced_and_transformed_calls_keep_the_tensor_library_form():
+    from torch.autograd import forward_ad
+
+    from ghost_flow_b200.nn import Embedding
+
+    e = Embedding(6, 8, device="cuda").requires_grad_(False)
+    ids, other = torch.tensor([[1, 7, 2]], device="cuda"), torch.tensor([[5, 0, -1]], device="cuda")
+    want = e(other)
+    assert torch.equal(torch.vmap(e)(other), want)
+    with torch.no_grad():
+        assert torch.equal(torch.jit.trace(e, ids)(other), want)
+    with forward_ad.dual_level():
+        w = forward_ad.make_dual(e.weight.detach(), torch.ones_like(e.weight))
+        tangent = forward_ad.unpack_dual(torch.func.functional_call(e, {"weight": w}, (other,))).tangent
+    assert torch.equal(tangent, torch.ones_like(want) * (want.abs().sum(-1, keepdim=True) > 0))
+    e.weight = torch.nn.Parameter(torch.ones(8, 8, device="cuda"), requires_grad=False)    # more rows than ids that count
+    assert e(ids)[0, 1].count_nonzero().item() == 0
