@@ -143,11 +143,14 @@ class Optimizer:
         writes them where they lie; ``None`` when one of them has a layout, type or device that needs the flat copy."""
         if f["repeats"]:
             return None
-        out, dev = [], f["master"].device
+        out, dev, written = [], f["master"].device, set()
         for p, o, view in zip(f["params"], f["offs"], f["is_view"]):
             g = p.grad
-            if g is None:
+            if g is None or g.numel() == 0:
                 continue
+            if p.data_ptr() in written:         # two parameters over one storage: the copy back gives an order
+                return None
+            written.add(p.data_ptr())
             if g.dtype not in (torch.bfloat16, torch.float32) or g.device != dev or g.layout != torch.strided \
                     or not g.is_contiguous() or type(g) not in (torch.Tensor, torch.nn.Parameter):
                 return None

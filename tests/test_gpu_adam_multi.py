@@ -61,3 +61,20 @@ def test_layouts_that_need_the_flat_copy_give_the_same_result():
         oa.step()
         ob.step()
     assert torch.equal(a, b)
+
+
+def test_empty_parameters_and_shared_storage():
+    from ghost_flow_b200.optim import AdamW
+
+    w = torch.randn(64, device="cuda").bfloat16()
+    tied = [torch.nn.Parameter(w.clone()) for _ in range(2)]
+    tied[1].data = tied[0].data
+    alone = torch.nn.Parameter(w.clone())
+    empty = torch.nn.Parameter(torch.zeros(0, 3, device="cuda"))
+    for p in (*tied, alone, empty):
+        p.grad = torch.ones_like(p)
+    tied[0].grad.neg_()
+    AdamW([*tied, empty], lr=0.1).step()
+    AdamW([empty, alone], lr=0.1).step()
+    assert torch.equal(tied[0], alone)          # the second of the two parameters is written last
+    AdamW([empty], lr=0.1).step()
