@@ -1,6 +1,6 @@
 // gf_rmsnorm_bwd_noalloc: RMSNorm backward whose weight-gradient scratch lives in a fixed device
 // array of this module, for callers that cannot allocate (see gf_noalloc.h for who they are, the
-// size limit and the sharing rules). Same math as rmsnorm_bwd_kernel in norm.cu.
+// size limit and the sharing rules). Same math as the RMSNorm backward in norm.cu.
 #include "gf_noalloc.h"
 
 #include <mutex>
