@@ -69,10 +69,9 @@ class Embedding(Module):
 
     def forward(self, ids):
         idx = ids.long() if ids.is_floating_point() else ids
-        if self.weight.shape[0] == self.num_embeddings:
-            out = ops.embedding_rows(idx, self.weight)
-            if out is not None:
-                return out
+        out = ops.embedding_rows(idx, self.weight, self.num_embeddings)
+        if out is not None:
+            return out
         oob = (idx < 0) | (idx >= self.num_embeddings)
         out = F.embedding(idx.clamp(0, self.num_embeddings - 1), self.weight, self.padding_idx)
         # applied unconditionally: asking the device whether any id is out of range would stall the host on every
