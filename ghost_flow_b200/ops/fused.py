@@ -367,12 +367,13 @@ def _observed() -> bool:
 
 def embedding_rows(ids, table, rows: int | None = None):
     """``table[ids]`` with zero rows for ids outside the table, in one launch; ``None`` where the kernel does not apply
-    (CPU tensors, a gradient to record, rows that are no whole 16-byte vectors, tensors that are traced or transformed,
-    a table of other than ``rows`` rows)."""
+    (CPU tensors, a GPU that is not the current one, a gradient to record, rows that are no whole 16-byte vectors, tensors
+    that are traced or transformed, a table of other than ``rows`` rows)."""
     if type(ids) is not torch.Tensor or type(table) not in (torch.Tensor, torch.nn.Parameter) or _observed():
         return None
     if not (table.is_cuda and ids.is_cuda and ids.device == table.device and table.dim() == 2 and ids.numel() > 0
             and ids.dtype in (torch.int64, torch.int32) and table.dtype in (torch.bfloat16, torch.float32, torch.float16)
+            and table.device.index == torch.cuda.current_device()     # launches go to the current device
             and not (torch.is_grad_enabled() and table.requires_grad) and table.is_contiguous() and table.shape[0] > 0
             and rows in (None, table.shape[0])):
         return None

@@ -42,3 +42,17 @@ def test_traced_and_transformed_calls_keep_the_tensor_library_form():
     assert torch.equal(tangent, torch.ones_like(want) * (want.abs().sum(-1, keepdim=True) > 0))
     e.weight = torch.nn.Parameter(torch.ones(8, 8, device="cuda"), requires_grad=False)    # more rows than ids that count
     assert e(ids)[0, 1].count_nonzero().item() == 0
+
+
+def test_a_table_off_the_current_device_keeps_the_tensor_library_form(monkeypatch):
+    from ghost_flow_b200 import ops
+    from ghost_flow_b200.nn import Embedding
+    from ghost_flow_b200.ops import _lib
+
+    e = Embedding(6, 8, device="cuda").requires_grad_(False)
+    ids = torch.tensor([[1, 7, 2]], device="cuda")
+    want = e(ids)
+    other = torch.cuda.current_device() + 1
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: other)
+    n0 = _lib.launch_count()
+    assert ops.embedding_rows(ids, e.weight) is None and torch.equal(e(ids), want) and _lib.launch_count() == n0
