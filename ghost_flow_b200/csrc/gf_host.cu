@@ -63,17 +63,22 @@ int make_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int
   return GFH_OK;
 }
 
+// The device a thread selected is that thread's own; a thread that selected none (a plain C caller, a worker) follows the
+// last selection of any thread. Two threads that drive two GPUs would otherwise launch on each other's device.
 static std::atomic<int> g_device{-1};
+static thread_local int t_device = -1;
 static std::atomic<long long> g_launches{0};
 
 void note_extra_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-// Every exported launcher calls this first: it binds the calling thread to the process's device in
+int process_device() { return t_device >= 0 ? t_device : g_device.load(std::memory_order_relaxed); }
+
+// Every exported launcher calls this first: it binds the calling thread to its device in
 // this library's copy of the CUDA runtime (PyTorch keeps its own copy, with its own per-thread state).
 void enter() {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   thread_local int bound = -2;
-  const int d = g_device.load(std::memory_order_relaxed);
+  const int d = process_device();
   if (d < 0) {
     if (bound == -2) {
       cudaFree(0);
@@ -86,8 +91,6 @@ void enter() {
     bound = d;
   }
 }
-
-int process_device() { return g_device.load(std::memory_order_relaxed); }
 
 int sm_count() {
   static int cached[64] = {0};
@@ -134,7 +137,12 @@ void set_check_buffer(int device, int* p) {
 }  // namespace gf
 
 // ------------------------------------------------------------------ C surface
-GF_API void gf_set_device(int dev) { gf::g_device.store(dev); }
+GF_API void gf_set_device(int dev) {
+  gf::t_device = dev;
+  gf::g_device.store(dev);
+}
+// The device the calling thread's launches go to, -1 when none was selected.
+GF_API int gf_selected_device() { return gf::process_device(); }
 
 // Kernels launched by this library since load (every launcher counts its own kernels).
 GF_API long long gf_launch_count() { return gf::g_launches.load(); }

@@ -78,7 +78,7 @@ int attention_head_group_l2(int heads, long long bytes_per_head);
 void enter();
 // Launchers that start more than one kernel report the extra ones here (enter() counts one).
 void note_extra_launches(int n);
-// Device index selected with gf_set_device, or -1 when none was selected.
+// Device index selected with gf_set_device by this thread, else the last one selected by any, or -1.
 int process_device();
 
 // Asks for the largest shared-memory carve-out for a kernel that itself needs little shared memory. An SM

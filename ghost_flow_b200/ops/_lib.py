@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from pathlib import Path
 
@@ -27,6 +28,7 @@ _SIGS = {
     "gf_device_count": [],
     "gf_version": [],
     "gf_set_device": [I],
+    "gf_selected_device": [],
     "gf_gemm_bf16": [P, P, P, I, I, I, I, L, I, L, L, I, I, P, P, L, F, P, I, I, P, I, I, P],
     "gf_norm_bwd_grid": [I],
     "gf_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
@@ -132,19 +134,18 @@ def host_lib():
     return _HOST_LIB
 
 
-_BOUND_DEVICE = -1
+_BOUND = threading.local()     # .device: the one this thread last selected in the kernel library
 # the handle without the Python stream object around it (3 us of every launch); absent in some torch builds
 _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def stream_ptr() -> int:
     """Current CUDA stream handle; also keeps the kernel library's device in step with PyTorch's
-    (the library carries its own copy of the CUDA runtime, with its own current-device state)."""
-    global _BOUND_DEVICE
+    (the library carries its own copy of the CUDA runtime, with its own current-device state, per thread as PyTorch's is)."""
     dev = torch.cuda.current_device()
-    if dev != _BOUND_DEVICE:
+    if dev != getattr(_BOUND, "device", -1):
         cuda_lib().gf_set_device(dev)
-        _BOUND_DEVICE = dev
+        _BOUND.device = dev
     return _RAW_STREAM(dev) if _RAW_STREAM is not None else torch.cuda.current_stream().cuda_stream
 
 
