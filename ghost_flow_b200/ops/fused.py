@@ -195,6 +195,21 @@ def rope_ref(x, cos, sin, interleaved=False, pos_offset=0):
     return out.to(x.dtype)
 
 
+def check_rope_tables(device, S: int, D: int, cos, sin, pos_offset: int) -> None:
+    """Raises where the kernels, which index the tables by position without a bound, would read outside of them."""
+    if not (cos.device == sin.device == device and cos.dim() == sin.dim() == 2 and cos.shape[1] == sin.shape[1] == D // 2):
+        raise ValueError(f"rope tables must be [positions, {D // 2}] on {device}, got {list(cos.shape)} on {cos.device} "
+                         f"and {list(sin.shape)} on {sin.device}")
+    if pos_offset < 0 or pos_offset + S > min(cos.shape[0], sin.shape[0]):
+        raise ValueError(f"rope positions {pos_offset} .. {pos_offset + S - 1} are not in tables of "
+                         f"{min(cos.shape[0], sin.shape[0])} rows")
+
+
+def _rope_tables_fit_kernel(cos, sin) -> bool:
+    return (cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0)
+
+
 def _rope_launch(x, cos, sin, S, interleaved, pos_offset, backward):
     """In place on x viewed as [T, H, D] (unit stride over D; rows and heads may be strided)."""
     T, H, D = x.shape
@@ -232,7 +247,9 @@ class _RopeFn(torch.autograd.Function):
 def rope(x, cos, sin, interleaved: bool = False, pos_offset: int = 0, inplace: bool = False):
     """Rotary embedding on ``[B, S, H, D]``; half-split pairing by default, ``interleaved`` for (2i, 2i+1)."""
     if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] % 16 == 0:
-        return _call(_RopeFn, x, cos, sin, interleaved, pos_offset, inplace)
+        check_rope_tables(x.device, x.shape[-3], x.shape[-1], cos, sin, pos_offset)
+        if _rope_tables_fit_kernel(cos, sin):
+            return _call(_RopeFn, x, cos, sin, interleaved, pos_offset, inplace)
     return rope_ref(x, cos, sin, interleaved, pos_offset)
 
 
@@ -289,16 +306,19 @@ class _RopeQKVFn(torch.autograd.Function):
         return g, None, None, None, None, None, None
 
 
-def _rope_qkv_ok(qkv, cos, sin) -> bool:
-    return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.shape[-1] % 16 == 0 and qkv.numel() > 0
-            and cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
-            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0)
+def _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset) -> bool:
+    if qkv.shape[2] != H + 2 * Hk:
+        raise ValueError(f"a packed projection of {H} + 2 x {Hk} heads has {H + 2 * Hk} of them, not {qkv.shape[2]}")
+    if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.shape[-1] % 16 == 0 and qkv.numel() > 0):
+        return False
+    check_rope_tables(qkv.device, qkv.shape[1], qkv.shape[3], cos, sin, pos_offset)
+    return _rope_tables_fit_kernel(cos, sin)
 
 
 def rope_qkv(qkv, num_heads: int, num_kv_heads: int, cos, sin, interleaved: bool = False, pos_offset: int = 0):
     """``q, k, v`` of a packed projection output ``[B, S, H + 2 Hk, D]`` with q and k rotated (see :func:`rope`)."""
     H, Hk = num_heads, num_kv_heads
-    if _rope_qkv_ok(qkv, cos, sin):
+    if _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset):
         return _call(_RopeQKVFn, qkv, H, Hk, cos, sin, interleaved, pos_offset)
     q, k, v = split_qkv(qkv, H, Hk)
     return rope(q, cos, sin, interleaved, pos_offset), rope(k, cos, sin, interleaved, pos_offset), v
@@ -310,7 +330,7 @@ def rope_qkv_to_cache(qkv, num_heads: int, num_kv_heads: int, cos, sin, kcache, 
     ``[B, max_len, Hk, D]``. Inference only: nothing is recorded for autograd."""
     B, S, _, D = qkv.shape
     H, Hk = num_heads, num_kv_heads
-    if not torch.is_grad_enabled() and _rope_qkv_ok(qkv, cos, sin) and pos_offset + S <= kcache.shape[1] \
+    if not torch.is_grad_enabled() and _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset) and pos_offset + S <= kcache.shape[1] \
             and all(c.is_cuda and c.device == qkv.device and c.dtype == qkv.dtype and c.shape == (B, kcache.shape[1], Hk, D)
                     and c.stride(3) == 1 and c.stride(2) == D and c.stride(1) % 8 == 0 and c.stride(0) % 8 == 0
                     and c.data_ptr() % 16 == 0 for c in (kcache, vcache)):

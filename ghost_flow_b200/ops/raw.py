@@ -11,7 +11,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib
-from .fused import _scratch, rope_ref
+from .fused import _scratch, check_rope_tables, rope_ref
 from .gemm import gemm_raw
 
 
@@ -102,6 +102,7 @@ def rmsnorm_bwd(x, w, dy, rstd, dres=None, dw_out=None):
 def rope_(x3, cos, sin, S, interleaved=False, pos_offset=0, backward=False):
     T, H, D = x3.shape
     if _k(x3):
+        check_rope_tables(x3.device, S, D, cos, sin, pos_offset)
         _rc(_lib.cuda_lib().gf_rope(x3.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, H, D, x3.stride(0),
                                     x3.stride(1), S, pos_offset, 1 if interleaved else 0, 1 if backward else 0,
                                     _lib.stream_ptr()), "gf_rope")

@@ -60,3 +60,35 @@ def test_rope_qkv_to_cache(B, S, H, Hk, D, layout):
         rest = torch.ones(n, dtype=torch.bool)
         rest[pos:pos + S] = False
         assert torch.equal(c[:, rest], w[:, rest])
+
+
+def test_positions_outside_the_tables_are_refused_before_any_launch():
+    from ghost_flow_b200 import ops
+    from ghost_flow_b200.ops import _lib, raw
+
+    qkv = torch.randn(1, 4, 6, 64, device="cuda", dtype=torch.bfloat16)
+    kc, vc = (torch.zeros(1, 32, 2, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    tables = [(*ops.rope_tables(8, 64, 1e4, "cuda"), 5), (*ops.rope_tables(8, 64, 1e4, "cuda"), -1),
+              (*ops.rope_tables(8, 128, 1e4, "cuda"), 0), (*ops.rope_tables(8, 64, 1e4, "cpu"), 0)]
+    n0 = _lib.launch_count()
+    for cos, sin, pos in tables:
+        with torch.no_grad(), pytest.raises(ValueError):
+            ops.rope_qkv_to_cache(qkv, 2, 2, cos, sin, kc, vc, False, pos)
+        with pytest.raises(ValueError):
+            ops.rope_qkv(qkv, 2, 2, cos, sin, False, pos)
+        with pytest.raises(ValueError):
+            ops.rope(qkv, cos, sin, False, pos)
+        with pytest.raises(ValueError):
+            raw.rope_(qkv.view(4, 6, 64), cos, sin, 4, False, pos)
+    assert _lib.launch_count() == n0 and not kc.any() and not vc.any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float64])
+def test_tables_of_another_type_give_the_same_rotation(dtype):
+    from ghost_flow_b200 import ops
+
+    x = torch.randn(2, 5, 6, 64, device="cuda", dtype=torch.bfloat16)
+    cos, sin = (t.to(dtype) for t in ops.rope_tables(8, 64, 1e4, "cuda"))
+    got, want = ops.rope_qkv(x, 2, 2, cos, sin, False, 3), ops.rope_qkv(x, 2, 2, cos.float(), sin.float(), False, 3)
+    for g, w in zip(got, want):
+        assert _close(g, w)
