@@ -377,25 +377,33 @@ def swiglu(gu):
     return F.silu(g) * u
 
 
+# private names of torch (tracing, torch.func transforms, dispatch modes, function modes, forward-mode level); a torch build
+# without one of them counts as observed throughout, and the tensor-library form is taken
+_PROBES = tuple(getattr(torch._C, n, None) for n in ("_get_tracing_state", "_are_functorch_transforms_active",
+                                                      "_len_torch_dispatch_stack", "_len_torch_function_stack"))
+
+
 def _observed() -> bool:
     """Whether something follows the tensor operations of this call that a kernel launch would escape: tracing, compilation,
     ``torch.func`` transforms, dispatch or function modes, forward-mode gradients."""
-    return (torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active()
-            or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
-            or forward_ad._current_level >= 0 or torch.compiler.is_compiling())
+    if None in _PROBES:
+        return True
+    tracing, transforms, dispatch_modes, function_modes = _PROBES
+    return (tracing() is not None or transforms() or dispatch_modes() > 0 or function_modes() > 0
+            or getattr(forward_ad, "_current_level", 0) >= 0 or torch.compiler.is_compiling())
 
 
 def embedding_rows(ids, table, rows: int | None = None):
     """``table[ids]`` with zero rows for ids outside the table, in one launch; ``None`` where the kernel does not apply
     (CPU tensors, a GPU that is not the current one, a gradient to record, rows that are no whole 16-byte vectors, tensors
     that are traced or transformed, a table of other than ``rows`` rows)."""
-    if type(ids) is not torch.Tensor or type(table) not in (torch.Tensor, torch.nn.Parameter) or _observed():
+    if type(ids) is not torch.Tensor or type(table) not in (torch.Tensor, torch.nn.Parameter) or not table.is_cuda \
+            or (torch.is_grad_enabled() and table.requires_grad) or _observed():
         return None
-    if not (table.is_cuda and ids.is_cuda and ids.device == table.device and table.dim() == 2 and ids.numel() > 0
+    if not (ids.is_cuda and ids.device == table.device and table.dim() == 2 and ids.numel() > 0
             and ids.dtype in (torch.int64, torch.int32) and table.dtype in (torch.bfloat16, torch.float32, torch.float16)
             and table.device.index == torch.cuda.current_device()     # launches go to the current device
-            and not (torch.is_grad_enabled() and table.requires_grad) and table.is_contiguous() and table.shape[0] > 0
-            and rows in (None, table.shape[0])):
+            and table.is_contiguous() and table.shape[0] > 0 and rows in (None, table.shape[0])):
         return None
     row_bytes = table.shape[1] * table.element_size()
     if row_bytes == 0 or row_bytes % 16 or table.data_ptr() % 16:
