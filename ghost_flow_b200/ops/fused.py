@@ -330,13 +330,15 @@ def rope_qkv_to_cache(qkv, num_heads: int, num_kv_heads: int, cos, sin, kcache, 
     ``[B, max_len, Hk, D]``. Inference only: nothing is recorded for autograd."""
     B, S, _, D = qkv.shape
     H, Hk = num_heads, num_kv_heads
-    if not torch.is_grad_enabled() and _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset) and pos_offset + S <= kcache.shape[1] \
+    # what follows the assignments below (dispatch modes, transforms) would not see the kernel's writes
+    if not torch.is_grad_enabled() and not _observed() and _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset) and pos_offset + S <= kcache.shape[1] \
             and all(c.is_cuda and c.device == qkv.device and c.dtype == qkv.dtype and c.shape == (B, kcache.shape[1], Hk, D)
                     and c.stride(3) == 1 and c.stride(2) == D and c.stride(1) % 8 == 0 and c.stride(0) % 8 == 0
                     and c.data_ptr() % 16 == 0 for c in (kcache, vcache)):
         q = torch.empty((B, S, H, D), dtype=qkv.dtype, device=qkv.device)
         _rope_qkv_launch(qkv[:, :, :H], qkv[:, :, H:H + Hk], qkv[:, :, H + Hk:], q, kcache[:, pos_offset:pos_offset + S],
                          vcache[:, pos_offset:pos_offset + S], cos, sin, interleaved, pos_offset, False)
+        torch.autograd.graph.increment_version((kcache, vcache))     # a graph that saved a cache has to notice the write
         return q
     q, k, v = rope_qkv(qkv, H, Hk, cos, sin, interleaved, pos_offset)
     kcache[:, pos_offset:pos_offset + S] = k

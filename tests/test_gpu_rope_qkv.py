@@ -92,3 +92,38 @@ def test_tables_of_another_type_give_the_same_rotation(dtype):
     got, want = ops.rope_qkv(x, 2, 2, cos, sin, False, 3), ops.rope_qkv(x, 2, 2, cos.float(), sin.float(), False, 3)
     for g, w in zip(got, want):
         assert _close(g, w)
+
+
+def test_cache_writes_are_visible_to_autograd_and_to_dispatch_modes():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from ghost_flow_b200 import ops
+
+    cos, sin = ops.rope_tables(8, 64, 1e4, "cuda")
+    qkv = torch.randn(1, 1, 6, 64, device="cuda", dtype=torch.bfloat16)
+    kc, vc = (torch.randn(1, 8, 2, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    w = torch.ones_like(kc, requires_grad=True)
+    for saved in (kc, vc):
+        y = (saved * w).sum()
+        with torch.no_grad():
+            ops.rope_qkv_to_cache(qkv, 2, 2, cos, sin, kc, vc, False, 3)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            y.backward()
+    with torch.inference_mode():
+        ic = torch.zeros_like(kc), torch.zeros_like(vc)
+        ops.rope_qkv_to_cache(qkv, 2, 2, cos, sin, *ic, False, 3)
+    assert torch.equal(ic[0][:, 3], kc[:, 3]) and torch.equal(ic[1][:, 3], vc[:, 3])
+
+    written = []
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if func._schema.name == "aten::copy_":
+                written.append(args[0].untyped_storage().data_ptr())
+            return func(*args, **(kwargs or {}))
+
+    want = kc.clone(), vc.clone()
+    with torch.no_grad(), Mode():
+        ops.rope_qkv_to_cache(qkv, 2, 2, cos, sin, kc, vc, False, 3)
+    assert {kc.untyped_storage().data_ptr(), vc.untyped_storage().data_ptr()} <= set(written)
+    assert _close(kc, want[0]) and _close(vc, want[1])
