@@ -324,6 +324,30 @@ def rope_qkv(qkv, num_heads: int, num_kv_heads: int, cos, sin, interleaved: bool
     return rope(q, cos, sin, interleaved, pos_offset), rope(k, cos, sin, interleaved, pos_offset), v
 
 
+def _rows_apart(row: int, dims) -> bool:
+    """Whether rows of ``row`` elements repeated over ``dims`` = (stride, count) pairs share no element (sufficient: every
+    stride reaches over all that lies inside it)."""
+    extent = row
+    for st, n in sorted(dims):
+        if n > 1:
+            if st < extent:
+                return False
+            extent += st * (n - 1)
+    return True
+
+
+def _cache_rows_apart(kc, vc) -> bool:
+    """Whether no two rows of the caches ``[B, n, Hk, D]`` (packed heads) share memory: expanded caches are refused by the
+    assignments, and two that overlap are written by them one after the other."""
+    row = kc.shape[2] * kc.shape[3]
+    dims = [[(c.stride(i), c.shape[i]) for i in (0, 1)] for c in (kc, vc)]
+    a, b = (c.data_ptr() // c.element_size() for c in (kc, vc))
+    if dims[0] == dims[1]:               # the caches themselves are one more dimension, wherever it lies
+        return _rows_apart(row, [*dims[0], (abs(b - a), 2)])
+    ends = sorted((p, p + row + sum(st * (n - 1) for st, n in d)) for p, d in zip((a, b), dims))
+    return all(_rows_apart(row, d) for d in dims) and ends[0][1] <= ends[1][0]
+
+
 def rope_qkv_to_cache(qkv, num_heads: int, num_kv_heads: int, cos, sin, kcache, vcache, interleaved: bool = False,
                       pos_offset: int = 0):
     """Rotated q of a packed projection output; rotated k and v go to rows ``pos_offset ..`` of the caches
@@ -334,7 +358,7 @@ def rope_qkv_to_cache(qkv, num_heads: int, num_kv_heads: int, cos, sin, kcache, 
     if not torch.is_grad_enabled() and not _observed() and _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset) and pos_offset + S <= kcache.shape[1] \
             and all(c.is_cuda and c.device == qkv.device and c.dtype == qkv.dtype and c.shape == (B, kcache.shape[1], Hk, D)
                     and c.stride(3) == 1 and c.stride(2) == D and c.stride(1) % 8 == 0 and c.stride(0) % 8 == 0
-                    and c.data_ptr() % 16 == 0 for c in (kcache, vcache)):
+                    and c.data_ptr() % 16 == 0 for c in (kcache, vcache)) and _cache_rows_apart(kcache, vcache):
         q = torch.empty((B, S, H, D), dtype=qkv.dtype, device=qkv.device)
         _rope_qkv_launch(qkv[:, :, :H], qkv[:, :, H:H + Hk], qkv[:, :, H + Hk:], q, kcache[:, pos_offset:pos_offset + S],
                          vcache[:, pos_offset:pos_offset + S], cos, sin, interleaved, pos_offset, False)

@@ -127,3 +127,17 @@ def test_cache_writes_are_visible_to_autograd_and_to_dispatch_modes():
         ops.rope_qkv_to_cache(qkv, 2, 2, cos, sin, kc, vc, False, 3)
     assert {kc.untyped_storage().data_ptr(), vc.untyped_storage().data_ptr()} <= set(written)
     assert _close(kc, want[0]) and _close(vc, want[1])
+
+
+def test_caches_whose_rows_share_memory_take_the_assignments():
+    from ghost_flow_b200 import ops
+
+    cos, sin = ops.rope_tables(8, 64, 1e4, "cuda")
+    qkv = torch.randn(2, 1, 6, 64, device="cuda", dtype=torch.bfloat16)
+    mk = lambda b: torch.zeros(b, 8, 2, 64, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+    with torch.no_grad():
+        with pytest.raises(RuntimeError):                   # refused, as a write to an expanded tensor is
+            ops.rope_qkv_to_cache(qkv, 2, 2, cos, sin, mk(1).expand(2, -1, -1, -1), mk(2), False, 3)
+        both = mk(2)
+        ops.rope_qkv_to_cache(qkv, 2, 2, cos, sin, both, both, False, 3)
+    assert torch.equal(both[:, 3], qkv[:, 0, 4:])           # v is written last
