@@ -16,17 +16,11 @@ from torch.autograd import forward_ad
 
 from . import _lib
 
-_SCRATCH = {}
-
-
 def _scratch(device, nfloats: int) -> torch.Tensor:
-    """Grow-only fp32 workspace per device (partial sums of the norm backward kernels)."""
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    t = _SCRATCH.get(key)
-    if t is None or t.numel() < nfloats:
-        t = torch.empty(max(nfloats, 1 << 20), dtype=torch.float32, device=device)
-        _SCRATCH[key] = t
-    return t
+    """fp32 workspace of one call (partial sums of the norm backward kernels). From torch's allocator, so that it belongs to
+    the current stream, or to the graph's pool while a CUDA graph is recorded: one buffer kept for all calls would be
+    shared by streams, and a recorded graph would go on writing it after it was replaced by a larger one."""
+    return torch.empty(nfloats, dtype=torch.float32, device=device)
 
 
 def _cuda_bf16(*ts) -> bool:
