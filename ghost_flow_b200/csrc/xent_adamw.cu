@@ -134,7 +134,7 @@ xent_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targets, 
       red[k & 1][1][warp] = s;
     }
     if (!__syncthreads_and(ok)) {              // the copy never arrived: all threads give up together
-      if (status && threadIdx.x == 0) atomicCAS(status, 0, GF_ERR_WAIT_FULL);
+      if (threadIdx.x == 0) atomicCAS(status, 0, GF_ERR_WAIT_FULL);
       error_drain_pause();
       break;
     }
@@ -384,12 +384,13 @@ static inline int flat_grid(long long n) {
 
 using namespace gf;
 
-// dlogits may equal logits (in place) or be null (loss only). ld = row pitch in elements.
+// dlogits may equal logits (in place) or be null (loss only). ld = row pitch in elements. status: device int that receives a
+// code when the bounded wait for a row runs out (that CTA's remaining rows are then not written).
 GF_API int gf_xent_fused(const void* logits, const long long* targets, float* loss_rows, void* dlogits, int T, int V,
-                         long long ld, float grad_scale, long long ignore_index, void* stream) {
+                         long long ld, float grad_scale, long long ignore_index, int* status, void* stream) {
   gf::enter();
   const long long v8 = ((long long)V + 7) / 8 * 8;
-  if (V <= 0 || ld % 8 || ld < v8 || T <= 0) return GFH_BAD_ARG;
+  if (V <= 0 || ld % 8 || ld < v8 || T <= 0 || !status) return GFH_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(dlogits) & 15)) return GFH_BAD_ARG;
   const size_t smem = (size_t)v8 * 2;
   if (smem > 200 * 1024) return GFH_TOO_LARGE;
@@ -403,8 +404,7 @@ GF_API int gf_xent_fused(const void* logits, const long long* targets, float* lo
   per_sm = per_sm < 1 ? 1 : per_sm > XENT_CTAS ? XENT_CTAS : per_sm;
   const long long most = per_sm * sm_count();
   xent_kernel<<<(unsigned)(T < most ? T : most), XENT_THREADS, smem, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)logits, targets, loss_rows, (__nv_bfloat16*)dlogits, T, V, ld, grad_scale, ignore_index,
-      gf::check_buffer());
+      (const __nv_bfloat16*)logits, targets, loss_rows, (__nv_bfloat16*)dlogits, T, V, ld, grad_scale, ignore_index, status);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
 }
 

@@ -47,7 +47,7 @@ _SIGS = {
     "gf_binary": [P, P, P, L, I, F, I, P],
     "gf_reduce": [P, P, P, L, I, I, P],
     "gf_softmax_rows": [P, P, I, I, I, I, P],
-    "gf_xent_fused": [P, P, P, P, I, I, L, F, L, P],
+    "gf_xent_fused": [P, P, P, P, I, I, L, F, L, P, P],
     "gf_adam_flat": [P, P, P, P, P, L, F, F, F, F, F, I, F, I, I, P, P],
     "gf_adam_flat_dev": [P, P, P, P, P, L, F, F, F, F, F, I, F, I, I, P, P, P],
     "gf_adam_multi": [P, P, P, P, I, F, F, F, F, F, I, F, I, P],

@@ -533,7 +533,7 @@ class _XentFn(torch.autograd.Function):
         _rc(_lib.cuda_lib().gf_xent_fused(l2.data_ptr(), tg.data_ptr(), loss_rows.data_ptr(),
                                           dl.data_ptr() if dl is not None else None, T, V, l2.stride(0), scale,
                                           ignore_index if ignore_index is not None else -(1 << 62),
-                                          _lib.stream_ptr()), "gf_xent_fused")
+                                          _lib.status_word(l2.device).data_ptr(), _lib.stream_ptr()), "gf_xent_fused")
         loss = loss_rows.sum() * scale
         ctx.save_for_backward(dl if dl is not None else torch.empty(0, device=logits.device))
         ctx.shape = logits.shape

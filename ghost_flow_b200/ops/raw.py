@@ -203,7 +203,8 @@ def xent_fwd_bwd(logits, targets, grad_scale=None):
         loss_rows = torch.empty(T, dtype=torch.float32, device=logits.device)
         _rc(_lib.cuda_lib().gf_xent_fused(logits.data_ptr(), targets.data_ptr(), loss_rows.data_ptr(),
                                           logits.data_ptr(), T, V, logits.stride(0), float(scale), -(1 << 62),
-                                          _lib.stream_ptr()), "gf_xent_fused")
+                                          _lib.status_word(logits.device).data_ptr(), _lib.stream_ptr()),
+            "gf_xent_fused")
         return loss_rows.sum() * scale
     lf = logits.float()
     lse = torch.logsumexp(lf, -1)

@@ -60,3 +60,12 @@ def test_in_place_gradient_overwrites_the_logits():
     p[torch.arange(300), tg] -= 1
     raw.xent_fwd_bwd(x, tg)
     assert ((x.double() - p / 300).norm() / p.norm() * 300).item() < 4e-3
+
+
+def test_a_launch_without_a_status_word_is_refused():
+    from ghost_flow_b200.ops import _lib
+
+    x, tg, rows = torch.zeros(2, 64, device="cuda").bfloat16(), torch.zeros(2, dtype=torch.int64, device="cuda"), torch.zeros(2, device="cuda")
+    args = (x.data_ptr(), tg.data_ptr(), rows.data_ptr(), None, 2, 64, 64, 0.5, -100)
+    assert _lib.cuda_lib().gf_xent_fused(*args, None, _lib.stream_ptr()) == -1
+    assert _lib.cuda_lib().gf_xent_fused(*args, _lib.status_word().data_ptr(), _lib.stream_ptr()) == 0
