@@ -140,23 +140,40 @@ class Optimizer:
     @staticmethod
     def _tensors_in_place(f):
         """``(gradient, bf16 weight or None, offset)`` of every parameter with a gradient, for a kernel that reads and
-        writes them where they lie; ``None`` when one of them has a layout, type or device that needs the flat copy."""
+        writes them where they lie; ``None`` when one of them has a layout, type or device that needs the flat copy, or
+        when the kernel would write what it reads or writes elsewhere."""
         if f["repeats"]:
             return None
-        out, dev, written = [], f["master"].device, set()
+        m = f["master"]
+        out, dev = [], m.device
+        spans = [(m.data_ptr(), m.data_ptr() + 4 * m.numel(), True)]        # first and last byte; is it written?
         for p, o, view in zip(f["params"], f["offs"], f["is_view"]):
             g = p.grad
+            if not view and p.numel() > 0:
+                if not p.is_contiguous():
+                    return None
+                a = p.data_ptr()
+                spans.append((a, a + p.numel() * p.element_size(), True))
             if g is None or g.numel() == 0:
                 continue
-            if p.data_ptr() in written:         # two parameters over one storage: the copy back gives an order
-                return None
-            written.add(p.data_ptr())
             if g.dtype not in (torch.bfloat16, torch.float32) or g.device != dev or g.layout != torch.strided \
-                    or not g.is_contiguous() or type(g) not in (torch.Tensor, torch.nn.Parameter):
+                    or not g.is_contiguous() or g.is_neg() or type(g) not in (torch.Tensor, torch.nn.Parameter):
                 return None
-            if not view and (p.dtype != torch.bfloat16 or p.device != dev or not p.is_contiguous()):
+            if not view and (p.dtype != torch.bfloat16 or p.device != dev):
                 return None
+            a = g.data_ptr()
+            spans.append((a, a + g.numel() * g.element_size(), False))
             out.append((g, None if view else p, o))
+        # parameters over one storage are copied back one after the other, and a gradient that lies over a weight or the
+        # master copy is read before anything is written: one launch gives neither order
+        spans.sort()
+        end = end_written = 0
+        for a, b, written in spans:
+            if a < (end if written else end_written):
+                return None
+            end = max(end, b)
+            if written:
+                end_written = max(end_written, b)
         return out
 
     @staticmethod

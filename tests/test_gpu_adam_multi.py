@@ -78,3 +78,17 @@ def test_empty_parameters_and_shared_storage():
     AdamW([empty, alone], lr=0.1).step()
     assert torch.equal(tied[0], alone)          # the second of the two parameters is written last
     AdamW([empty], lr=0.1).step()
+
+
+def test_overlapping_weights_are_copied_back_in_order():
+    from ghost_flow_b200.optim import AdamW
+
+    w = torch.randn(96, device="cuda").bfloat16()
+    buf, alone = w.clone(), [torch.nn.Parameter(w[lo:lo + 64].clone()) for lo in (0, 32)]
+    ps = [torch.nn.Parameter(buf[lo:lo + 64]) for lo in (0, 32)]
+    for p, q in zip(ps, alone):
+        q.grad = torch.randn(64, device="cuda").bfloat16()
+        p.grad = q.grad.clone()
+    AdamW(ps, lr=0.1).step()
+    AdamW(alone, lr=0.1).step()
+    assert torch.equal(buf, torch.cat((alone[0].detach()[:32], alone[1].detach())))    # the second is written last
