@@ -177,10 +177,10 @@ class Optimizer:
         return out
 
     @staticmethod
-    def _scatter_params(f):
+    def _scatter_params(f, only_without_grad=False):
         m = f["master"]
         for i, (p, o) in enumerate(zip(f["params"], f["offs"])):
-            if not f["is_view"][i]:
+            if not f["is_view"][i] and not (only_without_grad and p.grad is not None):
                 p.data.copy_(m[o:o + p.numel()].view_as(p))
 
     def state_dict(self):
@@ -292,10 +292,11 @@ class Adam(Optimizer):
                 hyper = dict(lr=g["lr"], beta1=b1, beta2=b2, eps=g["eps"], weight_decay=g["weight_decay"], step=t,
                              decoupled=self.decoupled)
                 if tensors is not None:
-                    # a parameter that has no gradient keeps its bf16 value: its master copy did not move either
                     with torch.cuda.device(f["master"].device):
                         if tensors:
                             adam_multi(f["master"], *f["state"], tensors, **hyper)
+                    # the others show their master copy all the same: it may have been loaded since
+                    self._scatter_params(f, only_without_grad=True)
                 else:
                     grads, runs = self._gather_grads(f)
                     with torch.cuda.device(f["master"].device):

@@ -92,3 +92,23 @@ def test_overlapping_weights_are_copied_back_in_order():
     AdamW(ps, lr=0.1).step()
     AdamW(alone, lr=0.1).step()
     assert torch.equal(buf, torch.cat((alone[0].detach()[:32], alone[1].detach())))    # the second is written last
+
+
+def test_loaded_master_weights_reach_parameters_without_a_gradient():
+    from ghost_flow_b200.optim import AdamW
+
+    def make():
+        g = torch.Generator(device="cuda").manual_seed(3)
+        ps = [torch.nn.Parameter(torch.randn(40, generator=g, device="cuda").bfloat16()) for _ in range(3)]
+        return ps, AdamW(ps, lr=0.1)
+
+    ps, opt = make()
+    for p in ps:
+        p.grad = torch.ones_like(p)
+    opt.step()
+    saved, want = opt.state_dict(), [p.detach().clone() for p in ps]
+    qs, other = make()
+    other.load_state_dict(saved)                    # the optimizer alone: its master copies are the truth
+    qs[0].grad = torch.zeros_like(qs[0])
+    other.step()
+    assert torch.equal(qs[1], want[1]) and torch.equal(qs[2], want[2])
