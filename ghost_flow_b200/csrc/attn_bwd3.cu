@@ -85,34 +85,6 @@ struct FaBwd3Cfg {
   static constexpr int TMEM_COLS = 512;
 };
 
-// ---- two fp32 at a time (one issue slot for two results)
-__device__ __forceinline__ uint64_t pk2(uint32_t a, uint32_t b) { return (uint64_t)a | ((uint64_t)b << 32); }
-__device__ __forceinline__ uint64_t pk2f(float a, float b) { return pk2(__float_as_uint(a), __float_as_uint(b)); }
-__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
-__device__ __forceinline__ void bulk_load_1d_b3(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(smem_dst)),
-               "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
 template <int HD>
 __global__ void __launch_bounds__(B3_THREADS, 1)
 fa_bwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -225,8 +197,8 @@ fa_bwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             tma_load_2d(sQ + st * Cfg::TILE_BYTES + c * (B3_TILE * 128), &tmQ, &q_full[st], h * HD + c * 64,
                         row_base + i * B3_TILE);
           const long long soff = ((long long)b * p.Hq + h) * p.S + (long long)i * B3_TILE;
-          bulk_load_1d_b3(sStat + st * 2 * B3_TILE, p.nlse2 + soff, B3_TILE * 4, &q_full[st]);
-          bulk_load_1d_b3(sStat + st * 2 * B3_TILE + B3_TILE, p.ndelta + soff, B3_TILE * 4, &q_full[st]);
+          bulk_load_1d(sStat + st * 2 * B3_TILE, p.nlse2 + soff, B3_TILE * 4, &q_full[st]);
+          bulk_load_1d(sStat + st * 2 * B3_TILE + B3_TILE, p.ndelta + soff, B3_TILE * 4, &q_full[st]);
           if (!mbar_wait(do_empty, (it & 1) ^ 1)) {
             if (p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_EMPTY);
             break;

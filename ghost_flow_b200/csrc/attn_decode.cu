@@ -28,12 +28,6 @@ constexpr int DEC_MAX_G = 8;
 constexpr int DEC_KEYS = 16;     // keys of a block
 constexpr int DEC_STAGES = 3;
 
-__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -138,8 +132,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, const __n
     for (int t = 0; t < D / 16; ++t) {
       uint32_t a[4];
       ldmatrix_x4(a, tk + (lane & 15) * Cfg::ROW + (16 * t + (lane >> 4) * 8) * 2);
-      if (t & 1) mma_bf16_16816(sd, a, qb[t][0], qb[t][1]);
-      else mma_bf16_16816(sc, a, qb[t][0], qb[t][1]);
+      if (t & 1) mma_bf16_16816(sd, a[0], a[1], a[2], a[3], qb[t][0], qb[t][1]);
+      else mma_bf16_16816(sc, a[0], a[1], a[2], a[3], qb[t][0], qb[t][1]);
     }
     const int left = s1 - (s0 + (i * DEC_WARPS + warp) * DEC_KEYS);    // valid keys of the block, at least one
     float corr[2], p[4];
@@ -166,7 +160,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, const __n
       uint32_t a[4];
       ldmatrix_x4_trans(a, tv + ((lane & 7) + ((lane >> 4) << 3)) * Cfg::ROW + (16 * j + ((lane >> 3) & 1) * 8) * 2);
       o[j][0] *= corr[0]; o[j][1] *= corr[1]; o[j][2] *= corr[0]; o[j][3] *= corr[1];
-      mma_bf16_16816(o[j], a, b0, b1);
+      mma_bf16_16816(o[j], a[0], a[1], a[2], a[3], b0, b1);
     }
     __syncwarp();                  // the stage is filled again two blocks on
   }

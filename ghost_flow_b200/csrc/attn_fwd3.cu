@@ -43,23 +43,6 @@ constexpr int F3_REGS_SOFTMAX = 200;
 constexpr int F3_PARTS = 2;       // P V of a tile is issued in this many parts of the kv rows, each as soon as its P is there
 constexpr float F3_RESCALE_THRESHOLD = 8.0f;  // log2 units
 
-// ---- two fp32 at a time (one issue slot for two results)
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -351,18 +334,16 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
       const float mref_use = (m_ref == -INFINITY) ? 0.f : m_ref;  // row with no visible key yet
       const float mneg = -mref_use * sl2;
-      const uint64_t sl2x = pack2(sl2, sl2), mnegx = pack2(mneg, mneg);
+      const uint64_t sl2x = pk2f(sl2, sl2), mnegx = pk2f(mneg, mneg);
       uint64_t rsa = 0, rsb = 0;
       uint32_t sa[32], sb[32];
       auto chunk = [&](const uint32_t (&sv)[32], uint32_t dst) {
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p0, p1;
-          unpack2(fma2(pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2x, mnegx), p0, p1);
-          p0 = ex2_approx(p0);
-          p1 = ex2_approx(p1);
-          if (i & 2) rsa = add2(rsa, pack2(p0, p1)); else rsb = add2(rsb, pack2(p0, p1));
+          const uint64_t x = f2_fma(pk2(sv[i], sv[i + 1]), sl2x, mnegx);
+          const float p0 = ex2_approx(lo2(x)), p1 = ex2_approx(hi2(x));
+          if (i & 2) rsa = f2_add(rsa, pk2f(p0, p1)); else rsb = f2_add(rsb, pk2f(p0, p1));
           pk[i >> 1] = pack_bf16x2(p0, p1);
         }
         tmem_st16(dst, pk);
@@ -381,9 +362,8 @@ fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[t * F3_PARTS + c2]);
       }
-      float r0, r1;
-      unpack2(add2(rsa, rsb), r0, r1);
-      l += r0 + r1;
+      const uint64_t rs = f2_add(rsa, rsb);
+      l += lo2(rs) + hi2(rs);
     }
     // ---- epilogue: O / l
     if (ok && my_n > 0) {

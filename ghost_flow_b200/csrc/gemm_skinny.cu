@@ -28,14 +28,6 @@ __device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {   // read o
   return v;
 }
 
-__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                          uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // NT tiles of eight tokens, U k blocks of 64 in flight per warp
 template <int NT, int U>
 __global__ void __launch_bounds__(SK_WARPS * 32)
@@ -78,8 +70,8 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __n
     for (int h = 0; h < U * 2; ++h)
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        mma_16816(acc[t], u[h][0].x, u[h][1].x, u[h][0].y, u[h][1].y, x[h][t].x, x[h][t].y);
-        mma_16816(acc[t], u[h][0].z, u[h][1].z, u[h][0].w, u[h][1].w, x[h][t].z, x[h][t].w);
+        mma_bf16_16816(acc[t], u[h][0].x, u[h][1].x, u[h][0].y, u[h][1].y, x[h][t].x, x[h][t].y);
+        mma_bf16_16816(acc[t], u[h][0].z, u[h][1].z, u[h][0].w, u[h][1].w, x[h][t].z, x[h][t].w);
       }
   }
 #pragma unroll

@@ -26,34 +26,11 @@ constexpr int XENT_THREADS = 256;
 constexpr int XENT_CTAS = 6;
 constexpr size_t XENT_SMEM = 220 * 1024;    // of an SM, for rows
 
-__device__ __forceinline__ void bulk_load_row(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(smem_dst)),
-               "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-// ---- two fp32 at a time (one issue slot for two results)
-__device__ __forceinline__ uint64_t two(float a, float b) {
-  return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32);
-}
-__device__ __forceinline__ float first(uint64_t v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float second(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ uint64_t add_two(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul_two(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // e^(x + nm) of a packed pair of logits: the subtraction, the scaling by log2(e) and the exponential of __expf
 __device__ __forceinline__ uint64_t exp_two(uint32_t bf16_pair, uint64_t nm) {
-  const uint64_t x = two(__uint_as_float(bf16_pair << 16), __uint_as_float(bf16_pair & 0xffff0000u));
-  const uint64_t y = mul_two(add_two(x, nm), two(1.4426950408889634f, 1.4426950408889634f));
-  return two(ex2_approx(first(y)), ex2_approx(second(y)));
+  const uint64_t x = pk2f(__uint_as_float(bf16_pair << 16), __uint_as_float(bf16_pair & 0xffff0000u));
+  const uint64_t y = f2_mul(f2_add(x, nm), pk2f(1.4426950408889634f, 1.4426950408889634f));
+  return pk2f(ex2_approx(lo2(y)), ex2_approx(hi2(y)));
 }
 __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {     // a NaN leaves the other operand
   const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
@@ -88,7 +65,7 @@ xent_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targets, 
   __syncthreads();
   auto load = [&](long long row) {
     mbar_expect_tx(&full, row_bytes);
-    bulk_load_row(rowbuf, logits + row * ld, row_bytes, &full);
+    bulk_load_1d(rowbuf, logits + row * ld, row_bytes, &full);
   };
   if (threadIdx.x == 0 && blockIdx.x < T) load(blockIdx.x);
   uint4* xs = reinterpret_cast<uint4*>(rowbuf);
@@ -116,18 +93,18 @@ xent_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targets, 
     const float2 m2 = unpack_bf16x2(mp);
     float m = fmaxf(m2.x, m2.y);
     const float m0 = m == -INFINITY ? 0.f : -m;
-    const uint64_t nm0 = two(m0, m0);
+    const uint64_t nm0 = pk2f(m0, m0);
     uint64_t sa = 0, sb = 0;
 #pragma unroll 2
     for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
       const uint4 u = xs[v];
-      sa = add_two(sa, exp_two(u.x, nm0));
-      sb = add_two(sb, exp_two(u.y, nm0));
-      sa = add_two(sa, exp_two(u.z, nm0));
-      sb = add_two(sb, exp_two(u.w, nm0));
+      sa = f2_add(sa, exp_two(u.x, nm0));
+      sb = f2_add(sb, exp_two(u.y, nm0));
+      sa = f2_add(sa, exp_two(u.z, nm0));
+      sb = f2_add(sb, exp_two(u.w, nm0));
     }
-    sa = add_two(sa, sb);
-    float s = first(sa) + second(sa);
+    sa = f2_add(sa, sb);
+    float s = lo2(sa) + hi2(sa);
     warp_max_sum(m, s);
     if (lane == 0) {
       red[k & 1][0][warp] = m;
@@ -148,7 +125,7 @@ xent_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targets, 
       const float inv = ignored ? 0.f : grad_scale / s;
       uint4* dr = reinterpret_cast<uint4*>(dlogits + row * ld);
       const int tv = ignored ? -1 : (int)(tgt >> 3), tj = (int)(tgt & 7);
-      const uint64_t nm = two(-m, -m), inv2 = two(inv, inv);
+      const uint64_t nm = pk2f(-m, -m), inv2 = pk2f(inv, inv);
 #pragma unroll 2
       for (int v = threadIdx.x; v < nv; v += XENT_THREADS) {
         const uint4 u = xs[v];
@@ -156,8 +133,8 @@ xent_kernel(const __nv_bfloat16* logits, const long long* __restrict__ targets, 
         uint32_t o[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const uint64_t g = mul_two(exp_two(w[q], nm), inv2);
-          float g0 = first(g), g1 = second(g);
+          const uint64_t g = f2_mul(exp_two(w[q], nm), inv2);
+          float g0 = lo2(g), g1 = hi2(g);
           if (v == tv) {
             g0 -= 2 * q == tj ? grad_scale : 0.f;
             g1 -= 2 * q + 1 == tj ? grad_scale : 0.f;
