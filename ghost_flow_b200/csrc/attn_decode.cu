@@ -12,6 +12,10 @@
 // query heads as the 8 columns, so no half of an instruction is padding, and the heads of a lane's scores are those of
 // its output columns. K is read with ldmatrix, V with its transposing form, and P^T becomes the other operand with movmatrix.
 // (tcgen05 tiles would need 128 query rows.)
+// An operand has 8 bits and a probability 24, so P^T goes in as two bf16 numbers, the rounded value and what it left: the
+// error of a result is then its own rounding to bf16 (0.00165 .. 0.00168 of the norm for both head sizes, as with P in fp32; rounded
+// once, P makes it 0.0019 .. 0.0022). The second product costs nothing where memory bounds the kernel, 7 % at most where
+// 160 to 240 CTAs leave SMs half empty; a third changes no digit.
 // Measured, before -> now: 32 sequences of 1 .. 4096 keys, 32 / 8 heads of 128 77 -> 57 us (4.4 TB/s); 8 sequences of
 // 1501 keys, 32 / 32 heads of 128 58 -> 40 us; 64 of 2048 keys, 64 / 8 heads 156 -> 92 us (5.8 TB/s); 32 of 1 .. 4096 keys, 12 /
 // 12 heads of 64 295 -> 44 us (those went one key at a time).
@@ -27,6 +31,7 @@ constexpr int DEC_WARPS = 4;
 constexpr int DEC_MAX_G = 8;
 constexpr int DEC_KEYS = 16;     // keys of a block
 constexpr int DEC_STAGES = 3;
+constexpr int DEC_P_TERMS = 2;   // bf16 numbers that stand for a probability
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -153,14 +158,26 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, const __n
       p[2 + e] = ex2_approx(x1 - ref);
       l[e] = l[e] * corr[e] + p[e] + p[2 + e];
     }
-    const uint32_t b0 = transpose_8x8(pack_bf16x2(p[0], p[1])), b1 = transpose_8x8(pack_bf16x2(p[2], p[3]));
+    uint32_t pt[DEC_P_TERMS][2];
+#pragma unroll
+    for (int n = 0; n < DEC_P_TERMS; ++n) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t u = pack_bf16x2(p[2 * h], p[2 * h + 1]);
+        const float2 f = unpack_bf16x2(u);
+        p[2 * h] -= f.x;             // exact: what this term leaves
+        p[2 * h + 1] -= f.y;
+        pt[n][h] = transpose_8x8(u);
+      }
+    }
     // ---- O^T += V^T P^T
 #pragma unroll
     for (int j = 0; j < D / 16; ++j) {
       uint32_t a[4];
       ldmatrix_x4_trans(a, tv + ((lane & 7) + ((lane >> 4) << 3)) * Cfg::ROW + (16 * j + ((lane >> 3) & 1) * 8) * 2);
       o[j][0] *= corr[0]; o[j][1] *= corr[1]; o[j][2] *= corr[0]; o[j][3] *= corr[1];
-      mma_bf16_16816(o[j], a[0], a[1], a[2], a[3], b0, b1);
+#pragma unroll
+      for (int n = 0; n < DEC_P_TERMS; ++n) mma_bf16_16816(o[j], a[0], a[1], a[2], a[3], pt[n][0], pt[n][1]);
     }
     __syncwarp();                  // the stage is filled again two blocks on
   }
