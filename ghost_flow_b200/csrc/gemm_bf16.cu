@@ -919,7 +919,7 @@ static float* splitk_workspace(size_t floats) {
 namespace gf {
 // kernel for at most 16 rows (gemm_skinny.cu)
 bool gemm_skinny_wanted(const void* A, const void* W, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
-                        long long ldb, int accumulate);
+                        long long ldb, int accumulate, int split);
 int gemm_skinny_run(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                     int out_fp32, const void* bias, const void* residual, long long ldr, float alpha, int relu,
                     cudaStream_t st);
@@ -945,6 +945,28 @@ static void no_gather(gf::GemmParams& p) {
   p.conv_cpb = 0; p.conv_kw = 1; p.conv_pitch = 0; p.conv_pad = 0;
 }
 
+// Slices of K for a product with few output tiles and a long K (decode-sized M; weight gradients of narrow layers, [768, 2304]
+// over 8192 tokens): too few tiles to fill the machine, so K is split until there is about one work item per SM. 1: no split.
+static int splitk_slices(int M, int N, int K, int out_fp32, int accumulate, int act) {
+  if (K < 2048 || out_fp32 || accumulate || act != 0) return 1;
+  const int bn = N <= 128 ? 128 : 256;
+  const long long tiles = (long long)((M + gf::BM - 1) / gf::BM) * ((N + bn - 1) / bn);
+  const int sms = gf::sm_count();
+  if (tiles <= 0 || tiles * 2 > sms) return 1;
+  int split = (int)(sms / tiles);
+  if (split > K / 512) split = K / 512;
+  if (split > 16) split = 16;
+  return split;
+}
+
+// 1 when gf_gemm_bf16 (bf16 result, bn_hint and max_ctas 0) takes a workspace of M * N fp32 values, else 0. aligned: bases and
+// pitches of A and B are multiples of 16 bytes.
+GF_API int gf_gemm_bf16_splits(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate, int activation) {
+  const int split = splitk_slices(M, N, K, 0, accumulate, activation == 1 ? 1 : 0);
+  const long long pitch = aligned ? 8 : 1;
+  return split >= 2 && !gf::gemm_skinny_wanted(nullptr, nullptr, M, N, K, a_mn_major, pitch, b_mn_major, pitch, accumulate, split);
+}
+
 // lda/ldb: row pitch in elements of the matrix as stored.
 //   a_mn_major = 0: A stored [M, K] (K contiguous); 1: A stored [K, M] (M contiguous).
 //   b_mn_major = 0: B stored [N, K] (K contiguous); 1: B stored [K, N] (N contiguous).
@@ -958,42 +980,30 @@ GF_API int gf_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int
   no_gather(p);
   p.act = activation == 1 ? 1 : 0;   // epilogue activation after bias and residual: 0 none, 1 ReLU
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
+  const int split = bn_hint == 0 && max_ctas == 0 ? splitk_slices(M, N, K, out_fp32, accumulate, p.act) : 1;
   if (bn_hint == 0 && max_ctas == 0 &&
-      gf::gemm_skinny_wanted(A, B, M, N, K, a_mn_major, lda, b_mn_major, ldb, accumulate))
+      gf::gemm_skinny_wanted(A, B, M, N, K, a_mn_major, lda, b_mn_major, ldb, accumulate, split))
     return gf::gemm_skinny_run(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, bias, residual, ldr, alpha, p.act, st);
-  // Few output tiles and a long K (decode-sized M; weight gradients of narrow layers, [768, 2304] over 8192 tokens):
-  // too few tiles to fill the machine. Split K until there is about one work item per SM; the slices add into an
-  // fp32 workspace that a second kernel converts. The workspace is the caller's (splitk_ws, splitk_ws_floats >= M * N:
-  // a buffer that belongs to the calling stream, e.g. from a stream-ordered allocator) or, without one, a buffer
-  // this library keeps per device, which only one stream at a time may use.
-  const int bn_sk = N <= 128 ? 128 : 256;
-  const long long tiles_sk = (long long)((M + gf::BM - 1) / gf::BM) * ((N + bn_sk - 1) / bn_sk);
-  if (tiles_sk * 2 <= gf::sm_count() && !out_fp32 && !accumulate && K >= 2048 && bn_hint == 0 && max_ctas == 0 &&
-      p.act == 0) {
-    const int bn = bn_sk;
-    const long long tiles = tiles_sk;
-    const int sms = gf::sm_count();
-    int split = (int)(sms / (tiles > 0 ? tiles : 1));
-    if (split > K / 512) split = K / 512;
-    if (split > 16) split = 16;
-    if (split >= 2) {
-      float* ws = (splitk_ws && (long long)splitk_ws_floats >= (long long)M * N)
-                      ? reinterpret_cast<float*>(const_cast<int*>(splitk_ws))
-                      : gf::splitk_workspace((size_t)M * N);
-      if (ws) {
-        if (cudaMemsetAsync(ws, 0, sizeof(float) * (size_t)M * N, st) != cudaSuccess) return gf::GFH_CUDA;
-        p.split_k = split;
-        p.ws = ws;
-        int rc = gemm_core(A, B, C, M, N, K, a_mn_major, lda, b_mn_major, ldb, ldc, 0, 0, nullptr, nullptr, 0, alpha,
-                           status, bn, 0, p, st);
-        if (rc) return rc;
-        const long long n = (long long)M * N;
-        gf::splitk_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-            ws, reinterpret_cast<__nv_bfloat16*>(C), ldc, reinterpret_cast<const __nv_bfloat16*>(bias),
-            reinterpret_cast<const __nv_bfloat16*>(residual), ldr, M, N);
-        gf::note_extra_launches(1);
-        return cudaGetLastError() == cudaSuccess ? gf::GFH_OK : gf::GFH_CUDA;
-      }
+  // The slices add into an fp32 workspace that a second kernel converts. The workspace is the caller's (splitk_ws,
+  // splitk_ws_floats >= M * N: a buffer that belongs to the calling stream, e.g. from a stream-ordered allocator) or,
+  // without one, a buffer this library keeps per device, which only one stream at a time may use.
+  if (split >= 2) {
+    float* ws = (splitk_ws && (long long)splitk_ws_floats >= (long long)M * N)
+                    ? reinterpret_cast<float*>(const_cast<int*>(splitk_ws))
+                    : gf::splitk_workspace((size_t)M * N);
+    if (ws) {
+      if (cudaMemsetAsync(ws, 0, sizeof(float) * (size_t)M * N, st) != cudaSuccess) return gf::GFH_CUDA;
+      p.split_k = split;
+      p.ws = ws;
+      int rc = gemm_core(A, B, C, M, N, K, a_mn_major, lda, b_mn_major, ldb, ldc, 0, 0, nullptr, nullptr, 0, alpha,
+                         status, N <= 128 ? 128 : 256, 0, p, st);
+      if (rc) return rc;
+      const long long n = (long long)M * N;
+      gf::splitk_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+          ws, reinterpret_cast<__nv_bfloat16*>(C), ldc, reinterpret_cast<const __nv_bfloat16*>(bias),
+          reinterpret_cast<const __nv_bfloat16*>(residual), ldr, M, N);
+      gf::note_extra_launches(1);
+      return cudaGetLastError() == cudaSuccess ? gf::GFH_OK : gf::GFH_CUDA;
     }
   }
   // large plain products run on CTA pairs (256 x 256 tiles, half the operand bytes per SM and flop)

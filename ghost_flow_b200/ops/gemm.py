@@ -9,6 +9,8 @@ Reference counterparts: ``ghostflow-core/src/ops/matmul.rs:13-170`` (CPU blocked
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _lib
@@ -27,6 +29,12 @@ def _sm_count(device) -> int:
 
 def _is_dense_2d(t: torch.Tensor) -> bool:
     return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.size(1)
+
+
+@functools.lru_cache(maxsize=4096)
+def _splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu) -> bool:
+    """Whether the kernel library splits K for such a product: its rule, asked once for each combination of sizes."""
+    return bool(_lib.cuda_lib().gf_gemm_bf16_splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu))
 
 
 def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bfloat16, bias=None, residual=None,
@@ -56,12 +64,13 @@ def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bf
     # few output tiles and a long K: the kernel splits K and needs an fp32 [M, N] workspace. It comes from torch's
     # allocator, so it belongs to the current stream (and to the graph's pool while a CUDA graph is recorded).
     ws = None
-    if (K >= 2048 and (M > 16 or a_mn_major or b_mn_major or K % 8) and out.dtype is _BF16 and not accumulate and not relu and bn_hint == 0 and max_ctas == 0
-            and M * N < (1 << 31)
-            and 2 * ((M + 127) // 128) * ((N + (127 if N <= 128 else 255)) // (128 if N <= 128 else 256)) <= _sm_count(device)):
+    pa, pb = a.data_ptr(), b.data_ptr()
+    if K >= 2048 and not f32_out and bn_hint == 0 and max_ctas == 0 \
+            and _splits(M, N, K, bool(a_mn_major), bool(b_mn_major), not (pa | pb | 2 * sa[0] | 2 * sb[0]) & 15,
+                        bool(accumulate), bool(relu)):
         ws = torch.empty(M * N, dtype=torch.float32, device=device)
     rc = lib.gf_gemm_bf16(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K,
+        pa, pb, out.data_ptr(), M, N, K,
         1 if a_mn_major else 0, sa[0], 1 if b_mn_major else 0, sb[0], out.stride(0),
         1 if f32_out else 0, 1 if accumulate else 0,
         None if bias is None else bias.data_ptr(),
