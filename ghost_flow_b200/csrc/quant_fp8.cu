@@ -730,9 +730,16 @@ GF_API int gf_gemm_fp8(const void* A, const void* B, void* C, int M, int N, int 
   if (mode == 1 && (K & 127)) return GFH_BAD_ARG;
   // large products with row and column scales run on CTA pairs (gemm2sm_bf16.cu): half the operand bytes per SM and
   // instruction, where the single-CTA tiles ask shared memory for more than it delivers. The rule is that of the bf16 products
-  // (every pair has a tile of 256 x 256), but for at most 256 rows, which would leave half of a tile empty or one row of tiles.
-  // [4096, 4096] x [11008, 4096]^T 162 -> 145 us, 8192^3 466 -> 392 us, [2048, 4096] x [4096, 4096]^T 40 -> 35 us.
-  if (mode == 0 && M > 256 && gf::gemm2sm_wanted(M, N, K) && !(reinterpret_cast<uintptr_t>(sb) & 15))
+  // (every pair has a tile of 256 x 256), but for at most 256 rows, which would leave half of a tile empty or one row of tiles,
+  // and where the taller tiles leave the pairs more waves than the single CTAs have: a wave takes them 7/8 of the time.
+  // [4096, 4096] x [11008, 4096]^T 162 -> 145 us, 8192^3 466 -> 392 us, [2048, 4096] x [4096, 4096]^T 40 -> 35 us. Waves of single
+  // CTAs / pairs, us of each: [384, 4096] x [11008, 4096]^T 1 / 2, 23.7 / 29.5, [512, ...] 2 / 2, 35.6 / 29.9, [1040, 4096] x
+  // [4096, 4096]^T 1 / 2, 23.0 / 28.5, [640, 4096] x [22016, 4096]^T 3 / 4, 56.1 / 57.2, [784, ...] 5 / 5, 76 / 70.
+  const long long sms = gf::sm_count(), n_tiles = (N + 255) / 256;
+  const long long waves = ((M + 127) / 128 * n_tiles + sms - 1) / sms;
+  const long long pair_waves = ((M + 255) / 256 * n_tiles + sms / 2 - 1) / (sms / 2);
+  if (mode == 0 && M > 256 && gf::gemm2sm_wanted(M, N, K) && 7 * pair_waves <= 8 * waves &&
+      !(reinterpret_cast<uintptr_t>(sb) & 15))
     return gf::gemm2sm_run_fp8(A, B, C, M, N, K, lda, ldb, ldc, sa, sb, bias, status, (cudaStream_t)stream_v);
   const int bn = mode == 0 ? 256 : 128;
   CUtensorMap tmA, tmB;

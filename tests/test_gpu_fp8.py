@@ -142,7 +142,7 @@ def test_transposed_quantisation_equals_quantising_the_transpose(R, K):
 
 # 256 x 256 tiles for 74 pairs and one fewer, ragged in every dimension, K of one block and of a part of one
 @pytest.mark.parametrize("M,N,K", [(2048, 2368, 128), (2000, 2600, 528), (2560, 1800, 272), (2304, 2100, 1040), (256, 18944, 256),
-                                   (257, 9500, 256)])
+                                   (257, 9500, 256), (384, 11000, 272), (400, 11008, 272), (700, 22000, 256)])
 @pytest.mark.parametrize("with_bias", [True, False])
 def test_large_products_with_row_and_column_scales(M, N, K, with_bias, kernel_status):
     from ghost_flow_b200.ops import fp8
