@@ -1,14 +1,15 @@
 // RMSNorm and LayerNorm, forward and backward, bf16 in/out with fp32 arithmetic.
 //
 // Bound by memory: every tensor is read once and written once, as 16-byte vectors that stay packed in registers between
-// the passes over a row. Rows up to 1024 columns belong to one warp (sums are shuffles, eight rows to a CTA), longer ones
-// to one CTA of 256 threads with one barrier per reduction. The weight / bias gradients are cross-row sums: every CTA of a
+// the passes over a row. Rows up to 1024 columns belong to one warp (sums are shuffles, eight rows to a CTA) if there are
+// enough of them, all others to one CTA of 256 threads with one barrier per reduction. The weight / bias gradients are cross-row sums: every CTA of a
 // grid that fits the machine at once keeps them in registers over its rows, with the next row's loads in flight
 // behind the reduction of the current one, and writes one partial row to a scratch buffer; a second small kernel folds
 // the partial rows.
 //
 // Measured, before -> now: RMSNorm with residual of [8192, 4096] forward 58 -> 40 us, backward 70 -> 56 us (fold included);
-// LayerNorm of [8192, 768] forward 12.4 -> 7.6 us, backward 47 -> 16 us; four column sums of a GPT-2 block 56 -> 36 us. The
+// LayerNorm of [8192, 768] forward 12.4 -> 7.6 us, backward 47 -> 16 us, of [8192, 8192] (one CTA to an SM, no prefetch) backward
+// 264 -> 137 us, of [16, 8192] 15.8 -> 8.9 us; four column sums of a GPT-2 block 56 -> 36 us. The
 // forward pass read h back from memory right after storing it (to normalise what was stored); the backward pass had
 // 592 CTAs on 444 places, two barriers a row and, for short rows, eight warps adding into shared memory with atomics.
 //
@@ -393,9 +394,14 @@ static void launch_fold(const float* p0, void* o0, const float* p1, void* o1, in
       p0, (__nv_bfloat16*)o0, p1, (__nv_bfloat16*)o1, nparts, D, accumulate);
 }
 
+// A row to a warp, eight rows to a CTA, for rows that are short or many. Few rows of 264 columns and more (up to five for an SM
+// forward, one backward) leave SMs idle that way and take a CTA each. RMSNorm with residual, us as CTAs / as warps: forward [16, 1024] 2.1 / 3.1, [600, 1024] 2.7 / 3.5, [600, 264]
+// 2.6 / 2.6, [1200, 768] 3.6 / 3.1; backward [16, 1024] 4.2 / 6.1, [128, 264] 4.4 / 4.8, [300, 384] 5.6 / 5.1, [600, 1024] 7.3 / 6.9.
+static inline bool norm_row_per_warp(int T, int D, int few) { return D <= NORM_WARP_D && !(D > 256 && T <= few); }
+
 template <bool LN>
 static int launch_norm_fwd(const NormFwd& p, cudaStream_t st) {
-  if (p.D <= NORM_WARP_D) {   // one warp per row
+  if (norm_row_per_warp(p.T, p.D, sm_count() * 5)) {
     const int vpl = (p.D / 8 + 31) / 32, grid = (p.T + NORM_WARPS - 1) / NORM_WARPS;
     auto kern = vpl == 1 ? norm_fwd_warp_kernel<LN, 1> : vpl == 2 ? norm_fwd_warp_kernel<LN, 2>
                 : vpl == 3 ? norm_fwd_warp_kernel<LN, 3> : norm_fwd_warp_kernel<LN, 4>;
@@ -414,7 +420,7 @@ template <bool LN>
 static int launch_norm_bwd(const NormBwd& p, cudaStream_t st) {
   const int cap = norm_grid(p.T), sms = sm_count();
   int grid;
-  if (p.D <= NORM_WARP_D) {
+  if (norm_row_per_warp(p.T, p.D, sms)) {
     const int vpl = (p.D / 8 + 31) / 32;
     grid = at_most(at_most((p.T + NORM_WARPS - 1) / NORM_WARPS, cap), (long long)sms * (vpl == 1 ? 3 : 2));
     auto kern = vpl == 1 ? norm_bwd_warp_kernel<LN, 1> : vpl == 2 ? norm_bwd_warp_kernel<LN, 2>

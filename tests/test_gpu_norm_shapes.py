@@ -7,7 +7,9 @@ pytestmark = pytest.mark.gpu
 
 # row lengths around one warp's and one CTA's steps; row counts below, at and beyond a grid of rows
 SHAPES = [(1, 8), (3, 256), (9, 264), (17, 768), (8, 1016), (5, 1024), (5, 1032), (700, 2048), (3, 2056), (1500, 4096),
-          (2, 4104), (601, 8192), (5000, 128)]
+          (2, 4104), (601, 8192), (5000, 128),
+          # rows of 264 to 1024 columns: one to a CTA while there are few of them (740 forward, 148 backward), else one to a warp
+          (148, 264), (149, 264), (740, 768), (741, 768), (900, 1016), (1400, 1024)]
 
 
 def _rel(a, b):
