@@ -191,6 +191,9 @@ def rope_ref(x, cos, sin, interleaved=False, pos_offset=0):
 
 def check_rope_tables(device, S: int, D: int, cos, sin, pos_offset: int) -> None:
     """Raises where the kernels, which index the tables by position without a bound, would read outside of them."""
+    c = cos.shape
+    if c == sin.shape and len(c) == 2 and 2 * c[1] == D and 0 <= pos_offset <= c[0] - S and cos.device == sin.device == device:
+        return
     if not (cos.device == sin.device == device and cos.dim() == sin.dim() == 2 and cos.shape[1] == sin.shape[1] == D // 2):
         raise ValueError(f"rope tables must be [positions, {D // 2}] on {device}, got {list(cos.shape)} on {cos.device} "
                          f"and {list(sin.shape)} on {sin.device}")
@@ -257,21 +260,22 @@ def _packed_rows(t):
     return t, ld
 
 
-def _rope_qkv_launch(q, k, v, qd, kd, vd, cos, sin, interleaved, pos_offset, backward):
-    """Rotates ``q, k [B, S, *, D]`` into ``qd, kd`` and copies ``v`` into ``vd`` (``None``: left alone). Destinations are
-    ``[B, S, *, D]`` views with packed heads and free row and sequence pitch."""
-    B, S, H, D = q.shape
-    q, ldq = _packed_rows(q)
-    k, ldk = _packed_rows(k)
-    ldv = 0
-    if vd is not None:
-        v, ldv = _packed_rows(v)
-    table = (ctypes.c_longlong * 9)(ldq, ldk, ldv, qd.stride(1), qd.stride(0), kd.stride(1), kd.stride(0),
-                                    vd.stride(1) if vd is not None else 0, vd.stride(0) if vd is not None else 0)
-    _rc(_lib.cuda_lib().gf_rope_qkv(q.data_ptr(), k.data_ptr(), v.data_ptr() if vd is not None else None, qd.data_ptr(),
-                                    kd.data_ptr(), vd.data_ptr() if vd is not None else None, table, cos.data_ptr(),
-                                    sin.data_ptr(), B * S, S, H, k.shape[2], D, pos_offset, 1 if interleaved else 0,
+def _rope_qkv_launch(src, dst, B, S, H, Hk, D, cos, sin, interleaved, pos_offset, backward):
+    """Rotates q and k and copies v. ``src``: (address, row pitch) of each, heads packed; ``dst``: (address, row pitch,
+    sequence pitch) of each, v's ``None`` to leave it alone."""
+    (q, ldq), (k, ldk), (v, ldv) = src
+    qd, kd, vd = dst
+    table = (ctypes.c_longlong * 9)(ldq, ldk, ldv, qd[1], qd[2], kd[1], kd[2], *((0, 0) if vd is None else vd[1:]))
+    _rc(_lib.cuda_lib().gf_rope_qkv(q, k, v, qd[0], kd[0], None if vd is None else vd[0], table, cos.data_ptr(),
+                                    sin.data_ptr(), B * S, S, H, Hk, D, pos_offset, 1 if interleaved else 0,
                                     1 if backward else 0, _lib.stream_ptr()), "gf_rope_qkv")
+
+
+def _packed_qkv(qkv, H: int, Hk: int):
+    """q, k and v of a packed projection as sources of :func:`_rope_qkv_launch`, and the tensor they point into."""
+    t, ld = _packed_rows(qkv)
+    p, head = t.data_ptr(), 2 * t.shape[3]
+    return t, ((p, ld), (p + H * head, ld), (p + (H + Hk) * head, ld))
 
 
 class _RopeQKVFn(torch.autograd.Function):
@@ -284,7 +288,9 @@ class _RopeQKVFn(torch.autograd.Function):
         q = torch.empty((B, S, H, D), dtype=qkv.dtype, device=qkv.device)
         k = torch.empty((B, S, Hk, D), dtype=qkv.dtype, device=qkv.device)
         v = qkv[:, :, H + Hk:]
-        _rope_qkv_launch(qkv[:, :, :H], qkv[:, :, H:H + Hk], None, q, k, None, cos, sin, interleaved, pos_offset, False)
+        t, src = _packed_qkv(qkv, H, Hk)
+        _rope_qkv_launch(src, ((q.data_ptr(), H * D, S * H * D), (k.data_ptr(), Hk * D, S * Hk * D), None), B, S, H, Hk, D,
+                         cos, sin, interleaved, pos_offset, False)
         ctx.save_for_backward(cos, sin)
         ctx.args = (H, Hk, interleaved, pos_offset)
         return q, k, v
@@ -294,9 +300,13 @@ class _RopeQKVFn(torch.autograd.Function):
         cos, sin = ctx.saved_tensors
         H, Hk, interleaved, pos_offset = ctx.args
         B, S, _, D = dq.shape
-        g = torch.empty((B, S, H + 2 * Hk, D), dtype=dq.dtype, device=dq.device)
-        _rope_qkv_launch(dq, dk, dv, g[:, :, :H], g[:, :, H:H + Hk], g[:, :, H + Hk:], cos, sin, interleaved, pos_offset,
-                         True)
+        G = H + 2 * Hk
+        g = torch.empty((B, S, G, D), dtype=dq.dtype, device=dq.device)
+        p = g.data_ptr()
+        packed = [_packed_rows(t) for t in (dq, dk, dv)]
+        _rope_qkv_launch([(t.data_ptr(), ld) for t, ld in packed],
+                         [(p + 2 * h * D, G * D, S * G * D) for h in (0, H, H + Hk)], B, S, H, Hk, D, cos, sin, interleaved,
+                         pos_offset, True)
         return g, None, None, None, None, None, None
 
 
@@ -333,13 +343,22 @@ def _rows_apart(row: int, dims) -> bool:
 def _cache_rows_apart(kc, vc) -> bool:
     """Whether no two rows of the caches ``[B, n, Hk, D]`` (packed heads) share memory: expanded caches are refused by the
     assignments, and two that overlap are written by them one after the other."""
-    row = kc.shape[2] * kc.shape[3]
-    dims = [[(c.stride(i), c.shape[i]) for i in (0, 1)] for c in (kc, vc)]
-    a, b = (c.data_ptr() // c.element_size() for c in (kc, vc))
-    if dims[0] == dims[1]:               # the caches themselves are one more dimension, wherever it lies
-        return _rows_apart(row, [*dims[0], (abs(b - a), 2)])
-    ends = sorted((p, p + row + sum(st * (n - 1) for st, n in d)) for p, d in zip((a, b), dims))
+    (B, n, Hk, D), sk, sv = kc.shape, kc.stride(), vc.stride()
+    row, between = Hk * D, abs(kc.data_ptr() - vc.data_ptr()) // kc.element_size()
+    if sk == sv and sk[1] == row and sk[0] == n * row:        # two dense caches
+        return between >= B * sk[0]
+    dims = [(sk[0], B), (sk[1], n)], [(sv[0], B), (sv[1], n)]
+    if sk[:2] == sv[:2]:                 # the caches themselves are one more dimension, wherever it lies
+        return _rows_apart(row, [*dims[0], (between, 2)])
+    ends = sorted((c.data_ptr(), c.data_ptr() + c.element_size() * (row + sum(st * (n - 1) for st, n in d)))
+                  for c, d in zip((kc, vc), dims))
     return all(_rows_apart(row, d) for d in dims) and ends[0][1] <= ends[1][0]
+
+
+def _cache_fits_kernel(c, shape, device, dtype) -> bool:
+    s = c.stride()
+    return (c.shape == shape and s[3] == 1 and s[2] == shape[3] and not (s[0] | s[1]) & 7 and not c.data_ptr() & 15
+            and c.dtype is dtype and c.device == device)
 
 
 def rope_qkv_to_cache(qkv, num_heads: int, num_kv_heads: int, cos, sin, kcache, vcache, interleaved: bool = False,
@@ -347,15 +366,16 @@ def rope_qkv_to_cache(qkv, num_heads: int, num_kv_heads: int, cos, sin, kcache, 
     """Rotated q of a packed projection output; rotated k and v go to rows ``pos_offset ..`` of the caches
     ``[B, max_len, Hk, D]``. Inference only: nothing is recorded for autograd."""
     B, S, _, D = qkv.shape
-    H, Hk = num_heads, num_kv_heads
+    H, Hk, n, dtype, device = num_heads, num_kv_heads, kcache.shape[1], qkv.dtype, qkv.device
+    shape = (B, n, Hk, D)
     # what follows the assignments below (dispatch modes, transforms) would not see the kernel's writes
-    if not torch.is_grad_enabled() and not _observed() and _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset) and pos_offset + S <= kcache.shape[1] \
-            and all(c.is_cuda and c.device == qkv.device and c.dtype == qkv.dtype and c.shape == (B, kcache.shape[1], Hk, D)
-                    and c.stride(3) == 1 and c.stride(2) == D and c.stride(1) % 8 == 0 and c.stride(0) % 8 == 0
-                    and c.data_ptr() % 16 == 0 for c in (kcache, vcache)) and _cache_rows_apart(kcache, vcache):
-        q = torch.empty((B, S, H, D), dtype=qkv.dtype, device=qkv.device)
-        _rope_qkv_launch(qkv[:, :, :H], qkv[:, :, H:H + Hk], qkv[:, :, H + Hk:], q, kcache[:, pos_offset:pos_offset + S],
-                         vcache[:, pos_offset:pos_offset + S], cos, sin, interleaved, pos_offset, False)
+    if not torch.is_grad_enabled() and not _observed() and _rope_qkv_ok(qkv, H, Hk, cos, sin, pos_offset) \
+            and pos_offset + S <= n and _cache_fits_kernel(kcache, shape, device, dtype) \
+            and _cache_fits_kernel(vcache, shape, device, dtype) and _cache_rows_apart(kcache, vcache):
+        q = torch.empty((B, S, H, D), dtype=dtype, device=device)
+        t, src = _packed_qkv(qkv, H, Hk)
+        at = [(c.data_ptr() + 2 * pos_offset * s1, s1, s0) for c in (kcache, vcache) for s0, s1, _, _ in (c.stride(),)]
+        _rope_qkv_launch(src, ((q.data_ptr(), H * D, S * H * D), *at), B, S, H, Hk, D, cos, sin, interleaved, pos_offset, False)
         torch.autograd.graph.increment_version((kcache, vcache))     # a graph that saved a cache has to notice the write
         return q
     q, k, v = rope_qkv(qkv, H, Hk, cos, sin, interleaved, pos_offset)
