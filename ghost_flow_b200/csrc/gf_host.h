@@ -18,6 +18,7 @@ enum HostErr : int {
   GFH_CUDA = -2,
   GFH_TMAP = -3,
   GFH_TOO_LARGE = -4,
+  GFH_OVERLAP = -5,     // memory of the arguments overlaps: nothing was launched
 };
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

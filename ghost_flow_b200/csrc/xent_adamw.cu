@@ -9,6 +9,9 @@
 #include "gf_host.h"
 #include "gf_ptx.cuh"
 
+#include <algorithm>
+#include <new>
+
 namespace gf {
 
 // One CTA of 256 threads per row, as many on an SM as have room for their row in shared memory, each walking its rows: a bulk
@@ -412,9 +415,45 @@ GF_API int gf_adam_flat_dev(float* p, float* m, float* v, const void* g, void* p
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
 }
 
+// Whether a launch over this table would write memory that it also reads or writes elsewhere: weights over one storage (the
+// caller's copy back has an order, the launch has none), a gradient over a weight or over the flat buffers. Host only.
+static bool adam_table_overlaps(const float* p, const float* m, const float* v, const long long* table, int count) {
+  struct Span {
+    unsigned long long lo, hi;
+    bool written;
+  };
+  Span* s = new (std::nothrow) Span[2 * (size_t)count + 3];
+  if (!s) return true;
+  size_t k = 0;
+  long long all = 0;
+  for (int i = 0; i < count; ++i) {
+    const long long *r = table + 5 * i, n = r[3];
+    if (n <= 0) continue;
+    if (r[0]) all = all < r[2] + n ? r[2] + n : all;
+    if (r[1]) s[k++] = {(unsigned long long)r[1], (unsigned long long)(r[1] + n * (r[0] ? 2 : r[4])), true};
+    if (r[0]) s[k++] = {(unsigned long long)r[0], (unsigned long long)(r[0] + n * (r[4] ? 2 : 4)), false};
+  }
+  for (const float* f : {p, m, v})
+    if (all) s[k++] = {(unsigned long long)f, (unsigned long long)(f + all), true};
+  std::sort(s, s + k, [](const Span& a, const Span& b) { return a.lo < b.lo; });
+  unsigned long long end = 0, end_written = 0;
+  bool hit = false;
+  for (size_t i = 0; i < k && !hit; ++i) {
+    hit = s[i].lo < (s[i].written ? end : end_written);
+    if (s[i].hi > end) end = s[i].hi;
+    if (s[i].written && s[i].hi > end_written) end_written = s[i].hi;
+  }
+  delete[] s;
+  return hit;
+}
+GF_API int gf_adam_table_overlaps(const float* p, const float* m, const float* v, const long long* table, int count) {
+  return count > 0 && table && adam_table_overlaps(p, m, v, table, count) ? 1 : 0;
+}
+
 // Adam / AdamW over `count` tensors. p / m / v: fp32 flat buffers; table (host memory, read before the call returns):
 // five values per tensor {gradient pointer, bf16 weight pointer or 0, first element in the flat buffers (a multiple of
-// four), number of elements, 1 when the gradient is bf16 and 0 when it is fp32}.
+// four), number of elements, 1 when the gradient is bf16 and 0 when it is fp32}. A row without a gradient stands for a weight
+// that the caller writes itself, fifth value its bytes per element. GFH_OVERLAP, and nothing launched, when adam_table_overlaps.
 GF_API int gf_adam_multi(float* p, float* m, float* v, const long long* table, int count, float lr, float beta1,
                          float beta2, float eps, float wd, int step, float grad_scale, int decoupled, void* stream) {
   gf::enter();
@@ -427,13 +466,14 @@ GF_API int gf_adam_multi(float* p, float* m, float* v, const long long* table, i
   a.bc2 = 1.f - powf(beta2, (float)step);
   a.decoupled = decoupled;
   for (int i = 0; i < count; ++i)
-    if (!table[5 * i] || table[5 * i + 2] < 0 || (table[5 * i + 2] & 3) || table[5 * i + 3] < 0) return GFH_BAD_ARG;
+    if (table[5 * i + 2] < 0 || (table[5 * i + 2] & 3) || table[5 * i + 3] < 0) return GFH_BAD_ARG;
+  if (count && adam_table_overlaps(p, m, v, table, count)) return GFH_OVERLAP;
   AdamTable t;
   t.count = 0;
   long long ctas = 0;
   int launches = 0;
   for (int i = 0; i <= count; ++i) {
-    const long long n = i < count ? table[5 * i + 3] : 0;
+    const long long n = i < count && table[5 * i] ? table[5 * i + 3] : 0;
     const long long need = (n + ADAM_MULTI_CHUNK - 1) / ADAM_MULTI_CHUNK;
     if (need > 0x7fffffffLL) return GFH_TOO_LARGE;
     if (t.count && (i == count || t.count == ADAM_MULTI_TENSORS || ctas + need > 0x7fffffffLL)) {

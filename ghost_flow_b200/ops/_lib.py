@@ -51,6 +51,7 @@ _SIGS = {
     "gf_xent_fused": [P, P, P, P, I, I, L, F, L, P, P],
     "gf_adam_flat": [P, P, P, P, P, L, F, F, F, F, F, I, F, I, I, P, P],
     "gf_adam_flat_dev": [P, P, P, P, P, L, F, F, F, F, F, I, F, I, I, P, P, P],
+    "gf_adam_table_overlaps": [P, P, P, P, I],
     "gf_adam_multi": [P, P, P, P, I, F, F, F, F, F, I, F, I, P],
     "gf_counter_add": [P, I, P],
     "gf_colsum_bf16": [P, L, P, P, I, I, I, P],

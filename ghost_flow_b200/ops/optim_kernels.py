@@ -36,20 +36,33 @@ def adam_flat(p, m, v, g, p_lp=None, *, lr, beta1=0.9, beta2=0.999, eps=1e-8, we
     _lib.check_rc(rc, "gf_adam_flat")
 
 
-def adam_multi(p, m, v, tensors, *, lr, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0, step=1, grad_scale=1.0,
-               decoupled=True):
-    """Adam / AdamW over many tensors whose fp32 master weights and moments lie in the flat buffers ``p, m, v``.
-    ``tensors``: ``(gradient, bf16 weight or None, first element in the flat buffers)`` per tensor; gradients are
-    contiguous, bf16 or fp32, and read in place; the bf16 weight gets the rounded result."""
-    assert p.is_cuda and p.dtype == torch.float32 and p.is_contiguous()
+def adam_table(tensors, beside=()):
+    """The table of :func:`adam_multi` and its number of rows."""
     rows = []
     for g, w, off in tensors:
-        rows += (g.data_ptr(), w.data_ptr() if w is not None else 0, off, g.numel(), _gd(g))
+        rows += (g.data_ptr(), 0 if w is None else w.data_ptr(), off, g.numel(), _gd(g))
+    for w in beside:
+        rows += (0, w.data_ptr(), 0, w.numel(), w.element_size())
+    return (ctypes.c_longlong * len(rows))(*rows), len(rows) // 5
+
+
+def adam_multi(p, m, v, tensors, beside=(), *, lr, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0, step=1, grad_scale=1.0,
+               decoupled=True) -> bool:
+    """Adam / AdamW over many tensors whose fp32 master weights and moments lie in the flat buffers ``p, m, v``.
+    ``tensors``: ``(gradient, bf16 weight or None, first element in the flat buffers)`` per tensor; gradients are
+    contiguous, bf16 or fp32, and read in place; the bf16 weight gets the rounded result. ``beside``: contiguous weights
+    that the caller writes itself. ``False``, and nothing done, when a weight lies over another one or under a gradient, or
+    a gradient over the flat buffers."""
+    assert p.is_cuda and p.dtype == torch.float32 and p.is_contiguous()
+    table, rows = adam_table(tensors, beside)
     rc = _lib.cuda_lib().gf_adam_multi(
-        p.data_ptr(), m.data_ptr(), v.data_ptr(), (ctypes.c_longlong * len(rows))(*rows), len(tensors), float(lr),
+        p.data_ptr(), m.data_ptr(), v.data_ptr(), table, rows, float(lr),
         float(beta1), float(beta2), float(eps), float(weight_decay), int(step), float(grad_scale),
         1 if decoupled else 0, _lib.stream_ptr())
+    if rc == -5:
+        return False
     _lib.check_rc(rc, "gf_adam_multi")
+    return True
 
 
 def sgd_flat(p, buf, g, p_lp=None, *, lr, momentum=0.0, dampening=0.0, weight_decay=0.0, nesterov=False,

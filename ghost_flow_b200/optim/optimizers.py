@@ -31,6 +31,9 @@ class ParamGroup(dict):
     """``{params, lr, weight_decay, ...}`` (ghostflow-optim/src/optimizer.rs:24-43)."""
 
 
+_IN_PLACE_GRADS = (torch.bfloat16, torch.float32)
+
+
 class Optimizer:
     """Base class: ``step, zero_grad, get_lr, set_lr, parameters`` (ghostflow-optim/src/optimizer.rs:6-21)."""
 
@@ -140,41 +143,26 @@ class Optimizer:
     @staticmethod
     def _tensors_in_place(f):
         """``(gradient, bf16 weight or None, offset)`` of every parameter with a gradient, for a kernel that reads and
-        writes them where they lie; ``None`` when one of them has a layout, type or device that needs the flat copy, or
-        when the kernel would write what it reads or writes elsewhere."""
+        writes them where they lie, and the other parameters that have a master copy; ``None`` when one of them has a
+        layout, type or device that needs the flat copy."""
         if f["repeats"]:
             return None
-        m = f["master"]
-        out, dev = [], m.device
-        spans = [(m.data_ptr(), m.data_ptr() + 4 * m.numel(), True)]        # first and last byte; is it written?
+        out, beside, dev = [], [], f["master"].get_device()
         for p, o, view in zip(f["params"], f["offs"], f["is_view"]):
             g = p.grad
-            if not view and p.numel() > 0:
-                if not p.is_contiguous():
-                    return None
-                a = p.data_ptr()
-                spans.append((a, a + p.numel() * p.element_size(), True))
+            if not view and not p.is_contiguous():
+                return None
             if g is None or g.numel() == 0:
+                if not view:
+                    beside.append(p)
                 continue
-            if g.dtype not in (torch.bfloat16, torch.float32) or g.device != dev or g.layout != torch.strided \
+            if g.dtype not in _IN_PLACE_GRADS or g.get_device() != dev or g.layout != torch.strided \
                     or not g.is_contiguous() or g.is_neg() or type(g) not in (torch.Tensor, torch.nn.Parameter):
                 return None
-            if not view and (p.dtype != torch.bfloat16 or p.device != dev):
+            if not view and (p.dtype != torch.bfloat16 or p.get_device() != dev):
                 return None
-            a = g.data_ptr()
-            spans.append((a, a + g.numel() * g.element_size(), False))
             out.append((g, None if view else p, o))
-        # parameters over one storage are copied back one after the other, and a gradient that lies over a weight or the
-        # master copy is read before anything is written: one launch gives neither order
-        spans.sort()
-        end = end_written = 0
-        for a, b, written in spans:
-            if a < (end if written else end_written):
-                return None
-            end = max(end, b)
-            if written:
-                end_written = max(end_written, b)
-        return out
+        return out, beside
 
     @staticmethod
     def _scatter_params(f, only_without_grad=False):
@@ -288,15 +276,16 @@ class Adam(Optimizer):
                 from ..ops.optim_kernels import adam_flat, adam_multi
 
                 self._sync_master(f)
-                tensors = self._tensors_in_place(f)
+                in_place = self._tensors_in_place(f)
                 hyper = dict(lr=g["lr"], beta1=b1, beta2=b2, eps=g["eps"], weight_decay=g["weight_decay"], step=t,
                              decoupled=self.decoupled)
-                if tensors is not None:
+                done = False
+                if in_place is not None:
                     with torch.cuda.device(f["master"].device):
-                        if tensors:
-                            adam_multi(f["master"], *f["state"], tensors, **hyper)
-                    # the others show their master copy all the same: it may have been loaded since
-                    self._scatter_params(f, only_without_grad=True)
+                        done = not in_place[0] or adam_multi(f["master"], *f["state"], *in_place, **hyper)
+                if done:
+                    if in_place[1]:     # the others show their master copy all the same: it may have been loaded since
+                        self._scatter_params(f, only_without_grad=True)
                 else:
                     grads, runs = self._gather_grads(f)
                     with torch.cuda.device(f["master"].device):
