@@ -29,7 +29,7 @@ constexpr int XENT_THREADS = 256;
 constexpr int XENT_CTAS = 6;
 constexpr size_t XENT_SMEM = 220 * 1024;    // of an SM, for rows
 
-// e^(x + nm) of a packed pair of logits: the subtraction, the scaling by log2(e) and the exponential of __expf
+// e^(x + nm) of a packed pair of logits, as 2^((x + nm) log2 e) on the ex2 instruction
 __device__ __forceinline__ uint64_t exp_two(uint32_t bf16_pair, uint64_t nm) {
   const uint64_t x = pk2f(__uint_as_float(bf16_pair << 16), __uint_as_float(bf16_pair & 0xffff0000u));
   const uint64_t y = f2_mul(f2_add(x, nm), pk2f(1.4426950408889634f, 1.4426950408889634f));
