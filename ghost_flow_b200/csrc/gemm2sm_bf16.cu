@@ -49,8 +49,10 @@ constexpr int G2_BM = 128;        // rows of A per CTA
 constexpr int G2_BK = 64;
 // TMA warp, MMA warp, 8 epilogue warps: two for each quarter of the TMEM lanes, one per half of the tile's columns. With a
 // short K the epilogue outlasts the products of the next tile (K = 768: 6100 cycles): four warps took longer than that.
-// 8192 x 3072 x 768 with bias 71 -> 56 us, 8192 x 768 x 768 with bias and residual 36 -> 28 us.
-constexpr int G2_THREADS = 320;
+// 8192 x 3072 x 768 with bias 71 -> 56 us, 8192 x 768 x 768 with bias and residual 36 -> 28 us, a weight gradient of 11008 x 4096
+// over 256 rows added to what is there 120 -> 99 us. A product with nothing to add or scale has four: eight take its short loops
+// longer (4096 x 2048 x 256 21.1 -> 23.1 us, 11008 x 4096 over 256 rows 54 -> 57 us) and its long ones no less.
+constexpr int g2_threads(int epilogue_warps) { return 64 + 32 * epilogue_warps; }
 constexpr int G2_A_BYTES = G2_BM * G2_BK * 2;
 
 // BNH = rows of B (output columns) per CTA: 128 (256 x 256 tiles, seven stages) or 64 (256 x 128 tiles, nine
@@ -145,8 +147,9 @@ __device__ __forceinline__ void g2_tile_coords(const Gemm2Params& p, int tile, i
 
 // F8: e4m3 operands (both K-major). A k block is 128 bytes of every row either way, 64 bf16 or 128 e4m3 values, and so are
 // its four instructions (16 or 32 values deep): only counts, instruction and epilogue differ.
-template <int BNH, bool A_MN, bool B_MN, bool F8>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
+// EPI: epilogue warps, 4 or 8.
+template <int BNH, bool A_MN, bool B_MN, bool F8, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2_threads(EPI), 1)
 gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const Gemm2Params p) {
   using Cfg = G2Cfg<BNH>;
@@ -179,7 +182,7 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 16);    // eight epilogue warps of each CTA (used in the even CTA)
+      mbar_init(&tempty_bar[b], 2 * EPI);    // the epilogue warps of both CTAs (used in the even CTA)
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
@@ -291,9 +294,10 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..9 of both CTAs)
+    // ------------------------------------------------------------ epilogue (warps 2 .. 1 + EPI of both CTAs)
     const int lane_grp = warp & 3;  // TMEM lanes [32*lane_grp, +32) belong to this warp
-    const int half = (warp - 2) >> 2;  // and this half of the columns
+    constexpr int CHUNKS = G2_BN / 8 / EPI;             // of 32 columns: all of the tile's with four warps, a half with eight
+    const int part = EPI > 4 ? (warp - 2) >> 2 : 0;     // and this part of the columns
     const bool bias_wide = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
     const bool res_wide = (p.ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0;
     int it = 0;
@@ -313,7 +317,7 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * G2_BN + ((uint32_t)(lane_grp * 32) << 16);
 #pragma unroll 1
-      for (int c = half * (G2_BN / 64); c < (half + 1) * (G2_BN / 64); ++c) {
+      for (int c = part * CHUNKS; c < (part + 1) * CHUNKS; ++c) {
         const int col0 = n0 + c * 32;
         const bool full = (col0 + 32 <= p.N);
         const __nv_bfloat16* rp = p.residual + (long long)row * p.ldr + col0;
@@ -445,21 +449,21 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
 }
 
-template <int BNH, bool A_MN, bool B_MN, bool F8 = false>
-static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, cudaStream_t stream) {
+template <int BNH, bool A_MN, bool B_MN, bool F8, int EPI>
+static int launch_gemm2_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, cudaStream_t stream) {
   using Cfg = G2Cfg<BNH>;
   constexpr int G2_SMEM_BYTES = Cfg::SMEM_BYTES;
   constexpr int G2_BN = Cfg::BN;
   static gf::DeviceOnce configured;
   static int max_pairs = 0;
-  auto kern = gemm2sm_bf16_kernel<BNH, A_MN, B_MN, F8>;
+  auto kern = gemm2sm_bf16_kernel<BNH, A_MN, B_MN, F8, EPI>;
   if (configured.todo()) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_BYTES) != cudaSuccess)
       return GFH_CUDA;
     // how many CTA pairs the device can hold at once (a GPC with an odd number of free SMs strands one)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count() & ~1);
-    cfg.blockDim = dim3(G2_THREADS);
+    cfg.blockDim = dim3(g2_threads(EPI));
     cfg.dynamicSmemBytes = G2_SMEM_BYTES;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -479,8 +483,15 @@ static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Par
   int pairs = max_pairs < tiles ? max_pairs : tiles;
   if (pairs < 1) pairs = 1;
   p.band = p.tiles_m > 8 ? 8 : p.tiles_m;
-  kern<<<2 * pairs, G2_THREADS, G2_SMEM_BYTES, stream>>>(tmA, tmB, p);
+  kern<<<2 * pairs, g2_threads(EPI), G2_SMEM_BYTES, stream>>>(tmA, tmB, p);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
+}
+
+template <int BNH, bool A_MN, bool B_MN, bool F8 = false>
+static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, cudaStream_t stream) {
+  if constexpr (!F8)
+    if (!p.bias && !p.residual && !p.accumulate) return launch_gemm2_epi<BNH, A_MN, B_MN, false, 4>(tmA, tmB, p, stream);
+  return launch_gemm2_epi<BNH, A_MN, B_MN, F8, 8>(tmA, tmB, p, stream);
 }
 
 // 1 when plain GEMMs of this shape should run on CTA pairs. GF_GEMM_2SM=0 turns the path off, =1 forces it for
