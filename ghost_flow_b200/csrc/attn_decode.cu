@@ -14,11 +14,12 @@
 // (tcgen05 tiles would need 128 query rows.)
 // An operand has 8 bits and a probability 24, so P^T goes in as two bf16 numbers, the rounded value and what it left: the
 // error of a result is then its own rounding to bf16 (0.00165 .. 0.00168 of the norm for both head sizes, as with P in fp32; rounded
-// once, P makes it 0.0019 .. 0.0022). The second product costs nothing where memory bounds the kernel, 7 % at most where
-// 160 to 240 CTAs leave SMs half empty; a third changes no digit.
-// Measured, before -> now: 32 sequences of 1 .. 4096 keys, 32 / 8 heads of 128 77 -> 57 us (4.4 TB/s); 8 sequences of
-// 1501 keys, 32 / 32 heads of 128 58 -> 40 us; 64 of 2048 keys, 64 / 8 heads 156 -> 92 us (5.8 TB/s); 32 of 1 .. 4096 keys, 12 /
-// 12 heads of 64 295 -> 44 us (those went one key at a time).
+// once, P makes it 0.0019 .. 0.0022). The second product costs 2 % where memory bounds the kernel (32 sequences of 1 .. 4096 keys,
+// 32 / 8 heads of 128: 60.7 -> 61.5 us; 64 of 2048 keys, 64 / 8 heads: 90.0 -> 92.1), 7 % where 160 to 240 CTAs leave SMs half
+// empty; a third changes no digit.
+// Measured, before -> now: 32 sequences of 1 .. 4096 keys, 32 / 8 heads of 128 77 -> 58 us (4.4 TB/s); 8 sequences of
+// 1501 keys, 32 / 32 heads of 128 58 -> 38 us; 64 of 2048 keys, 64 / 8 heads 156 -> 92 us (5.8 TB/s); 8 of 4000 keys, 40 / 40
+// heads 133 -> 115 us (5.7 TB/s); 32 of 1 .. 4096 keys, 12 / 12 heads of 64 295 -> 44 us (those went one key at a time).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
