@@ -152,7 +152,7 @@ extern "C" int gf_rmsnorm_bwd_noalloc(const void* x, const void* w, const void* 
                                       const void* dres, void* dx, void* dw, int T, int D, int accumulate,
                                       void* stream) {
   using namespace gf;
-  // Bind this thread to the process's device in this library's runtime (no allocation involved). A plain
+  // Bind this thread to its selected device in this library's runtime (no allocation involved). A plain
   // C caller that never selected a device simply uses the runtime's current device.
   // Arguments first: a call that is refused must not touch the device state of the calling thread.
   if (T <= 0 || D <= 0 || (D % 8) != 0 || !x || !w || !dy || !rstd || !dx || !dw) return GFH_BAD_ARG;
