@@ -34,6 +34,7 @@ CUDA_SOURCES = [
     "gemm_bf16.cu",
     "gemm2sm_bf16.cu",
     "gemm_skinny.cu",
+    "gemm_rows.cu",
     "norm.cu",
     "pointwise.cu",
     "xent_adamw.cu",

@@ -11,6 +11,7 @@
 // Replaces the reference's fp32 shared-memory SGEMM and its wmma kernel
 // (ghostflow-cuda/src/optimized_kernels.cu:22-119) and the cuBLAS wrapper
 // (ghostflow-cuda/src/blas.rs:278-313).
+#include "gemm_rows.cuh"
 #include "gf_host.h"
 #include "gf_ptx.cuh"
 
@@ -959,7 +960,26 @@ static int splitk_slices(int M, int N, int K, int out_fp32, int accumulate, int 
   return split;
 }
 
-// 1 when gf_gemm_bf16 (bf16 result, bn_hint and max_ctas 0) takes a workspace of M * N fp32 values, else 0. aligned: bases and
+// Few-row products on gemm_rows.cu rather than gemm_skinny.cu (at most 16 rows) or the kernels with 128-row tiles. Its fixed cost is
+// about 2 us more than the first one's, which loads weights into registers and holds less of them in flight; it does not clear
+// and convert a workspace as the split product does. us there / here, back to back with cold weights ([M, K] x [N, K]^T, M N K):
+//   8 512 8192 17.7 / 10.5, 8 2048 5504 12.6 / 10.7, 8 4096 11008 22.5 / 20.8, 8 4096 4096 12.4 / 12.6, 8 8192 14336 40.2 / 41.3,
+//   8 22016 4096 32.9 / 36.8; 16 1024 512 5.4 / 7.7, 16 2048 2048 8.4 / 8.5, 16 11008 2048 16.6 / 14.6, 16 4096 11008 28.6 / 20.9,
+//   16 22016 4096 41.5 / 38.3; 32 512 256 10.5 / 8.9, 32 4096 4096 20.2 / 12.9, 32 32000 4096 55.9 / 52.5; 64 512 256 10.6 / 12.6,
+//   64 2048 2048 18.5 / 10.5, 64 12288 4096 35.1 / 29.3, 64 28672 4096 56.1 / 56.9, 64 32000 4096 57.6 / 60.0.
+static bool few_rows_wanted(int M, int N, int K) {
+  if (M <= 8) return K >= 5120 && N <= 6144;
+  if (M <= 16) return K >= 4096 || (K >= 2048 && N > 4096);
+  return M <= 32 || (M <= gf::ROWS_MAX_M && N <= 24576 && K >= 512);
+}
+
+// 1 when gf_gemm_bf16 (bn_hint and max_ctas 0) takes the few-row kernel, which needs no workspace.
+GF_API int gf_gemm_bf16_few_rows(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate) {
+  return !a_mn_major && !b_mn_major && !accumulate && few_rows_wanted(M, N, K) &&
+         gf::gemm_rows_takes(nullptr, aligned ? 8 : 1, nullptr, aligned ? 8 : 1, M, N, K);
+}
+
+// For products that gf_gemm_bf16_few_rows does not name: 1 when gf_gemm_bf16 (bf16 result, bn_hint and max_ctas 0) takes a workspace of M * N fp32 values, else 0. aligned: bases and
 // pitches of A and B are multiples of 16 bytes.
 GF_API int gf_gemm_bf16_splits(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate, int activation) {
   const int split = splitk_slices(M, N, K, 0, accumulate, activation == 1 ? 1 : 0);
@@ -981,6 +1001,11 @@ GF_API int gf_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int
   p.act = activation == 1 ? 1 : 0;   // epilogue activation after bias and residual: 0 none, 1 ReLU
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
   const int split = bn_hint == 0 && max_ctas == 0 ? splitk_slices(M, N, K, out_fp32, accumulate, p.act) : 1;
+  if (bn_hint == 0 && max_ctas == 0 && !a_mn_major && !b_mn_major && !accumulate && few_rows_wanted(M, N, K) &&
+      gf::gemm_rows_takes(A, lda, B, ldb, M, N, K)) {
+    gf::RowsGemm g{A, lda, B, ldb, C, ldc, out_fp32, M, N, K, gf::ROWS_PLAIN, nullptr, 0.f, bias, residual, ldr, alpha, p.act, status};
+    return gf::gemm_rows_run(g, 0, st);
+  }
   if (bn_hint == 0 && max_ctas == 0 &&
       gf::gemm_skinny_wanted(A, B, M, N, K, a_mn_major, lda, b_mn_major, ldb, accumulate, split))
     return gf::gemm_skinny_run(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, bias, residual, ldr, alpha, p.act, st);

@@ -30,6 +30,7 @@ _SIGS = {
     "gf_set_device": [I],
     "gf_selected_device": [],
     "gf_gemm_bf16_splits": [I, I, I, I, I, I, I, I],
+    "gf_gemm_bf16_few_rows": [I, I, I, I, I, I, I],
     "gf_gemm_bf16": [P, P, P, I, I, I, I, L, I, L, L, I, I, P, P, L, F, P, I, I, P, I, I, P],
     "gf_norm_bwd_grid": [I],
     "gf_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],

@@ -37,6 +37,13 @@ def _splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu) -> bool:
     return bool(_lib.cuda_lib().gf_gemm_bf16_splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu))
 
 
+@functools.lru_cache(maxsize=4096)
+def _needs_workspace(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu) -> bool:
+    """Whether the product takes an fp32 ``[M, N]`` workspace: it splits K, and not inside the few-row kernel."""
+    return not _lib.cuda_lib().gf_gemm_bf16_few_rows(M, N, K, a_mn_major, b_mn_major, aligned, accumulate) \
+        and _splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu)
+
+
 def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bfloat16, bias=None, residual=None,
              accumulate=False, alpha=1.0, bn_hint=0, max_ctas=0, relu=False):
     """Launches the kernel on 2-D row-major views.
@@ -66,8 +73,8 @@ def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bf
     ws = None
     pa, pb = a.data_ptr(), b.data_ptr()
     if K >= 2048 and not f32_out and bn_hint == 0 and max_ctas == 0 \
-            and _splits(M, N, K, bool(a_mn_major), bool(b_mn_major), not (pa | pb | 2 * sa[0] | 2 * sb[0]) & 15,
-                        bool(accumulate), bool(relu)):
+            and _needs_workspace(M, N, K, bool(a_mn_major), bool(b_mn_major), not (pa | pb | 2 * sa[0] | 2 * sb[0]) & 15,
+                                 bool(accumulate), bool(relu)):
         ws = torch.empty(M * N, dtype=torch.float32, device=device)
     rc = lib.gf_gemm_bf16(
         pa, pb, out.data_ptr(), M, N, K,
