@@ -263,6 +263,22 @@ def _even_slices(ctas: int, blocks: int, D: int, sms: int) -> int:
     return best
 
 
+def _decode_parts(B: int, Hkv: int, n: int, D: int, sms: int, per_seq: bool) -> int:
+    """How decode attention cuts the keys of ``B`` sequences of at most ``n`` keys: parts of each sequence, or, negative, the number of
+    parts of all sequences together (one wave of CTAs, whatever the lengths are)."""
+    heads = max(1, B * Hkv)
+    if not per_seq:
+        return _even_slices(heads, max(1, (n + 127) // 128), D, sms)
+    slots = sms * (2 if D > 64 else 4)
+    # With eight units of 64 keys to a CTA the shares of all sequences together are worth the scan of the lengths and the pieces
+    # that begin and end inside a sequence (about 5 us): us with slices of each sequence / together, 32 sequences of 1 .. 4096 keys,
+    # 32 / 8 heads of 128 60.0 / 55.0, 64 of 1 .. 2048, 64 / 8 heads 70.3 / 64.4, 64 of 1 .. 1000, 16 / 16 of 64 33.3 / 30.8; 16 of
+    # 1 .. 128, 32 / 32 of 128 10.8 / 14.7, 2 of 1 .. 4000, 12 / 12 of 64 15.9 / 14.6. Two waves are slower everywhere.
+    if heads * ((n + 63) // 64) >= 8 * slots:
+        return -max(1, slots // Hkv)
+    return max(1, min(32, -(-(sms * 8) // heads), (n + 127) // 128))
+
+
 def attn_decode(q, kcache, vcache, length, B, Hq, Hkv, D, scale=None, splits=None, out=None):
     """q [B, Hq * D]; caches [B, s_max, Hkv * D]; attends over the first ``length`` cache rows of every sequence
     (``length``: int, or an int32 tensor [B] of per-sequence lengths). Returns [B, Hq * D]."""
@@ -272,14 +288,12 @@ def attn_decode(q, kcache, vcache, length, B, Hq, Hkv, D, scale=None, splits=Non
         per_seq = torch.is_tensor(length)
         n = s_max if per_seq else int(length)
         if splits is None:
-            # Mixed lengths: about four waves, so that short sequences even out the long ones (32 sequences of 1 .. 4096 keys,
-            # 8 heads: 72 us with one slice, 56 with four or five). No slice is shorter than 128 cache rows.
-            sms, ctas = _sm_count(q.device), max(1, B * Hkv)
-            splits = max(1, min(32, -(-(sms * 8) // ctas), (n + 127) // 128)) if per_seq \
-                else _even_slices(ctas, max(1, (n + 127) // 128), D, sms)
+            splits = _decode_parts(B, Hkv, n, D, _sm_count(q.device), per_seq)
+        elif splits < 1:
+            raise ValueError(f"attn_decode cuts the keys of a head into one part or more, not {splits}")
         if out is None:
             out = torch.empty(B, Hq * D, dtype=q.dtype, device=q.device)
-        scratch = torch.empty(B * Hq * splits * (D + 2), dtype=torch.float32, device=q.device)
+        scratch = torch.empty((B * splits if splits > 0 else -2 * splits) * Hq * (D + 2), dtype=torch.float32, device=q.device)
         _rc(_lib.cuda_lib().gf_attn_decode(q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(), s_max,
                                            length.data_ptr() if per_seq else None, 0 if per_seq else n, out.data_ptr(),
                                            out.stride(0), B, Hq, Hkv, D, float(scale), splits, scratch.data_ptr(),
