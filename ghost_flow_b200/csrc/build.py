@@ -44,6 +44,7 @@ CUDA_SOURCES = [
     "attn_bwd.cu",
     "attn_bwd3.cu",
     "attn_decode.cu",
+    "decode_layer.cu",
     "comm_kernels.cu",
     "moe_kernels.cu",
     "quant_fp8.cu",

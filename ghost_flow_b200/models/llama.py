@@ -12,8 +12,8 @@ from __future__ import annotations
 import torch
 
 from .. import ops
-from ..nn.layers import Embedding, Linear, RMSNorm
-from ..nn.module import Module, ModuleList
+from ..nn.layers import Embedding, Linear, RMSNorm, SwiGLU
+from ..nn.module import Module, ModuleList, plain_modules
 from .configs import LLaMAConfig
 
 
@@ -69,14 +69,52 @@ class LLaMAAttention(Module):
 class LLaMADecoderLayer(Module):
     def __init__(self, cfg: LLaMAConfig, device=None, dtype=None):
         super().__init__()
-        from ..nn.layers import SwiGLU
-
         self.attn_norm = RMSNorm(cfg.hidden_size, cfg.rms_norm_eps, device, dtype)
         self.attn = LLaMAAttention(cfg, device, dtype)
         self.ffn_norm = RMSNorm(cfg.hidden_size, cfg.rms_norm_eps, device, dtype)
         self.mlp = SwiGLU(cfg.hidden_size, cfg.intermediate_size, False, device, dtype)
 
+    def _decodes_in_one_call(self, x, cos, sin, cache, start_pos):
+        """The operands of :func:`ops.raw.llama_decode_layer`, or ``None`` where the layer runs module by module: more than one
+        token, a gradient, other types or layouts, modules that were replaced or carry hooks, and calls that something
+        follows (tracing, transforms, modes), which would miss what happens inside."""
+        if x.dim() != 3 or x.shape[1] != 1 or x.dtype is not torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() \
+                or type(x) is not torch.Tensor or not 0 < x.shape[0] <= 64:
+            return None
+        m = self._modules
+        an, at, fn, mlp = m["attn_norm"], m["attn"], m["ffn_norm"], m["mlp"]
+        if not (type(an) is RMSNorm and type(at) is LLaMAAttention and type(fn) is RMSNorm and type(mlp) is SwiGLU):
+            return None
+        lin = at._modules["wqkv"], at._modules["wo"], mlp._modules["gate_up"], mlp._modules["down"]
+        if any(type(n) is not Linear or n.bias is not None for n in lin) or not plain_modules(an, at, fn, mlp, *lin):
+            return None
+        c, (kc, vc), (B, _, hidden), dev = at.cfg, cache, x.shape, x.device
+        H, Hk, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim
+        w = [an._parameters["weight"], lin[0]._parameters["weight"], lin[1]._parameters["weight"], fn._parameters["weight"],
+             lin[2]._parameters["weight"], lin[3]._parameters["weight"]]
+        inner = w[5].shape[1] if w[5].dim() == 2 else 0
+        shapes = (hidden,), ((H + 2 * Hk) * D, hidden), (hidden, H * D), (hidden,), (2 * inner, hidden), (hidden, inner)
+        if D not in (64, 128) or H % Hk or H // Hk > 8 or hidden % 8 or inner % 8 or inner == 0:
+            return None
+        for p, s in zip(w, shapes):
+            if p.shape != s or p.dtype is not torch.bfloat16 or p.device != dev or not p.is_contiguous() or p.data_ptr() & 15 \
+                    or type(p) not in (torch.Tensor, torch.nn.Parameter):
+                return None
+        if dev.index != torch.cuda.current_device() or not (x.is_contiguous() and x.data_ptr() & 15 == 0) \
+                or not ops.decode_cache_ok(kc, vc, cos, sin, (B, Hk, D), dev, start_pos):
+            return None
+        return (x.view(B, hidden), w[0], an.eps, w[1], w[2], w[3], fn.eps, w[4], w[5], cos, sin, kc, vc, H, Hk, D,
+                c.rope_interleaved, start_pos)
+
     def forward(self, x, cos, sin, cache=None, start_pos: int = 0):
+        if cache is not None:
+            args = self._decodes_in_one_call(x, cos, sin, cache, start_pos)
+            if args is not None:
+                from ..ops import raw
+
+                y = raw.llama_decode_layer(*args)
+                torch.autograd.graph.increment_version(cache)     # a graph that saved a cache has to notice the write
+                return y.view(x.shape)
         x = self.attn(self.attn_norm(x), cos, sin, residual=x, cache=cache, start_pos=start_pos)
         return self.mlp(self.ffn_norm(x), residual=x)
 

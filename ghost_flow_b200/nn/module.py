@@ -91,6 +91,20 @@ class Module(torch.nn.Module):
         return self.load_state_dict(sd, strict=strict)
 
 
+_GLOBAL_HOOKS = tuple(getattr(torch.nn.modules.module, n, None) for n in ("_global_forward_hooks", "_global_forward_pre_hooks"))
+
+
+def plain_modules(*modules) -> bool:
+    """Whether calling these modules does nothing but their class's ``forward``: no hooks of their own or of all modules, no
+    profiling of modules, no ``forward`` put on an instance. What computes several of them at once has to ask."""
+    if Module._profile_hook is not None or any(h is None or h for h in _GLOBAL_HOOKS):
+        return False
+    for m in modules:
+        if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+            return False
+    return True
+
+
 class Sequential(Module):
     """Ordered container. ``Sequential([a, b])``, ``Sequential(a, b)`` or ``Sequential().add_layer(a)``."""
 

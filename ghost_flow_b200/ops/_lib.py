@@ -61,6 +61,7 @@ _SIGS = {
     "gf_flash_attn_fwd": [P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, I, P, P],
     "gf_flash_attn_fwd2": [P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, I, P, P],
     "gf_flash_attn_fwd3": [P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, I, P, P],
+    "gf_llama_decode_layer": [P, P, F, P, P, P, F, P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, P, P],
     "gf_attn_decode": [P, L, P, P, I, P, I, P, L, I, I, I, I, F, I, P, P],
     "gf_flash_attn_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, F, I, P, P],
     "gf_attn_bwd_prep": [P, P, P, P, I, I, I, I, L, L, P],

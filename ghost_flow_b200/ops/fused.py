@@ -433,6 +433,20 @@ def _observed() -> bool:
             or getattr(forward_ad, "_current_level", 0) >= 0 or torch.compiler.is_compiling())
 
 
+def decode_cache_ok(kcache, vcache, cos, sin, heads, device, pos: int) -> bool:
+    """Whether a decoding kernel may write row ``pos`` of the caches ``[B, n, Hk, D]`` (``heads`` = B, Hk, D) and rotate with these
+    tables; positions that are not in the tables are an error."""
+    B, Hk, D = heads
+    if _observed() or kcache.dim() != 4 or not (kcache.is_contiguous() and vcache.is_contiguous()):
+        return False
+    shape = (B, kcache.shape[1], Hk, D)
+    if not (0 <= pos < shape[1] and _cache_fits_kernel(kcache, shape, device, torch.bfloat16)
+            and _cache_fits_kernel(vcache, shape, device, torch.bfloat16) and _cache_rows_apart(kcache, vcache)):
+        return False
+    check_rope_tables(device, 1, D, cos, sin, pos)
+    return _rope_tables_fit_kernel(cos, sin)
+
+
 def embedding_rows(ids, table, rows: int | None = None):
     """``table[ids]`` with zero rows for ids outside the table, in one launch; ``None`` where the kernel does not apply
     (CPU tensors, a GPU that is not the current one, a gradient to record, rows that are no whole 16-byte vectors, tensors

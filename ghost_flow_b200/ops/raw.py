@@ -312,3 +312,27 @@ def attn_decode(q, kcache, vcache, length, B, Hq, Hkv, D, scale=None, splits=Non
         out.copy_(res)
         return out
     return res
+
+
+# ------------------------------------------------------------------ one decoder layer, one token of each sequence
+def llama_decode_layer(x, attn_norm, attn_eps, wqkv, wo, ffn_norm, ffn_eps, gate_up, down, cos, sin, kcache, vcache, Hq, Hkv, D,
+                       interleaved, pos):
+    """A whole LLaMA decoder layer for one new token of each of at most 64 sequences, in one call of the kernel library (six
+    kernels or nine, most of them started while the one in front of them ends). ``x [B, hidden]`` and weights ``[out, in]`` dense bf16; caches
+    ``[B, s_max, Hkv, D]`` dense, row ``pos`` is written; tables fp32 with a row for ``pos``. Returns ``[B, hidden]``."""
+    B, hidden = x.shape
+    inner, s_max = down.shape[1], kcache.shape[1]
+    splits = _even_slices(B * Hkv, (pos + 128) // 128, D, _sm_count(x.device))
+    lib = _lib.cuda_lib()
+    y = torch.empty_like(x)
+    # workspaces of the layer: q, k, v; attention; its sum with x; gate and up; the parts of the attention (fp32)
+    ws = torch.empty(2 * B * ((2 * Hq + 2 * Hkv) * D + hidden + 2 * inner + max(hidden, inner))
+                     + 4 * B * Hq * splits * (D + 2) + 1536, dtype=torch.uint8, device=x.device)
+    _rc(lib.gf_llama_decode_layer(
+        x.data_ptr(), attn_norm.data_ptr(), float(attn_eps), wqkv.data_ptr(), wo.data_ptr(), ffn_norm.data_ptr(),
+        float(ffn_eps), gate_up.data_ptr(), down.data_ptr(), cos.data_ptr(), sin.data_ptr(), kcache.data_ptr(),
+        vcache.data_ptr(), s_max, y.data_ptr(), ws.data_ptr(), B, hidden, inner, Hq, Hkv, D, 1 if interleaved else 0, pos, splits,
+        _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()), "gf_llama_decode_layer")
+    if _lib.DEBUG_SYNC:
+        _lib.check_status(x.device)
+    return y
