@@ -164,19 +164,21 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_fwd_block_kernel(const Norm
 struct NormBwd {
   const __nv_bfloat16 *x, *w, *dy, *dres;
   const float *mean, *rstd;
-  __nv_bfloat16* dx;
+  __nv_bfloat16 *dx, *dx2;            // dx2: a second copy, for an input whose gradient is stored apart (may be null)
   float *dw_partial, *db_partial;     // one row of D per CTA
   int T, D;
 };
 
-template <int NV>
+// RES: there may be a dres. RMSNorm loads it with the row; LayerNorm, which has no registers left for that, where it is added,
+// and it has kernels without.
+template <int NV, bool EARLY>
 struct NormBwdRow {
-  uint4 x[NV], g[NV], r[NV];
+  uint4 x[NV], g[NV], r[EARLY ? NV : 1];
   float mean, rstd;
 };
 
 template <bool LN, int NV>
-__device__ __forceinline__ void norm_bwd_load(const NormBwd& p, NormBwdRow<NV>& t, int row, int v0, int stride) {
+__device__ __forceinline__ void norm_bwd_load(const NormBwd& p, NormBwdRow<NV, !LN>& t, int row, int v0, int stride) {
   const int nv = p.D >> 3;
   const long long base = (long long)row * p.D;
 #pragma unroll
@@ -185,19 +187,19 @@ __device__ __forceinline__ void norm_bwd_load(const NormBwd& p, NormBwdRow<NV>& 
     const bool in = v < nv;
     t.x[i] = in ? ldv(p.x + base + v * 8) : make_uint4(0, 0, 0, 0);
     t.g[i] = in ? ldv(p.dy + base + v * 8) : make_uint4(0, 0, 0, 0);
-    if (!LN && p.dres) t.r[i] = in ? ldv(p.dres + base + v * 8) : make_uint4(0, 0, 0, 0);
+    if (!LN && p.dres) t.r[LN ? 0 : i] = in ? ldv(p.dres + base + v * 8) : make_uint4(0, 0, 0, 0);
   }
   t.rstd = p.rstd[row];
   t.mean = LN ? p.mean[row] : 0.f;
 }
 
 // Rows row0, row0 + step, ... of one warp or CTA; the sums over rows end in dw / db. wv: this thread's weights, packed.
-template <bool LN, int NV, bool PREFETCH, typename Sum>
+template <bool LN, int NV, bool RES, bool PREFETCH, typename Sum>
 __device__ __forceinline__ void norm_bwd_rows(const NormBwd& p, int row0, int step, int v0, int stride, float (&dw)[NV][8],
                                               float (&db)[LN ? NV : 1][8], Sum sum) {
   const int nv = p.D >> 3;
   const float inv_d = 1.f / (float)p.D;
-  NormBwdRow<NV> cur, nxt;
+  NormBwdRow<NV, !LN> cur, nxt;
   if (PREFETCH && row0 < p.T) norm_bwd_load<LN, NV>(p, cur, row0, v0, stride);
   for (int row = row0; row < p.T; row += step) {
     if (!PREFETCH) norm_bwd_load<LN, NV>(p, cur, row, v0, stride);
@@ -236,13 +238,15 @@ __device__ __forceinline__ void norm_bwd_rows(const NormBwd& p, int row0, int st
         for (int j = 0; j < 8; ++j)
           o[j] = LN ? cur.rstd * (gv[j] * wv[j] - s1 - (xv[j] - cur.mean) * cur.rstd * c)
                     : cur.rstd * gv[j] * wv[j] - c * xv[j];
-        if (!LN && p.dres) {
+        if (RES && p.dres) {
           float rv[8];
-          unpack8(cur.r[i], rv);
+          unpack8(LN ? ldv(p.dres + (long long)row * p.D + v * 8) : cur.r[LN ? 0 : i], rv);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += rv[j];
         }
-        stv(p.dx + (long long)row * p.D + v * 8, pack8(o));
+        const uint4 out = pack8(o);
+        stv(p.dx + (long long)row * p.D + v * 8, out);
+        if (!LN && p.dx2) stv(p.dx2 + (long long)row * p.D + v * 8, out);
       }
     }
     if (PREFETCH) cur = nxt;
@@ -250,7 +254,7 @@ __device__ __forceinline__ void norm_bwd_rows(const NormBwd& p, int row0, int st
 }
 
 // One warp per row, D <= 1024. The eight warps' sums meet in shared memory, warp by warp in its own row of it.
-template <bool LN, int NV>
+template <bool LN, int NV, bool RES>
 __global__ void __launch_bounds__(NORM_THREADS, NV == 1 ? 3 : 2) norm_bwd_warp_kernel(const NormBwd p) {
   __shared__ float acc[NORM_WARPS][NORM_WARP_D];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = p.D >> 3;
@@ -262,7 +266,7 @@ __global__ void __launch_bounds__(NORM_THREADS, NV == 1 ? 3 : 2) norm_bwd_warp_k
       dw[i][j] = 0.f;
       if (LN) db[LN ? i : 0][j] = 0.f;
     }
-  norm_bwd_rows<LN, NV, NV <= 2>(p, blockIdx.x * NORM_WARPS + warp, gridDim.x * NORM_WARPS, lane, 32, dw, db,
+  norm_bwd_rows<LN, NV, RES, NV <= 2>(p, blockIdx.x * NORM_WARPS + warp, gridDim.x * NORM_WARPS, lane, 32, dw, db,
                               [](float v) { return warp_sum(v); });
   auto flush = [&](const float(&a)[NV][8], float* out) {
 #pragma unroll
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(NORM_THREADS, NV == 1 ? 3 : 2) norm_bwd_warp_k
 template <bool LN, int NV>
 constexpr int norm_bwd_ctas() { return NV == 1 ? 4 : NV == 2 ? 2 : LN ? 1 : 2; }
 
-template <bool LN, int NV>
+template <bool LN, int NV, bool RES>
 __global__ void __launch_bounds__(NORM_THREADS, norm_bwd_ctas<LN, NV>()) norm_bwd_block_kernel(const NormBwd p) {
   __shared__ float red[4][NORM_WARPS];
   const int nv = p.D >> 3;
@@ -305,7 +309,7 @@ __global__ void __launch_bounds__(NORM_THREADS, norm_bwd_ctas<LN, NV>()) norm_bw
       if (LN) db[LN ? i : 0][j] = 0.f;
     }
   int k = 0;
-  norm_bwd_rows<LN, NV, NV <= 2>(p, blockIdx.x, gridDim.x, threadIdx.x, NORM_THREADS, dw, db,
+  norm_bwd_rows<LN, NV, RES, NV <= 2>(p, blockIdx.x, gridDim.x, threadIdx.x, NORM_THREADS, dw, db,
                                  [&](float v) { return block_sum(v, red[k++ & 3]); });
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -428,25 +432,25 @@ static int launch_norm_fwd(const NormFwd& p, cudaStream_t st) {
 
 // Number of partial rows written: at most norm_grid(T), which sizes the caller's scratch, and no more CTAs than are
 // resident at once (a second wave would wait for the first one's row loops).
-template <bool LN>
+template <bool LN, bool RES>
 static int launch_norm_bwd(const NormBwd& p, cudaStream_t st) {
   const int cap = norm_grid(p.T), sms = sm_count();
   int grid;
   if (norm_row_per_warp(p.T, p.D, sms)) {
     const int vpl = (p.D / 8 + 31) / 32;
     grid = at_most(at_most((p.T + NORM_WARPS - 1) / NORM_WARPS, cap), (long long)sms * (vpl == 1 ? 3 : 2));
-    auto kern = vpl == 1 ? norm_bwd_warp_kernel<LN, 1> : vpl == 2 ? norm_bwd_warp_kernel<LN, 2>
-                : vpl == 3 ? norm_bwd_warp_kernel<LN, 3> : norm_bwd_warp_kernel<LN, 4>;
+    auto kern = vpl == 1 ? norm_bwd_warp_kernel<LN, 1, RES> : vpl == 2 ? norm_bwd_warp_kernel<LN, 2, RES>
+                : vpl == 3 ? norm_bwd_warp_kernel<LN, 3, RES> : norm_bwd_warp_kernel<LN, 4, RES>;
     kern<<<grid, NORM_THREADS, 0, st>>>(p);
   } else if (p.D <= NORM_THREADS * 8) {
     grid = at_most(cap, (long long)sms * norm_bwd_ctas<LN, 1>());
-    norm_bwd_block_kernel<LN, 1><<<grid, NORM_THREADS, 0, st>>>(p);
+    norm_bwd_block_kernel<LN, 1, RES><<<grid, NORM_THREADS, 0, st>>>(p);
   } else if (p.D <= NORM_THREADS * 16) {
     grid = at_most(cap, (long long)sms * norm_bwd_ctas<LN, 2>());
-    norm_bwd_block_kernel<LN, 2><<<grid, NORM_THREADS, 0, st>>>(p);
+    norm_bwd_block_kernel<LN, 2, RES><<<grid, NORM_THREADS, 0, st>>>(p);
   } else {
     grid = at_most(cap, (long long)sms * norm_bwd_ctas<LN, NORM_MAXV>());
-    norm_bwd_block_kernel<LN, NORM_MAXV><<<grid, NORM_THREADS, 0, st>>>(p);
+    norm_bwd_block_kernel<LN, NORM_MAXV, RES><<<grid, NORM_THREADS, 0, st>>>(p);
   }
   return grid;
 }
@@ -467,17 +471,22 @@ GF_API int gf_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y
 }
 
 // scratch: fp32 [gf_norm_bwd_grid(T), D]. dw is bf16 [D]; accumulate=1 adds into it.
-GF_API int gf_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, const void* dres,
-                          void* dx, void* dw, float* scratch, int T, int D, int accumulate, void* stream) {
+// dx2: the input gradient once more (may be null).
+GF_API int gf_rmsnorm_bwd2(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx, void* dx2,
+                           void* dw, float* scratch, int T, int D, int accumulate, void* stream) {
   gf::enter();
   if (D % 8 || D > NORM_THREADS * NORM_MAXV * 8 || T <= 0) return GFH_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   NormBwd p{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, nullptr,
-            rstd, (__nv_bfloat16*)dx, scratch, nullptr, T, D};
-  const int parts = launch_norm_bwd<false>(p, st);
+            rstd, (__nv_bfloat16*)dx, (__nv_bfloat16*)dx2, scratch, nullptr, T, D};
+  const int parts = launch_norm_bwd<false, true>(p, st);
   launch_fold(scratch, dw, nullptr, nullptr, parts, D, accumulate, st);
   gf::note_extra_launches(1);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
+}
+GF_API int gf_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, const void* dres,
+                          void* dx, void* dw, float* scratch, int T, int D, int accumulate, void* stream) {
+  return gf_rmsnorm_bwd2(x, w, dy, rstd, dres, dx, nullptr, dw, scratch, T, D, accumulate, stream);
 }
 
 // x: bf16 [T, D] with row pitch ld (elements, multiple of 8); out: bf16 [D]; scratch: fp32 [gf_norm_bwd_grid(T), D].
@@ -504,18 +513,23 @@ GF_API int gf_layernorm_fwd(const void* x, const void* w, const void* b, void* y
   return launch_norm_fwd<true>(p, (cudaStream_t)stream);
 }
 
-// scratch: fp32 [2, gf_norm_bwd_grid(T), D]
-GF_API int gf_layernorm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
-                            void* dx, void* dw, void* db, float* scratch, int T, int D, int accumulate,
-                            void* stream) {
+// scratch: fp32 [2, gf_norm_bwd_grid(T), D]. dres is added into dx (may be null).
+GF_API int gf_layernorm_bwd_res(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
+                                const void* dres, void* dx, void* dw, void* db, float* scratch, int T, int D, int accumulate,
+                                void* stream) {
   gf::enter();
   if (D % 8 || D > NORM_THREADS * NORM_MAXV * 8 || T <= 0) return GFH_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   float* s2 = scratch + (long long)norm_grid(T) * D;
-  NormBwd p{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, nullptr, mean,
-            rstd, (__nv_bfloat16*)dx, scratch, s2, T, D};
-  const int parts = launch_norm_bwd<true>(p, st);
+  NormBwd p{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, mean,
+            rstd, (__nv_bfloat16*)dx, nullptr, scratch, s2, T, D};
+  const int parts = dres ? launch_norm_bwd<true, true>(p, st) : launch_norm_bwd<true, false>(p, st);
   launch_fold(scratch, dw, s2, db, parts, D, accumulate, st);
   gf::note_extra_launches(1);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
+}
+GF_API int gf_layernorm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
+                            void* dx, void* dw, void* db, float* scratch, int T, int D, int accumulate,
+                            void* stream) {
+  return gf_layernorm_bwd_res(x, w, dy, mean, rstd, nullptr, dx, dw, db, scratch, T, D, accumulate, stream);
 }

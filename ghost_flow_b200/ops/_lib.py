@@ -35,6 +35,7 @@ _SIGS = {
     "gf_norm_bwd_grid": [I],
     "gf_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "gf_rmsnorm_bwd": [P, P, P, P, P, P, P, P, I, I, I, P],
+    "gf_rmsnorm_bwd2": [P, P, P, P, P, P, P, P, P, I, I, I, P],
     "gf_layernorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "gf_layernorm_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, P],
     "gf_rope": [P, P, P, I, I, I, L, L, I, I, I, I, P],

@@ -64,6 +64,7 @@ class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps, residual):
         D = x.shape[-1]
+        x_is_leaf = x.is_leaf
         x = _dense(x)
         T = x.numel() // D
         y = torch.empty_like(x)
@@ -79,6 +80,8 @@ class _RMSNormFn(torch.autograd.Function):
             _lib.stream_ptr()), "gf_rmsnorm_fwd")
         ctx.save_for_backward(h if h is not None else x, w, rstd)
         ctx.has_res = residual is not None
+        # two leaves keep their gradients apart: the kernel writes both, where autograd would copy one (a pass of its own)
+        ctx.two = residual is not None and x_is_leaf and residual.is_leaf
         return (y, h) if residual is not None else y
 
     @staticmethod
@@ -89,14 +92,16 @@ class _RMSNormFn(torch.autograd.Function):
         dy = _dense(dy)
         dres = _dense(dh) if (ctx.has_res and dh is not None) else None
         dx = torch.empty_like(x)
+        dx2 = torch.empty_like(x) if ctx.two and ctx.needs_input_grad[0] and ctx.needs_input_grad[3] else None
         dw = torch.empty_like(w)
         lib = _lib.cuda_lib()
         g = lib.gf_norm_bwd_grid(T)
         scratch = _scratch(x.device, g * D)
-        _rc(lib.gf_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(),
-                               None if dres is None else dres.data_ptr(), dx.data_ptr(), dw.data_ptr(),
-                               scratch.data_ptr(), T, D, 0, _lib.stream_ptr()), "gf_rmsnorm_bwd")
-        return dx, dw, None, dx if ctx.has_res else None
+        _rc(lib.gf_rmsnorm_bwd2(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(),
+                                None if dres is None else dres.data_ptr(), dx.data_ptr(),
+                                None if dx2 is None else dx2.data_ptr(), dw.data_ptr(), scratch.data_ptr(), T, D, 0,
+                                _lib.stream_ptr()), "gf_rmsnorm_bwd2")
+        return dx, dw, None, None if not ctx.has_res else dx if dx2 is None else dx2
 
 
 def rms_norm_ref(x, w, eps=1e-6):
