@@ -45,6 +45,7 @@ CUDA_SOURCES = [
     "attn_bwd3.cu",
     "attn_decode.cu",
     "decode_layer.cu",
+    "transformer_block.cu",
     "comm_kernels.cu",
     "moe_kernels.cu",
     "quant_fp8.cu",

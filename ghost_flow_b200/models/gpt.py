@@ -14,8 +14,8 @@ import torch
 from .. import ops
 from ..nn import init
 from ..nn.attention import MultiHeadAttention
-from ..nn.layers import Dropout, Embedding, LayerNorm, Linear
-from ..nn.module import Module, ModuleList
+from ..nn.layers import GELU, Dropout, Embedding, LayerNorm, Linear
+from ..nn.module import Module, ModuleList, plain_modules
 from ..nn.transformer import FeedForward
 from .configs import GPTConfig
 
@@ -43,9 +43,38 @@ class GPTBlock(Module):
         self.mlp = FeedForward(cfg.n_embd, cfg.n_inner, cfg.dropout, cfg.activation)
         self.drop = Dropout(cfg.dropout)
 
+    def _one_call(self, x):
+        """The operands of :func:`ops.gpt_block`, or ``None`` where the block runs layer by layer: other types, layouts or
+        activations, dropout, modules that were replaced or carry hooks."""
+        if not x.is_cuda or x.dtype is not torch.bfloat16 or x.dim() != 3 or x.numel() == 0:
+            return None
+        m = self._modules
+        ln1, at, ln2, mlp = m["ln1"], m["attn"], m["ln2"], m["mlp"]
+        if not (type(ln1) is LayerNorm and type(at) is MultiHeadAttention and type(ln2) is LayerNorm and type(mlp) is FeedForward):
+            return None
+        qkv, out, fc1, fc2 = at._modules["qkv"], at._modules["out_proj"], mlp._modules["fc1"], mlp._modules["fc2"]
+        act, drop = mlp._modules["act"], mlp._modules["drop"]
+        lin = qkv, out, fc1, fc2
+        if any(type(n) is not Linear for n in lin) or type(act) is not GELU or type(drop) is not Dropout \
+                or not plain_modules(ln1, at, ln2, mlp, act, drop, *lin):
+            return None
+        if (at.dropout > 0 and at.training) or (drop.p > 0 and drop.training) or ln1.weight is None or ln2.weight is None:
+            return None
+        B, S, E = x.shape
+        params = (ln1.weight, ln1.bias, qkv.weight, qkv.bias, out.weight, out.bias, ln2.weight, ln2.bias, fc1.weight, fc1.bias,
+                  fc2.weight, fc2.bias)
+        H = at.num_heads
+        if E != at.embed_dim or E % H or fc1.weight.dim() != 2:
+            return None
+        sizes = (B, S, E, fc1.weight.shape[0], H, at.num_kv_heads)
+        return (x, params, sizes, ln1.eps, ln2.eps, at.causal) if ops.gpt_block_ok(x, params, sizes) else None
+
     def forward(self, x):
         if self.pre_norm:
             if self.drop.p == 0 or not self.training:
+                args = self._one_call(x)
+                if args is not None:
+                    return ops.gpt_block(*args)
                 x = self.attn(self.ln1(x), residual=x)          # residual add fused into the GEMM epilogue
                 return self.mlp(self.ln2(x), residual=x)
             x = x + self.drop(self.attn(self.ln1(x)))

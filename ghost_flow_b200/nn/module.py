@@ -91,7 +91,8 @@ class Module(torch.nn.Module):
         return self.load_state_dict(sd, strict=strict)
 
 
-_GLOBAL_HOOKS = tuple(getattr(torch.nn.modules.module, n, None) for n in ("_global_forward_hooks", "_global_forward_pre_hooks"))
+_GLOBAL_HOOKS = tuple(getattr(torch.nn.modules.module, n, None) for n in (
+    "_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks"))
 
 
 def plain_modules(*modules) -> bool:
@@ -100,7 +101,7 @@ def plain_modules(*modules) -> bool:
     if Module._profile_hook is not None or any(h is None or h for h in _GLOBAL_HOOKS):
         return False
     for m in modules:
-        if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+        if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__:
             return False
     return True
 

@@ -62,6 +62,10 @@ _SIGS = {
     "gf_flash_attn_fwd": [P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, I, P, P],
     "gf_flash_attn_fwd2": [P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, I, P, P],
     "gf_flash_attn_fwd3": [P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, I, P, P],
+    "gf_gpt_block_bytes": [I, I, I, I, I, I, I],
+    "gf_gpt_block_fwd": [P, P, P, P, P, I, I, I, I, I, I, I, F, F, P, P],
+    "gf_gpt_block_bwd": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P],
+    "gf_flash_attn_backward": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, F, I, P, P],
     "gf_llama_decode_layer": [P, P, F, P, P, P, F, P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, P, P],
     "gf_attn_decode": [P, L, P, P, I, P, I, P, L, I, I, I, I, F, I, P, P],
     "gf_flash_attn_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, F, I, P, P],
@@ -80,7 +84,7 @@ def _bind(lib, sigs):
         except AttributeError:
             continue
         fn.argtypes = args
-        fn.restype = c_int
+        fn.restype = c_longlong if name == "gf_gpt_block_bytes" else c_int
     return lib
 
 
@@ -247,10 +251,10 @@ def flash_attn_backward(q, k, v, o, do, lse, dq, dk, dv, B, S, Hq, Hkv, D, ld, s
     st = stream_ptr()
     dev = q.device
     status = status_word(dev).data_ptr()
-    delta = torch.empty((B, Hq, S), dtype=torch.float32, device=dev)
-    dq_acc = torch.empty((B * S, Hq * D), dtype=torch.float32, device=dev)
     c = 1 if causal else 0
     if os.environ.get("GF_FA_BWD", "3") == "1":
+        delta = torch.empty((B, Hq, S), dtype=torch.float32, device=dev)
+        dq_acc = torch.empty((B * S, Hq * D), dtype=torch.float32, device=dev)
         check_rc(lib.gf_attn_bwd_prep(o.data_ptr(), do.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), B, S, Hq, D,
                                       ld["o"], ld["do"], st), "gf_attn_bwd_prep")
         check_rc(lib.gf_flash_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), do.data_ptr(), lse.data_ptr(),
@@ -259,15 +263,10 @@ def flash_attn_backward(q, k, v, o, do, lse, dq, dk, dv, B, S, Hq, Hkv, D, ld, s
                                        c, status, st), "gf_flash_attn_bwd")
         check_rc(lib.gf_cast_f32_to_bf16_2d(dq_acc.data_ptr(), dq.data_ptr(), B * S, Hq * D, Hq * D, ld["dq"], 1.0,
                                             st), "gf_cast_f32_to_bf16_2d")
-    else:
-        nlse2 = torch.empty((B, Hq, S), dtype=torch.float32, device=dev)
-        check_rc(lib.gf_attn_bwd_prep3(o.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-                                       nlse2.data_ptr(), dq_acc.data_ptr(), B, S, Hq, D, ld["o"], ld["do"], st),
-                 "gf_attn_bwd_prep3")
-        check_rc(lib.gf_flash_attn_bwd3(q.data_ptr(), k.data_ptr(), v.data_ptr(), do.data_ptr(), nlse2.data_ptr(),
-                                        delta.data_ptr(), dq_acc.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, S, Hq,
-                                        Hkv, D, ld["q"], ld["k"], ld["v"], ld["do"], ld["dk"], ld["dv"],
-                                        float(scale), c, status, st), "gf_flash_attn_bwd3")
-        # the main kernel leaves dQ / scale in the accumulator [B, Hq, S, D]
-        check_rc(lib.gf_dq_rows_to_bf16(dq_acc.data_ptr(), dq.data_ptr(), B, S, Hq, D, ld["dq"], float(scale), st),
-                 "gf_dq_rows_to_bf16")
+        return
+    # fp32 accumulator of dQ, -sum(o do) and -lse log2(e) of every row
+    ws = torch.empty(B * Hq * S * (D + 2), dtype=torch.float32, device=dev)
+    table = (c_longlong * 8)(ld["q"], ld["k"], ld["v"], ld["o"], ld["do"], ld["dq"], ld["dk"], ld["dv"])
+    check_rc(lib.gf_flash_attn_backward(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
+                                        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), B, S, Hq, Hkv, D, table,
+                                        float(scale), c, status, st), "gf_flash_attn_backward")

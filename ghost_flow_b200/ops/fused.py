@@ -8,7 +8,9 @@ numerical reference the GPU tests compare against.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
+import os
 
 import torch
 import torch.nn.functional as F
@@ -725,3 +727,82 @@ def flash_attention(q, k, v, causal: bool = True, scale: float | None = None):
     if _cuda_bf16(q, k, v) and D in (64, 128) and q.shape[1] == k.shape[1]:
         return _call(_FlashAttnFn, q, k, v, causal, scale)
     return attention_ref(q, k, v, causal, scale)
+
+
+# ------------------------------------------------------------------------------------------ a whole pre-norm block
+@functools.lru_cache(maxsize=1024)
+def _block_bytes(which, B, S, E, F, H, Hk) -> int:
+    return _lib.cuda_lib().gf_gpt_block_bytes(which, B, S, E, F, H, Hk)
+
+
+def _pointers(ts):
+    return (ctypes.c_void_p * len(ts))(*[None if t is None else t.data_ptr() for t in ts])
+
+
+class _GPTBlockFn(torch.autograd.Function):
+    """See :func:`gpt_block`. The launches of a pass are one call; what the backward pass reads again is one buffer."""
+
+    @staticmethod
+    def forward(ctx, x, sizes, eps1, eps2, causal, *params):
+        B, S, E, F_, H, Hk = sizes
+        y = torch.empty_like(x)
+        mem = lambda n: torch.empty(n, dtype=torch.uint8, device=x.device) if n else None  # noqa: E731
+        saved, ws = mem(_block_bytes(0, *sizes)), mem(_block_bytes(2, *sizes))
+        _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), saved.data_ptr(),
+                                             None if ws is None else ws.data_ptr(), *sizes, causal, eps1, eps2,
+                                             _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()), "gf_gpt_block_fwd")
+        ctx.save_for_backward(x, saved, *params)
+        ctx.args = sizes, causal
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, saved, *params = ctx.saved_tensors
+        sizes, causal = ctx.args
+        dy = _dense(dy)
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        dx = torch.empty_like(x)
+        # the norms' kernels always write theirs
+        grads = [torch.empty_like(p) if p is not None and (need or i in (0, 6)) else None
+                 for i, (p, need) in enumerate(zip(params, ctx.needs_input_grad[5:]))]
+        ws = torch.empty(_block_bytes(1, *sizes), dtype=torch.uint8, device=x.device)
+        _rc(_lib.cuda_lib().gf_gpt_block_bwd(x.data_ptr(), _pointers(params), dy.data_ptr(), saved.data_ptr(), dx.data_ptr(),
+                                             _pointers(grads), ws.data_ptr(), *sizes, causal,
+                                             _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()), "gf_gpt_block_bwd")
+        return (dx, None, None, None, None, *grads)
+
+
+def gpt_block(x, params, sizes, eps1: float, eps2: float, causal: bool):
+    """``h = x + Wo attention(LN1(x) Wqkv^T + bqkv) + bo``, ``y = h + W2 gelu(LN2(h) W1^T + b1) + b2`` on the kernels of the layers,
+    all launches of a pass from one call of the kernel library. ``params``: ln1 weight and bias, Wqkv, bqkv, Wo, bo, ln2
+    weight and bias, W1, b1, W2, b2 (biases may be ``None``); ``sizes``: batch, sequence, width, inner width, heads, KV heads."""
+    y = _call(_GPTBlockFn, x, sizes, float(eps1), float(eps2), 1 if causal else 0, *params)
+    if _lib.DEBUG_SYNC:
+        _lib.check_status()
+    return y
+
+
+def gpt_block_ok(x, params, sizes) -> bool:
+    """Whether :func:`gpt_block` takes these operands: dense bf16 CUDA tensors of the sizes, on 16-byte boundaries, with head
+    sizes and (where there is a gradient) a sequence that the attention kernels have, and nothing that follows the layers'
+    own calls."""
+    B, S, E, F_, H, Hk = sizes
+    if type(x) is not torch.Tensor or not _cuda_bf16(x) or not x.is_contiguous() or x.data_ptr() % 16 or E > 8192 or F_ > 8192 \
+            or (H + 2 * Hk) * (E // H) > 8192 or _block_bytes(0, *sizes) < 0 or x.device.index != torch.cuda.current_device():
+        return False
+    P = (H + 2 * Hk) * (E // H)
+    shapes = ((E,), (E,), (P, E), (P,), (E, E), (E,), (E,), (E,), (F_, E), (F_,), (E, F_), (E,))
+    grad = False
+    for p, s in zip(params, shapes):
+        if p is None:
+            if len(s) == 2:
+                return False
+        elif type(p) not in (torch.Tensor, torch.nn.Parameter) or p.shape != s or p.dtype is not torch.bfloat16 \
+                or p.device != x.device or not p.is_contiguous() or p.data_ptr() % 16:
+            return False
+        else:
+            grad = grad or p.requires_grad
+    if (grad or x.requires_grad) and torch.is_grad_enabled() and S % 128:
+        return False                        # the layers say what they miss
+    return not _observed() and os.environ.get("GF_FA_FWD", "3") == "3" and os.environ.get("GF_FA_BWD", "3") != "1"
