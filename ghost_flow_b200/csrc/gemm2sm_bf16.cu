@@ -18,7 +18,7 @@
 //
 // Plain GEMMs only (all four operand layouts, the epilogue options of the single-CTA kernel, e4m3 operands with row and
 // column scales); the fused roles
-// (all-gather, reduce-scatter, grouped, split-K, implicit convolution) stay in gemm_bf16.cu.
+// (all-gather, reduce-scatter, grouped, implicit convolution) stay in gemm_bf16.cu.
 // Replaces, like that file, ghostflow-cuda/src/optimized_kernels.cu:22-119 and ghostflow-cuda/src/blas.rs:278-313.
 #include "gf_host.h"
 #include "gf_ptx.cuh"
@@ -40,6 +40,8 @@ struct Gemm2Params {
   int tiles_m, tiles_n;     // 256 x BN tiles
   int band;                 // rows of tiles walked together (keeps one wave's A and B panels in L2)
   int act;                  // 0 none, 1 ReLU
+  // K in `slices` parts, each a product of its own into C (fp32) + slice * M * ldc
+  int slices;
   // e4m3 operands: C = sa[m] * sb[n] * A B^T + bias
   const float* sa;
   const float* sb;
@@ -54,6 +56,7 @@ constexpr int G2_BK = 64;
 // longer (4096 x 2048 x 256 21.1 -> 23.1 us, 11008 x 4096 over 256 rows 54 -> 57 us) and its long ones no less.
 constexpr int g2_threads(int epilogue_warps) { return 64 + 32 * epilogue_warps; }
 constexpr int G2_A_BYTES = G2_BM * G2_BK * 2;
+constexpr int G2_MAX_SLICES = 4;  // of K
 
 // BNH = rows of B (output columns) per CTA: 128 (256 x 256 tiles, seven stages) or 64 (256 x 128 tiles, nine
 // stages; twice as many tiles, for problems whose last wave of 256-wide tiles would leave most pairs idle).
@@ -171,7 +174,8 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int num_kb = (p.K + BKE - 1) / BKE;
-  const int num_tiles = p.tiles_m * p.tiles_n;
+  const int slice_tiles = p.tiles_m * p.tiles_n;
+  const int num_tiles = slice_tiles * p.slices;         // a tile of a slice is an item like any other
   const int pair = (int)blockIdx.x >> 1;
   const int npairs = (int)gridDim.x >> 1;
 
@@ -206,10 +210,12 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += npairs) {
         int tm, tn;
-        g2_tile_coords(p, tile, tm, tn);
+        const int slice = tile / slice_tiles;
+        g2_tile_coords(p, tile - slice * slice_tiles, tm, tn);
+        const int kb0 = (int)((long long)slice * num_kb / p.slices), kb1 = (int)((long long)(slice + 1) * num_kb / p.slices);
         const int m0 = tm * 2 * G2_BM + (int)rank * G2_BM;
         const int n0 = tn * G2_BN + (int)rank * G2_BNH;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
             if (p.status) atomicCAS(p.status, 0, GF_ERR_WAIT_EMPTY);
             ok = false;
@@ -259,7 +265,9 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * G2_BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int slice = tile / slice_tiles;
+        const int kbs = (int)((long long)(slice + 1) * num_kb / p.slices) - (int)((long long)slice * num_kb / p.slices);
+        for (int kb = 0; kb < kbs; ++kb) {
           if (!mbar_wait_warp(&full_bar[stage], phase)) {
             if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
             ok = false;
@@ -303,7 +311,8 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     int it = 0;
     for (int tile = pair; tile < num_tiles; tile += npairs) {
       int tm, tn;
-      g2_tile_coords(p, tile, tm, tn);
+      const int slice = tile / slice_tiles;
+      g2_tile_coords(p, tile - slice * slice_tiles, tm, tn);
       const int row = tm * 2 * G2_BM + (int)rank * G2_BM + lane_grp * 32 + lane;
       const int n0 = tn * G2_BN;
       const float row_scale = F8 ? (row < p.M ? p.sa[row] : 0.f) : p.alpha;
@@ -384,7 +393,7 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
           }
           if (p.out_fp32) {
-            float* cp = reinterpret_cast<float*>(p.C) + (long long)row * p.ldc + col0;
+            float* cp = reinterpret_cast<float*>(p.C) + ((long long)slice * p.M + row) * p.ldc + col0;
             if (full && ((p.ldc & 3) == 0)) {
 #pragma unroll
               for (int q = 0; q < 8; ++q) {
@@ -479,7 +488,7 @@ static int launch_gemm2_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm
   }
   p.tiles_m = (p.M + 2 * G2_BM - 1) / (2 * G2_BM);
   p.tiles_n = (p.N + G2_BN - 1) / G2_BN;
-  const int tiles = p.tiles_m * p.tiles_n;
+  const int tiles = p.tiles_m * p.tiles_n * p.slices;
   int pairs = max_pairs < tiles ? max_pairs : tiles;
   if (pairs < 1) pairs = 1;
   p.band = p.tiles_m > 8 ? 8 : p.tiles_m;
@@ -523,9 +532,94 @@ static int g2_pick_bn(int M, int N) {
   return N <= 128 ? 128 : 256;
 }
 
+// Parts of K for a product with too few 256 x 256 tiles for the pairs, such as the weight gradient of a narrow layer over many
+// tokens; 0 where it is not split here. The parts are stored as fp32 and added by gemm2sm_add_slices_kernel, in their order, so the
+// result does not depend on the schedule. The number with the least estimated time: 0.41 us for a pair's 256 x 256 x 64 block
+// (1.5 PFLOP/s on the machine), 0.44 for a CTA's 128 x 256 x 64, the sums written and read at 8 TB/s, 4 us for the second kernel.
+// Device time in us, with slices that are added into one buffer (cleared before, converted after) or as whole tiles of a CTA / here:
+// [2304, 768] over 8192 rows 41.0 / 38.2, [3072, 768] 45.7 / 41.0, [768, 3072] 45.5 / 39.9, [1024, 1024] 27.5 / 24.7, [3072, 1024]
+// 51.6 / 48.9, [1600, 1600] 51.6 / 46.7, [4096, 512] over 4096 31.1 / 25.6, [512, 4096] over 4096 30.1 / 27.3, [256, 4096] over 11008
+// 34.7 / 33.8. With fewer than 16 tiles, which take more than four parts, the sums cost more than they save: [768, 768] over 8192
+// 21.8 / 23.9, [1024, 768] over 3072 19.8 / 21.5.
+int gemm2sm_slices(int M, int N, int K) {
+  if (M < 256 || N < 256 || K < 2048 || gemm2sm_wanted(M, N, K) || getenv("GF_GEMM_2SM")) return 0;
+  const int pairs = sm_count() / 2, kb = (K + G2_BK - 1) / G2_BK;
+  const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256), ctas = (long long)((M + 127) / 128) * ((N + 255) / 256);
+  if (tiles < 16) return 0;
+  const double add = (double)M * N * 8 / 8e6;
+  double best = 0.;
+  int slices = 0;
+  for (int s = 2; s <= G2_MAX_SLICES && s * 512 <= K; ++s) {
+    const double t = (double)((tiles * s + pairs - 1) / pairs) * ((kb + s - 1) / s) * 0.41 + s * add + 4.;
+    if (!slices || t < best) { best = t; slices = s; }
+  }
+  const double whole = (double)((ctas + 2 * pairs - 1) / (2 * pairs)) * kb * 0.44;
+  return slices && best < 0.9 * whole ? slices : 0;
+}
+
+__global__ void __launch_bounds__(256)
+gemm2sm_add_slices_kernel(const float* __restrict__ ws, int slices, __nv_bfloat16* __restrict__ C, long long ldc,
+                          const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ residual, long long ldr, int M,
+                          int N, int quads) {
+  const int per_row = quads ? N / 4 : N;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x, stride = (long long)M * N;
+  if (i >= (long long)M * per_row) return;
+  const int r = (int)(i / per_row), c = (int)(i - (long long)r * per_row) * (quads ? 4 : 1);
+  const float* src = ws + (long long)r * N + c;
+  if (quads) {
+    float4 v[G2_MAX_SLICES];
+#pragma unroll
+    for (int s = 0; s < G2_MAX_SLICES; ++s)
+      if (s < slices) v[s] = *reinterpret_cast<const float4*>(src + s * stride);
+    float4 a = v[0];
+#pragma unroll
+    for (int s = 1; s < G2_MAX_SLICES; ++s)
+      if (s < slices) { a.x += v[s].x; a.y += v[s].y; a.z += v[s].z; a.w += v[s].w; }
+    float o[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (bias) o[e] += __bfloat162float(bias[c + e]);
+      if (residual) o[e] += __bfloat162float(residual[(long long)r * ldr + c + e]);
+    }
+    *reinterpret_cast<uint2*>(C + (long long)r * ldc + c) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+  } else {
+    float a = 0.f;
+    for (int s = 0; s < slices; ++s) a += src[s * stride];
+    if (bias) a += __bfloat162float(bias[c]);
+    if (residual) a += __bfloat162float(residual[(long long)r * ldr + c]);
+    C[(long long)r * ldc + c] = __float2bfloat16(a);
+  }
+}
+
+int gemm2sm_run_parts(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
+                      long long ldb, long long ldc, int out_fp32, int accumulate, const void* bias, const void* residual,
+                      long long ldr, float alpha, int* status, int activation, int slices, cudaStream_t stream);
+
+// slices from gemm2sm_slices; ws: slices * M * N fp32 on a 16-byte boundary.
+int gemm2sm_run_sliced(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
+                       long long ldb, long long ldc, const void* bias, const void* residual, long long ldr, float alpha, int slices,
+                       float* ws, int* status, cudaStream_t stream) {
+  const int rc = gemm2sm_run_parts(A, B, ws, M, N, K, a_mn_major, lda, b_mn_major, ldb, N, 1, 0, nullptr, nullptr, 0, alpha, status, 0,
+                                   slices, stream);
+  if (rc) return rc;
+  const int quads = N % 4 == 0 && ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0 && (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
+  const long long n = (long long)M * (quads ? N / 4 : N);
+  gemm2sm_add_slices_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
+      ws, slices, (__nv_bfloat16*)C, ldc, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, ldr, M, N, quads);
+  note_extra_launches(1);
+  return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;
+}
+
 int gemm2sm_run(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda,
                 int b_mn_major, long long ldb, long long ldc, int out_fp32, int accumulate, const void* bias,
                 const void* residual, long long ldr, float alpha, int* status, int activation, cudaStream_t stream) {
+  return gemm2sm_run_parts(A, B, C, M, N, K, a_mn_major, lda, b_mn_major, ldb, ldc, out_fp32, accumulate, bias, residual, ldr, alpha,
+                           status, activation, 1, stream);
+}
+
+int gemm2sm_run_parts(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
+                      long long ldb, long long ldc, int out_fp32, int accumulate, const void* bias, const void* residual,
+                      long long ldr, float alpha, int* status, int activation, int slices, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return GFH_BAD_ARG;
   const int bn = g2_pick_bn(M, N);
   CUtensorMap tmA, tmB;
@@ -541,7 +635,7 @@ int gemm2sm_run(const void* A, const void* B, void* C, int M, int N, int K, int 
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   p.ldr = ldr; p.alpha = alpha; p.status = status; p.act = activation == 1 ? 1 : 0;
-  p.sa = p.sb = nullptr;
+  p.sa = p.sb = nullptr; p.slices = slices;
 #define GF_G2_DISPATCH(BNH_)                                                                        \
   if (!a_mn_major && !b_mn_major) return launch_gemm2<BNH_, false, false>(tmA, tmB, p, stream);     \
   if (!a_mn_major && b_mn_major) return launch_gemm2<BNH_, false, true>(tmA, tmB, p, stream);       \
@@ -563,7 +657,7 @@ int gemm2sm_run_fp8(const void* A, const void* B, void* C, int M, int N, int K, 
   Gemm2Params p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_fp32 = 0; p.accumulate = 0;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
-  p.residual = nullptr; p.ldr = 0; p.alpha = 1.f; p.status = status; p.act = 0; p.sa = sa; p.sb = sb;
+  p.residual = nullptr; p.ldr = 0; p.alpha = 1.f; p.status = status; p.act = 0; p.sa = sa; p.sb = sb; p.slices = 1;
   return launch_gemm2<128, false, false, true>(tmA, tmB, p, stream);
 }
 

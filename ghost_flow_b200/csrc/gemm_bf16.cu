@@ -926,6 +926,10 @@ int gemm_skinny_run(const void* A, const void* W, void* C, int M, int N, int K, 
                     cudaStream_t st);
 // CTA-pair kernel for plain GEMMs (gemm2sm_bf16.cu)
 int gemm2sm_wanted(int M, int N, int K);
+int gemm2sm_slices(int M, int N, int K);
+int gemm2sm_run_sliced(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
+                       long long ldb, long long ldc, const void* bias, const void* residual, long long ldr, float alpha, int slices,
+                       float* ws, int* status, cudaStream_t stream);
 int gemm2sm_run(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda,
                 int b_mn_major, long long ldb, long long ldc, int out_fp32, int accumulate, const void* bias,
                 const void* residual, long long ldr, float alpha, int* status, int activation, cudaStream_t stream);
@@ -979,6 +983,15 @@ GF_API int gf_gemm_bf16_few_rows(int M, int N, int K, int a_mn_major, int b_mn_m
          gf::gemm_rows_takes(nullptr, aligned ? 8 : 1, nullptr, aligned ? 8 : 1, M, N, K);
 }
 
+// fp32 values that gf_gemm_bf16 (bn_hint and max_ctas 0) takes as workspace: none, or the sums of the parts of K.
+GF_API int gf_gemm_bf16_splits(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate, int activation);
+GF_API long long gf_gemm_bf16_workspace(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int out_fp32, int accumulate,
+                                        int activation) {
+  if (out_fp32 || accumulate || activation || gf_gemm_bf16_few_rows(M, N, K, a_mn_major, b_mn_major, aligned, accumulate)) return 0;
+  if (const int s = gf::gemm2sm_slices(M, N, K)) return (long long)s * M * N;
+  return gf_gemm_bf16_splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, activation) ? (long long)M * N : 0;
+}
+
 // For products that gf_gemm_bf16_few_rows does not name: 1 when gf_gemm_bf16 (bf16 result, bn_hint and max_ctas 0) takes a workspace of M * N fp32 values, else 0. aligned: bases and
 // pitches of A and B are multiples of 16 bytes.
 GF_API int gf_gemm_bf16_splits(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate, int activation) {
@@ -1009,6 +1022,13 @@ GF_API int gf_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int
   if (bn_hint == 0 && max_ctas == 0 &&
       gf::gemm_skinny_wanted(A, B, M, N, K, a_mn_major, lda, b_mn_major, ldb, accumulate, split))
     return gf::gemm_skinny_run(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, bias, residual, ldr, alpha, p.act, st);
+  // few tiles and many rows to contract, with a workspace for the sums of every part of K
+  if (bn_hint == 0 && max_ctas == 0 && !out_fp32 && !accumulate && p.act == 0 && splitk_ws) {
+    const int s = gf::gemm2sm_slices(M, N, K);
+    if (s && splitk_ws_floats / s / N >= M)
+      return gf::gemm2sm_run_sliced(A, B, C, M, N, K, a_mn_major, lda, b_mn_major, ldb, ldc, bias, residual, ldr, alpha, s,
+                                    reinterpret_cast<float*>(const_cast<int*>(splitk_ws)), status, st);
+  }
   // The slices add into an fp32 workspace that a second kernel converts. The workspace is the caller's (splitk_ws,
   // splitk_ws_floats >= M * N: a buffer that belongs to the calling stream, e.g. from a stream-ordered allocator) or,
   // without one, a buffer this library keeps per device, which only one stream at a time may use.

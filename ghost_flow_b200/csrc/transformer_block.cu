@@ -18,8 +18,8 @@ GF_API int gf_norm_bwd_grid(int T);
 GF_API int gf_colsum_bf16(const void* x, long long ld, void* out, float* scratch, int T, int D, int accumulate, void* stream);
 GF_API int gf_unary_fwd(const void* x, void* y, long long n, int op, int dtype, void* stream);
 GF_API int gf_unary_bwd_bf16(const void* x, const void* dy, void* dx, long long n, int op, void* stream);
-GF_API int gf_gemm_bf16_few_rows(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate);
-GF_API int gf_gemm_bf16_splits(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate, int activation);
+GF_API long long gf_gemm_bf16_workspace(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int out_fp32, int accumulate,
+                                        int activation);
 GF_API int gf_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
                         long long ldb, long long ldc, int out_fp32, int accumulate, const void* bias, const void* residual,
                         long long ldr, float alpha, int* status, int bn_hint, int max_ctas, const int* splitk_ws, int activation,
@@ -88,10 +88,7 @@ int widest(const Block& b) { return b.P > b.F ? b.P : b.F; }
 
 // fp32 values a product takes as workspace
 long long product_floats(int M, int N, int K, int a_mn_major, int b_mn_major) {
-  return !gf_gemm_bf16_few_rows(M, N, K, a_mn_major, b_mn_major, 1, 0) &&
-                 gf_gemm_bf16_splits(M, N, K, a_mn_major, b_mn_major, 1, 0, 0)
-             ? (long long)M * N
-             : 0;
+  return gf_gemm_bf16_workspace(M, N, K, a_mn_major, b_mn_major, 1, 0, 0, 0);
 }
 // The most that any of the block's products y = x W^T takes (pass 0), or of their gradients (pass 1).
 long long most_floats(const Block& b, int pass) {

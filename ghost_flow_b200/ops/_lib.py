@@ -31,6 +31,7 @@ _SIGS = {
     "gf_selected_device": [],
     "gf_gemm_bf16_splits": [I, I, I, I, I, I, I, I],
     "gf_gemm_bf16_few_rows": [I, I, I, I, I, I, I],
+    "gf_gemm_bf16_workspace": [I, I, I, I, I, I, I, I, I],
     "gf_gemm_bf16": [P, P, P, I, I, I, I, L, I, L, L, I, I, P, P, L, F, P, I, I, P, I, I, P],
     "gf_norm_bwd_grid": [I],
     "gf_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
@@ -84,7 +85,7 @@ def _bind(lib, sigs):
         except AttributeError:
             continue
         fn.argtypes = args
-        fn.restype = c_longlong if name == "gf_gpt_block_bytes" else c_int
+        fn.restype = c_longlong if name in ("gf_gpt_block_bytes", "gf_gemm_bf16_workspace") else c_int
     return lib
 
 

@@ -38,10 +38,9 @@ def _splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu) -> bool:
 
 
 @functools.lru_cache(maxsize=4096)
-def _needs_workspace(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu) -> bool:
-    """Whether the product takes an fp32 ``[M, N]`` workspace: it splits K, and not inside the few-row kernel."""
-    return not _lib.cuda_lib().gf_gemm_bf16_few_rows(M, N, K, a_mn_major, b_mn_major, aligned, accumulate) \
-        and _splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu)
+def _workspace(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, relu) -> int:
+    """fp32 values that the product takes as workspace: the sums of the parts of K, where the kernel library splits it."""
+    return _lib.cuda_lib().gf_gemm_bf16_workspace(M, N, K, a_mn_major, b_mn_major, aligned, 0, accumulate, relu)
 
 
 def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bfloat16, bias=None, residual=None,
@@ -68,14 +67,15 @@ def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bf
     lib = _lib.cuda_lib()
     device = a.device
     f32_out = out.dtype is torch.float32
-    # few output tiles and a long K: the kernel splits K and needs an fp32 [M, N] workspace. It comes from torch's
+    # few output tiles and a long K: the kernel splits K and needs an fp32 workspace. It comes from torch's
     # allocator, so it belongs to the current stream (and to the graph's pool while a CUDA graph is recorded).
-    ws = None
+    ws, floats = None, 0
     pa, pb = a.data_ptr(), b.data_ptr()
-    if K >= 2048 and not f32_out and bn_hint == 0 and max_ctas == 0 \
-            and _needs_workspace(M, N, K, bool(a_mn_major), bool(b_mn_major), not (pa | pb | 2 * sa[0] | 2 * sb[0]) & 15,
-                                 bool(accumulate), bool(relu)):
-        ws = torch.empty(M * N, dtype=torch.float32, device=device)
+    if K >= 2048 and not f32_out and bn_hint == 0 and max_ctas == 0:
+        floats = _workspace(M, N, K, bool(a_mn_major), bool(b_mn_major), not (pa | pb | 2 * sa[0] | 2 * sb[0]) & 15,
+                            bool(accumulate), bool(relu))
+        if floats:
+            ws = torch.empty(floats, dtype=torch.float32, device=device)
     rc = lib.gf_gemm_bf16(
         pa, pb, out.data_ptr(), M, N, K,
         1 if a_mn_major else 0, sa[0], 1 if b_mn_major else 0, sb[0], out.stride(0),
@@ -84,7 +84,7 @@ def gemm_raw(a, a_mn_major, b, b_mn_major, M, N, K, out=None, out_dtype=torch.bf
         None if residual is None else residual.data_ptr(),
         0 if residual is None else residual.stride(0),
         float(alpha), _lib.status_word(device).data_ptr(), bn_hint, max_ctas,
-        None if ws is None else ws.data_ptr(), 1 if relu else 0, 0 if ws is None else M * N,
+        None if ws is None else ws.data_ptr(), 1 if relu else 0, floats,
         _lib.stream_ptr(),
     )
     _lib.check_rc(rc, "gf_gemm_bf16")
