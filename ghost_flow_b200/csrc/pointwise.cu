@@ -174,57 +174,75 @@ embedding_rows_kernel(const I* __restrict__ ids, const uint4* __restrict__ table
 
 // ------------------------------------------------------------------ SwiGLU
 // gu is [T, 2F] (gate columns [0,F), up columns [F,2F)); y = silu(g) * u is [T, F].
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, long long T,
-                                  int F) {
-  const int vpr = F >> 3;
-  const long long total = T * vpr;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long t = idx / vpr;
-    const int v = (int)(idx % vpr);
-    const __nv_bfloat16* g = gu + t * 2 * F + v * 8;
-    uint4 ug = *reinterpret_cast<const uint4*>(g);
-    uint4 uu = *reinterpret_cast<const uint4*>(g + F);
-    const uint32_t* pg = reinterpret_cast<const uint32_t*>(&ug);
-    const uint32_t* pu = reinterpret_cast<const uint32_t*>(&uu);
+// Bound by memory: a thread has EW_BATCH vectors of each operand, 256 vectors apart, and issues their loads before it uses the first.
+// Index is a 32-bit type where the sizes allow it: the division by the row length was a 64-bit one for every vector.
+// [2048, 2 x 11008] forward 32 -> 26 us (5.2 TB/s), backward 40.5 -> 38.5 (5.9 TB/s).
+constexpr int EW_BATCH = 2;
+template <typename Index>
+__global__ void __launch_bounds__(256)
+swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, Index total, int F) {
+  const Index vpr = F >> 3, i0 = (Index)blockIdx.x * (256 * EW_BATCH) + threadIdx.x;
+  uint4 ug[EW_BATCH], uu[EW_BATCH];
+  long long at[EW_BATCH];
+#pragma unroll
+  for (int k = 0; k < EW_BATCH; ++k) {
+    const Index i = i0 + k * 256;
+    if (i >= total) break;
+    const Index t = i / vpr, v = i - t * vpr;
+    at[k] = (long long)t * F + (long long)v * 8;
+    const __nv_bfloat16* g = gu + at[k] + (long long)t * F;
+    ug[k] = *reinterpret_cast<const uint4*>(g);
+    uu[k] = *reinterpret_cast<const uint4*>(g + F);
+  }
+#pragma unroll
+  for (int k = 0; k < EW_BATCH; ++k) {
+    if (i0 + k * 256 >= total) break;
+    const uint32_t *pg = reinterpret_cast<const uint32_t*>(&ug[k]), *pu = reinterpret_cast<const uint32_t*>(&uu[k]);
     uint4 o;
     uint32_t* po = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      float2 a = unpack_bf16x2(pg[q]), b = unpack_bf16x2(pu[q]);
+      const float2 a = unpack_bf16x2(pg[q]), b = unpack_bf16x2(pu[q]);
       po[q] = pack_bf16x2(a.x * sigmoidf_(a.x) * b.x, a.y * sigmoidf_(a.y) * b.y);
     }
-    *reinterpret_cast<uint4*>(y + t * F + v * 8) = o;
+    *reinterpret_cast<uint4*>(y + at[k]) = o;
   }
 }
 // dgu[T,2F]: dg = dy * u * (sig + g*sig*(1-sig)) ; du = dy * g * sig
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dy,
-                                  __nv_bfloat16* __restrict__ dgu, long long T, int F) {
-  const int vpr = F >> 3;
-  const long long total = T * vpr;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long t = idx / vpr;
-    const int v = (int)(idx % vpr);
-    const __nv_bfloat16* g = gu + t * 2 * F + v * 8;
-    uint4 ug = *reinterpret_cast<const uint4*>(g);
-    uint4 uu = *reinterpret_cast<const uint4*>(g + F);
-    uint4 ud = *reinterpret_cast<const uint4*>(dy + t * F + v * 8);
-    const uint32_t* pg = reinterpret_cast<const uint32_t*>(&ug);
-    const uint32_t* pu = reinterpret_cast<const uint32_t*>(&uu);
-    const uint32_t* pd = reinterpret_cast<const uint32_t*>(&ud);
+template <typename Index>
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dgu,
+                  Index total, int F) {
+  const Index vpr = F >> 3, i0 = (Index)blockIdx.x * (256 * EW_BATCH) + threadIdx.x;
+  uint4 ug[EW_BATCH], uu[EW_BATCH], ud[EW_BATCH];
+  long long at[EW_BATCH];
+#pragma unroll
+  for (int k = 0; k < EW_BATCH; ++k) {
+    const Index i = i0 + k * 256;
+    if (i >= total) break;
+    const Index t = i / vpr, v = i - t * vpr;
+    const long long row = (long long)t * F;
+    at[k] = 2 * row + (long long)v * 8;
+    ug[k] = *reinterpret_cast<const uint4*>(gu + at[k]);
+    uu[k] = *reinterpret_cast<const uint4*>(gu + at[k] + F);
+    ud[k] = *reinterpret_cast<const uint4*>(dy + row + (long long)v * 8);
+  }
+#pragma unroll
+  for (int k = 0; k < EW_BATCH; ++k) {
+    if (i0 + k * 256 >= total) break;
+    const uint32_t *pg = reinterpret_cast<const uint32_t*>(&ug[k]), *pu = reinterpret_cast<const uint32_t*>(&uu[k]),
+                   *pd = reinterpret_cast<const uint32_t*>(&ud[k]);
     uint4 og, ou;
-    uint32_t* pog = reinterpret_cast<uint32_t*>(&og);
-    uint32_t* pou = reinterpret_cast<uint32_t*>(&ou);
+    uint32_t *pog = reinterpret_cast<uint32_t*>(&og), *pou = reinterpret_cast<uint32_t*>(&ou);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      float2 a = unpack_bf16x2(pg[q]), b = unpack_bf16x2(pu[q]), d = unpack_bf16x2(pd[q]);
+      const float2 a = unpack_bf16x2(pg[q]), b = unpack_bf16x2(pu[q]), d = unpack_bf16x2(pd[q]);
       const float s0 = sigmoidf_(a.x), s1 = sigmoidf_(a.y);
       pog[q] = pack_bf16x2(d.x * b.x * (s0 + a.x * s0 * (1.f - s0)), d.y * b.y * (s1 + a.y * s1 * (1.f - s1)));
       pou[q] = pack_bf16x2(d.x * a.x * s0, d.y * a.y * s1);
     }
-    *reinterpret_cast<uint4*>(dgu + t * 2 * F + v * 8) = og;
-    *reinterpret_cast<uint4*>(dgu + t * 2 * F + F + v * 8) = ou;
+    *reinterpret_cast<uint4*>(dgu + at[k]) = og;
+    *reinterpret_cast<uint4*>(dgu + at[k] + F) = ou;
   }
 }
 
@@ -279,35 +297,66 @@ __global__ void chain_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, lon
     stf(y, i, v);
   }
 }
-__global__ void unary_fwd_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
-                                        long long nvec, int op) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-       i += (long long)gridDim.x * blockDim.x) {
-    uint4 u = reinterpret_cast<const uint4*>(x)[i];
-    uint32_t* p = reinterpret_cast<uint32_t*>(&u);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float2 a = unpack_bf16x2(p[q]);
-      p[q] = pack_bf16x2(apply_op(op, a.x), apply_op(op, a.y));
-    }
-    reinterpret_cast<uint4*>(y)[i] = u;
+// bf16 in and out. GELU as x sigmoid(2 u), the same function as x (1 + tanh u) / 2: 1 + tanh u loses its digits where the
+// result is small, and tanhf is the longer code. [8192, 3072] forward 24.0 -> 22.2 us, backward 32.5 -> 31.0.
+template <int OP>
+__device__ __forceinline__ float op_bf16(float x) {
+  if constexpr (OP == OP_GELU) return x * sigmoidf_(2.f * 0.7978845608028654f * (x + 0.044715f * x * x * x));
+  else return apply_op(OP, x);
+}
+template <int OP>
+__device__ __forceinline__ float op_grad_bf16(float x) {
+  if constexpr (OP == OP_GELU) {
+    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+    const float s = sigmoidf_(2.f * k0 * (x + k1 * x * x * x));
+    return s + x * s * (1.f - s) * (2.f * k0 * (1.f + 3.f * k1 * x * x));
+  } else {
+    return apply_op_grad(OP, x);
   }
 }
-// dx = dy * f'(x)
-__global__ void unary_bwd_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                                        __nv_bfloat16* __restrict__ dx, long long nvec, int op) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-       i += (long long)gridDim.x * blockDim.x) {
-    uint4 u = reinterpret_cast<const uint4*>(x)[i];
-    uint4 d = reinterpret_cast<const uint4*>(dy)[i];
-    uint32_t* p = reinterpret_cast<uint32_t*>(&u);
-    uint32_t* pd = reinterpret_cast<uint32_t*>(&d);
+constexpr int UNARY_BATCH = 4;      // vectors of a thread, 256 apart, loaded before the first is used
+template <int OP>
+__global__ void __launch_bounds__(256)
+unary_fwd_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long nvec) {
+  const long long i0 = (long long)blockIdx.x * (256 * UNARY_BATCH) + threadIdx.x;
+  uint4 u[UNARY_BATCH];
+#pragma unroll
+  for (int k = 0; k < UNARY_BATCH; ++k)
+    if (i0 + k * 256 < nvec) u[k] = reinterpret_cast<const uint4*>(x)[i0 + k * 256];
+#pragma unroll
+  for (int k = 0; k < UNARY_BATCH; ++k) {
+    if (i0 + k * 256 >= nvec) break;
+    uint32_t* p = reinterpret_cast<uint32_t*>(&u[k]);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      float2 a = unpack_bf16x2(p[q]), g = unpack_bf16x2(pd[q]);
-      p[q] = pack_bf16x2(g.x * apply_op_grad(op, a.x), g.y * apply_op_grad(op, a.y));
+      const float2 a = unpack_bf16x2(p[q]);
+      p[q] = pack_bf16x2(op_bf16<OP>(a.x), op_bf16<OP>(a.y));
     }
-    reinterpret_cast<uint4*>(dx)[i] = u;
+    reinterpret_cast<uint4*>(y)[i0 + k * 256] = u[k];
+  }
+}
+// dx = dy * f'(x); dx may be dy or x
+template <int OP>
+__global__ void __launch_bounds__(256)
+unary_bwd_bf16x8_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bfloat16* dx, long long nvec) {
+  const long long i0 = (long long)blockIdx.x * (256 * UNARY_BATCH) + threadIdx.x;
+  uint4 u[UNARY_BATCH], d[UNARY_BATCH];
+#pragma unroll
+  for (int k = 0; k < UNARY_BATCH; ++k)
+    if (i0 + k * 256 < nvec) {
+      u[k] = reinterpret_cast<const uint4*>(x)[i0 + k * 256];
+      d[k] = reinterpret_cast<const uint4*>(dy)[i0 + k * 256];
+    }
+#pragma unroll
+  for (int k = 0; k < UNARY_BATCH; ++k) {
+    if (i0 + k * 256 >= nvec) break;
+    uint32_t *p = reinterpret_cast<uint32_t*>(&u[k]), *pd = reinterpret_cast<uint32_t*>(&d[k]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 a = unpack_bf16x2(p[q]), g = unpack_bf16x2(pd[q]);
+      p[q] = pack_bf16x2(g.x * op_grad_bf16<OP>(a.x), g.y * op_grad_bf16<OP>(a.y));
+    }
+    reinterpret_cast<uint4*>(dx)[i0 + k * 256] = u[k];
   }
 }
 template <typename T>
@@ -618,23 +667,43 @@ GF_API int gf_scale_by_dev_scalar(void* x, long long n, const float* scalar, voi
 GF_API int gf_swiglu_fwd(const void* gu, void* y, long long T, int F, void* stream) {
   gf::enter();
   if (F % 8) return GFH_BAD_ARG;
-  swiglu_fwd_kernel<<<ew_grid(T * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu,
-                                                                                (__nv_bfloat16*)y, T, F);
+  const long long n = T * (F / 8), blocks = (n + 256 * EW_BATCH - 1) / (256 * EW_BATCH);
+  if (n <= 0) return GFH_OK;
+  if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
+  if (n < 0x7fffffffll)
+    swiglu_fwd_kernel<unsigned><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)y,
+                                                                                  (unsigned)n, F);
+  else
+    swiglu_fwd_kernel<long long><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)y, n,
+                                                                                   F);
   GF_RET();
 }
 GF_API int gf_swiglu_bwd(const void* gu, const void* dy, void* dgu, long long T, int F, void* stream) {
   gf::enter();
   if (F % 8) return GFH_BAD_ARG;
-  swiglu_bwd_kernel<<<ew_grid(T * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dgu, T, F);
+  const long long n = T * (F / 8), blocks = (n + 256 * EW_BATCH - 1) / (256 * EW_BATCH);
+  if (n <= 0) return GFH_OK;
+  if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
+  if (n < 0x7fffffffll)
+    swiglu_bwd_kernel<unsigned><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dgu, (unsigned)n, F);
+  else
+    swiglu_bwd_kernel<long long><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dgu, n, F);
   GF_RET();
 }
 // dtype: 0 = fp32, 1 = bf16
 GF_API int gf_unary_fwd(const void* x, void* y, long long n, int op, int dtype, void* stream) {
   gf::enter();
   if (dtype == 1 && n % 8 == 0 && ((uintptr_t)x % 16 == 0) && ((uintptr_t)y % 16 == 0)) {
-    unary_fwd_bf16x8_kernel<<<ew_grid(n / 8, 256), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)x, (__nv_bfloat16*)y, n / 8, op);
+    const long long blocks = (n / 8 + 256 * UNARY_BATCH - 1) / (256 * UNARY_BATCH);
+    if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
+    if (n > 0) {
+      auto kern = op == OP_RELU ? unary_fwd_bf16x8_kernel<OP_RELU> : op == OP_GELU ? unary_fwd_bf16x8_kernel<OP_GELU>
+                  : op == OP_SIGMOID ? unary_fwd_bf16x8_kernel<OP_SIGMOID> : op == OP_TANH ? unary_fwd_bf16x8_kernel<OP_TANH>
+                                                                                            : unary_fwd_bf16x8_kernel<OP_SILU>;
+      kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, n / 8);
+    }
   } else {
     OpChain c;
     c.n = 1;
@@ -653,8 +722,14 @@ GF_API int gf_unary_fwd(const void* x, void* y, long long n, int op, int dtype, 
 GF_API int gf_unary_bwd_bf16(const void* x, const void* dy, void* dx, long long n, int op, void* stream) {
   gf::enter();
   if (n % 8) return GFH_BAD_ARG;
-  unary_bwd_bf16x8_kernel<<<ew_grid(n / 8, 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, n / 8, op);
+  const long long blocks = (n / 8 + 256 * UNARY_BATCH - 1) / (256 * UNARY_BATCH);
+  if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
+  if (n <= 0) return GFH_OK;
+  auto kern = op == OP_RELU ? unary_bwd_bf16x8_kernel<OP_RELU> : op == OP_GELU ? unary_bwd_bf16x8_kernel<OP_GELU>
+              : op == OP_SIGMOID ? unary_bwd_bf16x8_kernel<OP_SIGMOID> : op == OP_TANH ? unary_bwd_bf16x8_kernel<OP_TANH>
+                                                                                        : unary_bwd_bf16x8_kernel<OP_SILU>;
+  kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx,
+                                                          n / 8);
   GF_RET();
 }
 GF_API int gf_op_chain(const void* x, void* y, long long n, const int* ops, int nops, int dtype, void* stream) {
