@@ -12,7 +12,7 @@
 // kernel that has waited may read the results of all earlier ones.
 //
 // One layer of LLaMA-7B (hidden 4096, inner 11008, 32 heads, 1500 keys), device time in a graph, nine ordinary launches -> now: one sequence
-// 101 -> 101 us, 8 142 -> 121, 16 185 -> 154, 32 (800 keys) 208 -> 168, 64 (500 keys) 228 -> 199; enqueueing it takes the host 80 us
+// 101 -> 96 us, 8 142 -> 116, 16 185 -> 149, 32 (800 keys) 208 -> 168, 64 (500 keys) 228 -> 199; enqueueing it takes the host 80 us
 // instead of 260. What is left above the bytes (93 us at 8): each kernel ends before the next one's tokens can be read, and the
 // memory waits for about 4 us then.
 #include <math.h>

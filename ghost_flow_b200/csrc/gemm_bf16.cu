@@ -966,13 +966,15 @@ static int splitk_slices(int M, int N, int K, int out_fp32, int accumulate, int 
 
 // Few-row products on gemm_rows.cu rather than gemm_skinny.cu (at most 16 rows) or the kernels with 128-row tiles. Its fixed cost is
 // about 2 us more than the first one's, which loads weights into registers and holds less of them in flight; it does not clear
-// and convert a workspace as the split product does. us there / here, back to back with cold weights ([M, K] x [N, K]^T, M N K):
-//   8 512 8192 17.7 / 10.5, 8 2048 5504 12.6 / 10.7, 8 4096 11008 22.5 / 20.8, 8 4096 4096 12.4 / 12.6, 8 8192 14336 40.2 / 41.3,
-//   8 22016 4096 32.9 / 36.8; 16 1024 512 5.4 / 7.7, 16 2048 2048 8.4 / 8.5, 16 11008 2048 16.6 / 14.6, 16 4096 11008 28.6 / 20.9,
-//   16 22016 4096 41.5 / 38.3; 32 512 256 10.5 / 8.9, 32 4096 4096 20.2 / 12.9, 32 32000 4096 55.9 / 52.5; 64 512 256 10.6 / 12.6,
-//   64 2048 2048 18.5 / 10.5, 64 12288 4096 35.1 / 29.3, 64 28672 4096 56.1 / 56.9, 64 32000 4096 57.6 / 60.0.
+// and convert a workspace as the split product does. Device time in us with cold weights, there / here ([M, K] x [N, K]^T, M N K):
+//   8 512 8192 12.9 / 9.3, 8 2048 5504 11.3 / 9.7, 8 4096 11008 21.0 / 19.5, 8 4096 4096 10.5 / 10.2, 8 6144 4096 12.0 / 12.5,
+//   8 12288 4096 23.3 / 20.7, 8 15360 5120 31.4 / 28.7, 8 8192 14336 38.2 / 39.9, 8 22016 4096 32.3 / 32.1, 8 28672 4096 41.9 / 43.5, 8
+//   11008 2048 10.6 / 11.8; 16 1024 512 2.8 / 5.5, 16 2048 2048 6.2 / 6.7, 16 11008 2048 15.1 / 11.9, 16 4096 4096 11.7 / 10.5, 16 4096
+//   11008 24.0 / 19.7, 16 22016 4096 40.9 / 33.2. Back to back from the host: 32 512 256 10.5 / 8.9, 32 4096 4096 20.2 / 12.9, 32
+//   32000 4096 55.9 / 52.5; 64 512 256 10.6 / 12.6, 64 2048 2048 18.5 / 10.5, 64 12288 4096 35.1 / 29.3, 64 28672 4096 56.1 / 56.9,
+//   64 32000 4096 57.6 / 60.0.
 static bool few_rows_wanted(int M, int N, int K) {
-  if (M <= 8) return K >= 5120 && N <= 6144;
+  if (M <= 8) return (K >= 4096 && (N <= 4096 || (N > 8192 && N <= 16384))) || (K >= 5120 && N <= 6144);
   if (M <= 16) return K >= 4096 || (K >= 2048 && N > 4096);
   return M <= 32 || (M <= gf::ROWS_MAX_M && N <= 24576 && K >= 512);
 }

@@ -2,8 +2,8 @@
 // M <= 64.
 //
 // The weight is read once and is all that counts, so it is the 128-row operand: tcgen05.mma with 128 output features as the
-// rows and 16, 32 or 64 tokens as the columns. TMA fills a ring of 128 x 64 weight blocks, about 100 KB to a CTA and two CTAs to
-// an SM, and needs no registers for what is in flight. K is split over the CTAs of a cluster; they add their sums through
+// rows and 16, 32 or 64 tokens as the columns. TMA fills a ring of 128 x 64 weight blocks, about 200 KB on an SM for its two or three
+// CTAs, and needs no registers for what is in flight. K is split over the CTAs of a cluster; they add their sums through
 // distributed shared memory in the order of their ranks, so there is no workspace to clear, no atomic and no second kernel.
 //
 // The tokens' side of a block comes by TMA too, or (at most 16 rows) four warps compute it, so that the operation in front of the
@@ -13,6 +13,13 @@
 //
 // In a chain of launches the weight blocks are on their way before the kernel in front has finished (griddepcontrol): they
 // are nobody's output there. X, the residual and C are touched behind griddepcontrol.wait only.
+//
+// What bounds it: memory, behind a fixed cost of about 5 us (launch, TMEM, first block, cluster barriers). The rings hold up to 28 MB
+// in flight. Up to 16 tokens three smaller CTAs share an SM: more of them mean shorter parts of K and a better fit to the machine (a
+// layer of 8 sequences, hidden 4096 / 5120: two CTAs of six stages 121 / 134 us, three of four 116 / 112; half as many CTAs 138 / 182).
+// Device time in us with cold weights, the kernels that took these products before -> this one: [16, 4096] x [12288, 4096]^T 27.0 ->
+// 20.8 (4.8 TB/s), x [22016, 4096]^T 40.9 -> 33.2 (5.4 TB/s), [16, 11008] x [4096, 11008]^T 24.0 -> 19.7; back to back from the host
+// [32, 4096] x [22016, 4096]^T 54.2 -> 41.9, [64, 4096] x [4096, 4096]^T 21.9 -> 14.7, [64, 14336] x [8192, 14336]^T 55.6 -> 45.8.
 #include "gemm_rows.cuh"
 #include "gf_host.h"
 #include "gf_ptx.cuh"
@@ -28,7 +35,8 @@ template <int NT>
 struct RwCfg {
   static constexpr int X_BYTES = NT * RW_BK * 2;
   static constexpr int STAGE_BYTES = RW_W_BYTES + X_BYTES;
-  static constexpr int STAGES = NT == 16 ? 6 : NT == 32 ? 5 : 4;      // two CTAs to an SM
+  static constexpr int STAGES = NT == 32 ? 5 : 4;
+  static constexpr int CTAS = NT == 16 ? 3 : 2;                       // on an SM
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 512;
   static constexpr int VPT = NT / 16;                                 // 16-byte vectors of a block for each of 128 threads
   static constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
@@ -74,7 +82,7 @@ __device__ __forceinline__ float ld_peer_f32(uint32_t cluster_addr) {
 __device__ __forceinline__ float silu_mul(float g, float u) { return g * (1.f / (1.f + __expf(-g))) * u; }
 
 template <int NT, int INPUT>
-__global__ void __launch_bounds__(RW_THREADS, 2)
+__global__ void __launch_bounds__(RW_THREADS, RwCfg<NT>::CTAS)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                  const __grid_constant__ RowsParams p) {
   using Cfg = RwCfg<NT>;
@@ -167,7 +175,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     asm volatile("griddepcontrol.wait;" ::: "memory");
     bool ok = true;
     if constexpr (INPUT != ROWS_PLAIN) {
-    constexpr int V = Cfg::VPT, B = 4 / V;               // B: blocks whose loads are issued together
+    constexpr int V = Cfg::VPT, B = 2;                   // B: blocks whose loads are issued together
     float sq[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) sq[v] = 0.f;
@@ -348,12 +356,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   }
 }
 
-// CTAs of a cluster, each with a part of K of at least four blocks: as many as fit on the machine at once, two to an SM, and a power
-// of two (clusters of 3, 6 or 7 leave SMs of a GPC out: 6144 features on 48 clusters of 6 took 22.4 us, on 48 of 4 14.7).
-static int rows_slices(int N, int K) {
+// CTAs of a cluster, each with a part of K of at least four blocks: as many as fit on the machine at once, and a power of two
+// (clusters of 3, 6 or 7 leave SMs of a GPC out: 6144 features on 48 clusters of 6 took 22.4 us, on 48 of 4 14.7).
+static int rows_slices(int M, int N, int K) {
   const int tiles = (N + RW_BM - 1) / RW_BM, blocks = (K + RW_BK - 1) / RW_BK;
+  const int slots = sm_count() * (M <= 16 ? RwCfg<16>::CTAS : RwCfg<64>::CTAS);
   int s = 8;
-  while (s > 1 && (s * tiles > 2 * sm_count() || 4 * s > blocks)) s >>= 1;
+  while (s > 1 && (s * tiles > slots || 4 * s > blocks)) s >>= 1;
   return s;
 }
 
@@ -405,7 +414,7 @@ int gemm_rows_run(const RowsGemm& g, int chained, cudaStream_t stream) {
                     (!g.residual || (g.ldr % 4 == 0 && reinterpret_cast<uintptr_t>(g.residual) % 8 == 0));
   RowsParams p{(const __nv_bfloat16*)g.X, g.ldx, g.C, g.ldc, g.out_fp32, g.M, g.N, g.K, (const __nv_bfloat16*)g.norm_w, g.eps,
                (const __nv_bfloat16*)g.bias, (const __nv_bfloat16*)g.residual, g.ldr, g.alpha, g.relu, quads, g.status};
-  const int slices = rows_slices(g.N, g.K);
+  const int slices = rows_slices(g.M, g.N, g.K);
   if (g.input == ROWS_RMSNORM) return launch_rows_nt<ROWS_RMSNORM>(tm, tm, p, slices, chained, stream);
   if (g.input == ROWS_SWIGLU) return launch_rows_nt<ROWS_SWIGLU>(tm, tm, p, slices, chained, stream);
   CUtensorMap tx;
