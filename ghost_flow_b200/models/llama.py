@@ -134,13 +134,16 @@ class LLaMAModel(Module):
             self._rope = ops.rope_tables(n, self.cfg.head_dim, self.cfg.rope_theta, device)
         return self._rope
 
-    def forward(self, ids, caches=None, start_pos: int = 0):
+    def _before_norm(self, ids, caches, start_pos):
         S = ids.shape[1]
         cos, sin = self.rope(start_pos + S, ids.device)
         x = self.embed_tokens(ids)
         for i, layer in enumerate(self.layers):
             x = layer(x, cos, sin, None if caches is None else caches[i], start_pos)
-        return self.norm(x)
+        return x
+
+    def forward(self, ids, caches=None, start_pos: int = 0):
+        return self.norm(self._before_norm(ids, caches, start_pos))
 
 
 class LLaMAForCausalLM(Module):
@@ -162,7 +165,32 @@ class LLaMAForCausalLM(Module):
         if self.cfg.tie_word_embeddings:
             self.lm_head.weight = self.model.embed_tokens.weight
 
+    def _norm_in_the_head(self, ids) -> bool:
+        """Whether the last norm can run inside the head's product: one token of at most 16 sequences, no gradient, modules that do
+        nothing but their own forward, dense bf16 weights on the current GPU, and nothing that follows the calls."""
+        model, head = self._modules["model"], self._modules["lm_head"]
+        if type(ids) is not torch.Tensor or not ids.is_cuda or ids.dim() != 2 or ids.shape[1] != 1 or not 0 < ids.shape[0] <= 16 \
+                or torch.is_grad_enabled() or type(model) is not LLaMAModel or type(head) is not Linear or head.bias is not None:
+            return False
+        norm, w = model._modules["norm"], head.weight
+        if type(norm) is not RMSNorm or not plain_modules(model, norm, head) or ids.device.index != torch.cuda.current_device():
+            return False
+        for p, s in ((norm.weight, (self.cfg.hidden_size,)), (w, (w.shape[0], self.cfg.hidden_size))):
+            if type(p) not in (torch.Tensor, torch.nn.Parameter) or p.shape != s or p.dtype is not torch.bfloat16 \
+                    or p.device != ids.device or not p.is_contiguous() or p.data_ptr() & 15:
+                return False
+        return self.cfg.hidden_size % 8 == 0 and not ops.observed()
+
     def forward(self, ids, labels=None, caches=None, start_pos: int = 0):
+        if labels is None and caches is not None and self._norm_in_the_head(ids):
+            x = self.model._before_norm(ids, caches, start_pos)
+            if x.dtype is torch.bfloat16 and x.is_contiguous() and not x.data_ptr() & 15:
+                from ..ops import raw
+
+                norm, w = self.model.norm, self.lm_head.weight
+                y = raw.rmsnorm_gemm(x.view(x.shape[0], -1), norm.weight, norm.eps, w)
+                return y.unsqueeze(1)
+            return self.lm_head(self.model.norm(x))
         h = self.model(ids, caches, start_pos)
         logits = self.lm_head(h)
         if labels is None:

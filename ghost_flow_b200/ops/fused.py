@@ -440,6 +440,9 @@ def _observed() -> bool:
             or getattr(forward_ad, "_current_level", 0) >= 0 or torch.compiler.is_compiling())
 
 
+observed = _observed
+
+
 def decode_cache_ok(kcache, vcache, cos, sin, heads, device, pos: int) -> bool:
     """Whether a decoding kernel may write row ``pos`` of the caches ``[B, n, Hk, D]`` (``heads`` = B, Hk, D) and rotate with these
     tables; positions that are not in the tables are an error."""

@@ -118,3 +118,36 @@ def test_layer_in_a_cuda_graph_and_where_it_is_not_taken(calls):
         assert len(calls) == 2
     m, cfg, g = _layer(512, 1024, 4, 2, 0)
     assert m(x, cos, sin, cache=(kc.clone(), vc.clone()), start_pos=3).requires_grad and len(calls) == 2
+
+
+@pytest.mark.parametrize("vocab,B", [(64, 1), (1003, 3), (512, 16), (512, 17)])
+def test_norm_inside_the_head(vocab, B, monkeypatch):
+    """Logits of a decoding step with the last norm in front of the head's product, and module by module."""
+    from ghost_flow_b200.models import LLaMAConfig, LLaMAForCausalLM
+    from ghost_flow_b200.ops import raw
+
+    cfg = LLaMAConfig(vocab_size=vocab, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=4,
+                      num_key_value_heads=2, max_position_embeddings=128)
+    m = LLaMAForCausalLM(cfg, device="cuda", dtype=torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    seen, real = [], raw.rmsnorm_gemm
+    monkeypatch.setattr(raw, "rmsnorm_gemm", lambda *a: seen.append(a) or real(*a))
+    ids = torch.randint(0, vocab, (B, 1), generator=g, device="cuda")
+    with torch.no_grad():
+        m.model.norm.weight.copy_(1 + 0.1 * torch.randn(256, generator=g, device="cuda"))
+        mk = lambda: [tuple(torch.randn(B, 20, 2, 64, generator=torch.Generator(device="cuda").manual_seed(i), device="cuda")  # noqa: E731
+                            .bfloat16() for _ in range(2)) for i in range(2)]
+        y = m(ids, caches=mk(), start_pos=9)
+        assert len(seen) == (1 if B <= 16 else 0) and y.shape == (B, 1, vocab)
+        hidden = []
+        hook = m.model.norm.register_forward_hook(lambda mod, a, out: hidden.append(a[0]))
+        y2 = m(ids, caches=mk(), start_pos=9)
+        hook.remove()
+        assert len(seen) == (1 if B <= 16 else 0)
+        x = hidden[0].double()
+        want = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + m.model.norm.eps) * m.model.norm.weight.double()
+        want = want @ m.lm_head.weight.double().t()
+    # the operand is rounded once on either path, and the result
+    e, e2 = ((t.double() - want).norm() / want.norm() for t in (y, y2))
+    assert e < 4e-3 and e < 1.2 * e2 + 1e-4
+    assert torch.equal(m.generate(ids, 3)[:, :2], m.generate(ids, 1))
