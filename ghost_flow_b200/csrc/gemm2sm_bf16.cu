@@ -60,6 +60,19 @@ constexpr int G2_MAX_SLICES = 4;  // of K
 
 // BNH = rows of B (output columns) per CTA: 128 (256 x 256 tiles, seven stages) or 64 (256 x 128 tiles, nine
 // stages; twice as many tiles, for problems whose last wave of 256-wide tiles would leave most pairs idle).
+// Slice of K that an item belongs to, and its k blocks. Most products have one: no divisions between their tiles then.
+__device__ __forceinline__ int g2_slice(const Gemm2Params& p, int item, int slice_tiles, int num_kb, int& kb0, int& kb1) {
+  if (p.slices == 1) {
+    kb0 = 0;
+    kb1 = num_kb;
+    return 0;
+  }
+  const int slice = item / slice_tiles;
+  kb0 = slice * num_kb / p.slices;         // at most four slices: within 32 bits
+  kb1 = (slice + 1) * num_kb / p.slices;
+  return slice;
+}
+
 template <int BNH>
 struct G2Cfg {
   static constexpr int BN = 2 * BNH;
@@ -209,10 +222,9 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += npairs) {
-        int tm, tn;
-        const int slice = tile / slice_tiles;
+        int tm, tn, kb0, kb1;
+        const int slice = g2_slice(p, tile, slice_tiles, num_kb, kb0, kb1);
         g2_tile_coords(p, tile - slice * slice_tiles, tm, tn);
-        const int kb0 = (int)((long long)slice * num_kb / p.slices), kb1 = (int)((long long)(slice + 1) * num_kb / p.slices);
         const int m0 = tm * 2 * G2_BM + (int)rank * G2_BM;
         const int n0 = tn * G2_BN + (int)rank * G2_BNH;
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -265,8 +277,9 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * G2_BN;
-        const int slice = tile / slice_tiles;
-        const int kbs = (int)((long long)(slice + 1) * num_kb / p.slices) - (int)((long long)slice * num_kb / p.slices);
+        int kb0, kb1;
+        g2_slice(p, tile, slice_tiles, num_kb, kb0, kb1);
+        const int kbs = kb1 - kb0;
         for (int kb = 0; kb < kbs; ++kb) {
           if (!mbar_wait_warp(&full_bar[stage], phase)) {
             if (p.status && leader) atomicCAS(p.status, 0, GF_ERR_WAIT_FULL);
@@ -311,7 +324,7 @@ gemm2sm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     int it = 0;
     for (int tile = pair; tile < num_tiles; tile += npairs) {
       int tm, tn;
-      const int slice = tile / slice_tiles;
+      const int slice = p.slices == 1 ? 0 : tile / slice_tiles;
       g2_tile_coords(p, tile - slice * slice_tiles, tm, tn);
       const int row = tm * 2 * G2_BM + (int)rank * G2_BM + lane_grp * 32 + lane;
       const int n0 = tn * G2_BN;
