@@ -309,7 +309,8 @@ __device__ __forceinline__ float op_grad_bf16(float x) {
   if constexpr (OP == OP_GELU) {
     const float k0 = 0.7978845608028654f, k1 = 0.044715f;
     const float s = sigmoidf_(2.f * k0 * (x + k1 * x * x * x));
-    return s + x * s * (1.f - s) * (2.f * k0 * (1.f + 3.f * k1 * x * x));
+    // s (1 - s) is zero long before |x| = 16; x x, left alone, leaves fp32 and makes that 0 * inf
+    return s + x * s * (1.f - s) * (2.f * k0 * (1.f + 3.f * k1 * fminf(x * x, 256.f)));
   } else {
     return apply_op_grad(OP, x);
   }

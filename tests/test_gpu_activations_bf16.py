@@ -83,3 +83,18 @@ def test_infinities_and_nan(name):
     x = torch.tensor([float("inf"), float("nan"), 0.0, 3e38, -3e38, 1.0, -1.0, 2.0], device="cuda").bfloat16()
     y = ops.unary(x, name)
     assert y[0] == float("inf") and (torch.isnan(y[1]) or name == "relu") and y[2] == 0 and y[3] == x[3] and y[4] == 0
+
+
+@pytest.mark.parametrize("name", ["relu", "gelu", "sigmoid", "tanh", "silu"])
+def test_numbers_of_any_size(name):
+    """Beyond what ``test_every_number`` takes, up to the largest finite number, where squares and cubes leave fp32."""
+    from ghost_flow_b200 import ops
+
+    x = _every()
+    x = x[x.abs() >= 60]
+    x = torch.cat((x, x[:-x.numel() % 8])).requires_grad_()
+    y = ops.unary(x, name)
+    y.backward(torch.ones_like(y))
+    want, grad = _exact(x.detach(), name)          # 3e38 squared and cubed are finite in fp64
+    assert ((y.double() - want).abs() <= 2 ** -7.99 * want.abs() + 2 ** -20 * (name != "relu")).all()
+    assert ((x.grad.double() - grad).abs() <= 2 ** -7.99 * grad.abs() + 2 ** -18).all()
