@@ -48,12 +48,12 @@ class GPTBlock(Module):
         activations, dropout, modules that were replaced or carry hooks."""
         if not x.is_cuda or x.dtype is not torch.bfloat16 or x.dim() != 3 or x.numel() == 0:
             return None
-        m = self._modules
-        ln1, at, ln2, mlp = m["ln1"], m["attn"], m["ln2"], m["mlp"]
+        m = self._modules                    # a plain callable that stands for a module is not in here
+        ln1, at, ln2, mlp = m.get("ln1"), m.get("attn"), m.get("ln2"), m.get("mlp")
         if not (type(ln1) is LayerNorm and type(at) is MultiHeadAttention and type(ln2) is LayerNorm and type(mlp) is FeedForward):
             return None
-        qkv, out, fc1, fc2 = at._modules["qkv"], at._modules["out_proj"], mlp._modules["fc1"], mlp._modules["fc2"]
-        act, drop = mlp._modules["act"], mlp._modules["drop"]
+        qkv, out, fc1, fc2 = at._modules.get("qkv"), at._modules.get("out_proj"), mlp._modules.get("fc1"), mlp._modules.get("fc2")
+        act, drop = mlp._modules.get("act"), mlp._modules.get("drop")
         lin = qkv, out, fc1, fc2
         if any(type(n) is not Linear for n in lin) or type(act) is not GELU or type(drop) is not Dropout \
                 or not plain_modules(ln1, at, ln2, mlp, act, drop, *lin):

@@ -81,17 +81,16 @@ class LLaMADecoderLayer(Module):
         if x.dim() != 3 or x.shape[1] != 1 or x.dtype is not torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() \
                 or type(x) is not torch.Tensor or not 0 < x.shape[0] <= 64:
             return None
-        m = self._modules
-        an, at, fn, mlp = m["attn_norm"], m["attn"], m["ffn_norm"], m["mlp"]
+        m = self._modules                    # a plain callable that stands for a module is not in here
+        an, at, fn, mlp = m.get("attn_norm"), m.get("attn"), m.get("ffn_norm"), m.get("mlp")
         if not (type(an) is RMSNorm and type(at) is LLaMAAttention and type(fn) is RMSNorm and type(mlp) is SwiGLU):
             return None
-        lin = at._modules["wqkv"], at._modules["wo"], mlp._modules["gate_up"], mlp._modules["down"]
+        lin = at._modules.get("wqkv"), at._modules.get("wo"), mlp._modules.get("gate_up"), mlp._modules.get("down")
         if any(type(n) is not Linear or n.bias is not None for n in lin) or not plain_modules(an, at, fn, mlp, *lin):
             return None
         c, (kc, vc), (B, _, hidden), dev = at.cfg, cache, x.shape, x.device
         H, Hk, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim
-        w = [an._parameters["weight"], lin[0]._parameters["weight"], lin[1]._parameters["weight"], fn._parameters["weight"],
-             lin[2]._parameters["weight"], lin[3]._parameters["weight"]]
+        w = [an.weight, lin[0].weight, lin[1].weight, fn.weight, lin[2].weight, lin[3].weight]
         inner = w[5].shape[1] if w[5].dim() == 2 else 0
         shapes = (hidden,), ((H + 2 * Hk) * D, hidden), (hidden, H * D), (hidden,), (2 * inner, hidden), (hidden, inner)
         if D not in (64, 128) or H % Hk or H // Hk > 8 or hidden % 8 or inner % 8 or inner == 0:
@@ -168,11 +167,11 @@ class LLaMAForCausalLM(Module):
     def _norm_in_the_head(self, ids) -> bool:
         """Whether the last norm can run inside the head's product: one token of at most 16 sequences, no gradient, modules that do
         nothing but their own forward, dense bf16 weights on the current GPU, and nothing that follows the calls."""
-        model, head = self._modules["model"], self._modules["lm_head"]
+        model, head = self._modules.get("model"), self._modules.get("lm_head")
         if type(ids) is not torch.Tensor or not ids.is_cuda or ids.dim() != 2 or ids.shape[1] != 1 or not 0 < ids.shape[0] <= 16 \
                 or torch.is_grad_enabled() or type(model) is not LLaMAModel or type(head) is not Linear or head.bias is not None:
             return False
-        norm, w = model._modules["norm"], head.weight
+        norm, w = model._modules.get("norm"), head.weight
         if type(norm) is not RMSNorm or not plain_modules(model, norm, head) or ids.device.index != torch.cuda.current_device():
             return False
         for p, s in ((norm.weight, (self.cfg.hidden_size,)), (w, (w.shape[0], self.cfg.hidden_size))):

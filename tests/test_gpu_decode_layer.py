@@ -151,3 +151,48 @@ def test_norm_inside_the_head(vocab, B, monkeypatch):
     e, e2 = ((t.double() - want).norm() / want.norm() for t in (y, y2))
     assert e < 4e-3 and e < 1.2 * e2 + 1e-4
     assert torch.equal(m.generate(ids, 3)[:, :2], m.generate(ids, 1))
+
+
+def test_weights_and_modules_that_plain_attributes_replace(calls):
+    """A weight put on a module as a tensor is a weight; a callable in the place of a module is called."""
+    import copy
+
+    from ghost_flow_b200 import ops
+    from ghost_flow_b200.models import LLaMAForCausalLM
+
+    m, cfg, g = _layer(256, 512, 4, 2, 3)
+    cos, sin = ops.rope_tables(64, 64, 10000.0, "cuda")
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    x, caches = mk(2, 1, 256), (mk(2, 40, 2, 64), mk(2, 40, 2, 64))
+    step = lambda l: l(x, cos, sin, cache=tuple(c.clone() for c in caches), start_pos=7)  # noqa: E731
+    with torch.no_grad():
+        want = step(m)
+        for name in ("attn_norm", "attn.wqkv", "attn.wo", "ffn_norm", "mlp.gate_up", "mlp.down"):
+            r = copy.deepcopy(m)
+            n = r.get_submodule(name)
+            w = n.weight.detach()
+            del n.weight
+            n.weight = w
+            assert torch.equal(step(r), want), name
+        taken = len(calls)
+        for owner, name in (("", "attn_norm"), ("attn", "wqkv"), ("attn", "wo"), ("", "mlp"), ("mlp", "down")):
+            r = copy.deepcopy(m)
+            o = r.get_submodule(owner)
+            real = getattr(o, name)
+            delattr(o, name)
+            setattr(o, name, lambda *a, real=real, **k: real(*a, **k))
+            # roundings of a chain of bf16 tensors, as above
+            assert ((step(r).float() - want.float()).norm() / want.float().norm()) < 8e-3, name
+        assert len(calls) == taken
+
+        lm = LLaMAForCausalLM(cfg, device="cuda", dtype=torch.bfloat16)
+        ids = torch.randint(0, 64, (2, 1), generator=g, device="cuda")
+        logits = lambda l: l(ids, caches=[tuple(c.clone() for c in caches)], start_pos=7).float()  # noqa: E731
+        want = logits(lm)
+        for owner, name in (("", "lm_head"), ("model", "norm")):
+            r = copy.deepcopy(lm)
+            o = r.get_submodule(owner)
+            real = getattr(o, name)
+            delattr(o, name)
+            setattr(o, name, lambda *a, real=real: real(*a))
+            assert (logits(r) - want).norm() / want.norm() < 8e-3, name

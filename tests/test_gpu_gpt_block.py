@@ -129,3 +129,14 @@ def test_where_it_is_not_taken(calls):
     with torch.no_grad():
         m.cpu()(x.float().cpu())
     assert len(calls) == 1
+
+
+@pytest.mark.parametrize("owner,name", [("", "ln1"), ("", "attn"), ("", "mlp"), ("attn", "qkv"), ("mlp", "fc2"), ("mlp", "act")])
+def test_callables_in_the_place_of_modules_are_called(owner, name, calls):
+    m, g = _block(256, 512, 4, 1)
+    x = torch.randn(2, 128, 256, generator=g, device="cuda").bfloat16()
+    want, o = m(x), m.get_submodule(owner)
+    real = getattr(o, name)
+    delattr(o, name)
+    setattr(o, name, lambda *a, **k: real(*a, **k))
+    assert torch.equal(m(x), want) and len(calls) == 1           # the layers' kernels on the same operands
