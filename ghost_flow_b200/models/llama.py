@@ -79,7 +79,7 @@ class LLaMADecoderLayer(Module):
         token, a gradient, other types or layouts, modules that were replaced or carry hooks, and calls that something
         follows (tracing, transforms, modes), which would miss what happens inside."""
         if x.dim() != 3 or x.shape[1] != 1 or x.dtype is not torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() \
-                or type(x) is not torch.Tensor or not 0 < x.shape[0] <= 64:
+                or type(x) is not torch.Tensor or not 0 < x.shape[0] <= 64 or not isinstance(start_pos, int):
             return None
         m = self._modules                    # a plain callable that stands for a module is not in here
         an, at, fn, mlp = m.get("attn_norm"), m.get("attn"), m.get("ffn_norm"), m.get("mlp")

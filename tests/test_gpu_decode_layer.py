@@ -1,4 +1,5 @@
 """A LLaMA decoder layer for one token in one call (``gf_llama_decode_layer``) against fp64 and against the modules one by one."""
+import ctypes
 import math
 
 import pytest
@@ -196,3 +197,18 @@ def test_weights_and_modules_that_plain_attributes_replace(calls):
             delattr(o, name)
             setattr(o, name, lambda *a, real=real: real(*a))
             assert (logits(r) - want).norm() / want.norm() < 8e-3, name
+
+
+def test_positions_that_are_no_int_are_refused(calls):
+    import numpy as np
+
+    from ghost_flow_b200 import ops
+
+    m, _, g = _layer(256, 512, 4, 2, 3)
+    cos, sin = ops.rope_tables(64, 64, 10000.0, "cuda")
+    x, kc, vc = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((2, 1, 256), (2, 40, 2, 64), (2, 40, 2, 64)))
+    with torch.no_grad():
+        for pos in (np.int64(7), torch.tensor(7), 7.0):
+            with pytest.raises((TypeError, ctypes.ArgumentError)):
+                m(x, cos, sin, cache=(kc, vc), start_pos=pos)
+    assert not calls
