@@ -8,6 +8,8 @@
 // device had work for 780 (8192 tokens of width 768).
 #include <math.h>
 
+#include <algorithm>
+
 #include "gf_host.h"
 
 GF_API int gf_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int T, int D, float eps,
@@ -63,13 +65,35 @@ struct Block {
   }
 };
 
-// What the backward pass reads again.
-struct Saved {
+// fp32 values a product takes as workspace
+long long product_floats(int M, int N, int K, int a_mn_major, int b_mn_major) {
+  return gf_gemm_bf16_workspace(M, N, K, a_mn_major, b_mn_major, 1, 0, 0, 0);
+}
+// The most that the products y = x W^T of the forward pass take, and the two gradients of one of them, W [N, K].
+long long forward_floats(const Block& b) {
+  return std::max({product_floats(b.T, b.P, b.E, 0, 0), product_floats(b.T, b.E, b.E, 0, 0), product_floats(b.T, b.F, b.E, 0, 0),
+                   product_floats(b.T, b.E, b.F, 0, 0)});
+}
+long long gradient_floats(const Block& b, int N, int K) {
+  return std::max(product_floats(b.T, K, N, 0, 1), product_floats(N, K, b.T, 1, 1));
+}
+
+// Results of the forward pass. With `keep` all of them have a place of their own and the backward pass reads them again. Without, only
+// what is still to be read has: n1, o and n2 take turns in y, which is written last; pre follows q, k, v.
+struct Results {
   void *n1, *qkv, *o, *h, *n2, *pre, *act;
-  float *stats1, *lse, *stats2;
+  float *stats1 = nullptr, *lse = nullptr, *stats2 = nullptr;
   long long bytes;
-  Saved(const Block& b, void* base) {
+  Results(const Block& b, bool keep, void* base, void* y) {
     Carve c{(uint8_t*)base};
+    if (!keep) {
+      n1 = o = n2 = y;
+      qkv = pre = c.take(2ll * b.T * std::max(b.P, b.F));
+      h = c.take(2ll * b.T * b.E);
+      act = c.take(2ll * b.T * b.F);
+      bytes = c.used;
+      return;
+    }
     n1 = c.take(2ll * b.T * b.E);
     stats1 = (float*)c.take(8ll * b.T);
     qkv = c.take(2ll * b.T * b.P);
@@ -84,42 +108,26 @@ struct Saved {
   }
 };
 
-int widest(const Block& b) { return b.P > b.F ? b.P : b.F; }
-
-// fp32 values a product takes as workspace
-long long product_floats(int M, int N, int K, int a_mn_major, int b_mn_major) {
-  return gf_gemm_bf16_workspace(M, N, K, a_mn_major, b_mn_major, 1, 0, 0, 0);
-}
-// The most that any of the block's products y = x W^T takes (pass 0), or of their gradients (pass 1).
-long long most_floats(const Block& b, int pass) {
-  long long most = 0;
-  const int shapes[4][2] = {{b.P, b.E}, {b.E, b.E}, {b.F, b.E}, {b.E, b.F}};
-  for (auto& s : shapes) {
-    const int N = s[0], K = s[1];
-    const long long n[2] = {pass ? product_floats(b.T, K, N, 0, 1) : product_floats(b.T, N, K, 0, 0),
-                            pass ? product_floats(N, K, b.T, 1, 1) : 0};
-    for (long long v : n)
-      if (v > most) most = v;
-  }
-  return most;
-}
-
+// Temporaries of the backward pass. The gradient of h lives where the one of x is written in the end; the second layer's
+// (`wide` and its products' workspace) are done with when the attention's, in the same place, begin.
 struct Temps {
-  void *wide, *dn, *dh, *dqkv;
-  float *ndelta, *nlse2, *dq_acc, *sums, *ws;
+  void *wide, *dn, *dqkv;
+  float *ndelta, *nlse2, *dq_acc, *sums, *ws_mlp, *ws_out, *ws_qkv;
   long long bytes;
   Temps(const Block& b, void* base) {
     Carve c{(uint8_t*)base};
-    wide = c.take(2ll * b.T * b.F);              // gradient of the activation, then of its input
     dn = c.take(2ll * b.T * b.E);                // of a norm's output, then of the attention output
-    dh = c.take(2ll * b.T * b.E);
-    dqkv = c.take(2ll * b.T * b.P);
     ndelta = (float*)c.take(4ll * b.T * b.H);
     nlse2 = (float*)c.take(4ll * b.T * b.H);
-    dq_acc = (float*)c.take(4ll * b.T * b.E);
-    sums = (float*)c.take(4ll * gf_norm_bwd_grid(b.T) * (2 * b.E > widest(b) ? 2 * b.E : widest(b)));
-    ws = (float*)c.take(4 * most_floats(b, 1));
-    bytes = c.used;
+    sums = (float*)c.take(4ll * gf_norm_bwd_grid(b.T) * std::max({2 * b.E, b.P, b.F}));
+    Carve mlp = c, out = c, att = c;
+    wide = mlp.take(2ll * b.T * b.F);            // gradient of the activation, then of its input
+    ws_mlp = (float*)mlp.take(4 * std::max(gradient_floats(b, b.F, b.E), gradient_floats(b, b.E, b.F)));
+    ws_out = (float*)out.take(4 * gradient_floats(b, b.E, b.E));
+    dqkv = att.take(2ll * b.T * b.P);
+    const long long ws_bytes = 4 * gradient_floats(b, b.P, b.E), acc_bytes = 4ll * b.T * b.E;
+    dq_acc = ws_qkv = (float*)att.take(std::max(acc_bytes, ws_bytes));
+    bytes = std::max({mlp.used, out.used, att.used});
   }
 };
 
@@ -127,22 +135,27 @@ struct Temps {
 }  // namespace gf
 
 // Bytes of the buffer `saved` that the forward pass fills for the backward pass (which = 0), of the backward pass's workspace
-// (which = 1) and of the forward pass's (which = 2, often none). -1: sizes that are not taken.
+// (which = 1), and of the forward pass's with `saved` (which = 2, often none) and without (which = 3). -1: sizes that are not
+// taken.
 GF_API long long gf_gpt_block_bytes(int which, int B, int S, int E, int F, int H, int Hk) {
   gf::Block b(B, S, E, F, H, Hk);
   if (!b.ok()) return -1;
-  return which == 0 ? gf::Saved(b, nullptr).bytes : which == 1 ? gf::Temps(b, nullptr).bytes : 4 * gf::most_floats(b, 0);
+  if (which == 0) return gf::Results(b, true, nullptr, nullptr).bytes;
+  if (which == 1) return gf::Temps(b, nullptr).bytes;
+  const long long ws = (4 * gf::forward_floats(b) + 255) & ~255ll;
+  return which == 2 ? ws : ws + gf::Results(b, false, nullptr, nullptr).bytes;
 }
 
 // params: {ln1 weight, bias, Wqkv, bqkv, Wo, bo, ln2 weight, bias, W1, b1, W2, b2}, biases may be null; dense bf16.
-// x, y: dense bf16 [B * S, E].
+// x, y: dense bf16 [B * S, E]. saved: null where there is no backward pass.
 GF_API int gf_gpt_block_fwd(const void* x, const void* const* params, void* y, void* saved, void* ws, int B, int S, int E, int F,
                             int H, int Hk, int causal, float eps1, float eps2, int* status, void* stream) {
   using namespace gf;
   enter();
   const Block b(B, S, E, F, H, Hk);
-  if (!b.ok() || !x || !y || !saved) return GFH_BAD_ARG;
-  const Saved s(b, saved);
+  if (!b.ok() || !x || !y || (!saved && !ws)) return GFH_BAD_ARG;
+  const long long ws_bytes = (4 * forward_floats(b) + 255) & ~255ll;
+  const Results s(b, saved != nullptr, saved ? saved : (uint8_t*)ws + ws_bytes, y);
   const int T = b.T, P = b.P, D = b.D;
   int rc;
   auto linear = [&](const void* in, int K, const void* w, const void* bias, const void* res, void* out, int N) {
@@ -151,14 +164,15 @@ GF_API int gf_gpt_block_fwd(const void* x, const void* const* params, void* y, v
     return gf_gemm_bf16(in, w, out, T, N, K, 0, K, 0, K, N, 0, 0, bias, res, res ? N : 0, 1.f, status, 0, 0,
                         fl ? (const int*)ws : nullptr, 0, (int)fl, stream);
   };
-  if ((rc = gf_layernorm_fwd(x, params[0], params[1], s.n1, s.stats1, s.stats1 + T, T, E, eps1, stream))) return rc;
+  if ((rc = gf_layernorm_fwd(x, params[0], params[1], s.n1, s.stats1, s.stats1 ? s.stats1 + T : nullptr, T, E, eps1, stream))) return rc;
   if ((rc = linear(s.n1, E, params[2], params[3], nullptr, s.qkv, P))) return rc;
   const uint8_t* q = (const uint8_t*)s.qkv;
   if ((rc = gf_flash_attn_fwd3(q, q + 2ll * E, q + 2ll * (E + Hk * D), s.o, s.lse, B, S, H, Hk, D, P, P, P, E,
                                1.f / sqrtf((float)D), causal, status, stream)))
     return rc;
   if ((rc = linear(s.o, E, params[4], params[5], x, s.h, E))) return rc;
-  if ((rc = gf_layernorm_fwd(s.h, params[6], params[7], s.n2, s.stats2, s.stats2 + T, T, E, eps2, stream))) return rc;
+  if ((rc = gf_layernorm_fwd(s.h, params[6], params[7], s.n2, s.stats2, s.stats2 ? s.stats2 + T : nullptr, T, E, eps2, stream)))
+    return rc;
   if ((rc = linear(s.n2, E, params[8], params[9], nullptr, s.pre, F))) return rc;
   if ((rc = gf_unary_fwd(s.pre, s.act, (long long)T * F, ACT_GELU, 1, stream))) return rc;
   return linear(s.act, F, params[10], params[11], s.h, y, E);
@@ -173,29 +187,30 @@ GF_API int gf_gpt_block_bwd(const void* x, const void* const* params, const void
   enter();
   const Block b(B, S, E, F, H, Hk);
   if (!b.ok() || !x || !dy || !saved || !ws || !dx || !grads[0] || !grads[6] || S % 128) return GFH_BAD_ARG;
-  const Saved s(b, const_cast<void*>(saved));
+  const Results s(b, true, const_cast<void*>(saved), nullptr);
   const Temps t(b, ws);
   const int T = b.T, P = b.P, D = b.D;
   const float scale = 1.f / sqrtf((float)D);
   int rc;
   // gradients of y = in W^T + bias at dy [T, N]: of in (to `din`), W and bias
-  auto linear = [&](const void* g, int N, const void* in, int K, const void* w, void* din, void* dw, void* db) {
+  auto linear = [&](const void* g, int N, const void* in, int K, const void* w, void* din, void* dw, void* db, float* ws_at) {
     auto product = [&](const void* A, int a_mn, int lda, const void* W, int ldw, void* out, int m, int n, int k) {
       const long long fl = product_floats(m, n, k, a_mn, 1);
       return gf_gemm_bf16(A, W, out, m, n, k, a_mn, lda, 1, ldw, n, 0, 0, nullptr, nullptr, 0, 1.f, status, 0, 0,
-                          fl ? (const int*)t.ws : nullptr, 0, (int)fl, stream);
+                          fl ? (const int*)ws_at : nullptr, 0, (int)fl, stream);
     };
     if ((rc = product(g, 0, N, w, K, din, T, K, N))) return rc;
     if (dw && (rc = product(g, 1, N, in, K, dw, N, K, T))) return rc;
     if (db) rc = gf_colsum_bf16(g, N, db, t.sums, T, N, 0, stream);
     return rc;
   };
-  if (linear(dy, E, s.act, F, params[10], t.wide, grads[10], grads[11])) return rc;
+  void* dh = dx;                     // of h: until the last launch, which reads it where it writes dx
+  if (linear(dy, E, s.act, F, params[10], t.wide, grads[10], grads[11], t.ws_mlp)) return rc;
   if ((rc = gf_unary_bwd_bf16(s.pre, t.wide, t.wide, (long long)T * F, ACT_GELU, stream))) return rc;
-  if (linear(t.wide, F, s.n2, E, params[8], t.dn, grads[8], grads[9])) return rc;
-  if ((rc = gf_layernorm_bwd_res(s.h, params[6], t.dn, s.stats2, s.stats2 + T, dy, t.dh, grads[6], grads[7], t.sums, T, E, 0, stream)))
+  if (linear(t.wide, F, s.n2, E, params[8], t.dn, grads[8], grads[9], t.ws_mlp)) return rc;
+  if ((rc = gf_layernorm_bwd_res(s.h, params[6], t.dn, s.stats2, s.stats2 + T, dy, dh, grads[6], grads[7], t.sums, T, E, 0, stream)))
     return rc;
-  if (linear(t.dh, E, s.o, E, params[4], t.dn, grads[4], grads[5])) return rc;
+  if (linear(dh, E, s.o, E, params[4], t.dn, grads[4], grads[5], t.ws_out)) return rc;
   const uint8_t* q = (const uint8_t*)s.qkv;
   uint8_t* dq = (uint8_t*)t.dqkv;
   const long long ok = 2ll * E, ov = 2ll * (E + Hk * D);
@@ -204,8 +219,8 @@ GF_API int gf_gpt_block_bwd(const void* x, const void* const* params, const void
                                scale, causal, status, stream)))
     return rc;
   if ((rc = gf_dq_rows_to_bf16(t.dq_acc, dq, B, S, H, D, P, scale, stream))) return rc;
-  if (linear(t.dqkv, P, s.n1, E, params[2], t.dn, grads[2], grads[3])) return rc;
-  return gf_layernorm_bwd_res(x, params[0], t.dn, s.stats1, s.stats1 + T, t.dh, dx, grads[0], grads[1], t.sums, T, E, 0, stream);
+  if (linear(t.dqkv, P, s.n1, E, params[2], t.dn, grads[2], grads[3], t.ws_qkv)) return rc;
+  return gf_layernorm_bwd_res(x, params[0], t.dn, s.stats1, s.stats1 + T, dh, dx, grads[0], grads[1], t.sums, T, E, 0, stream);
 }
 
 // The three launches of the attention backward pass; ws: fp32, B Hq S (D + 2) values on a 16-byte boundary (accumulator first).

@@ -750,10 +750,11 @@ class _GPTBlockFn(torch.autograd.Function):
         B, S, E, F_, H, Hk = sizes
         y = torch.empty_like(x)
         mem = lambda n: torch.empty(n, dtype=torch.uint8, device=x.device) if n else None  # noqa: E731
-        saved, ws = mem(_block_bytes(0, *sizes)), mem(_block_bytes(2, *sizes))
-        _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), saved.data_ptr(),
-                                             None if ws is None else ws.data_ptr(), *sizes, causal, eps1, eps2,
-                                             _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()), "gf_gpt_block_fwd")
+        graph = type(ctx) is not _NoGraph            # without one the layers' results share a small workspace
+        saved, ws = (mem(_block_bytes(0, *sizes)), mem(_block_bytes(2, *sizes))) if graph else (None, mem(_block_bytes(3, *sizes)))
+        _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), *_pointers((saved, ws)), *sizes, causal,
+                                             eps1, eps2, _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()),
+            "gf_gpt_block_fwd")
         ctx.save_for_backward(x, saved, *params)
         ctx.args = sizes, causal
         return y

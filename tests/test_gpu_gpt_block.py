@@ -140,3 +140,37 @@ def test_callables_in_the_place_of_modules_are_called(owner, name, calls):
     delattr(o, name)
     setattr(o, name, lambda *a, **k: real(*a, **k))
     assert torch.equal(m(x), want) and len(calls) == 1           # the layers' kernels on the same operands
+
+
+@pytest.mark.parametrize("train,most", [(False, 1.02), (True, 1.25)])
+def test_memory_of_a_pass_is_about_the_layers(train, most, calls):
+    """Most memory held during a pass. Without a gradient nothing is kept for one; in the backward pass, which holds all results
+    until its end where the layers let go of theirs one by one, temporaries share what they can (in rows of width 768, 2 bytes: 50
+    against 42)."""
+    m, g = _block(768, 3072, 12, 1)
+    x, dy = (torch.randn(8, 1024, 768, generator=g, device="cuda").bfloat16() for _ in range(2))
+    x.requires_grad_(train)
+
+    def most_held():
+        peak = 0
+        for _ in range(2):                                               # the first one settles what is allocated once
+            m.zero_grad()
+            x.grad = None
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            with torch.set_grad_enabled(train):
+                y = m(x)
+            if train:
+                y.backward(dy)
+            torch.cuda.synchronize()
+            peak = torch.cuda.max_memory_allocated() - before
+            del y
+        return peak
+
+    one = most_held()
+    assert len(calls) == 2
+    hook = m.mlp.fc1.register_forward_hook(lambda *a: None)              # layer by layer
+    layers = most_held()
+    hook.remove()
+    assert len(calls) == 2 and one <= most * layers, (one / 1e6, layers / 1e6)
