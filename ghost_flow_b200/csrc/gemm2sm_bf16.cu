@@ -518,12 +518,16 @@ static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Par
 
 // 1 when plain GEMMs of this shape should run on CTA pairs. GF_GEMM_2SM=0 turns the path off, =1 forces it for
 // every shape it can take.
-int gemm2sm_wanted(int M, int N, int K) {
-  static int mode = -1;
-  if (mode < 0) {
+// Read once: workspaces are sized by the same rule that the launches follow later.
+static int g2_mode() {
+  static const int mode = [] {
     const char* e = getenv("GF_GEMM_2SM");
-    mode = e ? atoi(e) : 2;
-  }
+    return e ? atoi(e) : 2;
+  }();
+  return mode;
+}
+int gemm2sm_wanted(int M, int N, int K) {
+  const int mode = g2_mode();
   if (mode == 0) return 0;
   if (mode == 1) return 1;
   // default: problems with enough 256 x 256 tiles to give every pair work
@@ -555,7 +559,7 @@ static int g2_pick_bn(int M, int N) {
 // 34.7 / 33.8. With fewer than 16 tiles, which take more than four parts, the sums cost more than they save: [768, 768] over 8192
 // 21.8 / 23.9, [1024, 768] over 3072 19.8 / 21.5.
 int gemm2sm_slices(int M, int N, int K) {
-  if (M < 256 || N < 256 || K < 2048 || gemm2sm_wanted(M, N, K) || getenv("GF_GEMM_2SM")) return 0;
+  if (M < 256 || N < 256 || K < 2048 || gemm2sm_wanted(M, N, K) || g2_mode() != 2) return 0;
   const int pairs = sm_count() / 2, kb = (K + G2_BK - 1) / G2_BK;
   const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256), ctas = (long long)((M + 127) / 128) * ((N + 255) / 256);
   if (tiles < 16) return 0;

@@ -148,19 +148,21 @@ GF_API long long gf_gpt_block_bytes(int which, int B, int S, int E, int F, int H
 
 // params: {ln1 weight, bias, Wqkv, bqkv, Wo, bo, ln2 weight, bias, W1, b1, W2, b2}, biases may be null; dense bf16.
 // x, y: dense bf16 [B * S, E]. saved: null where there is no backward pass.
-GF_API int gf_gpt_block_fwd(const void* x, const void* const* params, void* y, void* saved, void* ws, int B, int S, int E, int F,
-                            int H, int Hk, int causal, float eps1, float eps2, int* status, void* stream) {
+// saved_bytes, ws_bytes: what the caller allocated; less than gf_gpt_block_bytes is refused before the first launch.
+GF_API int gf_gpt_block_fwd(const void* x, const void* const* params, void* y, void* saved, long long saved_bytes, void* ws,
+                            long long ws_bytes, int B, int S, int E, int F, int H, int Hk, int causal, float eps1, float eps2,
+                            int* status, void* stream) {
   using namespace gf;
   enter();
   const Block b(B, S, E, F, H, Hk);
-  if (!b.ok() || !x || !y || (!saved && !ws)) return GFH_BAD_ARG;
-  const long long ws_bytes = (4 * forward_floats(b) + 255) & ~255ll;
-  const Results s(b, saved != nullptr, saved ? saved : (uint8_t*)ws + ws_bytes, y);
+  if (!b.ok() || !x || !y) return GFH_BAD_ARG;
+  const long long product_bytes = (4 * forward_floats(b) + 255) & ~255ll;
+  const Results s(b, saved != nullptr, saved ? saved : (uint8_t*)ws + product_bytes, y);
+  if (saved ? saved_bytes < s.bytes || ws_bytes < product_bytes : ws_bytes < product_bytes + s.bytes) return GFH_BAD_ARG;
   const int T = b.T, P = b.P, D = b.D;
   int rc;
   auto linear = [&](const void* in, int K, const void* w, const void* bias, const void* res, void* out, int N) {
     const long long fl = product_floats(T, N, K, 0, 0);
-    if (fl && !ws) return (int)GFH_BAD_ARG;
     return gf_gemm_bf16(in, w, out, T, N, K, 0, K, 0, K, N, 0, 0, bias, res, res ? N : 0, 1.f, status, 0, 0,
                         fl ? (const int*)ws : nullptr, 0, (int)fl, stream);
   };
@@ -179,16 +181,17 @@ GF_API int gf_gpt_block_fwd(const void* x, const void* const* params, void* y, v
 }
 
 // grads: where the gradients of params go, null for those that are not wanted; the norms' are always written. dx likewise.
-// ws: gf_gpt_block_bytes(1, ...) bytes. S must be a multiple of 128.
-GF_API int gf_gpt_block_bwd(const void* x, const void* const* params, const void* dy, const void* saved, void* dx,
-                            void* const* grads, void* ws, int B, int S, int E, int F, int H, int Hk, int causal, int* status,
-                            void* stream) {
+// ws: gf_gpt_block_bytes(1, ...) bytes; the sizes of both buffers are checked as above. S must be a multiple of 128.
+GF_API int gf_gpt_block_bwd(const void* x, const void* const* params, const void* dy, const void* saved, long long saved_bytes,
+                            void* dx, void* const* grads, void* ws, long long ws_bytes, int B, int S, int E, int F, int H, int Hk,
+                            int causal, int* status, void* stream) {
   using namespace gf;
   enter();
   const Block b(B, S, E, F, H, Hk);
-  if (!b.ok() || !x || !dy || !saved || !ws || !dx || !grads[0] || !grads[6] || S % 128) return GFH_BAD_ARG;
+  if (!b.ok() || !x || !dy || !saved || !ws || !dx || !grads || !grads[0] || !grads[6] || S % 128) return GFH_BAD_ARG;
   const Results s(b, true, const_cast<void*>(saved), nullptr);
   const Temps t(b, ws);
+  if (saved_bytes < s.bytes || ws_bytes < t.bytes) return GFH_BAD_ARG;
   const int T = b.T, P = b.P, D = b.D;
   const float scale = 1.f / sqrtf((float)D);
   int rc;

@@ -734,8 +734,13 @@ def flash_attention(q, k, v, causal: bool = True, scale: float | None = None):
 
 # ------------------------------------------------------------------------------------------ a whole pre-norm block
 @functools.lru_cache(maxsize=1024)
-def _block_bytes(which, B, S, E, F, H, Hk) -> int:
+def _block_bytes(device: int, which, B, S, E, F, H, Hk) -> int:
+    """Bytes of a buffer of the block on a device (the number of SMs decides which products split K)."""
     return _lib.cuda_lib().gf_gpt_block_bytes(which, B, S, E, F, H, Hk)
+
+
+def _nbytes(t) -> int:
+    return 0 if t is None else t.numel() * t.element_size()
 
 
 def _pointers(ts):
@@ -750,11 +755,13 @@ class _GPTBlockFn(torch.autograd.Function):
         B, S, E, F_, H, Hk = sizes
         y = torch.empty_like(x)
         mem = lambda n: torch.empty(n, dtype=torch.uint8, device=x.device) if n else None  # noqa: E731
+        size = lambda which: _block_bytes(x.device.index, which, *sizes)  # noqa: E731
         graph = type(ctx) is not _NoGraph            # without one the layers' results share a small workspace
-        saved, ws = (mem(_block_bytes(0, *sizes)), mem(_block_bytes(2, *sizes))) if graph else (None, mem(_block_bytes(3, *sizes)))
-        _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), *_pointers((saved, ws)), *sizes, causal,
-                                             eps1, eps2, _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()),
-            "gf_gpt_block_fwd")
+        saved, ws = (mem(size(0)), mem(size(2))) if graph else (None, mem(size(3)))
+        at = _pointers((saved, ws))
+        _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), at[0], _nbytes(saved), at[1], _nbytes(ws),
+                                             *sizes, causal, eps1, eps2, _lib.status_word(x.device).data_ptr(),
+                                             _lib.stream_ptr()), "gf_gpt_block_fwd")
         ctx.save_for_backward(x, saved, *params)
         ctx.args = sizes, causal
         return y
@@ -770,9 +777,9 @@ class _GPTBlockFn(torch.autograd.Function):
         # the norms' kernels always write theirs
         grads = [torch.empty_like(p) if p is not None and (need or i in (0, 6)) else None
                  for i, (p, need) in enumerate(zip(params, ctx.needs_input_grad[5:]))]
-        ws = torch.empty(_block_bytes(1, *sizes), dtype=torch.uint8, device=x.device)
-        _rc(_lib.cuda_lib().gf_gpt_block_bwd(x.data_ptr(), _pointers(params), dy.data_ptr(), saved.data_ptr(), dx.data_ptr(),
-                                             _pointers(grads), ws.data_ptr(), *sizes, causal,
+        ws = torch.empty(_block_bytes(x.device.index, 1, *sizes), dtype=torch.uint8, device=x.device)
+        _rc(_lib.cuda_lib().gf_gpt_block_bwd(x.data_ptr(), _pointers(params), dy.data_ptr(), saved.data_ptr(), _nbytes(saved),
+                                             dx.data_ptr(), _pointers(grads), ws.data_ptr(), _nbytes(ws), *sizes, causal,
                                              _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()), "gf_gpt_block_bwd")
         return (dx, None, None, None, None, *grads)
 
@@ -793,7 +800,7 @@ def gpt_block_ok(x, params, sizes) -> bool:
     own calls."""
     B, S, E, F_, H, Hk = sizes
     if type(x) is not torch.Tensor or not _cuda_bf16(x) or not x.is_contiguous() or x.data_ptr() % 16 or E > 8192 or F_ > 8192 \
-            or (H + 2 * Hk) * (E // H) > 8192 or _block_bytes(0, *sizes) < 0 or x.device.index != torch.cuda.current_device():
+            or (H + 2 * Hk) * (E // H) > 8192 or _block_bytes(x.device.index, 0, *sizes) < 0 or x.device.index != torch.cuda.current_device():
         return False
     P = (H + 2 * Hk) * (E // H)
     shapes = ((E,), (E,), (P, E), (P,), (E, E), (E,), (E,), (E,), (F_, E), (F_,), (E, F_), (E,))
