@@ -576,8 +576,10 @@ int attn_decode_append(const void* qkv, long long ldq, void* kcache, void* vcach
                        const float* sin_row, int interleaved, void* out, long long ldo, int B, int Hq, int Hkv, int D, float scale,
                        int splits, float* scratch, int chained, cudaStream_t st) {
   if (B <= 0 || Hkv <= 0 || Hq % Hkv || Hq / Hkv > DEC_MAX_G || (D != 64 && D != 128) || splits < 1 || !scratch || len < 1 ||
-      len > s_max)
+      len > s_max || ldq % 8)
     return GFH_BAD_ARG;
+  for (const void* x : {qkv, (const void*)kcache, (const void*)vcache})       // the new token's rows are read and written as vectors
+    if (!x || (reinterpret_cast<uintptr_t>(x) & 15)) return GFH_BAD_ARG;
   DecParams p{{nullptr, len, s_max, B, Hkv, 0, splits}, (const __nv_bfloat16*)qkv, ldq, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache,
               Hq, scale * 1.4426950408889634f, scratch, (__nv_bfloat16*)out, ldo, cos_row, sin_row, interleaved};
   return D == 128 ? launch_decode<128, true>(p, chained, st) : launch_decode<64, true>(p, chained, st);

@@ -40,8 +40,13 @@ GF_API int gf_llama_decode_layer(const void* x, const void* attn_norm, float att
   using namespace gf;
   enter();
   if (B < 1 || B > ROWS_MAX_M || hidden <= 0 || inner <= 0 || Hq <= 0 || Hkv <= 0 || pos < 0 || pos >= s_max || splits < 1 ||
-      (reinterpret_cast<uintptr_t>(ws) & 255))
+      !ws || (reinterpret_cast<uintptr_t>(ws) & 255))
     return GFH_BAD_ARG;
+  // all that the kernels check or read as 16-byte vectors, before the first of them writes anything
+  if ((D != 64 && D != 128) || Hq % Hkv || hidden % 8 || inner % 8) return GFH_BAD_ARG;
+  for (const void* p : {x, attn_norm, wqkv, wo, ffn_norm, gate_up, down, (const void*)kcache, (const void*)vcache, (const void*)y})
+    if (!p || (reinterpret_cast<uintptr_t>(p) & 15)) return GFH_BAD_ARG;
+  if (!cos_t || !sin_t) return GFH_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   const int att = Hq * D, packed = (Hq + 2 * Hkv) * D;
   uint8_t* at = reinterpret_cast<uint8_t*>(ws);

@@ -404,8 +404,15 @@ static int launch_rows_nt(const CUtensorMap& tm, const CUtensorMap& tx, const Ro
   else return launch_rows<64, INPUT>(tm, tx, p, slices, chained, stream);
 }
 
+// What the kernel reads as 16-byte vectors beside X and W, and the kinds that there are.
+static bool gemm_rows_input_ok(const RowsGemm& g) {
+  if (g.input == ROWS_PLAIN) return true;
+  if (g.M > ROWS_MAX_M_FUSED) return false;
+  return g.input == ROWS_SWIGLU || (g.input == ROWS_RMSNORM && g.norm_w && (reinterpret_cast<uintptr_t>(g.norm_w) & 15) == 0);
+}
+
 int gemm_rows_run(const RowsGemm& g, int chained, cudaStream_t stream) {
-  if (!gemm_rows_takes(g.X, g.ldx, g.W, g.ldw, g.M, g.N, g.K)) return GFH_BAD_ARG;
+  if (!gemm_rows_takes(g.X, g.ldx, g.W, g.ldw, g.M, g.N, g.K) || !gemm_rows_input_ok(g)) return GFH_BAD_ARG;
   CUtensorMap tm;
   const int rc = make_tmap_2d(&tm, g.W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.N, g.K, g.ldw * 2, RW_BM, RW_BK);
   if (rc) return rc;

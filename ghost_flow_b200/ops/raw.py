@@ -342,6 +342,10 @@ def rmsnorm_gemm(x, norm_w, eps, w):
     """``rms_norm(x) @ w^T`` for at most 16 rows of dense bf16, in one kernel (the norm in front of the product). ``w [N, K]`` dense; rows
     of the result start on 16-byte boundaries."""
     (M, K), N = x.shape, w.shape[0]
+    for t, s in (x, (M, K)), (norm_w, (K,)), (w, (N, K)):
+        if t.shape != s or t.dtype is not torch.bfloat16 or t.device != x.device or not t.is_contiguous():
+            raise ValueError(f"rmsnorm_gemm takes dense bf16 tensors [M, K], [K], [N, K] on one device, not {list(x.shape)}, "
+                             f"{list(norm_w.shape)}, {list(w.shape)}")
     y = torch.empty((M, N if N % 8 == 0 else (N + 63) // 64 * 64), dtype=x.dtype, device=x.device)[:, :N]
     _rc(_lib.cuda_lib().gf_gemm_rows(x.data_ptr(), K, w.data_ptr(), K, y.data_ptr(), y.stride(0), 0, M, N, K, 1, norm_w.data_ptr(),
                                      float(eps), None, None, 0, 1.0, 0, _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()),
