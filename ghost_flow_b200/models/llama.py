@@ -79,7 +79,8 @@ class LLaMADecoderLayer(Module):
         token, a gradient, other types or layouts, modules that were replaced or carry hooks, and calls that something
         follows (tracing, transforms, modes), which would miss what happens inside."""
         if x.dim() != 3 or x.shape[1] != 1 or x.dtype is not torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() \
-                or type(x) is not torch.Tensor or not 0 < x.shape[0] <= 64 or not isinstance(start_pos, int):
+                or type(x) is not torch.Tensor or not 0 < x.shape[0] <= 64 or not isinstance(start_pos, int) \
+                or ops.observed():            # before anything asks a tensor for its memory: transformed ones have none
             return None
         m = self._modules                    # a plain callable that stands for a module is not in here
         an, at, fn, mlp = m.get("attn_norm"), m.get("attn"), m.get("ffn_norm"), m.get("mlp")
@@ -169,7 +170,8 @@ class LLaMAForCausalLM(Module):
         nothing but their own forward, dense bf16 weights on the current GPU, and nothing that follows the calls."""
         model, head = self._modules.get("model"), self._modules.get("lm_head")
         if type(ids) is not torch.Tensor or not ids.is_cuda or ids.dim() != 2 or ids.shape[1] != 1 or not 0 < ids.shape[0] <= 16 \
-                or torch.is_grad_enabled() or type(model) is not LLaMAModel or type(head) is not Linear or head.bias is not None:
+                or torch.is_grad_enabled() or ops.observed() or type(model) is not LLaMAModel or type(head) is not Linear \
+                or head.bias is not None:
             return False
         norm, w = model._modules.get("norm"), head.weight
         if type(norm) is not RMSNorm or not plain_modules(model, norm, head) or ids.device.index != torch.cuda.current_device():
@@ -178,7 +180,7 @@ class LLaMAForCausalLM(Module):
             if type(p) not in (torch.Tensor, torch.nn.Parameter) or p.shape != s or p.dtype is not torch.bfloat16 \
                     or p.device != ids.device or not p.is_contiguous() or p.data_ptr() & 15:
                 return False
-        return self.cfg.hidden_size % 8 == 0 and not ops.observed()
+        return self.cfg.hidden_size % 8 == 0
 
     def forward(self, ids, labels=None, caches=None, start_pos: int = 0):
         if labels is None and caches is not None and self._norm_in_the_head(ids):

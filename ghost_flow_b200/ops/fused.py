@@ -445,9 +445,9 @@ observed = _observed
 
 def decode_cache_ok(kcache, vcache, cos, sin, heads, device, pos: int) -> bool:
     """Whether a decoding kernel may write row ``pos`` of the caches ``[B, n, Hk, D]`` (``heads`` = B, Hk, D) and rotate with these
-    tables; positions that are not in the tables are an error."""
+    tables; positions that are not in the tables are an error. For calls that nothing follows (:func:`observed`)."""
     B, Hk, D = heads
-    if _observed() or kcache.dim() != 4 or not (kcache.is_contiguous() and vcache.is_contiguous()):
+    if kcache.dim() != 4 or not (kcache.is_contiguous() and vcache.is_contiguous()):
         return False
     shape = (B, kcache.shape[1], Hk, D)
     if not (0 <= pos < shape[1] and _cache_fits_kernel(kcache, shape, device, torch.bfloat16)
@@ -799,6 +799,8 @@ def gpt_block_ok(x, params, sizes) -> bool:
     sizes and (where there is a gradient) a sequence that the attention kernels have, and nothing that follows the layers'
     own calls."""
     B, S, E, F_, H, Hk = sizes
+    if _observed():                         # before anything asks a tensor for its memory: transformed ones have none
+        return False
     if type(x) is not torch.Tensor or not _cuda_bf16(x) or not x.is_contiguous() or x.data_ptr() % 16 or E > 8192 or F_ > 8192 \
             or (H + 2 * Hk) * (E // H) > 8192 or _block_bytes(x.device.index, 0, *sizes) < 0 or x.device.index != torch.cuda.current_device():
         return False
@@ -816,4 +818,4 @@ def gpt_block_ok(x, params, sizes) -> bool:
             grad = grad or p.requires_grad
     if (grad or x.requires_grad) and torch.is_grad_enabled() and S % 128:
         return False                        # the layers say what they miss
-    return not _observed() and os.environ.get("GF_FA_FWD", "3") == "3" and os.environ.get("GF_FA_BWD", "3") != "1"
+    return os.environ.get("GF_FA_FWD", "3") == "3" and os.environ.get("GF_FA_BWD", "3") != "1"
