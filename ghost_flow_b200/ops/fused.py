@@ -15,6 +15,7 @@ import os
 import torch
 import torch.nn.functional as F
 from torch.autograd import forward_ad
+from torch.utils._device import DeviceContext
 
 from . import _lib
 
@@ -430,13 +431,23 @@ _PROBES = tuple(getattr(torch._C, n, None) for n in ("_get_tracing_state", "_are
                                                       "_len_torch_dispatch_stack", "_len_torch_function_stack"))
 
 
+_FUNCTION_MODES = getattr(torch.overrides, "_get_current_function_mode_stack", None)
+
+
+def _only_device_contexts() -> bool:
+    """Whether every function mode is a ``with torch.device(...)`` or ``torch.set_default_device``: they say where new tensors
+    go, and follow nothing. Allocations next to a launch name their device."""
+    return _FUNCTION_MODES is not None and all(type(m) is DeviceContext for m in _FUNCTION_MODES())
+
+
 def _observed() -> bool:
     """Whether something follows the tensor operations of this call that a kernel launch would escape: tracing, compilation,
     ``torch.func`` transforms, dispatch or function modes, forward-mode gradients."""
     if None in _PROBES:
         return True
     tracing, transforms, dispatch_modes, function_modes = _PROBES
-    return (tracing() is not None or transforms() or dispatch_modes() > 0 or function_modes() > 0
+    return (tracing() is not None or transforms() or dispatch_modes() > 0
+            or (function_modes() > 0 and not _only_device_contexts())
             or getattr(forward_ad, "_current_level", 0) >= 0 or torch.compiler.is_compiling())
 
 

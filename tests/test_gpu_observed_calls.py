@@ -124,3 +124,15 @@ def test_transforms_without_gradients_never_meet_the_call(what, taken):
     with torch.no_grad(), pytest.raises(RuntimeError):
         torch.func.vmap(f, randomness="same")(torch.stack((a, a)))
     assert not taken
+
+
+@pytest.mark.parametrize("what", ["gpt", "layer", "model"])
+def test_device_contexts_change_nothing(what, taken, kernel_status):
+    _, f, a = _case(what)
+    with torch.no_grad():
+        want = f(a)
+        n = len(taken)
+        for device in ("cuda", "cpu", "meta"):            # every allocation next to a launch names its device
+            with torch.device(device):
+                assert torch.equal(f(a), want)
+        assert len(taken) == 4 * n
