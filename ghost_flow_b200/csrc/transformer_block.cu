@@ -106,6 +106,15 @@ struct Results {
     act = c.take(2ll * b.T * b.F);
     bytes = c.used;
   }
+  static constexpr int PARTS = 10;
+  void get(const void** p) const {
+    const void* all[PARTS] = {n1, stats1, qkv, o, lse, h, n2, stats2, pre, act};
+    std::copy(all, all + PARTS, p);
+  }
+  void set(const void* const* p) {
+    n1 = (void*)p[0]; stats1 = (float*)p[1]; qkv = (void*)p[2]; o = (void*)p[3]; lse = (float*)p[4];
+    h = (void*)p[5]; n2 = (void*)p[6]; stats2 = (float*)p[7]; pre = (void*)p[8]; act = (void*)p[9];
+  }
 };
 
 // Temporaries of the backward pass. The gradient of h lives where the one of x is written in the end; the second layer's
@@ -146,6 +155,19 @@ GF_API long long gf_gpt_block_bytes(int which, int B, int S, int E, int F, int H
   return which == 2 ? ws : ws + gf::Results(b, false, nullptr, nullptr).bytes;
 }
 
+// Where in `saved` its ten tensors begin (bytes), in the order n1 [T, E], statistics [2, T] fp32, q k v [T, (H + 2 Hk) D], o [T, E],
+// lse [B, H, S] fp32, h [T, E], n2 [T, E], statistics [2, T] fp32, pre [T, F], act [T, F].
+GF_API int gf_gpt_block_parts(long long* offsets, int B, int S, int E, int F, int H, int Hk) {
+  using namespace gf;
+  const Block b(B, S, E, F, H, Hk);
+  if (!b.ok() || !offsets) return GFH_BAD_ARG;
+  uint8_t* base = reinterpret_cast<uint8_t*>(256);         // only differences are taken
+  const void* at[Results::PARTS];
+  Results(b, true, base, nullptr).get(at);
+  for (int i = 0; i < Results::PARTS; ++i) offsets[i] = (const uint8_t*)at[i] - base;
+  return GFH_OK;
+}
+
 // params: {ln1 weight, bias, Wqkv, bqkv, Wo, bo, ln2 weight, bias, W1, b1, W2, b2}, biases may be null; dense bf16.
 // x, y: dense bf16 [B * S, E]. saved: null where there is no backward pass.
 // saved_bytes, ws_bytes: what the caller allocated; less than gf_gpt_block_bytes is refused before the first launch.
@@ -181,17 +203,19 @@ GF_API int gf_gpt_block_fwd(const void* x, const void* const* params, void* y, v
 }
 
 // grads: where the gradients of params go, null for those that are not wanted; the norms' are always written. dx likewise.
+// saved: as the forward pass left it, or null and `parts`: its ten tensors one by one, where something moved them in between.
 // ws: gf_gpt_block_bytes(1, ...) bytes; the sizes of both buffers are checked as above. S must be a multiple of 128.
 GF_API int gf_gpt_block_bwd(const void* x, const void* const* params, const void* dy, const void* saved, long long saved_bytes,
-                            void* dx, void* const* grads, void* ws, long long ws_bytes, int B, int S, int E, int F, int H, int Hk,
+                            const void* const* parts, void* dx, void* const* grads, void* ws, long long ws_bytes, int B, int S, int E, int F, int H, int Hk,
                             int causal, int* status, void* stream) {
   using namespace gf;
   enter();
   const Block b(B, S, E, F, H, Hk);
-  if (!b.ok() || !x || !dy || !saved || !ws || !dx || !grads || !grads[0] || !grads[6] || S % 128) return GFH_BAD_ARG;
-  const Results s(b, true, const_cast<void*>(saved), nullptr);
+  if (!b.ok() || !x || !dy || (!saved && !parts) || !ws || !dx || !grads || !grads[0] || !grads[6] || S % 128) return GFH_BAD_ARG;
+  Results s(b, true, const_cast<void*>(saved), nullptr);
   const Temps t(b, ws);
-  if (saved_bytes < s.bytes || ws_bytes < t.bytes) return GFH_BAD_ARG;
+  if ((saved && saved_bytes < s.bytes) || ws_bytes < t.bytes) return GFH_BAD_ARG;
+  if (!saved) s.set(parts);
   const int T = b.T, P = b.P, D = b.D;
   const float scale = 1.f / sqrtf((float)D);
   int rc;

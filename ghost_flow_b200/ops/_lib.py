@@ -66,7 +66,8 @@ _SIGS = {
     "gf_flash_attn_fwd3": [P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, I, P, P],
     "gf_gpt_block_bytes": [I, I, I, I, I, I, I],
     "gf_gpt_block_fwd": [P, P, P, P, L, P, L, I, I, I, I, I, I, I, F, F, P, P],
-    "gf_gpt_block_bwd": [P, P, P, P, L, P, P, P, L, I, I, I, I, I, I, I, P, P],
+    "gf_gpt_block_parts": [P, I, I, I, I, I, I],
+    "gf_gpt_block_bwd": [P, P, P, P, L, P, P, P, P, L, I, I, I, I, I, I, I, P, P],
     "gf_flash_attn_backward": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, F, I, P, P],
     "gf_llama_decode_layer": [P, P, F, P, P, P, F, P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, P, P],
     "gf_attn_decode": [P, L, P, P, I, P, I, P, L, I, I, I, I, F, I, P, P],

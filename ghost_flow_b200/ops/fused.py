@@ -750,8 +750,33 @@ def _block_bytes(device: int, which, B, S, E, F, H, Hk) -> int:
     return _lib.cuda_lib().gf_gpt_block_bytes(which, B, S, E, F, H, Hk)
 
 
+@functools.lru_cache(maxsize=1024)
+def _block_parts(B, S, E, F, H, Hk):
+    """The tensors in the buffer that a forward pass leaves for its backward pass: first byte, last, type and shape of each."""
+    first = (ctypes.c_longlong * 10)()
+    _rc(_lib.cuda_lib().gf_gpt_block_parts(first, B, S, E, F, H, Hk), "gf_gpt_block_parts")
+    bf16, fp32 = torch.bfloat16, torch.float32
+    kinds = ((bf16, (B, S, E)), (fp32, (2, B * S)), (bf16, (B, S, H + 2 * Hk, E // H)), (bf16, (B, S, E)), (fp32, (B, H, S)),
+             (bf16, (B, S, E)), (bf16, (B, S, E)), (fp32, (2, B * S)), (bf16, (B, S, F)), (bf16, (B, S, F)))
+    return [(n, n + math.prod(s) * t.itemsize, t, s) for n, (t, s) in zip(first, kinds)]
+
+
+# private name of torch: the hooks that saved tensors go through, if any; without the name they count as present
+_SAVED_HOOKS = getattr(torch._C._autograd, "_top_saved_tensors_default_hooks", None)
+
+
+def _saved_tensors_are_hooked() -> bool:
+    return _SAVED_HOOKS is None or _SAVED_HOOKS(True) is not None
+
+
 def _nbytes(t) -> int:
     return 0 if t is None else t.numel() * t.element_size()
+
+
+def _dense16(t):
+    """``t`` itself where it is dense on a 16-byte boundary, else a copy that is."""
+    t = _dense(t)
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def _pointers(ts):
@@ -759,7 +784,8 @@ def _pointers(ts):
 
 
 class _GPTBlockFn(torch.autograd.Function):
-    """See :func:`gpt_block`. The launches of a pass are one call; what the backward pass reads again is one buffer."""
+    """See :func:`gpt_block`. The launches of a pass are one call; what the backward pass reads again is one buffer, which hooks on
+    saved tensors get as the typed tensors that it holds: a hook may do with a tensor what its type and shape tell it."""
 
     @staticmethod
     def forward(ctx, x, sizes, eps1, eps2, causal, *params):
@@ -773,24 +799,34 @@ class _GPTBlockFn(torch.autograd.Function):
         _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), at[0], _nbytes(saved), at[1], _nbytes(ws),
                                              *sizes, causal, eps1, eps2, _lib.status_word(x.device).data_ptr(),
                                              _lib.stream_ptr()), "gf_gpt_block_fwd")
-        ctx.save_for_backward(x, saved, *params)
-        ctx.args = sizes, causal
+        parts = _block_parts(*sizes) if graph and _saved_tensors_are_hooked() else None
+        kept = (saved,) if parts is None else [saved[n:e].view(t).view(s) for n, e, t, s in parts]
+        ctx.save_for_backward(x, *kept, *params)
+        ctx.args = sizes, causal, len(kept)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, saved, *params = ctx.saved_tensors
-        sizes, causal = ctx.args
-        dy = _dense(dy)
-        if dy.data_ptr() % 16:
-            dy = dy.clone()
+        sizes, causal, n = ctx.args
+        x, *kept = ctx.saved_tensors
+        x, params = _dense16(x), [None if p is None else _dense16(p) for p in kept[n:]]     # hooks may bring them back in another layout
+        kept = kept[:n]
+        saved, parts = kept[0], None
+        if n > 1:
+            for k, (_, _, t, s) in zip(kept, _block_parts(*sizes)):
+                if k.dtype is not t or k.shape != s or k.device != x.device:
+                    raise RuntimeError(f"a hook returned a saved tensor of {k.dtype} {list(k.shape)} on {k.device} for one of {t} "
+                                       f"{list(s)} on {x.device}")
+            kept = [_dense16(k) for k in kept]
+            saved, parts = None, _pointers(kept)
+        dy = _dense16(dy)
         dx = torch.empty_like(x)
         # the norms' kernels always write theirs
         grads = [torch.empty_like(p) if p is not None and (need or i in (0, 6)) else None
                  for i, (p, need) in enumerate(zip(params, ctx.needs_input_grad[5:]))]
         ws = torch.empty(_block_bytes(x.device.index, 1, *sizes), dtype=torch.uint8, device=x.device)
-        _rc(_lib.cuda_lib().gf_gpt_block_bwd(x.data_ptr(), _pointers(params), dy.data_ptr(), saved.data_ptr(), _nbytes(saved),
-                                             dx.data_ptr(), _pointers(grads), ws.data_ptr(), _nbytes(ws), *sizes, causal,
+        _rc(_lib.cuda_lib().gf_gpt_block_bwd(x.data_ptr(), _pointers(params), dy.data_ptr(), *_pointers((saved,)), _nbytes(saved),
+                                             parts, dx.data_ptr(), _pointers(grads), ws.data_ptr(), _nbytes(ws), *sizes, causal,
                                              _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()), "gf_gpt_block_bwd")
         return (dx, None, None, None, None, *grads)
 

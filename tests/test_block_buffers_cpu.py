@@ -21,7 +21,7 @@ def _call(saved_bytes, ws_bytes, backward=False, saved=1 << 20):
     lib, p = _lib.cuda_lib(), 1 << 20
     table = (ctypes.c_void_p * 12)(*[p] * 12)
     if backward:
-        return lib.gf_gpt_block_bwd(p, table, p, saved, saved_bytes, p, table, p, ws_bytes, *SIZES, 1, None, None)
+        return lib.gf_gpt_block_bwd(p, table, p, saved, saved_bytes, None, p, table, p, ws_bytes, *SIZES, 1, None, None)
     return lib.gf_gpt_block_fwd(p, table, p, saved, saved_bytes, p, ws_bytes, *SIZES, 1, 1e-5, 1e-5, None, None)
 
 
@@ -31,6 +31,17 @@ def test_buffers_that_are_too_small_are_refused(short):
     assert _call(_bytes(0) - 256 * short[0], _bytes(1) - short[1], backward=True) == BAD_ARG
     if short[1]:
         assert _call(0, _bytes(3) - 1, saved=None) == BAD_ARG
+
+
+def test_parts_of_the_buffer_are_apart_and_inside_it():
+    from ghost_flow_b200.ops.fused import _block_parts
+
+    for sizes in (SIZES, (1, 128, 128, 136, 2, 2), (3, 100, 256, 512, 4, 2)):
+        end = 0
+        for first, last, _, _ in _block_parts(*sizes):
+            assert first % 256 == 0 and end <= first < last
+            end = last
+        assert end <= _lib.cuda_lib().gf_gpt_block_bytes(0, *sizes) < end + 256
 
 
 def test_without_a_gradient_less_is_held():

@@ -3,6 +3,7 @@ import math
 
 import pytest
 import torch
+import torch.utils.checkpoint
 
 pytestmark = pytest.mark.gpu
 
@@ -174,3 +175,34 @@ def test_memory_of_a_pass_is_about_the_layers(train, most, calls):
     layers = most_held()
     hook.remove()
     assert len(calls) == 2 and one <= most * layers, (one / 1e6, layers / 1e6)
+
+
+def test_hooks_on_saved_tensors_get_typed_tensors(calls, kernel_status):
+    """A hook that stores what it is given in another form goes by type and shape; bytes would be nothing to go by."""
+    m, g = _block(256, 512, 4, 1)
+    x, dy = (torch.randn(2, 128, 256, generator=g, device="cuda").bfloat16() for _ in range(2))
+    y, full = _pass(m, x, dy)
+    seen = []
+
+    def through_the_host(t):
+        seen.append((t.dtype, tuple(t.shape)))
+        return t.t().contiguous().t().cpu() if t.dim() == 2 else t.double().cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (t.dtype, through_the_host(t)), lambda p: p[1].cuda().to(p[0])):
+        y2, grads = _pass(m, x, dy)
+    assert len(calls) == 2 and torch.equal(y, y2)
+    for n in full:
+        assert torch.equal(grads[n], full[n]), n
+    bf16, fp32 = torch.bfloat16, torch.float32
+    assert {t for t, _ in seen} == {bf16, fp32}
+    for want in ((bf16, (2, 128, 256)), (bf16, (2, 128, 512)), (bf16, (2, 128, 12, 64)), (fp32, (2, 4, 128)), (fp32, (2, 256))):
+        assert want in seen
+    y3 = torch.utils.checkpoint.checkpoint(m, x.clone().requires_grad_(), use_reentrant=False)
+    m.zero_grad()
+    y3.backward(dy)
+    for n, p in m.named_parameters():
+        assert torch.equal(p.grad, full[n]), n
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.float() if t.shape == (2, 128, 512) else t):
+        y4 = m(x.clone().requires_grad_())
+    with pytest.raises(RuntimeError, match="a hook returned a saved tensor"):
+        y4.backward(dy)
