@@ -38,7 +38,7 @@ GF_API int gf_llama_decode_layer(const void* x, const void* attn_norm, float att
                                  int B, int hidden, int inner, int Hq, int Hkv, int D, int interleaved, int pos, int splits,
                                  int* status, void* stream) {
   using namespace gf;
-  enter();
+  bind();
   if (B < 1 || B > ROWS_MAX_M || hidden <= 0 || inner <= 0 || Hq <= 0 || Hkv <= 0 || pos < 0 || pos >= s_max || splits < 1 ||
       !ws || (reinterpret_cast<uintptr_t>(ws) & 255))
     return GFH_BAD_ARG;
@@ -89,6 +89,6 @@ GF_API int gf_llama_decode_layer(const void* x, const void* attn_norm, float att
     g.X = tmp; g.ldx = inner; g.input = ROWS_PLAIN;
   }
   rc = gemm_rows_run(g, 1, st);
-  note_extra_launches(4);
+  note_extra_launches(5);                    // four products and the attention; its merge, norms and SwiGLU count themselves
   return rc;
 }

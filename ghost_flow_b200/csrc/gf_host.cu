@@ -23,7 +23,7 @@ EncodeTiledFn get_encode_fn() {
 int make_tmap_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int elem_size, uint64_t rows,
                  uint64_t cols, uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_cols,
                  CUtensorMapSwizzle swz) {
-  enter();
+  bind();
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return GFH_TMAP;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_stride_bytes & 15)) return GFH_BAD_ARG;
@@ -45,7 +45,7 @@ int make_tmap_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int
 int make_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int elem_size, uint64_t d2,
                  uint64_t rows, uint64_t cols, uint64_t row_stride_bytes, uint64_t d2_stride_bytes,
                  uint32_t box_d2, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swz) {
-  enter();
+  bind();
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return GFH_TMAP;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_stride_bytes & 15) || (d2_stride_bytes & 15))
@@ -73,10 +73,9 @@ void note_extra_launches(int n) { g_launches.fetch_add(n, std::memory_order_rela
 
 int process_device() { return t_device >= 0 ? t_device : g_device.load(std::memory_order_relaxed); }
 
-// Every exported launcher calls this first: it binds the calling thread to its device in
-// this library's copy of the CUDA runtime (PyTorch keeps its own copy, with its own per-thread state).
-void enter() {
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+// Binds the calling thread to its device in this library's copy of the CUDA runtime (PyTorch keeps its own copy, with its own
+// per-thread state).
+void bind() {
   thread_local int bound = -2;
   const int d = process_device();
   if (d < 0) {
@@ -90,6 +89,12 @@ void enter() {
     cudaSetDevice(d);
     bound = d;
   }
+}
+
+// Every exported launcher of a kernel calls this first.
+void enter() {
+  note_extra_launches(1);
+  bind();
 }
 
 int sm_count() {

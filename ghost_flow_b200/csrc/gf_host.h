@@ -76,6 +76,8 @@ int attention_head_group(int heads);
 int attention_head_group_l2(int heads, long long bytes_per_head);
 
 // Binds the calling thread to the device selected with gf_set_device (see gf_host.cu).
+void bind();
+// The same, and counts one kernel. What only calls other launchers binds, and they count.
 void enter();
 // Launchers that start more than one kernel report the extra ones here (enter() counts one).
 void note_extra_launches(int n);

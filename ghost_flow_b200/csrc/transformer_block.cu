@@ -175,7 +175,7 @@ GF_API int gf_gpt_block_fwd(const void* x, const void* const* params, void* y, v
                             long long ws_bytes, int B, int S, int E, int F, int H, int Hk, int causal, float eps1, float eps2,
                             int* status, void* stream) {
   using namespace gf;
-  enter();
+  bind();
   const Block b(B, S, E, F, H, Hk);
   if (!b.ok() || !x || !y) return GFH_BAD_ARG;
   const long long product_bytes = (4 * forward_floats(b) + 255) & ~255ll;
@@ -209,7 +209,7 @@ GF_API int gf_gpt_block_bwd(const void* x, const void* const* params, const void
                             const void* const* parts, void* dx, void* const* grads, void* ws, long long ws_bytes, int B, int S, int E, int F, int H, int Hk,
                             int causal, int* status, void* stream) {
   using namespace gf;
-  enter();
+  bind();
   const Block b(B, S, E, F, H, Hk);
   if (!b.ok() || !x || !dy || (!saved && !parts) || !ws || !dx || !grads || !grads[0] || !grads[6] || S % 128) return GFH_BAD_ARG;
   Results s(b, true, const_cast<void*>(saved), nullptr);
@@ -255,7 +255,7 @@ GF_API int gf_gpt_block_bwd(const void* x, const void* const* params, const void
 GF_API int gf_flash_attn_backward(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                                   void* dq, void* dk, void* dv, float* ws, int B, int S, int Hq, int Hkv, int D, const long long* ld,
                                   float scale, int causal, int* status, void* stream) {
-  gf::enter();
+  gf::bind();
   if (B <= 0 || S <= 0 || Hq <= 0 || S % 128 || !ws) return gf::GFH_BAD_ARG;
   const long long rows = (long long)B * Hq * S;
   float *acc = ws, *ndelta = ws + rows * D, *nlse2 = ndelta + rows;
