@@ -20,6 +20,8 @@
 // Device time in us with cold weights, the kernels that took these products before -> this one: [16, 4096] x [12288, 4096]^T 27.0 ->
 // 20.8 (4.8 TB/s), x [22016, 4096]^T 40.9 -> 33.2 (5.4 TB/s), [16, 11008] x [4096, 11008]^T 24.0 -> 19.7; back to back from the host
 // [32, 4096] x [22016, 4096]^T 54.2 -> 41.9, [64, 4096] x [4096, 4096]^T 21.9 -> 14.7, [64, 14336] x [8192, 14336]^T 55.6 -> 45.8.
+#include <atomic>
+
 #include "gemm_rows.cuh"
 #include "gf_host.h"
 #include "gf_ptx.cuh"
@@ -356,23 +358,69 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   }
 }
 
-// CTAs of a cluster, each with a part of K of at least four blocks: as many as fit on the machine at once, and a power of two
-// (clusters of 3, 6 or 7 leave SMs of a GPC out: 6144 features on 48 clusters of 6 took 22.4 us, on 48 of 4 14.7).
-static int rows_slices(int M, int N, int K) {
-  const int tiles = (N + RW_BM - 1) / RW_BM, blocks = (K + RW_BK - 1) / RW_BK;
-  const int slots = sm_count() * (M <= 16 ? RwCfg<16>::CTAS : RwCfg<64>::CTAS);
-  int s = 8;
-  while (s > 1 && (s * tiles > slots || 4 * s > blocks)) s >>= 1;
-  return s;
-}
-
 bool gemm_rows_takes(const void* X, long long ldx, const void* W, long long ldw, int M, int N, int K) {
   return M > 0 && M <= ROWS_MAX_M && N > 0 && K > 0 && K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 &&
          ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
 }
 
+static void rows_attributes(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&at)[2], int grid, int smem, int slices, int chained) {
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(RW_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)slices; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = chained ? 2 : 1;
+}
+
+// Never launched: the CTAs of this one share an SM as those of the kernel do (shared memory is what counts), and are counted so. For a
+// kernel with tensor memory the runtime counts one CTA to an SM.
+template <int NT>
+__global__ void __launch_bounds__(RW_THREADS, RwCfg<NT>::CTAS) rows_occupancy_kernel(int* p) {
+  extern __shared__ int part[];
+  if (p) *p = part[threadIdx.x];
+}
+
+// Clusters of `slices` CTAs that the current device holds at once: fewer than SMs x CTAs / slices, since a cluster lies within a
+// GPC. Asked once for each size and device.
+template <int NT>
+static int rows_clusters(int slices) {
+  using Cfg = RwCfg<NT>;
+  static std::atomic<int> known[64][4];
+  std::atomic<int>& k = known[gf::DeviceOnce::device()][slices >= 8 ? 3 : slices >> 1];
+  int n = k.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    rows_attributes(cfg, at, slices * sm_count() * Cfg::CTAS, Cfg::SMEM_BYTES, slices, 0);
+    auto kern = rows_occupancy_kernel<NT>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      return sm_count() * Cfg::CTAS / slices;
+    }
+    k.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// CTAs of a cluster, each with a part of K of at least four blocks: as many as leave all clusters on the machine at once, and a power
+// of two (clusters of 3, 6 or 7 leave SMs of a GPC out: 6144 features on 48 clusters of 6 took 22.4 us, on 48 of 4 14.7). Up to 16
+// tokens 48 clusters of 8 fit, 104 of 4, 222 of 2; with more tokens 33, 71 and 148. One more is a second wave: [8, 4096] x [N, 4096]^T, N =
+// 6272 17.1 us on 49 of 8, 13.7 on 49 of 4; 13824 27.6 on 108 of 4, 22.7 on 108 of 2; 24 tokens, 4352 16.0 on 34 of 8, 12.0 on 34
+// of 4; 9216 23.9 on 72 of 4, 17.7 on 72 of 2.
+template <int NT>
+static int rows_slices(int N, int K) {
+  const int tiles = (N + RW_BM - 1) / RW_BM, blocks = (K + RW_BK - 1) / RW_BK;
+  int s = 8;
+  while (s > 1 && (4 * s > blocks || tiles > rows_clusters<NT>(s))) s >>= 1;
+  return s;
+}
+
 template <int NT, int INPUT>
-static int launch_rows(const CUtensorMap& tm, const CUtensorMap& tx, const RowsParams& p, int slices, int chained, cudaStream_t stream) {
+static int launch_rows(const CUtensorMap& tm, const CUtensorMap& tx, const RowsParams& p, int chained, cudaStream_t stream) {
   using Cfg = RwCfg<NT>;
   auto kern = gemm_rows_kernel<NT, INPUT>;
   static gf::DeviceOnce configured;
@@ -381,27 +429,20 @@ static int launch_rows(const CUtensorMap& tm, const CUtensorMap& tx, const RowsP
       return GFH_CUDA;
     configured.mark();
   }
+  const int slices = rows_slices<NT>(p.N, p.K);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((p.N + RW_BM - 1) / RW_BM * slices));
-  cfg.blockDim = dim3(RW_THREADS);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  cfg.stream = stream;
   cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)slices; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = chained ? 2 : 1;
+  rows_attributes(cfg, at, (p.N + RW_BM - 1) / RW_BM * slices, Cfg::SMEM_BYTES, slices, chained);
+  cfg.stream = stream;
   return cudaLaunchKernelEx(&cfg, kern, tm, tx, p) == cudaSuccess ? GFH_OK : GFH_CUDA;
 }
 
 template <int INPUT>
-static int launch_rows_nt(const CUtensorMap& tm, const CUtensorMap& tx, const RowsParams& p, int slices, int chained, cudaStream_t stream) {
-  if (p.M <= 16) return launch_rows<16, INPUT>(tm, tx, p, slices, chained, stream);
+static int launch_rows_nt(const CUtensorMap& tm, const CUtensorMap& tx, const RowsParams& p, int chained, cudaStream_t stream) {
+  if (p.M <= 16) return launch_rows<16, INPUT>(tm, tx, p, chained, stream);
   if constexpr (INPUT != ROWS_PLAIN) return GFH_BAD_ARG;
-  else if (p.M <= 32) return launch_rows<32, INPUT>(tm, tx, p, slices, chained, stream);
-  else return launch_rows<64, INPUT>(tm, tx, p, slices, chained, stream);
+  else if (p.M <= 32) return launch_rows<32, INPUT>(tm, tx, p, chained, stream);
+  else return launch_rows<64, INPUT>(tm, tx, p, chained, stream);
 }
 
 // What the kernel reads as 16-byte vectors beside X and W, and the kinds that there are.
@@ -421,14 +462,13 @@ int gemm_rows_run(const RowsGemm& g, int chained, cudaStream_t stream) {
                     (!g.residual || (g.ldr % 4 == 0 && reinterpret_cast<uintptr_t>(g.residual) % 8 == 0));
   RowsParams p{(const __nv_bfloat16*)g.X, g.ldx, g.C, g.ldc, g.out_fp32, g.M, g.N, g.K, (const __nv_bfloat16*)g.norm_w, g.eps,
                (const __nv_bfloat16*)g.bias, (const __nv_bfloat16*)g.residual, g.ldr, g.alpha, g.relu, quads, g.status};
-  const int slices = rows_slices(g.M, g.N, g.K);
-  if (g.input == ROWS_RMSNORM) return launch_rows_nt<ROWS_RMSNORM>(tm, tm, p, slices, chained, stream);
-  if (g.input == ROWS_SWIGLU) return launch_rows_nt<ROWS_SWIGLU>(tm, tm, p, slices, chained, stream);
+  if (g.input == ROWS_RMSNORM) return launch_rows_nt<ROWS_RMSNORM>(tm, tm, p, chained, stream);
+  if (g.input == ROWS_SWIGLU) return launch_rows_nt<ROWS_SWIGLU>(tm, tm, p, chained, stream);
   CUtensorMap tx;
   const uint32_t rows = g.M <= 16 ? 16 : g.M <= 32 ? 32 : 64;
   const int rx = make_tmap_2d(&tx, g.X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.M, g.K, g.ldx * 2, rows, RW_BK);
   if (rx) return rx;
-  return launch_rows_nt<ROWS_PLAIN>(tm, tx, p, slices, chained, stream);
+  return launch_rows_nt<ROWS_PLAIN>(tm, tx, p, chained, stream);
 }
 
 }  // namespace gf
@@ -440,4 +480,15 @@ GF_API int gf_gemm_rows(const void* X, long long ldx, const void* W, long long l
   gf::enter();
   gf::RowsGemm g{X, ldx, W, ldw, C, ldc, out_fp32, M, N, K, (gf::RowsInput)input, norm_w, eps, bias, residual, ldr, alpha, relu, status};
   return gf::gemm_rows_run(g, 0, (cudaStream_t)stream);
+}
+
+// On the current device: the CTAs of a cluster that such a product takes (slices = 0), or the clusters of `slices`
+// CTAs that are on the machine at once.
+GF_API int gf_gemm_rows_clusters(int M, int N, int K, int slices) {
+  using namespace gf;
+  if (M < 1 || M > ROWS_MAX_M || N < 1 || K < 1 || slices < 0 || slices > 8 || (slices & (slices - 1))) return GFH_BAD_ARG;
+  bind();
+  if (slices)
+    return M <= 16 ? rows_clusters<16>(slices) : M <= 32 ? rows_clusters<32>(slices) : rows_clusters<64>(slices);
+  return M <= 16 ? rows_slices<16>(N, K) : M <= 32 ? rows_slices<32>(N, K) : rows_slices<64>(N, K);
 }

@@ -31,6 +31,7 @@ _SIGS = {
     "gf_selected_device": [],
     "gf_gemm_bf16_splits": [I, I, I, I, I, I, I, I],
     "gf_gemm_rows": [P, L, P, L, P, L, I, I, I, I, I, P, F, P, P, L, F, I, P, P],
+    "gf_gemm_rows_clusters": [I, I, I, I],
     "gf_gemm_bf16_few_rows": [I, I, I, I, I, I, I],
     "gf_gemm_bf16_workspace": [I, I, I, I, I, I, I, I, I],
     "gf_gemm_bf16": [P, P, P, I, I, I, I, L, I, L, L, I, I, P, P, L, F, P, I, I, P, I, I, P],

@@ -69,3 +69,27 @@ def test_nothing_finite_hides_what_is_not():
         assert _run(x, w, out, 8, 200, 256, inp, norm_w, None, None, 1.0, 0) == 0
         bad = ~torch.isfinite(out).all(1)
         assert bad.tolist() == [i in (2, 5) for i in range(8)] and torch.isnan(out[5]).all()
+
+
+@pytest.mark.parametrize("M,ctas", [(16, 3), (32, 2), (64, 2)])
+def test_all_clusters_of_a_product_fit_on_the_machine(M, ctas, kernel_status):
+    """Clusters lie within GPCs, so fewer of them fit than SMs and CTAs to an SM say: one that does not fit is a second wave."""
+    from ghost_flow_b200.ops import _lib
+
+    ask = _lib.cuda_lib().gf_gemm_rows_clusters
+    slots = ctas * torch.cuda.get_device_properties(0).multi_processor_count
+    fit = {s: ask(M, 1, 1, s) for s in (1, 2, 4, 8)}
+    assert all(0 < fit[s] <= slots // s for s in fit) and fit[8] <= fit[4] <= fit[2] <= fit[1] == slots
+    for K in (64, 512, 1024, 2048, 4096):
+        # around the numbers of tiles where a cluster size stops to fit, by machine and by slots
+        for tiles in {t + d for s in (2, 4, 8) for t in (fit[s], slots // s) for d in (0, 1)} | {1}:
+            most = max(s for s in (1, 2, 4, 8) if s == 1 or (tiles <= fit[s] and 4 * s <= K // 64))
+            assert ask(M, 128 * tiles, K, 0) == ask(M, 128 * tiles - 127, K, 0) == most, (K, tiles)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for tiles in (fit[8] + 1, fit[4] + 1, fit[2] + 1):
+        x, w = (torch.randn(n, 2048, generator=g, device="cuda").bfloat16() for n in (M, 128 * tiles))
+        out = torch.empty(M, 128 * tiles, device="cuda", dtype=torch.bfloat16)
+        assert _run(x, w, out, M, 128 * tiles, 2048, 0, None, None, None, 1.0, 0) == 0
+        want = x.double() @ w.double().t()
+        # fp32 sums of 2048 products, about 2048 * 2^-22 with room, and the rounding of the result
+        assert ((out.double() - want).abs() <= 2048 * 2 ** -22 + 2 ** -8 * want.abs()).all()
