@@ -919,8 +919,8 @@ static float* splitk_workspace(size_t floats) {
 
 namespace gf {
 // kernel for at most 16 rows (gemm_skinny.cu)
-bool gemm_skinny_wanted(const void* A, const void* W, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
-                        long long ldb, int accumulate, int split);
+bool gemm_skinny_takes(const void* A, const void* W, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
+                       long long ldb, int accumulate);
 int gemm_skinny_run(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                     int out_fp32, const void* bias, const void* residual, long long ldr, float alpha, int relu,
                     cudaStream_t st);
@@ -964,19 +964,31 @@ static int splitk_slices(int M, int N, int K, int out_fp32, int accumulate, int 
   return split;
 }
 
+// At most 16 rows, a long K and few features: gemm_skinny.cu has too few CTAs, each with a long chain (1.5 us per 1024 of K with at
+// most 8 rows, 2.2 with more, until all together reach the memory's speed).
+static bool few_long_rows(int M, int N, int K) { return M <= 8 ? K > 6144 && 4ll * N < K : K > 4096 && 2ll * N < K; }
+
 // Few-row products on gemm_rows.cu rather than gemm_skinny.cu (at most 16 rows) or the kernels with 128-row tiles. Its fixed cost is
-// about 2 us more than the first one's, which loads weights into registers and holds less of them in flight; it does not clear
-// and convert a workspace as the split product does. Device time in us with cold weights, there / here ([M, K] x [N, K]^T, M N K):
-//   8 512 8192 12.9 / 9.3, 8 2048 5504 11.3 / 9.7, 8 4096 11008 21.0 / 19.5, 8 4096 4096 10.5 / 10.2, 8 6144 4096 12.0 / 12.5,
-//   8 12288 4096 23.3 / 20.7, 8 15360 5120 31.4 / 28.7, 8 8192 14336 38.2 / 39.9, 8 22016 4096 32.3 / 32.1, 8 28672 4096 41.9 / 43.5, 8
-//   11008 2048 10.6 / 11.8; 16 1024 512 2.8 / 5.5, 16 2048 2048 6.2 / 6.7, 16 11008 2048 15.1 / 11.9, 16 4096 4096 11.7 / 10.5, 16 4096
-//   11008 24.0 / 19.7, 16 22016 4096 40.9 / 33.2. Back to back from the host: 32 512 256 10.5 / 8.9, 32 4096 4096 20.2 / 12.9, 32
-//   32000 4096 55.9 / 52.5; 64 512 256 10.6 / 12.6, 64 2048 2048 18.5 / 10.5, 64 12288 4096 35.1 / 29.3, 64 28672 4096 56.1 / 56.9,
-//   64 32000 4096 57.6 / 60.0.
+// about 5 us, the second one's 3; it has more weights in flight, and neither clears nor converts a workspace. Up to 16 rows it is the
+// better one where the other's last wave of CTAs (16 features; five to an SM with at most 8 rows, four with more) is too small to
+// fill the machine but takes as long as its K: up to two CTAs to an SM. Device time in us with cold weights, there / here:
+//   8 rows, K 4096: N 64 4.7 / 6.3, 128 6.1 / 6.4, 256 7.7 / 7.3, 2048 8.4 / 8.3, 4736 10.8 / 11.2 (two to an SM), 6144 11.9 / 12.6, 8192
+//   14.3 / 15.9, 11776 18.5 / 20.2 (a full wave), 11904 23.1 / 20.2, 12288 23.8 / 21.1, 15360 26.0 / 24.3, 16384 27.6 / 25.9 (two to an
+//   SM), 17408 28.3 / 26.8, 22016 32.4 / 32.6, 23552 34.8 / 35.0 (two waves), 23744 37.9 / 35.8, 28416 43.0 / 39.9, 28672 42.6 / 44.4. One
+//   row: 8192 14.1 / 16.0, 11904 21.9 / 19.7, 16384 25.7 / 25.1, 17408 26.4 / 26.5, 28416 40.3 / 39.1, 28672 40.3 / 43.2.
+//   8 rows, K 14336: 4096 25.8 / 23.4, 5120 28.9 / 27.6, 6144 31.6 / 32.3; K 2048: 1024 4.7 / 6.0, 12288 13.7 / 12.7, 16384 15.5 / 15.2.
+//   16 rows, K 2048: 6144 8.2 / 9.3, 8192 9.5 / 10.4, 11904 15.6 / 12.8, 17408 18.1 / 16.5; K 4096: 64 5.4 / 6.2, 128 7.3 / 6.6, 6144 13.4
+//   / 13.1, 11904 26.7 / 20.4, 28416 46.2 / 40.4.
+// A weight of a megabyte (three quarters with more than 8 rows) does not fill the rings. More rows: 24, K 512: 64 7.3 / 5.4; K 4096: 4096 15.3 / 11.0, 32000 52.9 / 48.6;
+// 64, K 256: 4096 7.4 / 8.8; K 512: 4096 8.6 / 8.2; K 4096: 24576 52.4 / 43.7, 32000 54.6 / 53.6; K 1024: 32000 19.1 / 19.6.
 static bool few_rows_wanted(int M, int N, int K) {
-  if (M <= 8) return (K >= 4096 && (N <= 4096 || (N > 8192 && N <= 16384))) || (K >= 5120 && N <= 6144);
-  if (M <= 16) return K >= 4096 || (K >= 2048 && N > 4096);
-  return M <= 32 || (M <= gf::ROWS_MAX_M && N <= 24576 && K >= 512);
+  if (M > 16) return M <= 32 || (M <= gf::ROWS_MAX_M && N <= 24576 && K >= 512);
+  if (few_long_rows(M, N, K)) return true;
+  if ((long long)N * K <= (M <= 8 ? 4 : 3) << 17) return false;
+  const int ctas = (N + 15) / 16, sms = gf::sm_count(), wave = sms * (M <= 8 ? 5 : 4);
+  if (M > 8) return K >= 4096 || (K >= 2048 && (ctas > wave || (K >= 3072 && N > 4096)));
+  if (K < 4096) return false;
+  return ctas <= wave ? 4 * ctas <= sms * (K >= 8192 ? 9 : 8) : (ctas - 1) % wave < 2 * sms;
 }
 
 // 1 when gf_gemm_bf16 (bn_hint and max_ctas 0) takes the few-row kernel, which needs no workspace.
@@ -994,12 +1006,13 @@ GF_API long long gf_gemm_bf16_workspace(int M, int N, int K, int a_mn_major, int
   return gf_gemm_bf16_splits(M, N, K, a_mn_major, b_mn_major, aligned, accumulate, activation) ? (long long)M * N : 0;
 }
 
-// For products that gf_gemm_bf16_few_rows does not name: 1 when gf_gemm_bf16 (bf16 result, bn_hint and max_ctas 0) takes a workspace of M * N fp32 values, else 0. aligned: bases and
-// pitches of A and B are multiples of 16 bytes.
+// For products that gf_gemm_bf16_few_rows does not name: 1 when gf_gemm_bf16 (bf16 result, bn_hint and max_ctas 0) takes a workspace of
+// M * N fp32 values, else 0. aligned: bases and pitches of A and B are multiples of 16 bytes.
 GF_API int gf_gemm_bf16_splits(int M, int N, int K, int a_mn_major, int b_mn_major, int aligned, int accumulate, int activation) {
   const int split = splitk_slices(M, N, K, 0, accumulate, activation == 1 ? 1 : 0);
   const long long pitch = aligned ? 8 : 1;
-  return split >= 2 && !gf::gemm_skinny_wanted(nullptr, nullptr, M, N, K, a_mn_major, pitch, b_mn_major, pitch, accumulate, split);
+  return split >= 2 && (few_long_rows(M, N, K) ||
+                        !gf::gemm_skinny_takes(nullptr, nullptr, M, N, K, a_mn_major, pitch, b_mn_major, pitch, accumulate));
 }
 
 // lda/ldb: row pitch in elements of the matrix as stored.
@@ -1022,7 +1035,7 @@ GF_API int gf_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int
     return gf::gemm_rows_run(g, 0, st);
   }
   if (bn_hint == 0 && max_ctas == 0 &&
-      gf::gemm_skinny_wanted(A, B, M, N, K, a_mn_major, lda, b_mn_major, ldb, accumulate, split))
+      gf::gemm_skinny_takes(A, B, M, N, K, a_mn_major, lda, b_mn_major, ldb, accumulate))
     return gf::gemm_skinny_run(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, bias, residual, ldr, alpha, p.act, st);
   // few tiles and many rows to contract, with a workspace for the sums of every part of K
   if (bn_hint == 0 && max_ctas == 0 && !out_fp32 && !accumulate && p.act == 0 && splitk_ws) {

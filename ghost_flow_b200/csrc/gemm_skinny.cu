@@ -97,15 +97,9 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __n
   }
 }
 
-// Both operands K-major, rows on 16-byte boundaries, whole 16-byte vectors along K. `split`: the number of K slices that the
-// tcgen05 path would take, 1 for none. With slices it wins where a CTA here has a long K and there are few of them: a CTA takes
-// 1.5 us per 1024 of K with one tile and 2.2 us with two, whatever N is, until all of them together reach the memory's speed.
-// Cold L2, us here / with slices: [8, 6144] x [256, 6144]^T 11.1 / 12.1, [8, 8192] x [1024, 8192]^T 14.3 / 13.3, x [2048, 8192]^T
-// 14.9 / 15.5, [8, 16384] x [512, 16384]^T 28.0 / 15.7, x [4096, 16384]^T 29.5 / 29.8, [16, 4096] x [64, 4096]^T 10.2 / 13.3,
-// [16, 8192] x [2048, 8192]^T 19.5 / 15.8, x [4096, 8192]^T 20.3 / 20.5, [16, 11008] x [4096, 11008]^T 26.9 / 23.9.
-bool gemm_skinny_wanted(const void* A, const void* W, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
-                        long long ldb, int accumulate, int split) {
-  if (split >= 2 && (M <= 8 ? K > 6144 && 4ll * N < K : K > 4096 && 2ll * N < K)) return false;
+// At most 16 rows, both operands K-major, rows on 16-byte boundaries, whole 16-byte vectors along K.
+bool gemm_skinny_takes(const void* A, const void* W, int M, int N, int K, int a_mn_major, long long lda, int b_mn_major,
+                       long long ldb, int accumulate) {
   return M <= 16 && !a_mn_major && !b_mn_major && !accumulate && K % 8 == 0 && lda % 8 == 0 && ldb % 8 == 0 &&
          ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 && M > 0 && N > 0 && K > 0;
 }
