@@ -54,15 +54,18 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint3
   asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-template <int D>
+template <int D, bool SHARES>
 struct DecCfg {
-  static constexpr int ROW = D * 2;                    // 16-byte chunk c of row r lies at chunk c ^ (r % 8): ldmatrix meets every bank once
+  static constexpr int ROW = D * 2;
   static constexpr int TILE = DEC_KEYS * ROW;          // K or V of a block
   static constexpr int WARP_BYTES = DEC_STAGES * 2 * TILE;
   static constexpr int RING = DEC_WARPS * WARP_BYTES;
   static constexpr int PITCH = D + 4;                  // a head's sums, maximum and total; the pitch spreads a lane's heads over the banks
-  static constexpr int SMEM = RING + 2 * DEC_MAX_G * PITCH * 4;
+  static constexpr int SMEM = RING + (SHARES ? 2 * DEC_MAX_G * PITCH * 4 : 0);
   static constexpr int CTAS = D > 64 ? 2 : 4;          // on an SM
+  static_assert(DEC_WARPS * DEC_MAX_G * PITCH * 4 <= RING, "results fit in the ring");
+  // 16-byte chunk c of row r lies at chunk c ^ (r % 8): ldmatrix meets every bank once, and rows fill whole lines
+  __device__ __forceinline__ static int chunk(int row, int col) { return (col ^ (row & 7)) << 4; }
 };
 
 // How the keys are dealt out. A unit is 64 keys of one KV head (16 for each warp); an empty sequence has one. Neighbouring CTAs
@@ -150,7 +153,7 @@ struct DecParams {
   const __nv_bfloat16* q;       // [B, Hq * D], pitch ldq; with append: packed rows [Hq + 2 Hkv heads of D]
   long long ldq;
   __nv_bfloat16 *kc, *vc;       // [B, s_max, Hkv * D]
-  int Hq;
+  int Hq, G;                    // G = Hq / Hkv
   float scale_log2;
   float* part;                  // [slots][G heads][D sums, maximum, total]
   __nv_bfloat16* out;
@@ -175,33 +178,49 @@ __device__ __forceinline__ void rope_words(uint32_t& lo, uint32_t& hi, const flo
   }
 }
 
-template <int D, bool APPEND>
-__global__ void __launch_bounds__(DEC_WARPS * 32, DecCfg<D>::CTAS)
+enum DecKind : int {
+  DEC_SLICES = 0,    // splits > 0
+  DEC_APPEND = 1,    // the same, with the new token's row
+  DEC_SHARES = 2,    // splits == 0
+};
+
+// Kinds of one piece to a CTA are compiled without what goes from one sequence to the next. With it, calls that the memory does not
+// bound took 5 to 25 % longer: us with / without it, 4 sequences of 64 keys, 64 / 8 heads of 64 3.8 / 3.1, 32 of 800, 32 / 8 heads of 64 13.7
+// / 11.4, 32 of 200, 32 / 32 heads of 128 32.7 / 26.5. (Padded rows instead of the exchange of chunks are 10 % slower where memory
+// bounds it: 32 of 4096 keys, 32 / 8 heads of 128 93 / 82: cp.async then fills lines in two parts.)
+template <int D, int KIND>
+__global__ void __launch_bounds__(DEC_WARPS * 32, DecCfg<D, KIND == DEC_SHARES>::CTAS)
 attn_decode_kernel(const __grid_constant__ DecParams p) {
-  using Cfg = DecCfg<D>;
+  constexpr bool SHARES = KIND == DEC_SHARES, APPEND = KIND == DEC_APPEND;
+  using Cfg = DecCfg<D, SHARES>;
   extern __shared__ __align__(128) uint8_t ring[];
   const DecWork& w = p.work;
-  const int G = p.Hq / w.Hkv;
+  const int G = p.G;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = lane >> 2, c = lane & 3;
   if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int hk = blockIdx.x % w.Hkv, part = blockIdx.x / w.Hkv;
   DecAt at;
   int left_units;                  // of this CTA's part
-  if (w.splits > 0) {
-    at.b = part / w.splits;
-    const int sp = part - at.b * w.splits;
-    at.len = w.len(at.b);
-    at.n = DecWork::units(at.len);
-    at.blk = (int)((long long)sp * at.n / w.splits);
-    left_units = (int)((long long)(sp + 1) * at.n / w.splits) - at.blk;
-  } else {
+  if constexpr (SHARES) {
     int total;
     dec_units_before(w, 0, total);
     const int parts = min(w.parts, total);                       // none is empty
     const int u0 = (int)((long long)part * total / parts);
     left_units = part < parts ? (int)((long long)(part + 1) * total / parts) - u0 : 0;
     if (left_units > 0) at = dec_find(w, u0);
+  } else {
+    at.b = part;
+    if (w.splits > 1) at.b = part / w.splits;
+    at.len = w.len(at.b);
+    at.n = left_units = DecWork::units(at.len);
+    at.blk = 0;
+    if (w.splits > 1) {
+      const unsigned sp = part - at.b * w.splits, splits = w.splits;             // sp n / splits in 32 bits: splits < 2^16
+      const unsigned each = (unsigned)at.n / splits, rest = (unsigned)at.n - each * splits;
+      at.blk = (int)(sp * each + sp * rest / splits);
+      left_units = (int)((sp + 1) * each + (sp + 1) * rest / splits) - at.blk;
+    }
   }
   if (left_units <= 0) return;
   const long long row_stride = (long long)w.Hkv * D, batch_stride = (long long)w.s_max * row_stride;
@@ -209,19 +228,19 @@ attn_decode_kernel(const __grid_constant__ DecParams p) {
   const uint32_t my = smem_u32(ring) + warp * Cfg::WARP_BYTES;
   DecAt ahead = at;
   int ahead_units = left_units;
+  long long head = at.b * batch_stride + (long long)hk * D;      // of the sequence ahead
   // keys of this warp's next unit into stage `st`; one commit group per unit, empty ones behind the part
   auto load = [&](int st) {
     const int k0 = ahead.blk * 64 + warp * DEC_KEYS;
     if (ahead_units > 0 && k0 < ahead.len) {
       const uint32_t dst = my + st * (2 * Cfg::TILE);
-      const long long head = ahead.b * batch_stride + (long long)hk * D;
       const int lim = ahead.len - (APPEND ? 1 : 0);              // rows to read: the new token's comes from registers
 #pragma unroll
       for (int n = 0; n < DEC_KEYS * D / 8 / 32; ++n) {
         const int id = lane + n * 32, row = id / (D / 8), col = id % (D / 8);
         const int key = k0 + row;
         const long long off = head + (long long)max(0, min(key, lim - 1)) * row_stride + col * 8;
-        const uint32_t to = dst + row * Cfg::ROW + ((col ^ (row & 7)) << 4);
+        const uint32_t to = dst + row * Cfg::ROW + Cfg::chunk(row, col);
         if (wide) {
           const uint32_t bytes = key < lim ? 16u : 0u;
           cp_async_16(to, p.kc + off, bytes);
@@ -236,7 +255,15 @@ attn_decode_kernel(const __grid_constant__ DecParams p) {
         }
       }
     }
-    if (--ahead_units > 0) ahead.next(w);
+    --ahead_units;
+    if constexpr (SHARES) {
+      if (ahead_units > 0) {
+        ahead.next(w);
+        head = ahead.b * batch_stride + (long long)hk * D;
+      }
+    } else {
+      ++ahead.blk;
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
@@ -247,52 +274,48 @@ attn_decode_kernel(const __grid_constant__ DecParams p) {
   float o[D / 16][4];              // O^T: dims 16 j + r (+ 8), heads 2c, 2c + 1
   float m[2], l[2];
   uint4 k_new, v_new;              // append: chunk `lane` of the new token's rows, in the warp whose keys it belongs to
-  bool begins = false;             // the piece in work starts with its head's first unit
-  int st = 0, st_load = DEC_STAGES - 1;
-  for (bool first = true; left_units > 0; first = false) {
-    load(st_load);
-    if (++st_load == DEC_STAGES) st_load = 0;
-    if (first || at.blk == 0) {
-      begins = at.blk == 0;
-      const unsigned short* qp = reinterpret_cast<const unsigned short*>(
-          p.q + at.b * p.ldq + (long long)(hk * G + min(r, G - 1)) * D + 2 * c);
+  // ---- start of a piece
+  auto begin = [&] {
+    const unsigned short* qp = reinterpret_cast<const unsigned short*>(
+        p.q + at.b * p.ldq + (long long)(hk * G + min(r, G - 1)) * D + 2 * c);
 #pragma unroll
-      for (int t = 0; t < D / 16; ++t) {
-        qb[t][0] = r < G ? qp[16 * t] | ((uint32_t)qp[16 * t + 1] << 16) : 0u;
-        qb[t][1] = r < G ? qp[16 * t + 8] | ((uint32_t)qp[16 * t + 9] << 16) : 0u;
-      }
-      if (APPEND) {
-        if (lane < D / 8) {
-          const __nv_bfloat16* kn = p.q + at.b * p.ldq + (long long)(p.Hq + hk) * D;
-          const int pc = (lane + D / 16) % (D / 8);              // the chunk half a head away
-          k_new = *reinterpret_cast<const uint4*>(kn + lane * 8);
-          v_new = *reinterpret_cast<const uint4*>(kn + (long long)w.Hkv * D + lane * 8);
-          uint4 k_far = *reinterpret_cast<const uint4*>(kn + pc * 8);
-          uint32_t *x = reinterpret_cast<uint32_t*>(&k_new), *y = reinterpret_cast<uint32_t*>(&k_far);
-          const bool low = lane < D / 16;
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            rope_words(low ? x[e] : y[e], low ? y[e] : x[e], p.cos_row, p.sin_row, (low ? lane : pc) * 8 + 2 * e, D / 2,
-                       p.interleaved);
-        }
-#pragma unroll
-        for (int t = 0; t < D / 32; ++t)
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            rope_words(qb[t][h], qb[t + D / 32][h], p.cos_row, p.sin_row, 16 * t + 2 * c + 8 * h, D / 2, p.interleaved);
-      }
-#pragma unroll
-      for (int j = 0; j < D / 16; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-      m[0] = m[1] = -INFINITY;
-      l[0] = l[1] = 0.f;
+    for (int t = 0; t < D / 16; ++t) {
+      qb[t][0] = r < G ? qp[16 * t] | ((uint32_t)qp[16 * t + 1] << 16) : 0u;
+      qb[t][1] = r < G ? qp[16 * t + 8] | ((uint32_t)qp[16 * t + 9] << 16) : 0u;
     }
+    if (APPEND) {
+      if (lane < D / 8) {
+        const __nv_bfloat16* kn = p.q + at.b * p.ldq + (long long)(p.Hq + hk) * D;
+        const int pc = (lane + D / 16) % (D / 8);                // the chunk half a head away
+        k_new = *reinterpret_cast<const uint4*>(kn + lane * 8);
+        v_new = *reinterpret_cast<const uint4*>(kn + (long long)w.Hkv * D + lane * 8);
+        uint4 k_far = *reinterpret_cast<const uint4*>(kn + pc * 8);
+        uint32_t *x = reinterpret_cast<uint32_t*>(&k_new), *y = reinterpret_cast<uint32_t*>(&k_far);
+        const bool low = lane < D / 16;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          rope_words(low ? x[e] : y[e], low ? y[e] : x[e], p.cos_row, p.sin_row, (low ? lane : pc) * 8 + 2 * e, D / 2, p.interleaved);
+      }
+#pragma unroll
+      for (int t = 0; t < D / 32; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          rope_words(qb[t][h], qb[t + D / 32][h], p.cos_row, p.sin_row, 16 * t + 2 * c + 8 * h, D / 2, p.interleaved);
+    }
+#pragma unroll
+    for (int j = 0; j < D / 16; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+    m[0] = m[1] = -INFINITY;
+    l[0] = l[1] = 0.f;
+  };
+  // ---- the unit at `at`, in stage st
+  auto unit = [&](int st) {
     asm volatile("cp.async.wait_group %0;" ::"n"(DEC_STAGES - 1) : "memory");
     __syncwarp();
     const int left = at.len - (at.blk * 64 + warp * DEC_KEYS);    // valid keys of the block
     if (APPEND && left > 0 && left <= DEC_KEYS) {                 // the new token is the last valid key: into the ring and the caches
       if (lane < D / 8) {
         const int row = left - 1;
-        uint8_t* to = ring + (my - smem_u32(ring)) + st * (2 * Cfg::TILE) + row * Cfg::ROW + ((lane ^ (row & 7)) << 4);
+        uint8_t* to = ring + (my - smem_u32(ring)) + st * (2 * Cfg::TILE) + row * Cfg::ROW + Cfg::chunk(row, lane);
         *reinterpret_cast<uint4*>(to) = k_new;
         *reinterpret_cast<uint4*>(to + Cfg::TILE) = v_new;
         const long long off = at.b * batch_stride + (long long)(at.len - 1) * row_stride + (long long)hk * D + lane * 8;
@@ -303,12 +326,12 @@ attn_decode_kernel(const __grid_constant__ DecParams p) {
     }
     if (left > 0) {
       const uint32_t tk = my + st * (2 * Cfg::TILE), tv = tk + Cfg::TILE;
-      // ---- S^T: keys r, r + 8 by heads 2c, 2c + 1
+      // S^T: keys r, r + 8 by heads 2c, 2c + 1
       float sc[4] = {0.f, 0.f, 0.f, 0.f}, sd[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int t = 0; t < D / 16; ++t) {
         uint32_t a[4];
-        ldmatrix_x4(a, tk + (lane & 15) * Cfg::ROW + (((2 * t + (lane >> 4)) ^ (lane & 7)) << 4));
+        ldmatrix_x4(a, tk + (lane & 15) * Cfg::ROW + Cfg::chunk(lane, 2 * t + (lane >> 4)));
         if (t & 1) mma_bf16_16816(sd, a[0], a[1], a[2], a[3], qb[t][0], qb[t][1]);
         else mma_bf16_16816(sc, a[0], a[1], a[2], a[3], qb[t][0], qb[t][1]);
       }
@@ -341,113 +364,138 @@ attn_decode_kernel(const __grid_constant__ DecParams p) {
           pt[n][h] = transpose_8x8(x);
         }
       }
-      // ---- O^T += V^T P^T
+      // O^T += V^T P^T
 #pragma unroll
       for (int j = 0; j < D / 16; ++j) {
         uint32_t a[4];
-        ldmatrix_x4_trans(a, tv + ((lane & 7) + ((lane >> 4) << 3)) * Cfg::ROW +
-                                 (((2 * j + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+        ldmatrix_x4_trans(a, tv + ((lane & 7) + ((lane >> 4) << 3)) * Cfg::ROW + Cfg::chunk(lane, 2 * j + ((lane >> 3) & 1)));
         o[j][0] *= corr[0]; o[j][1] *= corr[1]; o[j][2] *= corr[0]; o[j][3] *= corr[1];
 #pragma unroll
         for (int n = 0; n < DEC_P_TERMS; ++n) mma_bf16_16816(o[j], a[0], a[1], a[2], a[3], pt[n][0], pt[n][1]);
       }
     }
     __syncwarp();                  // the stage is filled again two units on
-    if (++st == DEC_STAGES) st = 0;
-    const bool ends = at.blk == at.n - 1;
-    if (ends || left_units == 1) {
-      // ---- the warps' results meet: in the ring behind the last piece, else in two buffers of their own, in two steps (2 and 3
-      // give theirs to 0 and 1, then 1 to 0) while the ring fills with the next sequence
+  };
+  // ---- end of a piece: the warps' results meet, in the ring behind the CTA's last piece, else in two buffers of their own, in two
+  // steps (2 and 3 give theirs to 0 and 1, then 1 to 0) while the ring fills with the next sequence. whole: the piece is a sequence
+  auto finish = [&](const bool last, const bool whole, const long long slot_of) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      l[e] += __shfl_xor_sync(0xffffffffu, l[e], 4);
+      l[e] += __shfl_xor_sync(0xffffffffu, l[e], 8);
+      l[e] += __shfl_xor_sync(0xffffffffu, l[e], 16);
+    }
+    constexpr int BUF = DEC_MAX_G * Cfg::PITCH;
+    float* buf = reinterpret_cast<float*>(ring + (last ? 0 : Cfg::RING));
+    auto give = [&](float* to) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 4);
-        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 8);
-        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 16);
+        float* g = to + (2 * c + e) * Cfg::PITCH;
+#pragma unroll
+        for (int j = 0; j < D / 16; ++j) {
+          g[16 * j + r] = o[j][e];
+          g[16 * j + 8 + r] = o[j][2 + e];
+        }
+        if (r == 0) {
+          g[D] = m[e];
+          g[D + 1] = l[e];
+        }
       }
-      constexpr int BUF = DEC_MAX_G * Cfg::PITCH;
-      const bool last = left_units == 1;
-      float* buf = reinterpret_cast<float*>(ring + (last ? 0 : Cfg::RING));
-      auto give = [&](float* to) {
+    };
+    if (last) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      give(buf + warp * BUF);
+    } else {
+      auto take = [&](const float* from) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          float* g = to + (2 * c + e) * Cfg::PITCH;
+          const float* g = from + (2 * c + e) * Cfg::PITCH;
+          const float mo = g[D], mn = fmaxf(m[e], mo), ref = mn == -INFINITY ? 0.f : mn;
+          const float ca = ex2_approx(m[e] - ref), cb = ex2_approx(mo - ref);
+          m[e] = mn;
+          l[e] = l[e] * ca + g[D + 1] * cb;
 #pragma unroll
           for (int j = 0; j < D / 16; ++j) {
-            g[16 * j + r] = o[j][e];
-            g[16 * j + 8 + r] = o[j][2 + e];
-          }
-          if (r == 0) {
-            g[D] = m[e];
-            g[D + 1] = l[e];
+            o[j][e] = o[j][e] * ca + g[16 * j + r] * cb;
+            o[j][2 + e] = o[j][2 + e] * ca + g[16 * j + 8 + r] * cb;
           }
         }
+        __syncwarp();              // read by all lanes before the buffer is written again
       };
-      if (last) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        give(buf + warp * BUF);
-      } else {
-        auto take = [&](const float* from) {
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float* g = from + (2 * c + e) * Cfg::PITCH;
-            const float mo = g[D], mn = fmaxf(m[e], mo), ref = mn == -INFINITY ? 0.f : mn;
-            const float ca = ex2_approx(m[e] - ref), cb = ex2_approx(mo - ref);
-            m[e] = mn;
-            l[e] = l[e] * ca + g[D + 1] * cb;
-#pragma unroll
-            for (int j = 0; j < D / 16; ++j) {
-              o[j][e] = o[j][e] * ca + g[16 * j + r] * cb;
-              o[j][2 + e] = o[j][2 + e] * ca + g[16 * j + 8 + r] * cb;
-            }
-          }
-          __syncwarp();              // read by all lanes before the buffer is written again
-        };
-        if (warp >= 2) give(buf + (warp - 2) * BUF);
-        __syncthreads();
-        if (warp < 2) take(buf + warp * BUF);
-        if (warp == 1) give(buf + BUF);
-        __syncthreads();
-        if (warp == 0) {
-          take(buf + BUF);
-          give(buf);
-        }
-      }
+      if (warp >= 2) give(buf + (warp - 2) * BUF);
       __syncthreads();
-      const int have = last ? DEC_WARPS : 1;
-      __nv_bfloat16* to = p.out + at.b * p.ldo + (long long)hk * G * D;
-      float* slot = p.part + (long long)(w.splits > 0 ? blockIdx.x : 2 * blockIdx.x + begins) * G * (D + 2);
-      for (int i = threadIdx.x; i < G * D; i += DEC_WARPS * 32) {
-        const int g = i / D, d = i % D;
-        const float* x = buf + g * Cfg::PITCH;
-        float mm = x[D], ll = x[D + 1], ov = x[d];
-        if (have > 1) {
-#pragma unroll
-          for (int k = 1; k < DEC_WARPS; ++k) mm = fmaxf(mm, x[k * BUF + D]);
-          const float ref = mm == -INFINITY ? 0.f : mm;
-          float e = ex2_approx(x[D] - ref);
-          ll *= e;
-          ov *= e;
-#pragma unroll
-          for (int k = 1; k < DEC_WARPS; ++k) {
-            e = ex2_approx(x[k * BUF + D] - ref);
-            ll += x[k * BUF + D + 1] * e;
-            ov += x[k * BUF + d] * e;
-          }
-        }
-        if (begins && ends) {
-          to[i] = __float2bfloat16(ll > 0.f ? ov / ll : 0.f);
-        } else {
-          slot[g * (D + 2) + d] = ov;
-          if (d == 0) {
-            slot[g * (D + 2) + D] = mm;
-            slot[g * (D + 2) + D + 1] = ll;
-          }
-        }
-      }
+      if (warp < 2) take(buf + warp * BUF);
+      if (warp == 1) give(buf + BUF);
       __syncthreads();
+      if (warp == 0) {
+        take(buf + BUF);
+        give(buf);
+      }
     }
-    if (--left_units > 0) at.next(w);
+    __syncthreads();
+    const int have = last ? DEC_WARPS : 1;
+    __nv_bfloat16* to = p.out + at.b * p.ldo + (long long)hk * G * D;
+    float* slot = p.part + slot_of * G * (D + 2);
+    for (int i = threadIdx.x; i < G * D; i += DEC_WARPS * 32) {
+      const int g = i / D, d = i % D;
+      const float* x = buf + g * Cfg::PITCH;
+      float mm = x[D], ll = x[D + 1], ov = x[d];
+      if (have > 1) {
+#pragma unroll
+        for (int k = 1; k < DEC_WARPS; ++k) mm = fmaxf(mm, x[k * BUF + D]);
+        const float ref = mm == -INFINITY ? 0.f : mm;
+        float e = ex2_approx(x[D] - ref);
+        ll *= e;
+        ov *= e;
+#pragma unroll
+        for (int k = 1; k < DEC_WARPS; ++k) {
+          e = ex2_approx(x[k * BUF + D] - ref);
+          ll += x[k * BUF + D + 1] * e;
+          ov += x[k * BUF + d] * e;
+        }
+      }
+      if (whole) {
+        to[i] = __float2bfloat16(ll > 0.f ? ov / ll : 0.f);
+      } else {
+        slot[g * (D + 2) + d] = ov;
+        if (d == 0) {
+          slot[g * (D + 2) + D] = mm;
+          slot[g * (D + 2) + D + 1] = ll;
+        }
+      }
+    }
+  };
+
+  int st = 0, st_load = DEC_STAGES - 1;
+  if constexpr (!SHARES) {
+    const bool whole = left_units == at.n;
+    begin();
+    for (; left_units > 0; --left_units, ++at.blk) {
+      load(st_load);
+      if (++st_load == DEC_STAGES) st_load = 0;
+      unit(st);
+      if (++st == DEC_STAGES) st = 0;
+    }
+    finish(true, whole, blockIdx.x);
+  } else {
+    bool begins = false;           // the piece in work starts with its head's first unit
+    for (bool first = true; left_units > 0; first = false) {
+      load(st_load);
+      if (++st_load == DEC_STAGES) st_load = 0;
+      if (first || at.blk == 0) {
+        begins = at.blk == 0;
+        begin();
+      }
+      unit(st);
+      if (++st == DEC_STAGES) st = 0;
+      const bool ends = at.blk == at.n - 1;
+      if (ends || left_units == 1) {
+        finish(left_units == 1, begins && ends, 2 * (long long)blockIdx.x + begins);
+        __syncthreads();
+      }
+      if (--left_units > 0) at.next(w);
+    }
   }
 }
 
@@ -457,7 +505,7 @@ template <int D>
 __global__ void __launch_bounds__(D) attn_decode_merge_kernel(const __grid_constant__ DecParams p) {
   __shared__ float share[D];                       // exp2(maximum of piece k - maximum of all)
   const DecWork& w = p.work;
-  const int G = p.Hq / w.Hkv, b = blockIdx.x, h = blockIdx.y, hk = h / G, g = h - hk * G, d = threadIdx.x;
+  const int G = p.G, b = blockIdx.x, h = blockIdx.y, hk = h / G, g = h - hk * G, d = threadIdx.x;
   const long long piece = (long long)G * (D + 2);
   const float *first, *rest;                       // the first piece's sums, and where piece k > 0 is: rest + k * step
   long long step;
@@ -542,12 +590,13 @@ __global__ void __launch_bounds__(D) attn_decode_merge_kernel(const __grid_const
   p.out[b * p.ldo + (long long)h * D + d] = __float2bfloat16(l > 0.f ? o / l : 0.f);
 }
 
-template <int D, bool APPEND>
+template <int D, int KIND>
 static int launch_decode(const DecParams& p, int chained, cudaStream_t st) {
   static gf::DeviceOnce configured;
-  auto kern = attn_decode_kernel<D, APPEND>;
+  constexpr int SMEM = DecCfg<D, KIND == DEC_SHARES>::SMEM;
+  auto kern = attn_decode_kernel<D, KIND>;
   if (configured.todo()) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DecCfg<D>::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
       return GFH_CUDA;
     configured.mark();
   }
@@ -557,7 +606,7 @@ static int launch_decode(const DecParams& p, int chained, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((p.work.splits > 0 ? p.work.B * p.work.splits : p.work.parts) * p.work.Hkv));
   cfg.blockDim = dim3(DEC_WARPS * 32);
-  cfg.dynamicSmemBytes = DecCfg<D>::SMEM;
+  cfg.dynamicSmemBytes = SMEM;
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = chained ? 1 : 0;
@@ -578,11 +627,12 @@ int attn_decode_append(const void* qkv, long long ldq, void* kcache, void* vcach
   if (B <= 0 || Hkv <= 0 || Hq % Hkv || Hq / Hkv > DEC_MAX_G || (D != 64 && D != 128) || splits < 1 || !scratch || len < 1 ||
       len > s_max || ldq % 8)
     return GFH_BAD_ARG;
+  if (splits > 65535) splits = 65535;
   for (const void* x : {qkv, (const void*)kcache, (const void*)vcache})       // the new token's rows are read and written as vectors
     if (!x || (reinterpret_cast<uintptr_t>(x) & 15)) return GFH_BAD_ARG;
   DecParams p{{nullptr, len, s_max, B, Hkv, 0, splits}, (const __nv_bfloat16*)qkv, ldq, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache,
-              Hq, scale * 1.4426950408889634f, scratch, (__nv_bfloat16*)out, ldo, cos_row, sin_row, interleaved};
-  return D == 128 ? launch_decode<128, true>(p, chained, st) : launch_decode<64, true>(p, chained, st);
+              Hq, Hq / Hkv, scale * 1.4426950408889634f, scratch, (__nv_bfloat16*)out, ldo, cos_row, sin_row, interleaved};
+  return D == 128 ? launch_decode<128, DEC_APPEND>(p, chained, st) : launch_decode<64, DEC_APPEND>(p, chained, st);
 }
 
 }  // namespace gf
@@ -598,7 +648,10 @@ GF_API int gf_attn_decode(const void* q, long long ldq, const void* kcache, cons
                           float scale, int splits, float* scratch, void* stream) {
   gf::enter();
   if (B <= 0 || Hkv <= 0 || Hq % Hkv || Hq / Hkv > DEC_MAX_G || (D != 64 && D != 128) || splits == 0 || !scratch) return GFH_BAD_ARG;
+  if (splits > 65535) splits = 65535;
   DecParams p{{lens, len_all, s_max, B, Hkv, splits < 0 ? -splits : 0, splits > 0 ? splits : 0}, (const __nv_bfloat16*)q, ldq, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache,
-              Hq, scale * 1.4426950408889634f, scratch, (__nv_bfloat16*)out, ldo, nullptr, nullptr, 0};
-  return D == 128 ? launch_decode<128, false>(p, 0, (cudaStream_t)stream) : launch_decode<64, false>(p, 0, (cudaStream_t)stream);
+              Hq, Hq / Hkv, scale * 1.4426950408889634f, scratch, (__nv_bfloat16*)out, ldo, nullptr, nullptr, 0};
+  if (splits < 0)
+    return D == 128 ? launch_decode<128, DEC_SHARES>(p, 0, (cudaStream_t)stream) : launch_decode<64, DEC_SHARES>(p, 0, (cudaStream_t)stream);
+  return D == 128 ? launch_decode<128, DEC_SLICES>(p, 0, (cudaStream_t)stream) : launch_decode<64, DEC_SLICES>(p, 0, (cudaStream_t)stream);
 }
