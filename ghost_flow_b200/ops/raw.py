@@ -239,44 +239,58 @@ def adamw_flat(p32, m, v, g, p_lp, *, lr, beta1, beta2, eps, weight_decay, step,
 
 
 # ------------------------------------------------------------------ decode attention over a KV cache
+# up to eight the merge reads all pieces at once; of more, only 16 was ever the best
+_SLICES = 1, 2, 3, 4, 5, 6, 7, 8, 16
+
+
 @functools.lru_cache(maxsize=1024)
 def _even_slices(ctas: int, blocks: int, D: int, sms: int) -> int:
-    """Slices of the cache for sequences of one length (``blocks`` of 128 rows, the shortest slice), ``ctas`` CTAs to a slice:
-    the number with the least estimated time. That is a wave of CTAs after the other (two to an SM, four with D = 64), a full one at
-    memory speed, the last one as long as its fullest SM needs: one, two, three CTAs of an SM take .55 and .8 of a full
-    wave (D = 64: .31, .43, .56, then .9); as long as 60 rows for another wave, 80 for the merge and 5 for each slice in it.
-    Over 183 combinations of sizes the choice takes 0.5 % longer than the best one on average and 7 % at most.
-    Measured at 4000 keys, us with 1 / 2 / 3 / 4 / 5 slices: D = 128, 160 CTAs 80 / 86 / 63 / 69 / 61; 248 CTAs 82 / 89 / 91 /
-    91 / 93; 320 CTAs 159 / 128 / 118 / 113 / 113; 496 CTAs 165 / 168 / 166 / 161 / 165; D = 64, 240 CTAs 46 / 53 / 54 / 47 / 48, 636
-    CTAs 138 / 114 / 115 / 113 / 113. At 300 keys and 96 CTAs, 1 / 2: 7.4 / 9.0, D = 64 5.1 / 7.0."""
-    steps = (.55, .8) if D > 64 else (.31, .43, .56, .9)
+    """Slices of the cache for sequences of one length (``blocks`` of 128 rows, the shortest slice), ``ctas`` CTAs to a slice: the number
+    with the least estimated time. That is a wave of CTAs after the other (two to an SM, four with D = 64), a full one at
+    memory speed, the last one as long as its fullest SM needs: one, two, three CTAs of an SM take .53 and .72 of a full
+    wave (D = 64: .32, .44, .58, then .93); as long as 85 rows for another wave, 70 for the merge, 3 for each slice in it, 70 for more
+    than eight. Over 351 combinations of 1 to 64 sequences, 2 to 32 heads in the cache and 64 to 8000 keys the choice takes
+    0.3 % longer than the best one on average and 9 % at most. Measured, us with 1 / 2 / 3 / 4 / 8 / 16 slices: D = 128, 8 CTAs at 4000 keys
+    50.5 / 28.2 / 20.4 / 16.7 / 10.8 / 9.9; 160 CTAs at 4000 61.4 / 73.9 / 54.7 / 63.0 / 58.8; 248 CTAs at 4000 79.9 / 80.9 / 85.0 / 88.7 / 88.6; 96 CTAs at 300, 1 / 2
+    6.8 / 7.6; D = 64, 32 CTAs at 2048 18.0 / 12.0 / 9.7 / 8.5 / 7.9 / 10.8; 256 CTAs at 4000 42.9 / 47.6 / 52.8 / 46.9 / 48.6."""
+    steps = (.53, .72) if D > 64 else (.32, .44, .58, .93)
     slots, n = sms * len(steps), 128 * blocks
-    if 2 * ctas <= sms:                  # far from filling the machine: as many slices as there may be
-        return max(1, min(32, slots // ctas, blocks))
     best = cost = None
-    for s in range(1, min(8, blocks) + 1):
+    for s in _SLICES:
+        if s > max(1, blocks):
+            break
         waves, rest = divmod(ctas * s, slots)
         tail = max(steps[-(-rest // sms) - 1], rest / slots) if rest else 0.
-        c = -(-n // s) * (waves + tail) + 60 * (waves - (not rest)) + (80 + 5 * s if s > 1 else 0)
+        c = -(-n // s) * (waves + tail) + 85 * (waves - (not rest)) + (70 + 3 * s + 70 * (s > 8) if s > 1 else 0)
         if best is None or c < cost:
             best, cost = s, c
     return best
 
 
+@functools.lru_cache(maxsize=1024)
 def _decode_parts(B: int, Hkv: int, n: int, D: int, sms: int, per_seq: bool) -> int:
     """How decode attention cuts the keys of ``B`` sequences of at most ``n`` keys: parts of each sequence, or, negative, the number of
-    parts of all sequences together (one wave of CTAs, whatever the lengths are)."""
+    parts of all sequences together (one wave of CTAs, whatever the lengths are).
+
+    Lengths that differ are not known here. Slices of each sequence: a piece takes .34 of a full wave's time (D = 64: .2) and up to .15 more
+    as the machine fills, a wave of CTAs more as long as 150 rows, the merge 52, each slice in it 6, more than eight 110. Shares
+    of all sequences cost 5 us for finding a share's sequences and the pieces that begin and end inside one, and are taken where there
+    are 40 units of 64 keys to a CTA and sequences of 2048 keys: lengths far apart then matter more. Over 219 combinations of 2 to
+    64 sequences and 130 to 8000 keys, with lengths uniform / one in eight long and the others a 16th / all full, the choice takes 3 /
+    6 / 6 % longer than the best of all on average. us with 1 / 2 / 4 / 8 slices / shares, uniform lengths: 62 sequences of 1 .. 300, 64 /
+    8 heads of 128 15.6 / 25.8 / 33.2 / - / 28.2; 4 of 1 .. 4000, 64 / 8 heads of 128 39.1 / 23.8 / 15.7 / 13.0 / 16.5; 8 of 1 .. 4000, 32 / 8 heads
+    of 64 24.4 / 15.5 / 12.2 / 11.0 / 14.2; 32 of 1 .. 4000, 32 / 8 heads of 128 62.1 / 59.9 / 53.8 / 57.1 / 54.8, one in eight long
+    55.6 / 41.7 / 34.9 / 31.2 / 28.8."""
     heads = max(1, B * Hkv)
     if not per_seq:
         return _even_slices(heads, max(1, (n + 127) // 128), D, sms)
-    slots = sms * (2 if D > 64 else 4)
-    # With eight units of 64 keys to a CTA the shares of all sequences together are worth the scan of the lengths and the pieces
-    # that begin and end inside a sequence (about 5 us): us with slices of each sequence / together, 32 sequences of 1 .. 4096 keys,
-    # 32 / 8 heads of 128 60.0 / 55.0, 64 of 1 .. 2048, 64 / 8 heads 70.3 / 64.4, 64 of 1 .. 1000, 16 / 16 of 64 33.3 / 30.8; 16 of
-    # 1 .. 128, 32 / 32 of 128 10.8 / 14.7, 2 of 1 .. 4000, 12 / 12 of 64 15.9 / 14.6. Two waves are slower everywhere.
-    if heads * ((n + 63) // 64) >= 8 * slots:
+    slots, units = sms * (2 if D > 64 else 4), (n + 63) // 64
+    if units >= 32 and heads * units >= 40 * slots:
         return -max(1, slots // Hkv)
-    return max(1, min(32, -(-(sms * 8) // heads), (n + 127) // 128))
+    piece = .34 if D > 64 else .2
+    cost = lambda s: (64 * -(-units // s) * (piece + .15 * min(1., heads * s / slots))  # noqa: E731
+                      + 150 * max(0., heads * s / slots - 1) + (52 + 6 * s + 110 * (s > 8) if s > 1 else 0))
+    return min((s for s in _SLICES if s <= max(1, units)), key=cost)
 
 
 def attn_decode(q, kcache, vcache, length, B, Hq, Hkv, D, scale=None, splits=None, out=None):
