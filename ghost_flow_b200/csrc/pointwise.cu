@@ -174,18 +174,21 @@ embedding_rows_kernel(const I* __restrict__ ids, const uint4* __restrict__ table
 
 // ------------------------------------------------------------------ SwiGLU
 // gu is [T, 2F] (gate columns [0,F), up columns [F,2F)); y = silu(g) * u is [T, F].
-// Bound by memory: a thread has EW_BATCH vectors of each operand, 256 vectors apart, and issues their loads before it uses the first.
-// Index is a 32-bit type where the sizes allow it: the division by the row length was a 64-bit one for every vector.
-// [2048, 2 x 11008] forward 32 -> 26 us (5.2 TB/s), backward 40.5 -> 38.5 (5.9 TB/s).
-constexpr int EW_BATCH = 2;
-template <typename Index>
+// Bound by memory: a thread has BATCH vectors of each operand, 256 vectors apart, and issues their loads before it uses the first. Index
+// is a 32-bit type where the sizes allow it: the division by the row length was a 64-bit one for every vector. Two vectors pay where
+// their loads wait for memory; a call that the L2 holds or that leaves the machine partly empty has more threads with one. us with one / two:
+// forward [1, 2 x 11008] 2.1 / 2.7, [256, 2 x 5504] 3.1 / 3.6, [512, 2 x 11008] 8.3 / 8.5, [700, 2 x 11008] 10.4 / 10.0, [2048, 2 x 11008] 26.9
+// / 24.9, [8192, 2 x 14336] 121.7 / 108.8; backward [256, 2 x 5504] 3.8 / 4.4, [1024, 2 x 11008] 19.1 / 19.6, [2048, 2 x 11008] 36.2 / 36.2,
+// [8192, 2 x 14336] 170.3 / 168.3.
+constexpr long long SWIGLU_FWD_ONE = 6 << 20, SWIGLU_BWD_ONE = 32 << 20;   // elements of the result, below which a thread has one
+template <typename Index, int BATCH>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, Index total, int F) {
-  const Index vpr = F >> 3, i0 = (Index)blockIdx.x * (256 * EW_BATCH) + threadIdx.x;
-  uint4 ug[EW_BATCH], uu[EW_BATCH];
-  long long at[EW_BATCH];
+  const Index vpr = F >> 3, i0 = (Index)blockIdx.x * (256 * BATCH) + threadIdx.x;
+  uint4 ug[BATCH], uu[BATCH];
+  long long at[BATCH];
 #pragma unroll
-  for (int k = 0; k < EW_BATCH; ++k) {
+  for (int k = 0; k < BATCH; ++k) {
     const Index i = i0 + k * 256;
     if (i >= total) break;
     const Index t = i / vpr, v = i - t * vpr;
@@ -195,7 +198,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
     uu[k] = *reinterpret_cast<const uint4*>(g + F);
   }
 #pragma unroll
-  for (int k = 0; k < EW_BATCH; ++k) {
+  for (int k = 0; k < BATCH; ++k) {
     if (i0 + k * 256 >= total) break;
     const uint32_t *pg = reinterpret_cast<const uint32_t*>(&ug[k]), *pu = reinterpret_cast<const uint32_t*>(&uu[k]);
     uint4 o;
@@ -209,15 +212,15 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
   }
 }
 // dgu[T,2F]: dg = dy * u * (sig + g*sig*(1-sig)) ; du = dy * g * sig
-template <typename Index>
+template <typename Index, int BATCH>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dgu,
                   Index total, int F) {
-  const Index vpr = F >> 3, i0 = (Index)blockIdx.x * (256 * EW_BATCH) + threadIdx.x;
-  uint4 ug[EW_BATCH], uu[EW_BATCH], ud[EW_BATCH];
-  long long at[EW_BATCH];
+  const Index vpr = F >> 3, i0 = (Index)blockIdx.x * (256 * BATCH) + threadIdx.x;
+  uint4 ug[BATCH], uu[BATCH], ud[BATCH];
+  long long at[BATCH];
 #pragma unroll
-  for (int k = 0; k < EW_BATCH; ++k) {
+  for (int k = 0; k < BATCH; ++k) {
     const Index i = i0 + k * 256;
     if (i >= total) break;
     const Index t = i / vpr, v = i - t * vpr;
@@ -228,7 +231,7 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __r
     ud[k] = *reinterpret_cast<const uint4*>(dy + row + (long long)v * 8);
   }
 #pragma unroll
-  for (int k = 0; k < EW_BATCH; ++k) {
+  for (int k = 0; k < BATCH; ++k) {
     if (i0 + k * 256 >= total) break;
     const uint32_t *pg = reinterpret_cast<const uint32_t*>(&ug[k]), *pu = reinterpret_cast<const uint32_t*>(&uu[k]),
                    *pd = reinterpret_cast<const uint32_t*>(&ud[k]);
@@ -298,34 +301,39 @@ __global__ void chain_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, lon
   }
 }
 // bf16 in and out. GELU as x sigmoid(2 u), the same function as x (1 + tanh u) / 2: 1 + tanh u loses its digits where the
-// result is small, and tanhf is the longer code. [8192, 3072] forward 24.0 -> 22.2 us, backward 32.5 -> 31.0.
+// result is small, and tanhf is the longer code. [8192, 3072] forward 24.0 -> 22.2 us, backward 32.5 -> 31.0. The short division (2 ulp of
+// fp32, zero for a divisor above 2^126, where the result is below 2^-120) is a quarter of a small call's time.
 template <int OP>
 __device__ __forceinline__ float op_bf16(float x) {
-  if constexpr (OP == OP_GELU) return x * sigmoidf_(2.f * 0.7978845608028654f * (x + 0.044715f * x * x * x));
+  if constexpr (OP == OP_GELU) return __fdividef(x, 1.f + __expf(-2.f * 0.7978845608028654f * (x + 0.044715f * x * x * x)));
   else return apply_op(OP, x);
 }
 template <int OP>
 __device__ __forceinline__ float op_grad_bf16(float x) {
   if constexpr (OP == OP_GELU) {
     const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    const float s = sigmoidf_(2.f * k0 * (x + k1 * x * x * x));
+    const float s = __fdividef(1.f, 1.f + __expf(-2.f * k0 * (x + k1 * x * x * x)));
     // s (1 - s) is zero long before |x| = 16; x x, left alone, leaves fp32 and makes that 0 * inf
     return s + x * s * (1.f - s) * (2.f * k0 * (1.f + 3.f * k1 * fminf(x * x, 256.f)));
   } else {
     return apply_op_grad(OP, x);
   }
 }
-constexpr int UNARY_BATCH = 4;      // vectors of a thread, 256 apart, loaded before the first is used
-template <int OP>
+// Vectors of a thread, 256 apart, loaded before the first is used: one for calls that the L2 holds or that leave the machine partly
+// empty, two and then (forward) four where loads wait for memory. GELU forward, us with 1 / 2 / 4: 65536 elements 2.1 / 2.6 / 4.0, 3 Mi
+// 4.9 / 5.4 / 5.9, 8 Mi 9.4 / 9.4 / 10.1, 16 Mi 16.5 / 15.8 / 16.5, 24 Mi 24.9 / 23.0 / 23.4 (tanh 22.8 / 20.0 / 18.7), 96 Mi 89.1 / 78.9 /
+// 77.1; backward 65536 2.1 / 2.8 / 4.2, 8 Mi 11.7 / 11.6 / 12.4, 96 Mi 118.4 / 108.8 / 109.7.
+static int unary_batch(long long n, bool forward) { return n < (8 << 20) ? 1 : n < (20 << 20) || !forward ? 2 : 4; }
+template <int OP, int BATCH>
 __global__ void __launch_bounds__(256)
 unary_fwd_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long nvec) {
-  const long long i0 = (long long)blockIdx.x * (256 * UNARY_BATCH) + threadIdx.x;
-  uint4 u[UNARY_BATCH];
+  const long long i0 = (long long)blockIdx.x * (256 * BATCH) + threadIdx.x;
+  uint4 u[BATCH];
 #pragma unroll
-  for (int k = 0; k < UNARY_BATCH; ++k)
+  for (int k = 0; k < BATCH; ++k)
     if (i0 + k * 256 < nvec) u[k] = reinterpret_cast<const uint4*>(x)[i0 + k * 256];
 #pragma unroll
-  for (int k = 0; k < UNARY_BATCH; ++k) {
+  for (int k = 0; k < BATCH; ++k) {
     if (i0 + k * 256 >= nvec) break;
     uint32_t* p = reinterpret_cast<uint32_t*>(&u[k]);
 #pragma unroll
@@ -337,19 +345,19 @@ unary_fwd_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
   }
 }
 // dx = dy * f'(x); dx may be dy or x
-template <int OP>
+template <int OP, int BATCH>
 __global__ void __launch_bounds__(256)
 unary_bwd_bf16x8_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bfloat16* dx, long long nvec) {
-  const long long i0 = (long long)blockIdx.x * (256 * UNARY_BATCH) + threadIdx.x;
-  uint4 u[UNARY_BATCH], d[UNARY_BATCH];
+  const long long i0 = (long long)blockIdx.x * (256 * BATCH) + threadIdx.x;
+  uint4 u[BATCH], d[BATCH];
 #pragma unroll
-  for (int k = 0; k < UNARY_BATCH; ++k)
+  for (int k = 0; k < BATCH; ++k)
     if (i0 + k * 256 < nvec) {
       u[k] = reinterpret_cast<const uint4*>(x)[i0 + k * 256];
       d[k] = reinterpret_cast<const uint4*>(dy)[i0 + k * 256];
     }
 #pragma unroll
-  for (int k = 0; k < UNARY_BATCH; ++k) {
+  for (int k = 0; k < BATCH; ++k) {
     if (i0 + k * 256 >= nvec) break;
     uint32_t *p = reinterpret_cast<uint32_t*>(&u[k]), *pd = reinterpret_cast<uint32_t*>(&d[k]);
 #pragma unroll
@@ -665,46 +673,62 @@ GF_API int gf_scale_by_dev_scalar(void* x, long long n, const float* scalar, voi
   scale_by_dev_scalar_kernel<<<ew_grid(n / 8 + 1, 256), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)x, n, scalar);
   GF_RET();
 }
+template <typename Index, int BATCH>
+static int launch_swiglu(const void* gu, const void* dy, void* out, long long n, int F, cudaStream_t st) {
+  const long long blocks = (n + 256 * BATCH - 1) / (256 * BATCH);
+  if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
+  if (dy)
+    swiglu_bwd_kernel<Index, BATCH><<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dy,
+                                                                     (__nv_bfloat16*)out, (Index)n, F);
+  else
+    swiglu_fwd_kernel<Index, BATCH><<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, (Index)n, F);
+  GF_RET();
+}
+static int run_swiglu(const void* gu, const void* dy, void* out, long long T, int F, cudaStream_t st) {
+  if (F % 8) return GFH_BAD_ARG;
+  const long long n = T * (F / 8);
+  if (n <= 0) return GFH_OK;
+  if (8 * n < (dy ? SWIGLU_BWD_ONE : SWIGLU_FWD_ONE)) return launch_swiglu<unsigned, 1>(gu, dy, out, n, F, st);
+  return n < 0x7fffffffll ? launch_swiglu<unsigned, 2>(gu, dy, out, n, F, st) : launch_swiglu<long long, 2>(gu, dy, out, n, F, st);
+}
 GF_API int gf_swiglu_fwd(const void* gu, void* y, long long T, int F, void* stream) {
   gf::enter();
-  if (F % 8) return GFH_BAD_ARG;
-  const long long n = T * (F / 8), blocks = (n + 256 * EW_BATCH - 1) / (256 * EW_BATCH);
-  if (n <= 0) return GFH_OK;
-  if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
-  if (n < 0x7fffffffll)
-    swiglu_fwd_kernel<unsigned><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)y,
-                                                                                  (unsigned)n, F);
-  else
-    swiglu_fwd_kernel<long long><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)y, n,
-                                                                                   F);
-  GF_RET();
+  return run_swiglu(gu, nullptr, y, T, F, (cudaStream_t)stream);
 }
 GF_API int gf_swiglu_bwd(const void* gu, const void* dy, void* dgu, long long T, int F, void* stream) {
   gf::enter();
-  if (F % 8) return GFH_BAD_ARG;
-  const long long n = T * (F / 8), blocks = (n + 256 * EW_BATCH - 1) / (256 * EW_BATCH);
-  if (n <= 0) return GFH_OK;
+  if (!dy) return GFH_BAD_ARG;
+  return run_swiglu(gu, dy, dgu, T, F, (cudaStream_t)stream);
+}
+template <int BATCH>
+static int launch_unary_fwd(const void* x, void* y, long long nvec, int op, cudaStream_t st) {
+  const long long blocks = (nvec + 256 * BATCH - 1) / (256 * BATCH);
   if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
-  if (n < 0x7fffffffll)
-    swiglu_bwd_kernel<unsigned><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dgu, (unsigned)n, F);
-  else
-    swiglu_bwd_kernel<long long><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dgu, n, F);
+  auto kern = op == OP_RELU ? unary_fwd_bf16x8_kernel<OP_RELU, BATCH> : op == OP_GELU ? unary_fwd_bf16x8_kernel<OP_GELU, BATCH>
+              : op == OP_SIGMOID ? unary_fwd_bf16x8_kernel<OP_SIGMOID, BATCH> : op == OP_TANH ? unary_fwd_bf16x8_kernel<OP_TANH, BATCH>
+                                                                                               : unary_fwd_bf16x8_kernel<OP_SILU, BATCH>;
+  kern<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, nvec);
+  GF_RET();
+}
+template <int BATCH>
+static int launch_unary_bwd(const void* x, const void* dy, void* dx, long long nvec, int op, cudaStream_t st) {
+  const long long blocks = (nvec + 256 * BATCH - 1) / (256 * BATCH);
+  if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
+  auto kern = op == OP_RELU ? unary_bwd_bf16x8_kernel<OP_RELU, BATCH> : op == OP_GELU ? unary_bwd_bf16x8_kernel<OP_GELU, BATCH>
+              : op == OP_SIGMOID ? unary_bwd_bf16x8_kernel<OP_SIGMOID, BATCH> : op == OP_TANH ? unary_bwd_bf16x8_kernel<OP_TANH, BATCH>
+                                                                                               : unary_bwd_bf16x8_kernel<OP_SILU, BATCH>;
+  kern<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, nvec);
   GF_RET();
 }
 // dtype: 0 = fp32, 1 = bf16
 GF_API int gf_unary_fwd(const void* x, void* y, long long n, int op, int dtype, void* stream) {
   gf::enter();
   if (dtype == 1 && n % 8 == 0 && ((uintptr_t)x % 16 == 0) && ((uintptr_t)y % 16 == 0)) {
-    const long long blocks = (n / 8 + 256 * UNARY_BATCH - 1) / (256 * UNARY_BATCH);
-    if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
-    if (n > 0) {
-      auto kern = op == OP_RELU ? unary_fwd_bf16x8_kernel<OP_RELU> : op == OP_GELU ? unary_fwd_bf16x8_kernel<OP_GELU>
-                  : op == OP_SIGMOID ? unary_fwd_bf16x8_kernel<OP_SIGMOID> : op == OP_TANH ? unary_fwd_bf16x8_kernel<OP_TANH>
-                                                                                            : unary_fwd_bf16x8_kernel<OP_SILU>;
-      kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, n / 8);
-    }
+    if (n <= 0) return GFH_OK;
+    const int batch = unary_batch(n, true);
+    return batch == 1 ? launch_unary_fwd<1>(x, y, n / 8, op, (cudaStream_t)stream)
+           : batch == 2 ? launch_unary_fwd<2>(x, y, n / 8, op, (cudaStream_t)stream)
+                        : launch_unary_fwd<4>(x, y, n / 8, op, (cudaStream_t)stream);
   } else {
     OpChain c;
     c.n = 1;
@@ -723,15 +747,9 @@ GF_API int gf_unary_fwd(const void* x, void* y, long long n, int op, int dtype, 
 GF_API int gf_unary_bwd_bf16(const void* x, const void* dy, void* dx, long long n, int op, void* stream) {
   gf::enter();
   if (n % 8) return GFH_BAD_ARG;
-  const long long blocks = (n / 8 + 256 * UNARY_BATCH - 1) / (256 * UNARY_BATCH);
-  if (blocks > 0x7fffffffll) return GFH_TOO_LARGE;
   if (n <= 0) return GFH_OK;
-  auto kern = op == OP_RELU ? unary_bwd_bf16x8_kernel<OP_RELU> : op == OP_GELU ? unary_bwd_bf16x8_kernel<OP_GELU>
-              : op == OP_SIGMOID ? unary_bwd_bf16x8_kernel<OP_SIGMOID> : op == OP_TANH ? unary_bwd_bf16x8_kernel<OP_TANH>
-                                                                                        : unary_bwd_bf16x8_kernel<OP_SILU>;
-  kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx,
-                                                          n / 8);
-  GF_RET();
+  return unary_batch(n, false) == 1 ? launch_unary_bwd<1>(x, dy, dx, n / 8, op, (cudaStream_t)stream)
+                                    : launch_unary_bwd<2>(x, dy, dx, n / 8, op, (cudaStream_t)stream);
 }
 GF_API int gf_op_chain(const void* x, void* y, long long n, const int* ops, int nops, int dtype, void* stream) {
   gf::enter();

@@ -98,3 +98,35 @@ def test_numbers_of_any_size(name):
     want, grad = _exact(x.detach(), name)          # 3e38 squared and cubed are finite in fp64
     assert ((y.double() - want).abs() <= 2 ** -7.99 * want.abs() + 2 ** -20 * (name != "relu")).all()
     assert ((x.grad.double() - grad).abs() <= 2 ** -7.99 * grad.abs() + 2 ** -18).all()
+
+
+@pytest.mark.parametrize("n", [(8 << 20) - 8, 8 << 20, (8 << 20) + 8, (20 << 20) - 8, (20 << 20) + 2056])
+@pytest.mark.parametrize("name", ["gelu", "silu"])
+def test_numbers_of_vectors_to_a_thread(n, name):
+    """Around the sizes where a thread gets more vectors."""
+    from ghost_flow_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, generator=g, device="cuda").bfloat16().requires_grad_()
+    dy = torch.randn(n, generator=g, device="cuda").bfloat16()
+    y = ops.unary(x, name)
+    y.backward(dy)
+    want, grad = _exact(x.detach(), name)
+    assert torch.allclose(y.double(), want, rtol=2 ** -8, atol=2 ** -20)
+    assert torch.allclose(x.grad.double(), grad * dy.double(), rtol=2 ** -8, atol=2 ** -17)
+
+
+@pytest.mark.parametrize("T,F", [(6143, 1024), (6144, 1024), (6145, 1024), (4095, 8192), (4096, 8192), (700, 11008)])
+def test_swiglu_numbers_of_vectors(T, F):
+    from ghost_flow_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T + F)
+    gu = torch.randn(T, 2 * F, generator=g, device="cuda").bfloat16().requires_grad_()
+    dy = torch.randn(T, F, generator=g, device="cuda").bfloat16()
+    y = ops.swiglu(gu)
+    y.backward(dy)
+    a, b = gu.detach().double().chunk(2, -1)
+    s = torch.sigmoid(a)
+    assert torch.allclose(y.double(), a * s * b, rtol=2 ** -8, atol=2 ** -20)
+    want = torch.cat((dy.double() * b * (s + a * s * (1 - s)), dy.double() * a * s), -1)
+    assert torch.allclose(gu.grad.double(), want, rtol=2 ** -8, atol=2 ** -17)
