@@ -170,7 +170,7 @@ struct NormBwd {
 };
 
 // RES: there may be a dres. RMSNorm loads it with the row; LayerNorm, which has no registers left for that, where it is added,
-// and it has kernels without.
+// and it has kernels without. TWO: dx2 is written, which no other call pays for ([8192, 1024] 16.2 us, 17.3 with a test in the loop).
 template <int NV, bool EARLY>
 struct NormBwdRow {
   uint4 x[NV], g[NV], r[EARLY ? NV : 1];
@@ -194,7 +194,7 @@ __device__ __forceinline__ void norm_bwd_load(const NormBwd& p, NormBwdRow<NV, !
 }
 
 // Rows row0, row0 + step, ... of one warp or CTA; the sums over rows end in dw / db. wv: this thread's weights, packed.
-template <bool LN, int NV, bool RES, bool PREFETCH, typename Sum>
+template <bool LN, int NV, bool RES, bool TWO, bool PREFETCH, typename Sum>
 __device__ __forceinline__ void norm_bwd_rows(const NormBwd& p, int row0, int step, int v0, int stride, float (&dw)[NV][8],
                                               float (&db)[LN ? NV : 1][8], Sum sum) {
   const int nv = p.D >> 3;
@@ -246,7 +246,7 @@ __device__ __forceinline__ void norm_bwd_rows(const NormBwd& p, int row0, int st
         }
         const uint4 out = pack8(o);
         stv(p.dx + (long long)row * p.D + v * 8, out);
-        if (!LN && p.dx2) stv(p.dx2 + (long long)row * p.D + v * 8, out);
+        if (TWO) stv(p.dx2 + (long long)row * p.D + v * 8, out);
       }
     }
     if (PREFETCH) cur = nxt;
@@ -254,7 +254,7 @@ __device__ __forceinline__ void norm_bwd_rows(const NormBwd& p, int row0, int st
 }
 
 // One warp per row, D <= 1024. The eight warps' sums meet in shared memory, warp by warp in its own row of it.
-template <bool LN, int NV, bool RES>
+template <bool LN, int NV, bool RES, bool TWO>
 __global__ void __launch_bounds__(NORM_THREADS, NV == 1 ? 3 : 2) norm_bwd_warp_kernel(const NormBwd p) {
   __shared__ float acc[NORM_WARPS][NORM_WARP_D];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = p.D >> 3;
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(NORM_THREADS, NV == 1 ? 3 : 2) norm_bwd_warp_k
       dw[i][j] = 0.f;
       if (LN) db[LN ? i : 0][j] = 0.f;
     }
-  norm_bwd_rows<LN, NV, RES, NV <= 2>(p, blockIdx.x * NORM_WARPS + warp, gridDim.x * NORM_WARPS, lane, 32, dw, db,
+  norm_bwd_rows<LN, NV, RES, TWO, NV <= 2>(p, blockIdx.x * NORM_WARPS + warp, gridDim.x * NORM_WARPS, lane, 32, dw, db,
                               [](float v) { return warp_sum(v); });
   auto flush = [&](const float(&a)[NV][8], float* out) {
 #pragma unroll
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(NORM_THREADS, NV == 1 ? 3 : 2) norm_bwd_warp_k
 template <bool LN, int NV>
 constexpr int norm_bwd_ctas() { return NV == 1 ? 4 : NV == 2 ? 2 : LN ? 1 : 2; }
 
-template <bool LN, int NV, bool RES>
+template <bool LN, int NV, bool RES, bool TWO>
 __global__ void __launch_bounds__(NORM_THREADS, norm_bwd_ctas<LN, NV>()) norm_bwd_block_kernel(const NormBwd p) {
   __shared__ float red[4][NORM_WARPS];
   const int nv = p.D >> 3;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(NORM_THREADS, norm_bwd_ctas<LN, NV>()) norm_bw
       if (LN) db[LN ? i : 0][j] = 0.f;
     }
   int k = 0;
-  norm_bwd_rows<LN, NV, RES, NV <= 2>(p, blockIdx.x, gridDim.x, threadIdx.x, NORM_THREADS, dw, db,
+  norm_bwd_rows<LN, NV, RES, TWO, NV <= 2>(p, blockIdx.x, gridDim.x, threadIdx.x, NORM_THREADS, dw, db,
                                  [&](float v) { return block_sum(v, red[k++ & 3]); });
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -432,25 +432,25 @@ static int launch_norm_fwd(const NormFwd& p, cudaStream_t st) {
 
 // Number of partial rows written: at most norm_grid(T), which sizes the caller's scratch, and no more CTAs than are
 // resident at once (a second wave would wait for the first one's row loops).
-template <bool LN, bool RES>
+template <bool LN, bool RES, bool TWO = false>
 static int launch_norm_bwd(const NormBwd& p, cudaStream_t st) {
   const int cap = norm_grid(p.T), sms = sm_count();
   int grid;
   if (norm_row_per_warp(p.T, p.D, sms)) {
     const int vpl = (p.D / 8 + 31) / 32;
     grid = at_most(at_most((p.T + NORM_WARPS - 1) / NORM_WARPS, cap), (long long)sms * (vpl == 1 ? 3 : 2));
-    auto kern = vpl == 1 ? norm_bwd_warp_kernel<LN, 1, RES> : vpl == 2 ? norm_bwd_warp_kernel<LN, 2, RES>
-                : vpl == 3 ? norm_bwd_warp_kernel<LN, 3, RES> : norm_bwd_warp_kernel<LN, 4, RES>;
+    auto kern = vpl == 1 ? norm_bwd_warp_kernel<LN, 1, RES, TWO> : vpl == 2 ? norm_bwd_warp_kernel<LN, 2, RES, TWO>
+                : vpl == 3 ? norm_bwd_warp_kernel<LN, 3, RES, TWO> : norm_bwd_warp_kernel<LN, 4, RES, TWO>;
     kern<<<grid, NORM_THREADS, 0, st>>>(p);
   } else if (p.D <= NORM_THREADS * 8) {
     grid = at_most(cap, (long long)sms * norm_bwd_ctas<LN, 1>());
-    norm_bwd_block_kernel<LN, 1, RES><<<grid, NORM_THREADS, 0, st>>>(p);
+    norm_bwd_block_kernel<LN, 1, RES, TWO><<<grid, NORM_THREADS, 0, st>>>(p);
   } else if (p.D <= NORM_THREADS * 16) {
     grid = at_most(cap, (long long)sms * norm_bwd_ctas<LN, 2>());
-    norm_bwd_block_kernel<LN, 2, RES><<<grid, NORM_THREADS, 0, st>>>(p);
+    norm_bwd_block_kernel<LN, 2, RES, TWO><<<grid, NORM_THREADS, 0, st>>>(p);
   } else {
     grid = at_most(cap, (long long)sms * norm_bwd_ctas<LN, NORM_MAXV>());
-    norm_bwd_block_kernel<LN, NORM_MAXV, RES><<<grid, NORM_THREADS, 0, st>>>(p);
+    norm_bwd_block_kernel<LN, NORM_MAXV, RES, TWO><<<grid, NORM_THREADS, 0, st>>>(p);
   }
   return grid;
 }
@@ -479,7 +479,7 @@ GF_API int gf_rmsnorm_bwd2(const void* x, const void* w, const void* dy, const f
   cudaStream_t st = (cudaStream_t)stream;
   NormBwd p{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, nullptr,
             rstd, (__nv_bfloat16*)dx, (__nv_bfloat16*)dx2, scratch, nullptr, T, D};
-  const int parts = launch_norm_bwd<false, true>(p, st);
+  const int parts = dx2 ? launch_norm_bwd<false, true, true>(p, st) : launch_norm_bwd<false, true>(p, st);
   launch_fold(scratch, dw, nullptr, nullptr, parts, D, accumulate, st);
   gf::note_extra_launches(1);
   return cudaGetLastError() == cudaSuccess ? GFH_OK : GFH_CUDA;

@@ -83,7 +83,8 @@ class _RMSNormFn(torch.autograd.Function):
             _lib.stream_ptr()), "gf_rmsnorm_fwd")
         ctx.save_for_backward(h if h is not None else x, w, rstd)
         ctx.has_res = residual is not None
-        # two leaves keep their gradients apart: the kernel writes both, where autograd would copy one (a pass of its own)
+        # A call on two leaves only (inside a model both are results of other modules): they keep their gradients apart, so the kernel
+        # writes both, where autograd would copy one (a pass of its own).
         ctx.two = residual is not None and x_is_leaf and residual.is_leaf
         return (y, h) if residual is not None else y
 
