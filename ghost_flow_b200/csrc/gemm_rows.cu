@@ -411,9 +411,14 @@ static int rows_clusters(int slices) {
 // tokens 48 clusters of 8 fit, 104 of 4, 222 of 2; with more tokens 33, 71 and 148. One more is a second wave: [8, 4096] x [N, 4096]^T, N =
 // 6272 17.1 us on 49 of 8, 13.7 on 49 of 4; 13824 27.6 on 108 of 4, 22.7 on 108 of 2; 24 tokens, 4352 16.0 on 34 of 8, 12.0 on 34
 // of 4; 9216 23.9 on 72 of 4, 17.7 on 72 of 2.
+// Tiles that do not fit at once even whole: the last ones stream all of K from a few CTAs, so a long K is cut in two where they are few
+// (up to 16 tokens, where the second half overlaps with more, always). us whole / in two: [8, 8192] x [57344, 8192]^T (448 tiles) 162.1 /
+// 146.7, x [73728, 8192]^T 180.7 / 176.8, x [128256, 8192]^T 303.2 / 301.1; K 4096: 83.4 / 77.1, 95.6 / 92.1, 158.0 / 152.6; K 2048: 45.4 / 45.4, 51.5 /
+// 53.6; 24 tokens, K 8192: [38016] 119.0 / 107.8, [43008] 124.9 / 116.1, [57344] 144.4 / 152.2; 64 tokens [57344] 155.7 / 172.5.
 template <int NT>
 static int rows_slices(int N, int K) {
-  const int tiles = (N + RW_BM - 1) / RW_BM, blocks = (K + RW_BK - 1) / RW_BK;
+  const int tiles = (N + RW_BM - 1) / RW_BM, blocks = (K + RW_BK - 1) / RW_BK, whole = rows_clusters<NT>(1);
+  if (tiles > whole) return blocks >= 64 && (NT == 16 || (tiles - 1) % whole < whole / 4) ? 2 : 1;
   int s = 8;
   while (s > 1 && (4 * s > blocks || tiles > rows_clusters<NT>(s))) s >>= 1;
   return s;

@@ -93,3 +93,27 @@ def test_all_clusters_of_a_product_fit_on_the_machine(M, ctas, kernel_status):
         want = x.double() @ w.double().t()
         # fp32 sums of 2048 products, about 2048 * 2^-22 with room, and the rounding of the result
         assert ((out.double() - want).abs() <= 2048 * 2 ** -22 + 2 ** -8 * want.abs()).all()
+
+
+def test_tiles_that_never_fit_at_once(kernel_status):
+    """More tiles than the machine holds whole: a long K is cut in two where the last ones are few."""
+    from ghost_flow_b200.ops import _lib
+
+    ask = _lib.cuda_lib().gf_gemm_rows_clusters
+    for M in (16, 32, 64):
+        whole = ask(M, 1, 1, 1)
+        for K, tiles, want in ((4096, whole + 1, 2), (4096, whole + whole // 4, 2), (4032, whole + 1, 1), (4096, 2 * whole, 2 if M == 16 else 1),
+                               (8192, whole, 1)):
+            assert ask(M, 128 * tiles, K, 0) == want, (M, K, tiles)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    M, N, K = 16, 128 * (ask(16, 1, 1, 1) + 3) - 5, 4096
+    x, w, norm_w = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((M, K), (N, K), (K,)))
+    out = torch.empty(M, N + 5, device="cuda", dtype=torch.bfloat16)[:, :N]
+    for inp in (0, 1):
+        assert _run(x, w, out, M, N, K, inp, norm_w, None, None, 1.0, 0) == 0
+        xd = x.double()
+        if inp:
+            xd = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5) * norm_w.double()
+        want = xd @ w.double().t()
+        size = (xd.square() @ w.double().t().square()).sqrt()                # tolerances as above
+        assert ((out.double() - want).abs() <= K * 2 ** -22 + (6 * 2 ** -9 * size if inp else 0) + 2 ** -8 * want.abs()).all()
