@@ -1,20 +1,25 @@
-// One LLaMA decoder layer for one new token of each sequence: six kernels from one call (nine with more than 16 sequences).
+// One LLaMA decoder layer for one new token of each sequence: seven kernels from one call (nine with more than 16 sequences;
+// one less where the attention needs no merge).
 //
 //   q, k, v   = rms_norm(x) Wqkv^T                 gemm_rows.cu, the norm in front of the product
 //   attention over the caches, rotation of q and k, and the new cache row (attn_decode.cu), and its merge
 //   h         = x + attention Wo^T
 //   gate, up  = rms_norm(h) Wgu^T
-//   y         = h + (silu(gate) * up) Wdown^T      SwiGLU in front of the product
+//   a         = silu(gate) * up                    pointwise.cu
+//   y         = h + a Wdown^T
 //
 // The first launch is an ordinary one, so all earlier work of the stream is complete when it runs. Every further kernel may
-// start while the one in front of it ends (programmatic stream serialization; norm and SwiGLU kernels do not) and fetches what no
-// kernel of the layer writes, weights and older cache rows, before it waits for that one. Each kernel waits for the one in front of it before it ends, so a
-// kernel that has waited may read the results of all earlier ones.
+// start while the one in front of it ends (programmatic stream serialization; the norms of more than 16 sequences do not) and
+// fetches what no kernel of the layer writes, weights and older cache rows, before it waits for that one. Each kernel waits for
+// the one in front of it before it ends, so a kernel that has waited may read the results of all earlier ones.
 //
-// One layer of LLaMA-7B (hidden 4096, inner 11008, 32 heads, 1500 keys), device time in a graph, nine ordinary launches -> now: one sequence
-// 101 -> 96 us, 8 142 -> 116, 16 185 -> 149, 32 (800 keys) 208 -> 168, 64 (500 keys) 228 -> 199; enqueueing it takes the host 80 us
-// instead of 260. What is left above the bytes (93 us at 8): each kernel ends before the next one's tokens can be read, and the
-// memory waits for about 4 us then.
+// Device time in a graph, us, nine ordinary launches of the layers / here: LLaMA-7B (hidden 4096, inner 11008, 32 heads), one
+// sequence of 1500 keys 104 / 88, 8 145 / 111, 16 of 300 140 / 96, 32 of 800 207 / 167, 64 of 300 200 / 168; 70B (8192, 28672,
+// 64 / 8 heads), one of 1500 283 / 282, 16 of 300 366 / 289; hidden 1024, one of 100 26.3 / 23.7, and 256 18.1 / 21.6, where
+// the products' fixed cost is all there is; enqueueing it takes the host 60 us instead of 205. SwiGLU inside the last product,
+// computed by every CTA for its part of K, costs more than the kernel and its launch: 88 -> 96 us for one sequence of the
+// first, 282 -> 329 of the second. What is left above the bytes (93 us at 8): each kernel ends before the next one's tokens can
+// be read, and the memory waits for about 4 us then.
 #include <math.h>
 
 #include "gemm_rows.cuh"
@@ -24,10 +29,10 @@ namespace gf {
 int attn_decode_append(const void* qkv, long long ldq, void* kcache, void* vcache, int s_max, int len, const float* cos_row,
                        const float* sin_row, int interleaved, void* out, long long ldo, int B, int Hq, int Hkv, int D, float scale,
                        int splits, float* scratch, int chained, cudaStream_t st);
+int swiglu_chained(const void* gu, void* y, long long T, int F, cudaStream_t st);
 }
 GF_API int gf_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd, int T, int D, float eps,
                           void* stream);
-GF_API int gf_swiglu_fwd(const void* gu, void* y, long long T, int F, void* stream);
 
 // x, y dense bf16 [B, hidden], dense weights [out, in], caches [B, s_max, Hkv, D], tables [positions, D / 2].
 // ws: 256-byte aligned, 2 B ((2 Hq + 2 Hkv) D + hidden + 2 inner + max(hidden, inner)) + 4 B Hq splits (D + 2) + 1536
@@ -63,8 +68,8 @@ GF_API int gf_llama_decode_layer(const void* x, const void* attn_norm, float att
   float* parts = reinterpret_cast<float*>(take(4ll * B * Hq * splits * (D + 2)));
   const long long half = (long long)pos * (D / 2);
 
-  // Up to 16 rows the norms and SwiGLU run in front of the products that read them. With more, every CTA would compute more of
-  // them than it has time for beside its weights, and they are kernels of their own.
+  // Up to 16 rows the norms run in front of the products that read them. With more, every CTA would compute more of them than
+  // it has time for beside its weights, and they are kernels of their own.
   const bool fused = B <= ROWS_MAX_M_FUSED;
   int rc = GFH_OK;
   auto normed_gemm = [&](const void* in, long long ld, const void* w_norm, float eps, const void* w, void* out, int n, int chained) {
@@ -83,12 +88,9 @@ GF_API int gf_llama_decode_layer(const void* x, const void* attn_norm, float att
   RowsGemm g{o, att, wo, att, h, hidden, 0, B, hidden, att, ROWS_PLAIN, nullptr, 0.f, nullptr, x, hidden, 1.f, 0, status};
   if ((rc = gemm_rows_run(g, 1, st))) return rc;
   if (normed_gemm(h, hidden, ffn_norm, ffn_eps, gate_up, gu, 2 * inner, 1)) return rc;
-  g = RowsGemm{gu, 2 * inner, down, inner, y, hidden, 0, B, hidden, inner, ROWS_SWIGLU, nullptr, 0.f, nullptr, h, hidden, 1.f, 0, status};
-  if (!fused) {
-    if ((rc = gf_swiglu_fwd(gu, tmp, B, inner, st))) return rc;
-    g.X = tmp; g.ldx = inner; g.input = ROWS_PLAIN;
-  }
+  if ((rc = swiglu_chained(gu, tmp, B, inner, st))) return rc;
+  g = RowsGemm{tmp, inner, down, inner, y, hidden, 0, B, hidden, inner, ROWS_PLAIN, nullptr, 0.f, nullptr, h, hidden, 1.f, 0, status};
   rc = gemm_rows_run(g, 1, st);
-  note_extra_launches(5);                    // four products and the attention; its merge, norms and SwiGLU count themselves
+  note_extra_launches(5);                    // four products and the attention; its merge, norms and SwiGLU are counted where they start
   return rc;
 }

@@ -1,25 +1,29 @@
-// bf16 GEMM of a few rows (one token of each sequence of a batch): C[M, N] = act(alpha * f(X)[M, K] W[N, K]^T + bias + residual),
-// M <= 64.
+// bf16 GEMM of a few rows (one token of each sequence of a batch): C[M, N] = act(alpha * f(X)[M, K] W[N, K]^T + bias +
+// residual), M <= 64.
 //
 // The weight is read once and is all that counts, so it is the 128-row operand: tcgen05.mma with 128 output features as the
-// rows and 16, 32 or 64 tokens as the columns. TMA fills a ring of 128 x 64 weight blocks, about 200 KB on an SM for its two or three
-// CTAs, and needs no registers for what is in flight. K is split over the CTAs of a cluster; they add their sums through
+// rows and 16, 32 or 64 tokens as the columns. TMA fills a ring of 128 x 64 weight blocks, about 200 KB on an SM for its two or
+// three CTAs, and needs no registers for what is in flight. K is split over the CTAs of a cluster; they add their sums through
 // distributed shared memory in the order of their ranks, so there is no workspace to clear, no atomic and no second kernel.
 //
-// The tokens' side of a block comes by TMA too, or (at most 16 rows) four warps compute it, so that the operation in front of the
-// product needs no launch and no trip through memory: an RMS norm (the operand is x * w rounded to bf16, and the row's factor
-// 1 / rms scales the sums; the squares are added up from the same loads) or SwiGLU. With more rows each CTA would compute more than
-// it has time for beside its weights: fused, 64 rows of a LLaMA-7B layer took 286 us, with a norm kernel in front 214.
+// The tokens' side of a block comes by TMA too, or (at most 16 rows) four warps compute it, so that the operation in front of
+// the product needs no launch and no trip through memory: an RMS norm (the operand is x * w rounded to bf16, and the row's
+// factor 1 / rms scales the sums; the squares are added up from the same loads) or SwiGLU. The norm costs 0.2 us. SwiGLU, an
+// exponential and a division for each element in every CTA that reads it, costs more than the 2 us of its own kernel: [1,
+// 28672] x [8192, 28672]^T 73 -> 106 us, [8, 11008] x [4096, 11008]^T 19.4 -> 26.1, [1, 688] x [256, 688]^T 5.6 -> 8.6; the
+// decoder layer uses the kernel. With more rows each CTA would compute more than it has time for beside its weights: fused, 64
+// rows of a LLaMA-7B layer took 286 us, with a norm kernel in front 214.
 //
-// In a chain of launches the weight blocks are on their way before the kernel in front has finished (griddepcontrol): they
-// are nobody's output there. X, the residual and C are touched behind griddepcontrol.wait only.
+// In a chain of launches the weight blocks are on their way before the kernel in front has finished (griddepcontrol): they are
+// nobody's output there. X, the residual and C are touched behind griddepcontrol.wait only.
 //
-// What bounds it: memory, behind a fixed cost of about 5 us (launch, TMEM, first block, cluster barriers). The rings hold up to 28 MB
-// in flight. Up to 16 tokens three smaller CTAs share an SM: more of them mean shorter parts of K and a better fit to the machine (a
-// layer of 8 sequences, hidden 4096 / 5120: two CTAs of six stages 121 / 134 us, three of four 116 / 112; half as many CTAs 138 / 182).
-// Device time in us with cold weights, the kernels that took these products before -> this one: [16, 4096] x [12288, 4096]^T 27.0 ->
-// 20.8 (4.8 TB/s), x [22016, 4096]^T 40.9 -> 33.2 (5.4 TB/s), [16, 11008] x [4096, 11008]^T 24.0 -> 19.7; back to back from the host
-// [32, 4096] x [22016, 4096]^T 54.2 -> 41.9, [64, 4096] x [4096, 4096]^T 21.9 -> 14.7, [64, 14336] x [8192, 14336]^T 55.6 -> 45.8.
+// What bounds it: memory, behind a fixed cost of about 5 us (launch, TMEM, first block, cluster barriers). The rings hold up to
+// 28 MB in flight. Up to 16 tokens three smaller CTAs share an SM: more of them mean shorter parts of K and a better fit to the
+// machine (a layer of 8 sequences, hidden 4096 / 5120: two CTAs of six stages 121 / 134 us, three of four 116 / 112; half as
+// many CTAs 138 / 182). Device time in us with cold weights, the kernels that took these products before -> this one: [16,
+// 4096] x [12288, 4096]^T 27.0 -> 20.8 (4.8 TB/s), x [22016, 4096]^T 40.9 -> 33.2 (5.4 TB/s), [16, 11008] x [4096, 11008]^T
+// 24.0 -> 19.7; back to back from the host [32, 4096] x [22016, 4096]^T 54.2 -> 41.9, [64, 4096] x [4096, 4096]^T 21.9 -> 14.7,
+// [64, 14336] x [8192, 14336]^T 55.6 -> 45.8.
 #include <atomic>
 
 #include "gemm_rows.cuh"
@@ -375,8 +379,8 @@ static void rows_attributes(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&at)[2
   cfg.numAttrs = chained ? 2 : 1;
 }
 
-// Never launched: the CTAs of this one share an SM as those of the kernel do (shared memory is what counts), and are counted so. For a
-// kernel with tensor memory the runtime counts one CTA to an SM.
+// Never launched: the CTAs of this one share an SM as those of the kernel do (shared memory is what counts), and are counted
+// so. For a kernel with tensor memory the runtime counts one CTA to an SM.
 template <int NT>
 __global__ void __launch_bounds__(RW_THREADS, RwCfg<NT>::CTAS) rows_occupancy_kernel(int* p) {
   extern __shared__ int part[];
@@ -406,15 +410,16 @@ static int rows_clusters(int slices) {
   return n;
 }
 
-// CTAs of a cluster, each with a part of K of at least four blocks: as many as leave all clusters on the machine at once, and a power
-// of two (clusters of 3, 6 or 7 leave SMs of a GPC out: 6144 features on 48 clusters of 6 took 22.4 us, on 48 of 4 14.7). Up to 16
-// tokens 48 clusters of 8 fit, 104 of 4, 222 of 2; with more tokens 33, 71 and 148. One more is a second wave: [8, 4096] x [N, 4096]^T, N =
-// 6272 17.1 us on 49 of 8, 13.7 on 49 of 4; 13824 27.6 on 108 of 4, 22.7 on 108 of 2; 24 tokens, 4352 16.0 on 34 of 8, 12.0 on 34
-// of 4; 9216 23.9 on 72 of 4, 17.7 on 72 of 2.
-// Tiles that do not fit at once even whole: the last ones stream all of K from a few CTAs, so a long K is cut in two where they are few
-// (up to 16 tokens, where the second half overlaps with more, always). us whole / in two: [8, 8192] x [57344, 8192]^T (448 tiles) 162.1 /
-// 146.7, x [73728, 8192]^T 180.7 / 176.8, x [128256, 8192]^T 303.2 / 301.1; K 4096: 83.4 / 77.1, 95.6 / 92.1, 158.0 / 152.6; K 2048: 45.4 / 45.4, 51.5 /
-// 53.6; 24 tokens, K 8192: [38016] 119.0 / 107.8, [43008] 124.9 / 116.1, [57344] 144.4 / 152.2; 64 tokens [57344] 155.7 / 172.5.
+// CTAs of a cluster, each with a part of K of at least four blocks: as many as leave all clusters on the machine at once, and a
+// power of two (clusters of 3, 6 or 7 leave SMs of a GPC out: 6144 features on 48 clusters of 6 took 22.4 us, on 48 of 4 14.7).
+// Up to 16 tokens 48 clusters of 8 fit, 104 of 4, 222 of 2; with more tokens 33, 71 and 148. One more is a second wave: [8,
+// 4096] x [N, 4096]^T, N = 6272 17.1 us on 49 of 8, 13.7 on 49 of 4; 13824 27.6 on 108 of 4, 22.7 on 108 of 2; 24 tokens, 4352
+// 16.0 on 34 of 8, 12.0 on 34 of 4; 9216 23.9 on 72 of 4, 17.7 on 72 of 2. Tiles that do not fit at once even whole: the last
+// ones stream all of K from a few CTAs, so a long K is cut in two where they are few (up to 16 tokens, where the second half
+// overlaps with more, always). us whole / in two: [8, 8192] x [57344, 8192]^T (448 tiles) 162.1 / 146.7, x [73728, 8192]^T
+// 180.7 / 176.8, x [128256, 8192]^T 303.2 / 301.1; K 4096: 83.4 / 77.1, 95.6 / 92.1, 158.0 / 152.6; K 2048: 45.4 / 45.4, 51.5 /
+// 53.6; 24 tokens, K 8192: [38016] 119.0 / 107.8, [43008] 124.9 / 116.1, [57344] 144.4 / 152.2; 64 tokens [57344] 155.7 /
+// 172.5.
 template <int NT>
 static int rows_slices(int N, int K) {
   const int tiles = (N + RW_BM - 1) / RW_BM, blocks = (K + RW_BK - 1) / RW_BK, whole = rows_clusters<NT>(1);

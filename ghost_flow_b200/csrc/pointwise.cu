@@ -173,17 +173,23 @@ embedding_rows_kernel(const I* __restrict__ ids, const uint4* __restrict__ table
 }
 
 // ------------------------------------------------------------------ SwiGLU
-// gu is [T, 2F] (gate columns [0,F), up columns [F,2F)); y = silu(g) * u is [T, F].
-// Bound by memory: a thread has BATCH vectors of each operand, 256 vectors apart, and issues their loads before it uses the first. Index
-// is a 32-bit type where the sizes allow it: the division by the row length was a 64-bit one for every vector. Two vectors pay where
-// their loads wait for memory; a call that the L2 holds or that leaves the machine partly empty has more threads with one. us with one / two:
-// forward [1, 2 x 11008] 2.1 / 2.7, [256, 2 x 5504] 3.1 / 3.6, [512, 2 x 11008] 8.3 / 8.5, [700, 2 x 11008] 10.4 / 10.0, [2048, 2 x 11008] 26.9
-// / 24.9, [8192, 2 x 14336] 121.7 / 108.8; backward [256, 2 x 5504] 3.8 / 4.4, [1024, 2 x 11008] 19.1 / 19.6, [2048, 2 x 11008] 36.2 / 36.2,
-// [8192, 2 x 14336] 170.3 / 168.3.
+// gu is [T, 2F] (gate columns [0,F), up columns [F,2F)); y = silu(g) * u is [T, F]. Bound by memory: a thread has BATCH vectors
+// of each operand, 256 vectors apart, and issues their loads before it uses the first. Index is a 32-bit type where the sizes
+// allow it: the division by the row length was a 64-bit one for every vector. Two vectors pay where their loads wait for
+// memory; a call that the L2 holds or that leaves the machine partly empty has more threads with one. us with one / two:
+// forward [1, 2 x 11008] 2.1 / 2.7, [256, 2 x 5504] 3.1 / 3.6, [512, 2 x 11008] 8.3 / 8.5, [700, 2 x 11008] 10.4 / 10.0, [2048,
+// 2 x 11008] 26.9 / 24.9, [8192, 2 x 14336] 121.7 / 108.8; backward [256, 2 x 5504] 3.8 / 4.4, [1024, 2 x 11008] 19.1 / 19.6,
+// [2048, 2 x 11008] 36.2 / 36.2, [8192, 2 x 14336] 170.3 / 168.3.
 constexpr long long SWIGLU_FWD_ONE = 6 << 20, SWIGLU_BWD_ONE = 32 << 20;   // elements of the result, below which a thread has one
-template <typename Index, int BATCH>
+// CHAIN: between two launches of a chain (see decode_layer.cu), so the next kernel may start now and the last one's result is
+// waited for.
+template <typename Index, int BATCH, bool CHAIN = false>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, Index total, int F) {
+  if constexpr (CHAIN) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
   const Index vpr = F >> 3, i0 = (Index)blockIdx.x * (256 * BATCH) + threadIdx.x;
   uint4 ug[BATCH], uu[BATCH];
   long long at[BATCH];
@@ -301,8 +307,9 @@ __global__ void chain_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, lon
   }
 }
 // bf16 in and out. GELU as x sigmoid(2 u), the same function as x (1 + tanh u) / 2: 1 + tanh u loses its digits where the
-// result is small, and tanhf is the longer code. [8192, 3072] forward 24.0 -> 22.2 us, backward 32.5 -> 31.0. The short division (2 ulp of
-// fp32, zero for a divisor above 2^126, where the result is below 2^-120) is a quarter of a small call's time.
+// result is small, and tanhf is the longer code. [8192, 3072] forward 24.0 -> 22.2 us, backward 32.5 -> 31.0. The short
+// division (2 ulp of fp32, zero for a divisor above 2^126, where the result is below 2^-120) is a quarter of a small call's
+// time.
 template <int OP>
 __device__ __forceinline__ float op_bf16(float x) {
   if constexpr (OP == OP_GELU) return __fdividef(x, 1.f + __expf(-2.f * 0.7978845608028654f * (x + 0.044715f * x * x * x)));
@@ -319,10 +326,10 @@ __device__ __forceinline__ float op_grad_bf16(float x) {
     return apply_op_grad(OP, x);
   }
 }
-// Vectors of a thread, 256 apart, loaded before the first is used: one for calls that the L2 holds or that leave the machine partly
-// empty, two and then (forward) four where loads wait for memory. GELU forward, us with 1 / 2 / 4: 65536 elements 2.1 / 2.6 / 4.0, 3 Mi
-// 4.9 / 5.4 / 5.9, 8 Mi 9.4 / 9.4 / 10.1, 16 Mi 16.5 / 15.8 / 16.5, 24 Mi 24.9 / 23.0 / 23.4 (tanh 22.8 / 20.0 / 18.7), 96 Mi 89.1 / 78.9 /
-// 77.1; backward 65536 2.1 / 2.8 / 4.2, 8 Mi 11.7 / 11.6 / 12.4, 96 Mi 118.4 / 108.8 / 109.7.
+// Vectors of a thread, 256 apart, loaded before the first is used: one for calls that the L2 holds or that leave the machine
+// partly empty, two and then (forward) four where loads wait for memory. GELU forward, us with 1 / 2 / 4: 65536 elements 2.1 /
+// 2.6 / 4.0, 3 Mi 4.9 / 5.4 / 5.9, 8 Mi 9.4 / 9.4 / 10.1, 16 Mi 16.5 / 15.8 / 16.5, 24 Mi 24.9 / 23.0 / 23.4 (tanh 22.8 / 20.0
+// / 18.7), 96 Mi 89.1 / 78.9 / 77.1; backward 65536 2.1 / 2.8 / 4.2, 8 Mi 11.7 / 11.6 / 12.4, 96 Mi 118.4 / 108.8 / 109.7.
 static int unary_batch(long long n, bool forward) { return n < (8 << 20) ? 1 : n < (20 << 20) || !forward ? 2 : 4; }
 template <int OP, int BATCH>
 __global__ void __launch_bounds__(256)
@@ -691,6 +698,25 @@ static int run_swiglu(const void* gu, const void* dy, void* out, long long T, in
   if (8 * n < (dy ? SWIGLU_BWD_ONE : SWIGLU_FWD_ONE)) return launch_swiglu<unsigned, 1>(gu, dy, out, n, F, st);
   return n < 0x7fffffffll ? launch_swiglu<unsigned, 2>(gu, dy, out, n, F, st) : launch_swiglu<long long, 2>(gu, dy, out, n, F, st);
 }
+namespace gf {
+// The forward pass of a few rows behind a launch of the same chain, which may still run.
+int swiglu_chained(const void* gu, void* y, long long T, int F, cudaStream_t st) {
+  const long long n = T * (F / 8);
+  if (F % 8 || n <= 0 || 8 * n >= SWIGLU_FWD_ONE) return GFH_BAD_ARG;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((n + 255) / 256));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  note_extra_launches(1);
+  return cudaLaunchKernelEx(&cfg, swiglu_fwd_kernel<unsigned, 1, true>, (const __nv_bfloat16*)gu, (__nv_bfloat16*)y, (unsigned)n, F) ==
+                 cudaSuccess ? GFH_OK : GFH_CUDA;
+}
+}  // namespace gf
 GF_API int gf_swiglu_fwd(const void* gu, void* y, long long T, int F, void* stream) {
   gf::enter();
   return run_swiglu(gu, nullptr, y, T, F, (cudaStream_t)stream);

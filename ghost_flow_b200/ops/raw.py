@@ -331,8 +331,8 @@ def attn_decode(q, kcache, vcache, length, B, Hq, Hkv, D, scale=None, splits=Non
 # ------------------------------------------------------------------ one decoder layer, one token of each sequence
 def llama_decode_layer(x, attn_norm, attn_eps, wqkv, wo, ffn_norm, ffn_eps, gate_up, down, cos, sin, kcache, vcache, Hq, Hkv, D,
                        interleaved, pos):
-    """A whole LLaMA decoder layer for one new token of each of at most 64 sequences, in one call of the kernel library (six
-    kernels or nine, most of them started while the one in front of them ends). ``x [B, hidden]`` and weights ``[out, in]`` dense bf16; caches
+    """A whole LLaMA decoder layer for one new token of each of at most 64 sequences, in one call of the kernel library (seven kernels
+    or nine, most of them started while the one in front of them ends). ``x [B, hidden]`` and weights ``[out, in]`` dense bf16; caches
     ``[B, s_max, Hkv, D]`` dense, row ``pos`` is written; tables fp32 with a row for ``pos``. Returns ``[B, hidden]``."""
     B, hidden = x.shape
     inner, s_max = down.shape[1], kcache.shape[1]
