@@ -12,6 +12,7 @@ from __future__ import annotations
 import torch
 
 from .. import ops
+from ..ops import raw
 from ..nn.layers import Embedding, Linear, RMSNorm, SwiGLU
 from ..nn.module import Module, ModuleList, plain_modules
 from .configs import LLaMAConfig
@@ -44,8 +45,6 @@ class LLaMAAttention(Module):
             elif kernels and S == 1:
                 q = ops.rope_qkv_to_cache(qkv, H, Hk, cos, sin, kc, vc, c.rope_interleaved, start_pos)
                 # one new token per sequence: the decode kernel streams the cache once (GQA groups share the reads)
-                from ..ops import raw
-
                 o = raw.attn_decode(q.reshape(B, H * D), kc.view(B, kc.shape[1], Hk * D), vc.view(B, vc.shape[1], Hk * D),
                                     start_pos + 1, B, H, Hk, D).view(B, 1, H, D)
             else:
@@ -64,6 +63,12 @@ class LLaMAAttention(Module):
             q, k, v = ops.rope_qkv(qkv, H, Hk, cos, sin, c.rope_interleaved, start_pos)
             o = ops.flash_attention(q, k, v, causal=True)
         return self.wo(o.reshape(B, S, H * D), residual)
+
+
+def _weight(module):
+    """A module's weight: its parameter without the search of an attribute, or what else bears the name."""
+    p = module._parameters.get("weight")
+    return module.weight if p is None else p
 
 
 class LLaMADecoderLayer(Module):
@@ -87,11 +92,14 @@ class LLaMADecoderLayer(Module):
         if not (type(an) is RMSNorm and type(at) is LLaMAAttention and type(fn) is RMSNorm and type(mlp) is SwiGLU):
             return None
         lin = at._modules.get("wqkv"), at._modules.get("wo"), mlp._modules.get("gate_up"), mlp._modules.get("down")
-        if any(type(n) is not Linear or n.bias is not None for n in lin) or not plain_modules(an, at, fn, mlp, *lin):
+        for n in lin:
+            if type(n) is not Linear or n.bias is not None:
+                return None
+        if not plain_modules(an, at, fn, mlp, *lin):
             return None
         c, (kc, vc), (B, _, hidden), dev = at.cfg, cache, x.shape, x.device
         H, Hk, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim
-        w = [an.weight, lin[0].weight, lin[1].weight, fn.weight, lin[2].weight, lin[3].weight]
+        w = [_weight(n) for n in (an, lin[0], lin[1], fn, lin[2], lin[3])]
         inner = w[5].shape[1] if w[5].dim() == 2 else 0
         shapes = (hidden,), ((H + 2 * Hk) * D, hidden), (hidden, H * D), (hidden,), (2 * inner, hidden), (hidden, inner)
         if D not in (64, 128) or H % Hk or H // Hk > 8 or hidden % 8 or inner % 8 or inner == 0:
@@ -110,8 +118,6 @@ class LLaMADecoderLayer(Module):
         if cache is not None:
             args = self._decodes_in_one_call(x, cos, sin, cache, start_pos)
             if args is not None:
-                from ..ops import raw
-
                 y = raw.llama_decode_layer(*args)
                 torch.autograd.graph.increment_version(cache)     # a graph that saved a cache has to notice the write
                 return y.view(x.shape)
@@ -186,8 +192,6 @@ class LLaMAForCausalLM(Module):
         if labels is None and caches is not None and self._norm_in_the_head(ids):
             x = self.model._before_norm(ids, caches, start_pos)
             if x.dtype is torch.bfloat16 and x.is_contiguous() and not x.data_ptr() & 15:
-                from ..ops import raw
-
                 norm, w = self.model.norm, self.lm_head.weight
                 y = raw.rmsnorm_gemm(x.view(x.shape[0], -1), norm.weight, norm.eps, w)
                 return y.unsqueeze(1)
