@@ -206,3 +206,37 @@ def test_hooks_on_saved_tensors_get_typed_tensors(calls, kernel_status):
         y4 = m(x.clone().requires_grad_())
     with pytest.raises(RuntimeError, match="a hook returned a saved tensor"):
         y4.backward(dy)
+
+
+def test_a_ragged_sequence_with_a_gradient_is_not_taken(calls):
+    """Dense operands: it is the sequence, which the backward kernels do not have, that the layers are asked about."""
+    m, g = _block(256, 512, 4, 1)
+    x = torch.randn(2, 100, 256, generator=g, device="cuda").bfloat16()
+    assert x.is_contiguous()
+    y = m(x)
+    assert not calls and y.requires_grad
+    with pytest.raises(RuntimeError, match="multiple of 128"):
+        y.backward(torch.ones_like(y))
+    m.requires_grad_(False)
+    m(x)
+    assert len(calls) == 1                                               # nothing to differentiate: taken
+
+
+# one token, rows that go to the few-row kernels (alone and as a batch), lengths around a query tile, sequences that end inside one
+@pytest.mark.parametrize("B,S", [(1, 1), (1, 17), (3, 20), (1, 64), (2, 100), (1, 129), (5, 127), (1, 300)])
+@pytest.mark.parametrize("E,F,H,causal", [(256, 512, 4, True), (768, 3072, 12, False), (256, 4096, 2, True)])
+def test_any_length_without_a_gradient(B, S, E, F, H, causal, calls, kernel_status):
+    m, g = _block(E, F, H, S, causal=causal)
+    x = torch.randn(B, S, E, generator=g, device="cuda").bfloat16()
+    want, _ = _want(m, x, torch.ones_like(x))
+    with torch.no_grad():
+        y = m(x)
+        assert len(calls) == 1
+        hook = m.mlp.fc1.register_forward_hook(lambda *a: None)          # layer by layer
+        y2 = m(x)
+        hook.remove()
+        assert len(calls) == 1
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()  # noqa: E731
+    assert rel(y, want) < 8e-3 and rel(y, want) < 1.02 * rel(y2, want)   # as above
+    if F < 2048:
+        assert torch.equal(y, y2)
