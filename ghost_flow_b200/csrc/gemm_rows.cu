@@ -44,7 +44,6 @@ struct RwCfg {
   static constexpr int STAGES = NT == 32 ? 5 : 4;
   static constexpr int CTAS = NT == 16 ? 3 : 2;                       // on an SM
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 512;
-  static constexpr int VPT = NT / 16;                                 // 16-byte vectors of a block for each of 128 threads
   static constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
   static_assert(NT * RW_BM * 4 <= STAGES * STAGE_BYTES, "partial sums fit in the ring");
 };
@@ -181,82 +180,65 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     asm volatile("griddepcontrol.wait;" ::: "memory");
     bool ok = true;
     if constexpr (INPUT != ROWS_PLAIN) {
-    constexpr int V = Cfg::VPT, B = 2;                   // B: blocks whose loads are issued together
-    float sq[V];
+      static_assert(NT == 16, "a vector of a block for each of 128 threads");
+      constexpr int B = 2;                 // blocks whose loads are issued together
+      float sq = 0.f;
+      uint4 x[2][B], y[2][B];              // y: up projection, or the norm's weight
+      auto load = [&](int kb, uint4 (&xr)[B], uint4 (&yr)[B]) {
 #pragma unroll
-    for (int v = 0; v < V; ++v) sq[v] = 0.f;
-    uint4 x[2][B][V], y[2][B][V];         // y: up projection, or the norm's weight in [..][0]
-    auto load = [&](int kb, uint4 (&xr)[B][V], uint4 (&yr)[B][V]) {
-#pragma unroll
-      for (int i = 0; i < B; ++i) {
-        const int k = (kb + i) * RW_BK + vec * 8;
-        const bool in = kb + i < kb1 && k < p.K;               // K is a multiple of eight
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          const int m = tok + 16 * v;
-          const __nv_bfloat16* src = p.X + (long long)m * p.ldx + k;
-          xr[i][v] = in && m < p.M ? *reinterpret_cast<const uint4*>(src) : make_uint4(0, 0, 0, 0);
-          if (INPUT == ROWS_SWIGLU)
-            yr[i][v] = in && m < p.M ? *reinterpret_cast<const uint4*>(src + p.K) : make_uint4(0, 0, 0, 0);
+        for (int i = 0; i < B; ++i) {
+          const int k = (kb + i) * RW_BK + vec * 8;
+          const bool in = kb + i < kb1 && k < p.K;             // K is a multiple of eight
+          const __nv_bfloat16* src = p.X + (long long)tok * p.ldx + k;
+          xr[i] = in && tok < p.M ? *reinterpret_cast<const uint4*>(src) : make_uint4(0, 0, 0, 0);
+          if (INPUT == ROWS_SWIGLU) yr[i] = in && tok < p.M ? *reinterpret_cast<const uint4*>(src + p.K) : make_uint4(0, 0, 0, 0);
+          if (INPUT == ROWS_RMSNORM) yr[i] = in ? *reinterpret_cast<const uint4*>(p.norm_w + k) : make_uint4(0, 0, 0, 0);
         }
-        if (INPUT == ROWS_RMSNORM)
-          yr[i][0] = in ? *reinterpret_cast<const uint4*>(p.norm_w + k) : make_uint4(0, 0, 0, 0);
-      }
-    };
-    int st = 0;
-    uint32_t ph = 1;
-    auto store = [&](int kb, const uint4 (&xr)[B][V], const uint4 (&yr)[B][V]) {
+      };
+      int st = 0;
+      uint32_t ph = 1;
+      auto store = [&](int kb, const uint4 (&xr)[B], const uint4 (&yr)[B]) {
 #pragma unroll
-      for (int i = 0; i < B; ++i) {
-        if (kb + i >= kb1 || !ok) break;
-        if (!mbar_wait_warp_tight(&empty[st], ph)) {
-          if (p.status && lane == 0) atomicCAS(p.status, 0, GF_ERR_WAIT_EMPTY);
-          ok = false;
-          break;
-        }
-        uint8_t* dst = smem + st * Cfg::STAGE_BYTES + RW_W_BYTES;
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          uint4 o = xr[i][v];
+        for (int i = 0; i < B; ++i) {
+          if (kb + i >= kb1 || !ok) break;
+          if (!mbar_wait_warp_tight(&empty[st], ph)) {
+            if (p.status && lane == 0) atomicCAS(p.status, 0, GF_ERR_WAIT_EMPTY);
+            ok = false;
+            break;
+          }
+          uint4 o = xr[i];
           uint32_t* po = reinterpret_cast<uint32_t*>(&o);
-          {
-            const uint32_t* pw = reinterpret_cast<const uint32_t*>(&yr[i][INPUT == ROWS_RMSNORM ? 0 : v]);
+          const uint32_t* pw = reinterpret_cast<const uint32_t*>(&yr[i]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 a = unpack_bf16x2(po[e]), w = unpack_bf16x2(pw[e]);
-              if (INPUT == ROWS_RMSNORM) {
-                sq[v] += a.x * a.x + a.y * a.y;
-                po[e] = pack_bf16x2(a.x * w.x, a.y * w.y);
-              } else {
-                po[e] = pack_bf16x2(silu_mul(a.x, w.x), silu_mul(a.y, w.y));
-              }
+          for (int e = 0; e < 4; ++e) {
+            const float2 a = unpack_bf16x2(po[e]), w = unpack_bf16x2(pw[e]);
+            if (INPUT == ROWS_RMSNORM) {
+              sq += a.x * a.x + a.y * a.y;
+              po[e] = pack_bf16x2(a.x * w.x, a.y * w.y);
+            } else {
+              po[e] = pack_bf16x2(silu_mul(a.x, w.x), silu_mul(a.y, w.y));
             }
           }
-          *reinterpret_cast<uint4*>(dst + sw128_offset(tok + 16 * v, vec)) = o;
+          *reinterpret_cast<uint4*>(smem + st * Cfg::STAGE_BYTES + RW_W_BYTES + sw128_offset(tok, vec)) = o;
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full[st]);
+          if (++st == Cfg::STAGES) { st = 0; ph ^= 1; }
         }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&full[st]);
-        if (++st == Cfg::STAGES) { st = 0; ph ^= 1; }
+      };
+      load(kb0, x[0], y[0]);
+      for (int kb = kb0; kb < kb1 && ok; kb += 2 * B) {
+        load(kb + B, x[1], y[1]);
+        store(kb, x[0], y[0]);
+        load(kb + 2 * B, x[0], y[0]);
+        store(kb + B, x[1], y[1]);
       }
-    };
-    load(kb0, x[0], y[0]);
-    for (int kb = kb0; kb < kb1 && ok; kb += 2 * B) {
-      load(kb + B, x[1], y[1]);
-      store(kb, x[0], y[0]);
-      load(kb + 2 * B, x[0], y[0]);
-      store(kb + B, x[1], y[1]);
-    }
-    if (INPUT == ROWS_RMSNORM) {
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        float s = sq[v];
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        if (vec == 0) row_sum[tok + 16 * v] = s;
+      if (INPUT == ROWS_RMSNORM) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+        sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+        sq += __shfl_xor_sync(0xffffffffu, sq, 4);
+        if (vec == 0) row_sum[tok] = sq;
       }
-    }
     }
     // ---------------------------------------------------------------- sums of this CTA: [token][feature] over the ring
     if (ok && !mbar_wait_warp_tight(acc_full, 0)) {

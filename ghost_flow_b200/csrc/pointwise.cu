@@ -16,13 +16,6 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
   return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
 }
-__device__ __forceinline__ float gelu_tanh_grad(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float u = k0 * (x + k1 * x * x * x);
-  const float t = tanhf(u);
-  const float du = k0 * (1.f + 3.f * k1 * x * x);
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
-}
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf(-x)); }
 
 // ------------------------------------------------------------------ RoPE
@@ -266,10 +259,10 @@ __device__ __forceinline__ float apply_op(int op, float x) {
     default: return x * sigmoidf_(x);
   }
 }
+// of all but GELU, which has op_grad_bf16 below
 __device__ __forceinline__ float apply_op_grad(int op, float x) {
   switch (op) {
     case OP_RELU: return x > 0.f ? 1.f : 0.f;
-    case OP_GELU: return gelu_tanh_grad(x);
     case OP_SIGMOID: { const float s = sigmoidf_(x); return s * (1.f - s); }
     case OP_TANH: { const float t = tanhf(x); return 1.f - t * t; }
     default: { const float s = sigmoidf_(x); return s + x * s * (1.f - s); }
