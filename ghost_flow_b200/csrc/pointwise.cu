@@ -695,7 +695,11 @@ namespace gf {
 // The forward pass of a few rows behind a launch of the same chain, which may still run.
 int swiglu_chained(const void* gu, void* y, long long T, int F, cudaStream_t st) {
   const long long n = T * (F / 8);
-  if (F % 8 || n <= 0 || 8 * n >= SWIGLU_FWD_ONE) return GFH_BAD_ARG;
+  if (F % 8 || n <= 0) return GFH_BAD_ARG;
+  if (n >= 0x7fffffffll) {                       // no chain, but no limit either
+    note_extra_launches(1);
+    return run_swiglu(gu, nullptr, y, T, F, st);
+  }
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;

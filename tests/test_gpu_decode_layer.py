@@ -212,3 +212,19 @@ def test_positions_that_are_no_int_are_refused(calls):
             with pytest.raises((TypeError, ctypes.ArgumentError)):
                 m(x, cos, sin, cache=(kc, vc), start_pos=pos)
     assert not calls
+
+
+def test_wide_inner_layer(calls):
+    """More activations between the last two products than a thread of their kernel usually has vectors for."""
+    from ghost_flow_b200 import ops
+    from ghost_flow_b200.ops import _lib
+
+    m, cfg, g = _layer(64, 131072, 1, 1, 5)
+    cos, sin = ops.rope_tables(64, 64, 10000.0, "cuda")
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    x, kc, vc = mk(64, 1, 64), mk(64, 9, 1, 64), mk(64, 9, 1, 64)
+    want, _, _ = _want(m, cfg, x, kc, vc, cos, sin, 7)
+    with torch.no_grad():
+        y = m(x, cos, sin, cache=(kc, vc), start_pos=7)
+    _lib.check_status()
+    assert len(calls) == 1 and (y.double() - want).norm() / want.norm() < 8e-3      # as above
