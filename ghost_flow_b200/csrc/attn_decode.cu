@@ -1,27 +1,28 @@
 // Single-query attention over a KV cache (the decode step of generation), grouped-query aware.
 //
 // The reference decodes by recomputing full attention on the CPU (ghostflow-nn/src/gpt.rs generate loop,
-// ghostflow-nn/src/attention.rs:11-49). Here one CTA handles one KV head of a part of the keys (see DecWork); the G = Hq / Hkv <= 8
-// query heads that share the KV head are processed together, so each cache row is read once, and softmax is kept online.
-// The pieces of a sequence are merged by a second kernel, which is on the machine before the first one ends. The cache read is the
-// only traffic that matters, and what bounds the kernel is how much of it is in flight, and where: every warp has its own ring of
-// DEC_STAGES blocks of 16 keys (K and V) filled by cp.async two blocks ahead, 128 KB on an SM, and neighbouring CTAs read the same
-// keys of neighbouring heads, which are one piece of memory (a head's row is 256 bytes; with the CTAs of a sequence at different keys, 32
-// sequences of 4096 keys took 98 us instead of 86). A CTA that goes from one sequence to the next loses about 4 us of its own.
+// ghostflow-nn/src/attention.rs:11-49). Here one CTA handles one KV head of a part of the keys (see DecWork); the G = Hq / Hkv
+// <= 8 query heads that share the KV head are processed together, so each cache row is read once, and softmax is kept online.
+// The pieces of a sequence are merged by a second kernel, which is on the machine before the first one ends. The cache read is
+// the only traffic that matters, and what bounds the kernel is how much of it is in flight, and where: every warp has its own
+// ring of DEC_STAGES blocks of 16 keys (K and V) filled by cp.async two blocks ahead, 128 KB on an SM, and neighbouring CTAs
+// read the same keys of neighbouring heads, which are one piece of memory (a head's row is 256 bytes; with the CTAs of a
+// sequence at different keys, 32 sequences of 4096 keys took 98 us instead of 86). A CTA that goes from one sequence to the
+// next loses about 4 us of its own.
 //
 // The products run on mma.m16n8k16 with keys (S^T = K Q^T) and then head dimensions (O^T = V^T P^T) as the 16 rows and the
-// query heads as the 8 columns, so no half of an instruction is padding, and the heads of a lane's scores are those of
-// its output columns. K is read with ldmatrix, V with its transposing form, and P^T becomes the other operand with movmatrix.
-// (tcgen05 tiles would need 128 query rows.)
-// An operand has 8 bits and a probability 24, so P^T goes in as two bf16 numbers, the rounded value and what it left: the
-// error of a result is then its own rounding to bf16 (0.00165 .. 0.00168 of the norm for both head sizes, as with P in fp32; rounded
-// once, P makes it 0.0019 .. 0.0022). The second product costs 2 % where memory bounds the kernel (32 sequences of 1 .. 4096 keys,
-// 32 / 8 heads of 128: 60.7 -> 61.5 us; 64 of 2048 keys, 64 / 8 heads: 90.0 -> 92.1), 7 % where 160 to 240 CTAs leave SMs half
-// empty; a third changes no digit.
-// Measured, a grid over sequences with slices of equal number -> now: 32 sequences of 1 .. 4096 keys, 32 / 8 heads of 128 60.7 -> 55.2
-// us (5.0 TB/s); 8 of 1 .. 1501, 32 / 32 heads 31.4 -> 24.9; 32 of 1 .. 4096, 12 / 12 heads of 64 43.7 -> 39.5; one length: 32 of 4096,
-// 32 / 8 heads 95.6 -> 86.1 (6.2 TB/s); 8 of 1501, 32 / 32 heads 38.5 -> 35.3; 8 of 4000, 40 / 40 heads 116.6 -> 109.8; 32 of 4096,
-// 12 / 12 heads of 64 76.7 -> 62.8 (6.4 TB/s). 64 of 300, 16 / 2 heads of 64, which take no time either way, 7.0 -> 8.6.
+// query heads as the 8 columns, so no half of an instruction is padding, and the heads of a lane's scores are those of its
+// output columns. K is read with ldmatrix, V with its transposing form, and P^T becomes the other operand with movmatrix.
+// (tcgen05 tiles would need 128 query rows.) An operand has 8 bits and a probability 24, so P^T goes in as two bf16 numbers,
+// the rounded value and what it left: the error of a result is then its own rounding to bf16 (0.00165 .. 0.00168 of the norm
+// for both head sizes, as with P in fp32; rounded once, P makes it 0.0019 .. 0.0022). The second product costs 2 % where memory
+// bounds the kernel (32 sequences of 1 .. 4096 keys, 32 / 8 heads of 128: 60.7 -> 61.5 us; 64 of 2048 keys, 64 / 8 heads: 90.0
+// -> 92.1), 7 % where 160 to 240 CTAs leave SMs half empty; a third changes no digit. Device time with cold caches, us, a grid
+// over sequences with slices of equal number / this: 32 sequences of 1 .. 4096 keys, 32 / 8 heads of 128 58.0 / 56.1 (shares),
+// 8 of 1 .. 1501, 32 / 32 heads 23.6 / 19.5, 62 of 1 .. 300, 64 / 8 heads 28.5 / 15.4, 32 of 1 .. 4096, 12 / 12 heads of 64
+// 44.9 / 41.1; one length: 32 of 4096, 32 / 8 heads 90.8 / 82.8 (6.5 TB/s), 8 of 1501, 32 / 32 heads 36.3 / 32.6, 8 of 4000, 40
+// / 40 heads 112.2 / 103.9, 32 of 4096, 12 / 12 heads of 64 72.7 / 60.7 (6.6 TB/s), 64 of 300, 16 / 2 heads of 64 5.9 / 5.9, 4
+// of 64, 64 / 8 heads of 64 3.1 / 3.2.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -73,9 +74,9 @@ struct DecCfg {
 //   splits > 0   every sequence is cut into `splits` parts that differ by one unit at most. No merge with one part.
 //   splits == 0  the sequences, one behind the other, are cut into `parts` parts that differ by one unit at most, whatever
 //                the lengths are: a part may begin and end inside a sequence.
-// A CTA has one KV head of one part. A piece that is not a whole sequence leaves its sums in a slot: the CTA's own (splits > 0),
-// else the CTA's slot 0 where the sequence began in an earlier part and slot 1 where it began here and goes on in the next. A second
-// kernel adds them up.
+// A CTA has one KV head of one part. A piece that is not a whole sequence leaves its sums in a slot: the CTA's own (splits >
+// 0), else the CTA's slot 0 where the sequence began in an earlier part and slot 1 where it began here and goes on in the next.
+// A second kernel adds them up.
 struct DecWork {
   const int* lens;
   int len_all, s_max, B, Hkv, parts, splits;
@@ -184,10 +185,10 @@ enum DecKind : int {
   DEC_SHARES = 2,    // splits == 0
 };
 
-// Kinds of one piece to a CTA are compiled without what goes from one sequence to the next. With it, calls that the memory does not
-// bound took 5 to 25 % longer: us with / without it, 4 sequences of 64 keys, 64 / 8 heads of 64 3.8 / 3.1, 32 of 800, 32 / 8 heads of 64 13.7
-// / 11.4, 32 of 200, 32 / 32 heads of 128 32.7 / 26.5. (Padded rows instead of the exchange of chunks are 10 % slower where memory
-// bounds it: 32 of 4096 keys, 32 / 8 heads of 128 93 / 82: cp.async then fills lines in two parts.)
+// Kinds of one piece to a CTA are compiled without what goes from one sequence to the next. With it, calls that the memory does
+// not bound took 5 to 25 % longer: us with / without it, 4 sequences of 64 keys, 64 / 8 heads of 64 3.8 / 3.1, 32 of 800, 32 /
+// 8 heads of 64 13.7 / 11.4, 32 of 200, 32 / 32 heads of 128 32.7 / 26.5. (Padded rows instead of the exchange of chunks are 10
+// % slower where memory bounds it: 32 of 4096 keys, 32 / 8 heads of 128 93 / 82: cp.async then fills lines in two parts.)
 template <int D, int KIND>
 __global__ void __launch_bounds__(DEC_WARPS * 32, DecCfg<D, KIND == DEC_SHARES>::CTAS)
 attn_decode_kernel(const __grid_constant__ DecParams p) {
@@ -649,9 +650,10 @@ GF_API int gf_attn_decode(const void* q, long long ldq, const void* kcache, cons
   gf::enter();
   if (B <= 0 || Hkv <= 0 || Hq % Hkv || Hq / Hkv > DEC_MAX_G || (D != 64 && D != 128) || splits == 0 || !scratch) return GFH_BAD_ARG;
   if (splits > 65535) splits = 65535;
-  DecParams p{{lens, len_all, s_max, B, Hkv, splits < 0 ? -splits : 0, splits > 0 ? splits : 0}, (const __nv_bfloat16*)q, ldq, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache,
+  DecParams p{{lens, len_all, s_max, B, Hkv, splits < 0 ? -splits : 0, splits > 0 ? splits : 0}, (const __nv_bfloat16*)q, ldq,
+              (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache,
               Hq, Hq / Hkv, scale * 1.4426950408889634f, scratch, (__nv_bfloat16*)out, ldo, nullptr, nullptr, 0};
-  if (splits < 0)
-    return D == 128 ? launch_decode<128, DEC_SHARES>(p, 0, (cudaStream_t)stream) : launch_decode<64, DEC_SHARES>(p, 0, (cudaStream_t)stream);
-  return D == 128 ? launch_decode<128, DEC_SLICES>(p, 0, (cudaStream_t)stream) : launch_decode<64, DEC_SLICES>(p, 0, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (splits < 0) return D == 128 ? launch_decode<128, DEC_SHARES>(p, 0, st) : launch_decode<64, DEC_SHARES>(p, 0, st);
+  return D == 128 ? launch_decode<128, DEC_SLICES>(p, 0, st) : launch_decode<64, DEC_SLICES>(p, 0, st);
 }

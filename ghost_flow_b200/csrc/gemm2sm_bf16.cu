@@ -58,8 +58,6 @@ constexpr int g2_threads(int epilogue_warps) { return 64 + 32 * epilogue_warps; 
 constexpr int G2_A_BYTES = G2_BM * G2_BK * 2;
 constexpr int G2_MAX_SLICES = 4;  // of K
 
-// BNH = rows of B (output columns) per CTA: 128 (256 x 256 tiles, seven stages) or 64 (256 x 128 tiles, nine
-// stages; twice as many tiles, for problems whose last wave of 256-wide tiles would leave most pairs idle).
 // Slice of K that an item belongs to, and its k blocks. Most products have one: no divisions between their tiles then.
 __device__ __forceinline__ int g2_slice(const Gemm2Params& p, int item, int slice_tiles, int num_kb, int& kb0, int& kb1) {
   if (p.slices == 1) {
@@ -73,6 +71,8 @@ __device__ __forceinline__ int g2_slice(const Gemm2Params& p, int item, int slic
   return slice;
 }
 
+// BNH = rows of B (output columns) per CTA: 128 (256 x 256 tiles, seven stages) or 64 (256 x 128 tiles, nine
+// stages; twice as many tiles, for problems whose last wave of 256-wide tiles would leave most pairs idle).
 template <int BNH>
 struct G2Cfg {
   static constexpr int BN = 2 * BNH;

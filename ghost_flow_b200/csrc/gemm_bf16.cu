@@ -973,13 +973,15 @@ static bool few_long_rows(int M, int N, int K) { return M <= 8 ? K > 6144 && 4ll
 // rows it is the better one where the other's last wave of CTAs (16 features; five to an SM with at most 8 rows, four with
 // more) is too small to fill the machine but takes as long as its K: up to two CTAs to an SM. Device time in us with cold
 // weights, there / here:
-//   8 rows, K 4096: N 64 4.7 / 6.3, 128 6.1 / 6.4, 256 7.7 / 7.3, 2048 8.4 / 8.3, 4736 10.8 / 11.2 (two to an SM), 6144 11.9 / 12.6, 8192
-//   14.3 / 15.9, 11776 18.5 / 20.2 (a full wave), 11904 23.1 / 20.2, 12288 23.8 / 21.1, 15360 26.0 / 24.3, 16384 27.6 / 25.9 (two to an
-//   SM), 17408 28.3 / 26.8, 22016 32.4 / 32.6, 23552 34.8 / 35.0 (two waves), 23744 37.9 / 35.8, 28416 43.0 / 39.9, 28672 42.6 / 44.4. One
-//   row: 8192 14.1 / 16.0, 11904 21.9 / 19.7, 16384 25.7 / 25.1, 17408 26.4 / 26.5, 28416 40.3 / 39.1, 28672 40.3 / 43.2.
-//   8 rows, K 14336: 4096 25.8 / 23.4, 5120 28.9 / 27.6, 6144 31.6 / 32.3; K 2048: 1024 4.7 / 6.0, 12288 13.7 / 12.7, 16384 15.5 / 15.2.
-//   16 rows, K 2048: 6144 8.2 / 9.3, 8192 9.5 / 10.4, 11904 15.6 / 12.8, 17408 18.1 / 16.5; K 4096: 64 5.4 / 6.2, 128 7.3 / 6.6, 6144 13.4
-//   / 13.1, 11904 26.7 / 20.4, 28416 46.2 / 40.4.
+//   8 rows, K 4096: N 64 4.7 / 6.3, 128 6.1 / 6.4, 256 7.7 / 7.3, 2048 8.4 / 8.3, 4736 10.8 / 11.2 (two to an SM), 6144 11.9 /
+//   12.6, 8192 14.3 / 15.9, 11776 18.5 / 20.2 (a full wave), 11904 23.1 / 20.2, 12288 23.8 / 21.1, 15360 26.0 / 24.3, 16384 27.6
+//   / 25.9 (two to an SM), 17408 28.3 / 26.8, 22016 32.4 / 32.6, 23552 34.8 / 35.0 (two waves), 23744 37.9 / 35.8, 28416 43.0 /
+//   39.9, 28672 42.6 / 44.4. One row: 8192 14.1 / 16.0, 11904 21.9 / 19.7, 16384 25.7 / 25.1, 17408 26.4 / 26.5, 28416 40.3 /
+//   39.1, 28672 40.3 / 43.2.
+//   8 rows, K 14336: 4096 25.8 / 23.4, 5120 28.9 / 27.6, 6144 31.6 / 32.3; K 2048: 1024 4.7 / 6.0, 12288 13.7 / 12.7, 16384 15.5
+//   / 15.2.
+//   16 rows, K 2048: 6144 8.2 / 9.3, 8192 9.5 / 10.4, 11904 15.6 / 12.8, 17408 18.1 / 16.5; K 4096: 64 5.4 / 6.2, 128 7.3 / 6.6,
+//   6144 13.4 / 13.1, 11904 26.7 / 20.4, 28416 46.2 / 40.4.
 // A weight of a megabyte (three quarters with more than 8 rows) does not fill the rings. More rows: 24, K 512: 64 7.3 / 5.4; K
 // 4096: 4096 15.3 / 11.0, 32000 52.9 / 48.6; 64, K 256: 4096 7.4 / 8.8; K 512: 4096 8.6 / 8.2; K 4096: 24576 52.4 / 43.7, 32000
 // 54.6 / 53.6; K 1024: 32000 19.1 / 19.6.

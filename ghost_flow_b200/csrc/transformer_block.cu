@@ -3,9 +3,10 @@
 //   h = x + Wo attention(LN1(x) Wqkv^T + bqkv) + bo        y = h + W2 gelu(LN2(h) W1^T + b1) + b2
 //
 // Host code only: the launches are those of the layers one by one, in the same order with the same operands, so results are the
-// same bits; only the sums of a gradient with the one that arrives past the branch are taken inside the LayerNorm backward
-// kernels (rounded once instead of twice). From Python the layers' 38 launches kept the host busy for 1000 to 1200 us where the
-// device had work for 780 (8192 tokens of width 768).
+// same bits, with two exceptions: the sums of a gradient with the one that arrives past the branch are taken inside the
+// LayerNorm backward kernels (rounded once instead of twice), and products whose parts of K are added with atomics (few tiles
+// and a long K, see gemm_bf16.cu) differ from call to call as they do in the layers. From Python the layers' 38 launches kept
+// the host busy for 1000 to 1200 us where the device had work for 780 (8192 tokens of width 768).
 #include <math.h>
 
 #include <algorithm>
@@ -78,8 +79,8 @@ long long gradient_floats(const Block& b, int N, int K) {
   return std::max(product_floats(b.T, K, N, 0, 1), product_floats(N, K, b.T, 1, 1));
 }
 
-// Results of the forward pass. With `keep` all of them have a place of their own and the backward pass reads them again. Without, only
-// what is still to be read has: n1, o and n2 take turns in y, which is written last; pre follows q, k, v.
+// Results of the forward pass. With `keep` all of them have a place of their own and the backward pass reads them again.
+// Without, only what is still to be read has: n1, o and n2 take turns in y, which is written last; pre follows q, k, v.
 struct Results {
   void *n1, *qkv, *o, *h, *n2, *pre, *act;
   float *stats1 = nullptr, *lse = nullptr, *stats2 = nullptr;
@@ -155,8 +156,8 @@ GF_API long long gf_gpt_block_bytes(int which, int B, int S, int E, int F, int H
   return which == 2 ? ws : ws + gf::Results(b, false, nullptr, nullptr).bytes;
 }
 
-// Where in `saved` its ten tensors begin (bytes), in the order n1 [T, E], statistics [2, T] fp32, q k v [T, (H + 2 Hk) D], o [T, E],
-// lse [B, H, S] fp32, h [T, E], n2 [T, E], statistics [2, T] fp32, pre [T, F], act [T, F].
+// Where in `saved` its ten tensors begin (bytes), in the order n1 [T, E], statistics [2, T] fp32, q k v [T, (H + 2 Hk) D], o
+// [T, E], lse [B, H, S] fp32, h [T, E], n2 [T, E], statistics [2, T] fp32, pre [T, F], act [T, F].
 GF_API int gf_gpt_block_parts(long long* offsets, int B, int S, int E, int F, int H, int Hk) {
   using namespace gf;
   const Block b(B, S, E, F, H, Hk);
