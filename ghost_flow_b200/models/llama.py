@@ -111,7 +111,7 @@ class LLaMADecoderLayer(Module):
         if dev.index != torch.cuda.current_device() or not (x.is_contiguous() and x.data_ptr() & 15 == 0) \
                 or not ops.decode_cache_ok(kc, vc, cos, sin, (B, Hk, D), dev, start_pos):
             return None
-        return (x.view(B, hidden), w[0], an.eps, w[1], w[2], w[3], fn.eps, w[4], w[5], cos, sin, kc, vc, H, Hk, D,
+        return (x, w[0], an.eps, w[1], w[2], w[3], fn.eps, w[4], w[5], cos, sin, kc, vc, H, Hk, D,
                 c.rope_interleaved, start_pos)
 
     def forward(self, x, cos, sin, cache=None, start_pos: int = 0):
@@ -120,7 +120,7 @@ class LLaMADecoderLayer(Module):
             if args is not None:
                 y = raw.llama_decode_layer(*args)
                 torch.autograd.graph.increment_version(cache)     # a graph that saved a cache has to notice the write
-                return y.view(x.shape)
+                return y
         x = self.attn(self.attn_norm(x), cos, sin, residual=x, cache=cache, start_pos=start_pos)
         return self.mlp(self.ffn_norm(x), residual=x)
 

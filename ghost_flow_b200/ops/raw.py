@@ -332,9 +332,9 @@ def attn_decode(q, kcache, vcache, length, B, Hq, Hkv, D, scale=None, splits=Non
 def llama_decode_layer(x, attn_norm, attn_eps, wqkv, wo, ffn_norm, ffn_eps, gate_up, down, cos, sin, kcache, vcache, Hq, Hkv, D,
                        interleaved, pos):
     """A whole LLaMA decoder layer for one new token of each of at most 64 sequences, in one call of the kernel library (seven kernels
-    or nine, most of them started while the one in front of them ends). ``x [B, hidden]`` and weights ``[out, in]`` dense bf16; caches
-    ``[B, s_max, Hkv, D]`` dense, row ``pos`` is written; tables fp32 with a row for ``pos``. Returns ``[B, hidden]``."""
-    B, hidden = x.shape
+    or nine, most of them started while the one in front of them ends). ``x [B, hidden]`` or ``[B, 1, hidden]`` and weights ``[out, in]``
+    dense bf16; caches ``[B, s_max, Hkv, D]`` dense, row ``pos`` is written; tables fp32 with a row for ``pos``. Returns the shape of ``x``."""
+    B, hidden = x.shape[0], x.shape[-1]
     inner, s_max = down.shape[1], kcache.shape[1]
     splits = _even_slices(B * Hkv, (pos + 128) // 128, D, _sm_count(x.device))
     lib = _lib.cuda_lib()
@@ -356,10 +356,11 @@ def rmsnorm_gemm(x, norm_w, eps, w):
     """``rms_norm(x) @ w^T`` for at most 16 rows of dense bf16, in one kernel (the norm in front of the product). ``w [N, K]`` dense; rows
     of the result start on 16-byte boundaries."""
     (M, K), N = x.shape, w.shape[0]
-    for t, s in (x, (M, K)), (norm_w, (K,)), (w, (N, K)):
-        if t.shape != s or t.dtype is not torch.bfloat16 or t.device != x.device or not t.is_contiguous():
-            raise ValueError(f"rmsnorm_gemm takes dense bf16 tensors [M, K], [K], [N, K] on one device, not {list(x.shape)}, "
-                             f"{list(norm_w.shape)}, {list(w.shape)}")
+    bf16, dev = torch.bfloat16, x.device
+    if not (norm_w.shape == (K,) and w.shape == (N, K) and x.dtype is bf16 and norm_w.dtype is bf16 and w.dtype is bf16
+            and norm_w.device == dev and w.device == dev and x.is_contiguous() and norm_w.is_contiguous() and w.is_contiguous()):
+        raise ValueError(f"rmsnorm_gemm takes dense bf16 tensors [M, K], [K], [N, K] on one device, not {list(x.shape)}, "
+                         f"{list(norm_w.shape)}, {list(w.shape)}")
     y = torch.empty((M, N if N % 8 == 0 else (N + 63) // 64 * 64), dtype=x.dtype, device=x.device)[:, :N]
     _rc(_lib.cuda_lib().gf_gemm_rows(x.data_ptr(), K, w.data_ptr(), K, y.data_ptr(), y.stride(0), 0, M, N, K, 1, norm_w.data_ptr(),
                                      float(eps), None, None, 0, 1.0, 0, _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()),
