@@ -746,9 +746,11 @@ def flash_attention(q, k, v, causal: bool = True, scale: float | None = None):
 
 # ------------------------------------------------------------------------------------------ a whole pre-norm block
 @functools.lru_cache(maxsize=1024)
-def _block_bytes(device: int, which, B, S, E, F, H, Hk) -> int:
-    """Bytes of a buffer of the block on a device (the number of SMs decides which products split K)."""
-    return _lib.cuda_lib().gf_gpt_block_bytes(which, B, S, E, F, H, Hk)
+def _block_bytes(device: int, sizes) -> tuple:
+    """Bytes of the block's buffers on a device (the number of SMs decides which products split K): what a forward pass leaves for
+    the backward pass, the latter's workspace, the former's, and the one of a forward pass that leaves nothing. -1: sizes
+    that are not taken."""
+    return tuple(_lib.cuda_lib().gf_gpt_block_bytes(which, *sizes) for which in range(4))
 
 
 @functools.lru_cache(maxsize=1024)
@@ -770,10 +772,6 @@ def _saved_tensors_are_hooked() -> bool:
     return _SAVED_HOOKS is None or _SAVED_HOOKS(True) is not None
 
 
-def _nbytes(t) -> int:
-    return 0 if t is None else t.numel() * t.element_size()
-
-
 def _dense16(t):
     """``t`` itself where it is dense on a 16-byte boundary, else a copy that is."""
     t = _dense(t)
@@ -790,44 +788,49 @@ class _GPTBlockFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, sizes, eps1, eps2, causal, *params):
-        B, S, E, F_, H, Hk = sizes
-        y = torch.empty_like(x)
-        mem = lambda n: torch.empty(n, dtype=torch.uint8, device=x.device) if n else None  # noqa: E731
-        size = lambda which: _block_bytes(x.device.index, which, *sizes)  # noqa: E731
-        graph = type(ctx) is not _NoGraph            # without one the layers' results share a small workspace
-        saved, ws = (mem(size(0)), mem(size(2))) if graph else (None, mem(size(3)))
-        at = _pointers((saved, ws))
-        _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), at[0], _nbytes(saved), at[1], _nbytes(ws),
-                                             *sizes, causal, eps1, eps2, _lib.status_word(x.device).data_ptr(),
-                                             _lib.stream_ptr()), "gf_gpt_block_fwd")
-        parts = _block_parts(*sizes) if graph and _saved_tensors_are_hooked() else None
-        kept = (saved,) if parts is None else [saved[n:e].view(t).view(s) for n, e, t, s in parts]
-        ctx.save_for_backward(x, *kept, *params)
-        ctx.args = sizes, causal, len(kept)
+        y, dev, graph = torch.empty_like(x), x.device, type(ctx) is not _NoGraph
+        nsaved, nback, nws, alone = _block_bytes(dev.index, sizes)
+        if not graph:                      # the layers' results share a small workspace
+            nsaved, nws = 0, alone
+        saved = torch.empty(nsaved, dtype=torch.uint8, device=dev) if nsaved else None
+        ws = torch.empty(nws, dtype=torch.uint8, device=dev) if nws else None
+        _rc(_lib.cuda_lib().gf_gpt_block_fwd(x.data_ptr(), _pointers(params), y.data_ptr(), None if saved is None else saved.data_ptr(),
+                                             nsaved, None if ws is None else ws.data_ptr(), nws, *sizes, causal, eps1, eps2,
+                                             _lib.status_word(dev).data_ptr(), _lib.stream_ptr()), "gf_gpt_block_fwd")
+        hooked = graph and _saved_tensors_are_hooked()
+        if hooked:
+            ctx.save_for_backward(x, *(saved[n:e].view(t).view(s) for n, e, t, s in _block_parts(*sizes)), *params)
+        else:
+            ctx.save_for_backward(x, saved, *params)
+        ctx.args = sizes, causal, hooked, nback
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        sizes, causal, n = ctx.args
-        x, *kept = ctx.saved_tensors
-        x, params = _dense16(x), [None if p is None else _dense16(p) for p in kept[n:]]     # hooks may bring them back in another layout
-        kept = kept[:n]
-        saved, parts = kept[0], None
-        if n > 1:
-            for k, (_, _, t, s) in zip(kept, _block_parts(*sizes)):
+        sizes, causal, hooked, nws = ctx.args
+        parts = None
+        if not hooked:
+            x, saved, *params = ctx.saved_tensors
+            at, nsaved = saved.data_ptr(), saved.numel()
+        else:
+            x, *kept = ctx.saved_tensors
+            kinds, at, nsaved = _block_parts(*sizes), None, 0
+            kept, params = kept[:len(kinds)], kept[len(kinds):]
+            for k, (_, _, t, s) in zip(kept, kinds):
                 if k.dtype is not t or k.shape != s or k.device != x.device:
                     raise RuntimeError(f"a hook returned a saved tensor of {k.dtype} {list(k.shape)} on {k.device} for one of {t} "
                                        f"{list(s)} on {x.device}")
-            kept = [_dense16(k) for k in kept]
-            saved, parts = None, _pointers(kept)
+            # hooks may bring all of them back in another layout
+            kept, x, params = [_dense16(k) for k in kept], _dense16(x), [None if p is None else _dense16(p) for p in params]
+            parts = _pointers(kept)
         dy = _dense16(dy)
         dx = torch.empty_like(x)
         # the norms' kernels always write theirs
         grads = [torch.empty_like(p) if p is not None and (need or i in (0, 6)) else None
                  for i, (p, need) in enumerate(zip(params, ctx.needs_input_grad[5:]))]
-        ws = torch.empty(_block_bytes(x.device.index, 1, *sizes), dtype=torch.uint8, device=x.device)
-        _rc(_lib.cuda_lib().gf_gpt_block_bwd(x.data_ptr(), _pointers(params), dy.data_ptr(), *_pointers((saved,)), _nbytes(saved),
-                                             parts, dx.data_ptr(), _pointers(grads), ws.data_ptr(), _nbytes(ws), *sizes, causal,
+        ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
+        _rc(_lib.cuda_lib().gf_gpt_block_bwd(x.data_ptr(), _pointers(params), dy.data_ptr(), at, nsaved, parts, dx.data_ptr(),
+                                             _pointers(grads), ws.data_ptr(), nws, *sizes, causal,
                                              _lib.status_word(x.device).data_ptr(), _lib.stream_ptr()), "gf_gpt_block_bwd")
         return (dx, None, None, None, None, *grads)
 
@@ -850,7 +853,7 @@ def gpt_block_ok(x, params, sizes) -> bool:
     if _observed():                         # before anything asks a tensor for its memory: transformed ones have none
         return False
     if type(x) is not torch.Tensor or not _cuda_bf16(x) or not x.is_contiguous() or x.data_ptr() % 16 or E > 8192 or F_ > 8192 \
-            or (H + 2 * Hk) * (E // H) > 8192 or _block_bytes(x.device.index, 0, *sizes) < 0 or x.device.index != torch.cuda.current_device():
+            or (H + 2 * Hk) * (E // H) > 8192 or _block_bytes(x.device.index, sizes)[0] < 0 or x.device.index != torch.cuda.current_device():
         return False
     P = (H + 2 * Hk) * (E // H)
     shapes = ((E,), (E,), (P, E), (P,), (E, E), (E,), (E,), (E,), (F_, E), (F_,), (E, F_), (E,))
